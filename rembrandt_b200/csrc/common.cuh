@@ -16,8 +16,7 @@ __device__ __forceinline__ float bf2f(bf16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ bf16 f2bf(float v) { return __float2bfloat16_rn(v); }
 
 // 8 bf16 values <-> 8 floats through one 16-byte access
-__device__ __forceinline__ void load8(const bf16* p, float (&f)[8]) {
-  const uint4 v = *reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
   const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -25,6 +24,9 @@ __device__ __forceinline__ void load8(const bf16* p, float (&f)[8]) {
     f[2 * i] = t.x;
     f[2 * i + 1] = t.y;
   }
+}
+__device__ __forceinline__ void load8(const bf16* p, float (&f)[8]) {
+  unpack8(*reinterpret_cast<const uint4*>(p), f);
 }
 __device__ __forceinline__ void store8(bf16* p, const float (&f)[8]) {
   uint4 v;

@@ -55,7 +55,7 @@ class _BnConv:
         self.conv_out = torch.zeros((n, self.P, self.Q, self.kp), dtype=torch.bfloat16, device=dev)
         self.mean = torch.zeros(self.kp, device=dev)
         self.istd = torch.ones(self.kp, device=dev)
-        self.sums = torch.zeros(2 * self.kp, device=dev)
+        self.sums = torch.zeros(4 * self.kp + K.BN_SCRATCH_TAIL, device=dev)
         self.dconv = torch.zeros_like(self.conv_out) if net.training_capable else None
         self.wt16 = None
         if net.training_capable and need_dx_filters and self.gs == 1:
