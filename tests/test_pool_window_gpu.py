@@ -1,0 +1,42 @@
+"""Average pooling over windows large enough to be split over a block, against torch, where the channel groups or the
+window do not divide the block, with padding and several outputs per sample."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from rembrandt_b200.ops import native_ops as K
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("N,C,H,k,stride,pad,relu", [(3, 64, 8, 8, 1, 0, False), (1, 8, 4, 4, 1, 0, False),
+                                                     (2, 96, 7, 7, 7, 0, True), (5, 1024, 6, 6, 1, 0, False),
+                                                     (2, 160, 13, 5, 3, 2, True), (1, 136, 9, 9, 9, 0, False)])
+def test_large_window_average(N, C, H, k, stride, pad, relu):
+    g = torch.Generator(device=DEV).manual_seed(C + H)
+    P = (H + 2 * pad - k) // stride + 1
+    x = torch.randn((N, H, H, C), generator=g, device=DEV).bfloat16()
+    y = torch.full((N, P, P, C), float("nan"), device=DEV, dtype=torch.bfloat16)
+    K.pool_fwd(x, y, None, N, H, H, C, P, P, k, stride, pad, False, relu)
+    ref = F.avg_pool2d(x.double().permute(0, 3, 1, 2), k, stride, pad, count_include_pad=True).permute(0, 2, 3, 1)
+    ref = ref.relu() if relu else ref
+    # one rounding to bf16 (2^-9 of the value) after an fp32 sum
+    assert float(((y.double() - ref).abs() - ref.abs() * 2 ** -8).max()) < 1e-5
+
+
+@pytest.mark.parametrize("k,stride,H", [(2, 2, 16), (3, 2, 13), (3, 1, 9)])
+def test_recorded_offsets_carry_the_producers_relu(k, stride, H):
+    """Behind a ReLU, clamping in the max-pooling forward pass and no mask in backward give what the mask gives."""
+    g = torch.Generator(device=DEV).manual_seed(k + H)
+    N, C, P = 3, 64, (H - k) // stride + 1
+    x = torch.randn((N, H, H, C), generator=g, device=DEV).sub_(1.0).relu_().bfloat16()      # most windows hold zeros
+    dy = torch.randn((N, P, P, C), generator=g, device=DEV).bfloat16()
+    got = []
+    for clamp in (False, True):
+        y, idx = torch.empty_like(dy), torch.empty(dy.shape, dtype=torch.uint8, device=DEV)
+        dx = torch.full_like(x, float("nan"))
+        K.pool_fwd(x, y, idx, N, H, H, C, P, P, k, stride, 0, True, clamp)
+        K.pool_bwd(dy, idx, None, dx, None if clamp else x, N, H, H, C, P, P, k, stride, 0, True)
+        got.append((y, dx))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
