@@ -7,9 +7,10 @@
 // src/operator/input.rs:288-419) in a single kernel. Crop offsets and flip coins are per sample by
 // default; `per_batch` reproduces the reference's one-draw-per-batch behaviour.
 //
-// Space-to-depth by f (used for strided first layers): output pixel (Y,X) holds the f*f*C values of
-// source pixels (Y*f+dy, X*f+dx), channel = (dy*f+dx)*C + c, so an s-strided k x k convolution becomes
-// a stride-1 ceil(k/f) x ceil(k/f) convolution on f*f*C channels.
+// An output pixel (Y,X) holds the f*f*C values of source pixels (Y*stride+dy, X*stride+dx), channel = (dy*f+dx)*C + c.
+// With f == stride this is space-to-depth: an s-strided k x k convolution becomes a stride-1 ceil(k/f) x ceil(k/f)
+// convolution on f*f*C channels. With f = k and the convolution's own stride each output pixel holds the whole
+// receptive field of a first layer, which then is a plain matrix product.
 #include "launch.cuh"
 #include "common.cuh"
 
@@ -22,6 +23,9 @@ struct InputArgs {
   int N, C, H, W;
   int crop_h, crop_w;   // extent of the crop window
   int OH, OW, Cp, f;
+  int stride;           // source pixels between neighbouring output pixels (f: space-to-depth)
+  int border;           // this many rows / columns around the crop window are zeros, whatever the image holds there
+  int ones;             // channel that holds 1 in every pixel (-1: none)
   int lo_y, hi_y, lo_x, hi_x;  // inclusive range of the window's top-left corner (may be negative)
   int random_crop, random_flip, per_batch;
   float scale;          // 1/255 when normalising, else 1
@@ -63,6 +67,14 @@ __device__ __forceinline__ void sample_draw(const InputArgs& a, int n, int& oy, 
   }
 }
 
+// Value of crop-window position (y, x) in channel c; zero outside the window, in its border and outside the image.
+__device__ __forceinline__ bool input_source(const InputArgs& a, int y, int x, int oy, int ox, int flip, int& sy, int& sx) {
+  const bool in = y >= a.border && y < a.crop_h - a.border && x >= a.border && x < a.crop_w - a.border;
+  sy = oy + y;
+  sx = ox + (flip ? a.crop_w - 1 - x : x);
+  return in && sy >= 0 && sy < a.H && sx >= 0 && sx < a.W;
+}
+
 __global__ void input_kernel(InputArgs a) {
   pdl_prolog();
   const int groups = a.Cp / 8;
@@ -81,21 +93,16 @@ __global__ void input_kernel(InputArgs a) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int ch = gidx * 8 + j;
-      float v = 0.f;
+      float v = ch == a.ones ? 1.f : 0.f;
       const int blk = ch / a.C, c = ch - blk * a.C;
       if (blk < a.f * a.f) {
         const int dy = blk / a.f, dx = blk - dy * a.f;
-        const int y = Y * a.f + dy;
-        int x = X * a.f + dx;
-        if (y < a.crop_h && x < a.crop_w) {
-          if (flip) x = a.crop_w - 1 - x;
-          const int sy = oy + y, sx = ox + x;
-          if (sy >= 0 && sy < a.H && sx >= 0 && sx < a.W) {
-            const long long si = ((long long)c * a.H + sy) * a.W + sx;
-            v = (float)a.src[(long long)n * a.C * a.H * a.W + si] * a.scale;
-            if (a.mean) v -= a.mean_scale * a.mean[si];
-            if (c < 3) v += shift[c];
-          }
+        int sy, sx;
+        if (input_source(a, Y * a.stride + dy, X * a.stride + dx, oy, ox, flip, sy, sx)) {
+          const long long si = ((long long)c * a.H + sy) * a.W + sx;
+          v = (float)a.src[(long long)n * a.C * a.H * a.W + si] * a.scale;
+          if (a.mean) v -= a.mean_scale * a.mean[si];
+          if (c < 3) v += shift[c];
         }
       }
       out[j] = v;
@@ -104,108 +111,137 @@ __global__ void input_kernel(InputArgs a) {
   }
 }
 
-// Row-staged variant: one block per (sample, output row). The f source rows of every channel are read with
-// coalesced byte loads, converted (scale, mean, lighting shift, crop / flip / zero padding) into shared memory
-// as floats, then written out as 16-byte channel groups. The per-sample random draw is computed once per block.
-__global__ void __launch_bounds__(256) input_rows_kernel(InputArgs a) {
+// q = e / d by one multiply-high; exact for e * d < 2^32 (the host checks the largest e of a block).
+struct Divider {
+  uint32_t d, magic;
+};
+__device__ __forceinline__ uint32_t fast_div(uint32_t e, const Divider& v) { return v.d == 1u ? e : __umulhi(e, v.magic); }
+
+// Staged variant: one block per (sample, `rows` output rows). The source rows that these need are read four pixels at a
+// time (two aligned words, shifted), several loads in flight per thread, converted (scale, mean, lighting shift, crop /
+// flip / zero padding) and kept in shared memory as bf16 planes [row][channel][pitch]; then every thread writes 16-byte
+// channel groups. A thread keeps the same channel group throughout, so where its eight values lie relative to a pixel is
+// worked out once, in registers. A block moves a few KB: latency and instruction count are what it costs, not bandwidth.
+// The kernel before this one read single bytes, looked the eight offsets up in shared memory per group, and walked the
+// lines of more than four channels one after the other with as many threads as a row has pixels.
+__global__ void __launch_bounds__(256) input_tile_kernel(InputArgs a, int rows, int pitch, Divider by_q, Divider by_c,
+                                                         Divider by_ow) {
   pdl_prolog();
-  extern __shared__ float srow[];  // [f][C][seg_w]
+  extern __shared__ __align__(16) uint8_t input_smem[];
+  bf16* st = reinterpret_cast<bf16*>(input_smem);   // [0] = 0, [1] = 1, planes from [8]
   __shared__ int s_draw[3];
-  __shared__ float s_shift[3];
-  const int n = blockIdx.x / a.OH, Y = blockIdx.x % a.OH;
+  __shared__ float s_shift[4];
+  const int n = blockIdx.y, Y0 = blockIdx.x * rows;
+  const int nrow = min(rows, a.OH - Y0);
   if (threadIdx.x == 0) {
     int oy, ox, flip;
     float shift[3];
     sample_draw(a, n, oy, ox, flip, shift);
     s_draw[0] = oy; s_draw[1] = ox; s_draw[2] = flip;
-    s_shift[0] = shift[0]; s_shift[1] = shift[1]; s_shift[2] = shift[2];
+    s_shift[0] = shift[0]; s_shift[1] = shift[1]; s_shift[2] = shift[2]; s_shift[3] = 0.f;
+    st[0] = f2bf(0.f);
+    st[1] = f2bf(1.f);
   }
   __syncthreads();
   const int oy = s_draw[0], ox = s_draw[1], flip = s_draw[2];
-  const int seg_w = a.OW * a.f;
   const uint8_t* img = a.src + (long long)n * a.C * a.H * a.W;
-  // phase 1: (source row dy, channel c) lines, threads stride along x. No per-element divisions; the loads of two
-  // source rows (up to 8 lines) are issued before any of them is used, because a block moves only a few KB and
-  // what it costs is load latency and instruction count, not bandwidth.
-  const int Cn = a.C < 4 ? a.C : 4;
-  if (a.C <= 4) {
-    for (int dy0 = 0; dy0 < a.f; dy0 += 2) {
-      for (int xc = threadIdx.x; xc < seg_w; xc += blockDim.x) {
-        const int sx = ox + (flip ? a.crop_w - 1 - xc : xc);
-        const bool col_in = xc < a.crop_w && sx >= 0 && sx < a.W;
-        uint8_t px[8];
-        float mu[8];
-        bool ok[8];
+  const uint8_t* src_end = a.src + (long long)a.N * a.C * a.H * a.W;
+  const int lines = ((nrow - 1) * a.stride + a.f) * a.C;
+  const uint32_t quads = (uint32_t)lines * by_q.d;
+  constexpr int U = 4;
+  for (uint32_t e0 = threadIdx.x; e0 < quads; e0 += 256 * U) {
+    uint32_t lo[U], hi[U];   // the two words of four neighbouring source pixels, or those pixels one by one in `lo`
+    int sh[U], at[U], idx[U], ch[U];
+    uint32_t ok[U];          // which of the four positions hold a source pixel
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int dy = dy0 + (u >> 2), c = u & 3;
-          const int y = Y * a.f + dy;
-          const int sy = oy + y;
-          ok[u] = dy < a.f && c < Cn && col_in && y < a.crop_h && sy >= 0 && sy < a.H;
-          px[u] = 0;
-          mu[u] = 0.f;
-          if (ok[u]) {
-            const int idx = (c * a.H + sy) * a.W + sx;
-            px[u] = img[idx];
-            if (a.mean) mu[u] = a.mean[idx];
-          }
-        }
+    for (int u = 0; u < U; ++u) {
+      const uint32_t e = e0 + u * 256;
+      at[u] = -1;
+      ok[u] = 0u;
+      lo[u] = hi[u] = 0u;
+      sh[u] = 0;
+      idx[u] = 0;
+      ch[u] = 3;
+      if (e >= quads) continue;
+      const uint32_t line = fast_div(e, by_q);
+      const int x0 = 4 * (int)(e - line * by_q.d);
+      const int t = (int)fast_div(line, by_c);
+      const int c = (int)line - t * (int)by_c.d;
+      at[u] = 8 + (int)line * pitch + x0;
+      ch[u] = min(c, 3);
+      const int y = Y0 * a.stride + t, sy = oy + y;
+      if (y < a.border || y >= a.crop_h - a.border || sy < 0 || sy >= a.H) continue;
+      // source column of position x0 (not flipped) or x0 + 3 (flipped): the lowest of the four
+      const int sx = ox + (flip ? a.crop_w - 4 - x0 : x0);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int dy = dy0 + (u >> 2), c = u & 3;
-          if (dy < a.f && c < Cn) {
-            float v = 0.f;
-            if (ok[u]) v = (float)px[u] * a.scale - a.mean_scale * mu[u] + (c < 3 ? s_shift[c] : 0.f);
-            srow[(dy * a.C + c) * seg_w + xc] = v;
-          }
-        }
+      for (int k = 0; k < 4; ++k) {
+        const int x = x0 + k, sk = sx + (flip ? 3 - k : k);
+        if (x >= a.border && x < a.crop_w - a.border && sk >= 0 && sk < a.W) ok[u] |= 1u << k;
+      }
+      if (!ok[u]) continue;
+      idx[u] = (c * a.H + sy) * a.W + sx;
+      const uint8_t* px = img + idx[u];
+      const int off = (int)(reinterpret_cast<uintptr_t>(px) & 3u);
+      const uint8_t* w = px - off;
+      if (ok[u] == 15u && w >= a.src && w + 8 <= src_end) {
+        lo[u] = *reinterpret_cast<const uint32_t*>(w);
+        hi[u] = *reinterpret_cast<const uint32_t*>(w + 4);
+        sh[u] = off * 8;
+      } else {   // at an edge
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (ok[u] & (1u << (flip ? 3 - k : k))) lo[u] |= (uint32_t)px[k] << (8 * k);
       }
     }
-  } else {
-    for (int line = 0; line < a.f * a.C; ++line) {
-      const int dy = line / a.C, c = line - dy * a.C;
-      const int y = Y * a.f + dy;
-      const int sy = oy + y;
-      const bool row_in = y < a.crop_h && sy >= 0 && sy < a.H;
-      const long long rbase = ((long long)c * a.H + sy) * a.W;
-      for (int xc = threadIdx.x; xc < seg_w; xc += blockDim.x) {
-        float v = 0.f;
-        const int sx = ox + (flip ? a.crop_w - 1 - xc : xc);
-        if (row_in && xc < a.crop_w && sx >= 0 && sx < a.W) {
-          v = (float)img[rbase + sx] * a.scale;
-          if (a.mean) v -= a.mean_scale * a.mean[rbase + sx];
-          if (c < 3) v += s_shift[c];
-        }
-        srow[line * seg_w + xc] = v;
+    float mu[U][4];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        mu[u][k] = 0.f;
+        if (a.mean && (ok[u] & (1u << k))) mu[u][k] = a.mean[idx[u] + (flip ? 3 - k : k)];
       }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (at[u] < 0) continue;
+      uint32_t px = __funnelshift_r(lo[u], hi[u], sh[u]);
+      if (flip) px = __byte_perm(px, 0u, 0x0123);
+      const float shift = s_shift[ch[u]];
+      float v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        v[k] = (float)((px >> (8 * k)) & 255u) * a.scale - a.mean_scale * mu[u][k] + shift;
+        if (!(ok[u] & (1u << k))) v[k] = 0.f;
+      }
+      __nv_bfloat162 two[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+      *reinterpret_cast<uint2*>(st + at[u]) = *reinterpret_cast<uint2*>(two);
     }
   }
-  // channel -> offset of its source line in shared memory (or -1 for padded channels), built once per block
-  __shared__ int s_tab[512];
-  const int ff = a.f * a.f;
-  for (int ch = threadIdx.x; ch < a.Cp && ch < 512; ch += blockDim.x) {
+  const int groups = a.Cp / 8;
+  const int per = 256 / groups;                       // pixels per pass of the block
+  const int g = threadIdx.x % groups, first = threadIdx.x / groups;
+  int off[8], sel[8];                                 // sel: all ones where the value moves with the pixel
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int ch = g * 8 + j;
     const int blk = ch / a.C, c = ch - blk * a.C;
-    int off = -1;
-    if (blk < ff) {
-      const int dy = blk / a.f, dx = blk - dy * a.f;
-      off = (dy * a.C + c) * seg_w + dx;
-    }
-    s_tab[ch] = off;
+    const int dy = blk / a.f, dx = blk - dy * a.f;
+    sel[j] = blk < a.f * a.f ? -1 : 0;
+    off[j] = sel[j] ? 8 + (dy * a.C + c) * pitch + dx : (ch == a.ones ? 1 : 0);
   }
   __syncthreads();
-  const int groups = a.Cp / 8;
-  bf16* drow = a.dst + ((long long)n * a.OH + Y) * a.OW * a.Cp;
-  const int gshift = (groups & (groups - 1)) == 0 ? __ffs(groups) - 1 : -1;
-  for (int i = threadIdx.x; i < a.OW * groups; i += blockDim.x) {
-    const int X = gshift >= 0 ? (i >> gshift) : i / groups, g = i - X * groups;
-    const int xoff = X * a.f;
-    float out[8];
+  if (first >= per) return;
+  const int row_step = a.stride * a.C * pitch;
+  bf16* drow = a.dst + (((long long)n * a.OH + Y0) * a.OW) * a.Cp + g * 8;
+  const uint16_t* raw = reinterpret_cast<const uint16_t*>(st);
+  for (int i = first; i < nrow * a.OW; i += per) {
+    const int Y = (int)fast_div((uint32_t)i, by_ow), X = i - Y * a.OW;
+    const int base = Y * row_step + X * a.stride;
+    uint32_t v[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int off = s_tab[g * 8 + j];
-      out[j] = off >= 0 ? srow[off + xoff] : 0.f;
-    }
-    store8(drow + (long long)i * 8, out);
+    for (int j = 0; j < 8; ++j) v[j] = raw[off[j] + (base & sel[j])];
+    *reinterpret_cast<uint4*>(drow + (long long)i * a.Cp) =
+        make_uint4(v[0] | (v[1] << 16), v[2] | (v[3] << 16), v[4] | (v[5] << 16), v[6] | (v[7] << 16));
   }
 }
 
@@ -248,7 +284,7 @@ using namespace rb;
 extern "C" {
 
 int rb_input_u8(const void* src, const float* mean, void* dst, int N, int C, int H, int W, int crop_h, int crop_w,
-                int OH, int OW, int Cp, int f, int lo_y, int hi_y, int lo_x, int hi_x, int random_crop,
+                int OH, int OW, int Cp, int f, int stride, int border, int ones, int lo_y, int hi_y, int lo_x, int hi_x, int random_crop,
                 int random_flip, int per_batch, float scale, float mean_scale, float pca_sigma, const float* pca_vals,
                 const float* pca_vecs, unsigned long long seed, unsigned int step, const unsigned int* step_ptr,
                 cudaStream_t st) {
@@ -256,21 +292,37 @@ int rb_input_u8(const void* src, const float* mean, void* dst, int N, int C, int
   InputArgs a;
   a.src = (const uint8_t*)src; a.mean = mean; a.dst = (bf16*)dst;
   a.N = N; a.C = C; a.H = H; a.W = W; a.crop_h = crop_h; a.crop_w = crop_w;
-  a.OH = OH; a.OW = OW; a.Cp = Cp; a.f = f;
+  a.OH = OH; a.OW = OW; a.Cp = Cp; a.f = f; a.stride = stride; a.border = border; a.ones = ones;
   a.lo_y = lo_y; a.hi_y = hi_y; a.lo_x = lo_x; a.hi_x = hi_x;
   a.random_crop = random_crop; a.random_flip = random_flip; a.per_batch = per_batch;
   a.scale = scale; a.mean_scale = mean_scale; a.pca_sigma = pca_sigma;
   for (int i = 0; i < 3; ++i) a.pca_vals[i] = pca_vals ? pca_vals[i] : 0.f;
   for (int i = 0; i < 9; ++i) a.pca_vecs[i] = pca_vecs ? pca_vecs[i] : 0.f;
   a.seed = seed; a.step = step; a.step_ptr = step_ptr;
-  const long long total = (long long)N * OH * OW * (Cp / 8);
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  if (blocks < 1) blocks = 1;
-  const size_t row_smem = (size_t)f * C * OW * f * sizeof(float);
-  if (row_smem <= 40 * 1024 && Cp <= 512 && (long long)N * OH < 0x7FFFFFFF) {
-    launch_pdl(input_rows_kernel, N * OH, 256, row_smem, st, a);
+  // Output rows per block: as many as leave every SM eight blocks and the planes in 32 KB (fewer rows are staged twice
+  // when windows overlap, and a block's fixed cost is shared by more of them).
+  const int seg_w = (OW - 1) * stride + f;
+  const int quads = (seg_w + 3) / 4;
+  const int pitch = 4 * (quads | 1);
+  int rows = 0;
+  for (int r = 8; r >= 1; r >>= 1) {
+    const long long lines = ((long long)(r - 1) * stride + f) * C;
+    const long long smem = (8 + lines * pitch) * 2;
+    if (smem > (r == 1 ? 40 * 1024 : 32 * 1024)) continue;
+    if (lines * quads * quads >= 0xFFFFFFFFll || (long long)r * OW * OW >= 0xFFFFFFFFll) continue;   // see Divider
+    rows = r;
+    if ((long long)N * ((OH + r - 1) / r) >= 148 * 8) break;
+  }
+  if (rows > 0 && Cp <= 2048 && N <= 65535 && (long long)C * H * W < 0x7FFFFFFF) {
+    const size_t smem = (8 + (size_t)((rows - 1) * stride + f) * C * pitch) * 2;
+    auto divider = [](int d) { return Divider{(uint32_t)d, (uint32_t)((0x100000000ull + d - 1) / d)}; };
+    launch_pdl(input_tile_kernel, dim3((unsigned)((OH + rows - 1) / rows), (unsigned)N), dim3(256), smem, st, a, rows,
+               pitch, divider(quads), divider(C), divider(OW));
   } else {
+    const long long total = (long long)N * OH * OW * (Cp / 8);
+    long long blocks = (total + 255) / 256;
+    if (blocks > 148 * 16) blocks = 148 * 16;
+    if (blocks < 1) blocks = 1;
     launch_pdl(input_kernel, (int)blocks, 256, 0, st, a);
   }
   return RB_LAUNCH_OK();

@@ -335,12 +335,15 @@ def axpby(x, y, n, a, b):
 
 
 def input_u8(src, mean, dst, N, C, H, W, crop_h, crop_w, OH, OW, Cp, f, lo_y, hi_y, lo_x, hi_x, random_crop,
-             random_flip, per_batch, scale, mean_scale, pca_sigma, pca_vals, pca_vecs, seed, step, step_ptr=None):
+             random_flip, per_batch, scale, mean_scale, pca_sigma, pca_vals, pca_vecs, seed, step, step_ptr=None, stride=None,
+             border=0, ones=-1):
+    """Output pixel (Y, X) holds the f x f window of source pixels at (Y * stride, X * stride) (default: stride = f, space
+    to depth); `border` rows / columns around the crop window are zeros; channel `ones` holds 1."""
     import ctypes as C_
     pv = (C_.c_float * 3)(*pca_vals) if pca_vals is not None else None
     pe = (C_.c_float * 9)(*pca_vecs) if pca_vecs is not None else None
-    check(_native.cuda().rb_input_u8(ptr(src), ptr(mean), ptr(dst), N, C, H, W, crop_h, crop_w, OH, OW, Cp, f, lo_y,
-                                     hi_y, lo_x, hi_x, int(random_crop), int(random_flip), int(per_batch),
+    check(_native.cuda().rb_input_u8(ptr(src), ptr(mean), ptr(dst), N, C, H, W, crop_h, crop_w, OH, OW, Cp, f,
+                                     f if stride is None else int(stride), int(border), int(ones), lo_y, hi_y, lo_x, hi_x, int(random_crop), int(random_flip), int(per_batch),
                                      float(scale), float(mean_scale), float(pca_sigma),
                                      C_.cast(pv, C_.c_void_p) if pv is not None else None,
                                      C_.cast(pe, C_.c_void_p) if pe is not None else None,
