@@ -28,6 +28,7 @@ _CUDA_SIGS = {
                    vp, vp],
     "rb_conv_fprop_tc": [vp, i32, i32, i32, i32, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, i64, vp, i32, vp,
                          i32, i32, vp, i64, vp, vp],
+    "rb_conv_dgrad_tc": [vp, i32, i32, i32, i32, vp, vp] + [i32] * 10 + [vp, vp, vp, vp, i64, vp, vp],
     "rb_gemm_set_option": [vp, i32],
     "rb_gemm_get_option": [vp, vp],
     "rb_gemm_tune_mode": [i32],

@@ -148,19 +148,27 @@ __global__ void f32_to_bf16_kernel(const float* __restrict__ x, bf16* __restrict
 
 // wt[c][(R-1-r)*S + (S-1-s)][k] = w[k][r*S+s][c]   (k < Kout, c < Cp; padded k are zero)
 // Filters for the data-gradient, which runs as a forward convolution of dY with flipped taps.
-__global__ void pack_dgrad_filters_kernel(const bf16* __restrict__ w, bf16* __restrict__ wt, int Kout, int Kp, int RS,
-                                          int Cp) {
+// A transposition of k x c per tap: 32 x 32 tiles through shared memory, so that reads (c) and writes (k) are contiguous.
+// One thread per element with strided reads took 40 us for 512 x 9 x 512 (19 MB of sectors for 9 MB of data).
+__global__ void __launch_bounds__(256) pack_dgrad_filters_kernel(const bf16* __restrict__ w, bf16* __restrict__ wt, int Kout,
+                                                                 int Kp, int RS, int Cp) {
   pdl_prolog();
-  const long long total = (long long)Cp * RS * Kp;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int k = (int)(i % Kp);
-    long long t = i / Kp;
-    const int tap = (int)(t % RS);
-    const int c = (int)(t / RS);
-    bf16 v = f2bf(0.f);
-    if (k < Kout) v = w[((long long)k * RS + (RS - 1 - tap)) * Cp + c];
-    wt[i] = v;
+  __shared__ bf16 tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int kt = (Kp + 31) / 32, ct = (Cp + 31) / 32;
+  const int total = kt * ct * RS;
+  for (int t = blockIdx.x; t < total; t += gridDim.x) {
+    const int tap = t / (kt * ct), r = t - tap * (kt * ct);
+    const int c0 = (r / kt) * 32, k0 = (r - (r / kt) * kt) * 32;
+    __syncthreads();
+#pragma unroll
+    for (int i = ty; i < 32; i += 8)
+      tile[i][tx] =
+          k0 + i < Kout && c0 + tx < Cp ? w[((long long)(k0 + i) * RS + (RS - 1 - tap)) * Cp + c0 + tx] : f2bf(0.f);
+    __syncthreads();
+#pragma unroll
+    for (int i = ty; i < 32; i += 8)
+      if (c0 + i < Cp && k0 + tx < Kp) wt[((long long)(c0 + i) * RS + tap) * Kp + k0 + tx] = tile[tx][i];
   }
 }
 
@@ -303,8 +311,10 @@ int rb_f32_to_bf16(const float* x, void* y, long long n, cudaStream_t st) {
 }
 
 int rb_pack_dgrad_filters(const void* w, void* wt, int Kout, int Kp, int RS, int Cp, cudaStream_t st) {
-  launch_pdl(pack_dgrad_filters_kernel, grid_for((long long)Cp * RS * Kp, 256), 256, 0, st, (const bf16*)w, (bf16*)wt,
-             Kout, Kp, RS, Cp);
+  const long long tiles = (long long)((Kp + 31) / 32) * ((Cp + 31) / 32) * RS;
+  if (tiles >= 0x7FFFFFFFll) return -10;
+  launch_pdl(pack_dgrad_filters_kernel, (int)(tiles < 148 * 8 ? tiles : 148 * 8), 256, 0, st, (const bf16*)w, (bf16*)wt, Kout,
+             Kp, RS, Cp);
   return RB_LAUNCH_OK();
 }
 

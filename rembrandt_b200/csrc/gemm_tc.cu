@@ -157,6 +157,12 @@ __device__ __forceinline__ WorkItem decode_work(const GemmTcParams& p, int work,
   return w;
 }
 
+__device__ __forceinline__ int dgrad_tap(const GemmTcParams& p, int tap) {
+  if (p.dg_dv == 0) return tap;
+  const int u = tap / p.cv_S;
+  return p.dg_base + u * p.dg_du + (tap - u * p.cv_S) * p.dg_dv;
+}
+
 __device__ __forceinline__ void load_b(const GemmTcParams& p, uint8_t* sb, uint64_t* bar, int kb, int n0, int b_tap,
                                        int b_c0) {
   const int b_split = p.b_split > 0 ? p.b_split : 1;
@@ -168,7 +174,12 @@ __device__ __forceinline__ void load_b(const GemmTcParams& p, uint8_t* sb, uint6
     const int tap = kb / p.cv_cchunks;
     const int cc = kb - tap * p.cv_cchunks;
     for (int q = 0; q < b_split; ++q)
-      tma_load_3d(sb + q * b_rows * p.bk * 2, &p.tm_b, bar, cc * p.bk, tap, n0 + q * b_rows);
+      tma_load_3d(sb + q * b_rows * p.bk * 2, &p.tm_b, bar, cc * p.bk, dgrad_tap(p, tap), n0 + q * b_rows);
+  } else if (p.b_mode == B_DGRAD_MN) {
+    const int tap = kb / p.cv_cchunks;
+    const int cc = kb - tap * p.cv_cchunks;
+    for (int j = 0; j < p.bn_load / 64; ++j)
+      tma_load_3d(sb + j * p.bk * 128, &p.tm_b, bar, n0 + 64 * j, dgrad_tap(p, tap), cc * p.bk);
   } else if (p.b_mode == B_TILED_MN) {
     for (int j = 0; j < p.bn_load / 64; ++j) tma_load_2d(sb + j * p.bk * 128, &p.tm_b, bar, n0 + 64 * j, kb * p.bk);
   } else {  // B_IM2COL_MN
@@ -256,7 +267,10 @@ __device__ __forceinline__ bool issue_item(const IssueCtx& c, SharedCtl* ctl, un
 
 // PAIR: the instantiation that runs as clusters of two CTAs (p.pair != 0). It is a kernel of its own because a
 // kernel that contains cta_group::2 instructions can only be launched with an even cluster size.
-template <bool PAIR>
+// EXT: the instantiation whose bf16 epilogue can scatter rows and take an addend. The tests for these cost the epilogue of
+// every other launch what they do not use: 1 x 1 layers, which are bound by it, ran 8 % slower with them (NIN's training
+// step at 64 images: 1255 instead of 1186 us).
+template <bool PAIR, bool EXT>
 __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant__ GemmTcParams p) {
 #ifdef RB_GEMM_PROFILE
   const long long t_kernel0 = clock64();
@@ -404,7 +418,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       int nload;
       const int a_split = p.a_split > 0 ? p.a_split : 1, b_split = p.b_split > 0 ? p.b_split : 1;
       if (is_a) nload = box ? mt : (p.a_mode == A_TILED_MN ? 2 : a_split) * mt;
-      else if (p.b_mode == B_TILED_MN) nload = p.bn_load / 64;
+      else if (p.b_mode == B_TILED_MN || p.b_mode == B_DGRAD_MN) nload = p.bn_load / 64;
       else if (p.b_mode == B_IM2COL_MN) nload = p.wg_taps > 1 ? p.wg_taps * (p.wg_cw / 64) : p.bn_load / 64;
       else nload = b_split;
       // a pair counts every load on the leader's `full` barriers
@@ -453,7 +467,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
           uint8_t* sb = sa + mt * a_bytes;
           uint64_t* bar = &ctl->full[s];
           if (pair) {
-            // K-major operands only; the bytes are counted on the leader's barrier of this stage
+            // K-major A; K-major B or filters as they lie; the bytes are counted on the leader's barrier of this stage
             const uint32_t bar2 = full0_leader + (uint32_t)s * 8u;
             if (lane < nload) {
               const int tap = p.cv_cchunks > 0 ? kb / p.cv_cchunks : 0;   // filter tap (convolution operands)
@@ -467,11 +481,14 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                   const int sx = tap - r * p.cv_S;
                   tma2_load_im2col_4d(saj, &p.tm_a, bar2, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
                 }
+              } else if (p.b_mode == B_DGRAD_MN) {
+                tma2_load_3d(sb + lane * p.bk * 128, &p.tm_b, bar2, n0 + 64 * lane, dgrad_tap(p, tap),
+                             (kb - tap * p.cv_cchunks) * p.bk);
               } else {
                 const int b_rows = p.bn_load / b_split;
                 uint8_t* sbq = sb + lane * b_rows * p.bk * 2;
                 if (p.b_mode == B_TILED_K) tma2_load_2d(sbq, &p.tm_b, bar2, kb * p.bk, n0 + lane * b_rows);
-                else tma2_load_3d(sbq, &p.tm_b, bar2, (kb - tap * p.cv_cchunks) * p.bk, tap, n0 + lane * b_rows);
+                else tma2_load_3d(sbq, &p.tm_b, bar2, (kb - tap * p.cv_cchunks) * p.bk, dgrad_tap(p, tap), n0 + lane * b_rows);
               }
             }
           } else if (lane < nload) {
@@ -503,7 +520,11 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
               const int tap = kb / p.cv_cchunks;
               const int cc = kb - tap * p.cv_cchunks;
               const int b_rows = p.bn_load / b_split;
-              tma_load_3d(sb + lane * b_rows * p.bk * 2, &p.tm_b, bar, cc * p.bk, tap, n0 + lane * b_rows);
+              tma_load_3d(sb + lane * b_rows * p.bk * 2, &p.tm_b, bar, cc * p.bk, dgrad_tap(p, tap), n0 + lane * b_rows);
+            } else if (p.b_mode == B_DGRAD_MN) {
+              const int tap = kb / p.cv_cchunks;
+              tma_load_3d(sb + lane * p.bk * 128, &p.tm_b, bar, n0 + 64 * lane, dgrad_tap(p, tap),
+                          (kb - tap * p.cv_cchunks) * p.bk);
             } else if (p.b_mode == B_TILED_MN) {
               tma_load_2d(sb + lane * p.bk * 128, &p.tm_b, bar, n0 + 64 * lane, kb * p.bk);
             } else {  // B_IM2COL_MN
@@ -555,11 +576,11 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
     // ------------------------------ MMA issuer ------------------------------
     if (lane == 0 && cta_rank == 0) {   // of a pair, only the leader issues
       const bool a_mn = (p.a_mode == A_TILED_MN);
-      const bool b_mn = (p.b_mode == B_TILED_MN || p.b_mode == B_IM2COL_MN);
+      const bool b_mn = (p.b_mode == B_TILED_MN || p.b_mode == B_IM2COL_MN || p.b_mode == B_DGRAD_MN);
       // a tile wider than 256 columns is two MMAs side by side (256 + the rest) that share the A descriptor
       const uint32_t idesc = make_idesc_bf16(pair ? 2 * BM : BM, (uint32_t)min(p.bn, 256), a_mn ? 1u : 0u, b_mn ? 1u : 0u);
       const uint32_t idesc2 = p.bn > 256 ? make_idesc_bf16(BM, (uint32_t)(p.bn - 256), a_mn ? 1u : 0u, b_mn ? 1u : 0u) : 0u;
-      const uint64_t b_wide_off = (uint64_t)((256u * (uint32_t)p.bk * 2u) >> 4);   // K-major B: 256 rows further down
+      const uint64_t b_wide_off = (uint64_t)((256u * (uint32_t)p.bk * 2u) >> 4);   // 256 rows (K-major) or 4 blocks on
       // K-major: rows of bk*2 bytes, 8-row atoms -> SBO = 8*bk*2; swizzle 128B (bk=64) or 64B (bk=32)
       // MN-major: 64-element (128 B) rows per k, atoms of 8 k -> SBO = 1024, LBO = bk*128 between 64-wide blocks
       const uint32_t k_layout = (p.bk == 64) ? 2u : 4u;
@@ -724,6 +745,13 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
         const uint32_t t_addr =
             tmem_base + (uint32_t)acc * set_cols + (uint32_t)(j * p.acc_stride) + ((uint32_t)lane_base << 16);
         if (p.epi == EPI_BF16 && !tail) {
+          // row of D that this lane's row belongs to (-1: none); only scattered rows and an addend need it
+          const bool scatter = EXT && p.sc_stride != 0;
+          const bool addend = EXT && p.add_src != nullptr;
+          long long drow_of = -1;
+          if ((scatter || addend) && lane < band_rows && row0 + lane < p.M)
+            drow_of = scatter ? scatter_row(row0 + lane, p.cv_P, p.cv_Q, p.sc_stride, p.sc_a, p.sc_b, p.sc_H, p.sc_W)
+                              : (long long)(row0 + lane);
           // 64-column slabs: TMEM -> registers -> bias / ReLU / mask -> swizzled shared memory -> TMA store.
           // Each warp owns a 4 KB slab buffer and issues its own stores, so no cross-warp sync is needed.
           // the two warps of a lane quarter alternate slabs, starting with the other warp on the second sub-tile, so
@@ -734,7 +762,14 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
             __syncwarp();
             const int gcol = col0 + c;
             uint4 mreg[8];
-            if (p.mask_src) {
+            if (p.mask_src && scatter) {
+#pragma unroll
+              for (int ch = 0; ch < 8; ++ch) {
+                mreg[ch] = make_uint4(0u, 0u, 0u, 0u);
+                if (drow_of >= 0 && gcol + ch * 8 < p.n_store)
+                  mreg[ch] = *reinterpret_cast<const uint4*>(p.mask_src + drow_of * p.ldd + gcol + ch * 8);
+              }
+            } else if (p.mask_src) {
               // the mask slab arrives through TMA into the slab buffer (same box and swizzle as the output),
               // is copied to registers, and the buffer is then reused for the output
               if (lane == 0) {
@@ -768,6 +803,10 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                 uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
                 const uint4 mv = p.mask_src ? mreg[half * 4 + q] : make_uint4(0u, 0u, 0u, 0u);
                 const __nv_bfloat162* m2 = reinterpret_cast<const __nv_bfloat162*>(&mv);
+                uint4 av = make_uint4(0u, 0u, 0u, 0u);
+                if (addend && drow_of >= 0 && nbase + q * 8 < p.n_store)
+                  av = *reinterpret_cast<const uint4*>(p.add_src + drow_of * p.ldd + nbase + q * 8);
+                const uint32_t* aw = reinterpret_cast<const uint32_t*>(&av);
                 if (fast) {
                   // Two epilogue warps share a scheduler, so this is bound by instruction count and dependent-issue
                   // latency: packed fp32 adds for the bias, one conversion per pair, ReLU and the mask of the
@@ -785,6 +824,10 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                   for (int e = 0; e < 4; ++e) {
                     float x0 = __uint_as_float(v[q * 8 + 2 * e]), x1 = __uint_as_float(v[q * 8 + 2 * e + 1]);
                     if (has_bias) add2_f32(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1], bb[2 * e], bb[2 * e + 1], x0, x1);
+                    if (addend) {
+                      x0 += __uint_as_float(aw[e] << 16);
+                      x1 += __uint_as_float(aw[e] & 0xFFFF0000u);
+                    }
                     __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
                     if (p.relu) h = __hmax2(h, zero2);
                     uint32_t w = *reinterpret_cast<uint32_t*>(&h);
@@ -797,7 +840,9 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                   for (int e = 0; e < 8; ++e) {
                     const int n = nbase + q * 8 + e;
                     float x = 0.f;
-                    if (n < p.n_valid) x = fmaxf(__uint_as_float(v[q * 8 + e]) + (has_bias ? __ldg(p.bias + n) : 0.f), act_lo);
+                    const float extra = !addend ? 0.f : __uint_as_float((e & 1) ? (aw[e >> 1] & 0xFFFF0000u) : (aw[e >> 1] << 16));
+                    if (n < p.n_valid)
+                      x = fmaxf(__uint_as_float(v[q * 8 + e]) + (has_bias ? __ldg(p.bias + n) : 0.f) + extra, act_lo);
                     f[e] = x;
                   }
                   if (p.mask_src) {
@@ -821,6 +866,20 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
 #ifdef RB_GEMM_PROFILE
             const long long prof_t1_ = clock64();
 #endif
+            if (scatter) {
+              // eight lanes write the 128 bytes of a row, four rows at a time
+              __syncwarp();
+#pragma unroll
+              for (int it = 0; it < 8; ++it) {
+                const int rr = it * 4 + (lane >> 3), ch = lane & 7;
+                const long long dr = __shfl_sync(0xffffffffu, drow_of, rr);
+                if (dr >= 0 && gcol + ch * 8 < p.n_store)
+                  *reinterpret_cast<uint4*>(reinterpret_cast<bf16*>(p.D) + dr * p.ldd + gcol + ch * 8) =
+                      *reinterpret_cast<const uint4*>(buf + rr * 128 + ((ch ^ (rr & 7)) * 16));
+              }
+              __syncwarp();
+              continue;
+            }
             fence_proxy_async_smem();
             __syncwarp();
             if (band_rows < 32) {
@@ -939,11 +998,9 @@ static int ensure_driver_entry() {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDriverGetVersion(&g_driver_version);
-  if (cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) !=
-          cudaSuccess ||
-      cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) !=
-          cudaSuccess)
-    return -2;
+  for (auto kern : {gemm_tc_kernel<false, false>, gemm_tc_kernel<true, false>, gemm_tc_kernel<false, true>,
+                    gemm_tc_kernel<true, true>})
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) != cudaSuccess) return -2;
   {   // how many CTA pairs fit at once: the persistent loop of pair mode runs exactly that many clusters
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -958,7 +1015,7 @@ static int ensure_driver_entry() {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, gemm_tc_kernel<true>, &cfg) != cudaSuccess) nc = 0;
+    if (cudaOccupancyMaxActiveClusters(&nc, gemm_tc_kernel<true, true>, &cfg) != cudaSuccess) nc = 0;
     cudaGetLastError();   // a refused query must not be taken for a failed launch later
     g_pair_clusters = nc > g_num_sms / 2 ? g_num_sms / 2 : nc;
   }
@@ -1115,6 +1172,10 @@ struct Plan {
 static bool pair_ok(const GemmTcParams& p) {
   if (g_opt.force_pair == 0 || g_pair_clusters <= 0) return false;
   if (p.a_mode != A_TILED_K && p.a_mode != A_IM2COL_K) return false;
+  if (p.b_mode == B_DGRAD_MN) {
+    if (p.bn > 256 || p.bn % 128 != 0) return false;   // each CTA loads whole 64-column blocks
+    return p.M > 2 * BM;
+  }
   if (p.b_mode != B_TILED_K && p.b_mode != B_TILED_K3) return false;
   if (p.bn > 256 || p.bn % 16 != 0 || p.b_split < 2 || p.b_split % 2 != 0) return false;
   return p.M > 2 * BM;
@@ -1236,7 +1297,7 @@ static int apply_plan(GemmTcParams& p, const Plan& pl) {
     if (!pair_ok(p) || pl.resident || pl.tail || p.M <= BM * pl.mt) return 0;
     p.pair = 1;
     p.bn_load = p.bn / 2;      // rows of B per CTA
-    p.b_split = p.b_split / 2;
+    if (p.b_mode != B_DGRAD_MN) p.b_split = p.b_split / 2;
   }
   p.acc_stride = acc_stride_for(p.bn);
   p.acc_bufs = (2 * p.mt * p.acc_stride <= 512) ? 2 : 1;
@@ -1283,7 +1344,9 @@ struct TailFixArgs {
   const float* bias;
   const __nv_bfloat16* mask;
   long long ldd;
+  const __nv_bfloat16* add;
   int M, bn, rows_per_item, m_items, direct, tail_items, n_valid, n_store, relu;
+  int sc_stride, sc_a, sc_b, sc_H, sc_W;   // see GemmTcParams
   int box, P, Q, bx_rows, bx_groups, mt;   // box mode: rows of a sub-tile are whole output rows of one image
 };
 __global__ void tail_fix_kernel(const TailFixArgs a) {
@@ -1314,11 +1377,14 @@ __global__ void tail_fix_kernel(const TailFixArgs a) {
     src[0] = make_float4(0.f, 0.f, 0.f, 0.f);
     src[1] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (!live || row >= a.M || col >= a.n_store) continue;
+    if (a.sc_stride) row = scatter_row((int)row, a.P, a.Q, a.sc_stride, a.sc_a, a.sc_b, a.sc_H, a.sc_W);
+    float extra[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (a.add) load8(a.add + row * a.ldd + col, extra);
     float f[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int n = col + e;
-      f[e] = n < a.n_valid ? fmaxf(f[e] + (a.bias ? __ldg(a.bias + n) : 0.f), act_lo) : 0.f;
+      f[e] = n < a.n_valid ? fmaxf(f[e] + (a.bias ? __ldg(a.bias + n) : 0.f) + extra[e], act_lo) : 0.f;
     }
     if (a.mask) {
       float m[8];
@@ -1329,6 +1395,35 @@ __global__ void tail_fix_kernel(const TailFixArgs a) {
     }
     store8(a.D + row * a.ldd + col, f);
   }
+}
+
+// One output phase that no filter tap reaches: mask(add) or zeros. One thread per 8 channels.
+__global__ void fill_phase_kernel(const __nv_bfloat16* add, const __nv_bfloat16* __restrict__ mask, __nv_bfloat16* dx,
+                                  long long groups, int P, int Q, int stride, int a, int b, int H, int W, int Cp) {
+  pdl_prolog();
+  const int cg = Cp / 8;
+  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < groups; g += (long long)gridDim.x * blockDim.x) {
+    const int m = (int)(g / cg), c = (int)(g - (long long)m * cg) * 8;
+    const long long o = scatter_row(m, P, Q, stride, a, b, H, W) * Cp + c;
+    float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (add) load8(add + o, f);
+    if (mask) {
+      float k[8];
+      load8(mask + o, k);
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (!(k[e] > 0.f)) f[e] = 0.f;
+    }
+    store8(dx + o, f);
+  }
+}
+static int fill_phase(const __nv_bfloat16* add, const __nv_bfloat16* mask, __nv_bfloat16* dx, int N, int P, int Q, int stride,
+                      int a, int b, int H, int W, int Cp, cudaStream_t stream) {
+  const long long groups = (long long)N * P * Q * (Cp / 8);
+  long long blocks = (groups + 255) / 256;
+  if (blocks > 148 * 8) blocks = 148 * 8;
+  launch_pdl(fill_phase_kernel, (int)blocks, 256, 0, stream, add, mask, dx, groups, P, Q, stride, a, b, H, W, Cp);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
 // What the most recent launch of this process used (for benchmarks and tests; not synchronised between threads):
@@ -1364,8 +1459,10 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
     }
     cfg.attrs = n_at ? at : nullptr;
     cfg.numAttrs = (unsigned)n_at;
-    const cudaError_t e = p.pair ? cudaLaunchKernelEx(&cfg, gemm_tc_kernel<true>, p)
-                                 : cudaLaunchKernelEx(&cfg, gemm_tc_kernel<false>, p);
+    const bool ext = p.sc_stride != 0 || p.add_src != nullptr;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, p.pair ? (ext ? gemm_tc_kernel<true, true> : gemm_tc_kernel<true, false>)
+                                                          : (ext ? gemm_tc_kernel<false, true> : gemm_tc_kernel<false, false>),
+                                             p);
     if (e != cudaSuccess) {
       g_last_cuda_error = (int)e;
       cudaGetLastError();
@@ -1378,6 +1475,12 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
     f.D = reinterpret_cast<__nv_bfloat16*>(p.D);
     f.bias = p.bias;
     f.mask = p.mask_src;
+    f.add = p.add_src;
+    f.sc_stride = p.sc_stride;
+    f.sc_a = p.sc_a;
+    f.sc_b = p.sc_b;
+    f.sc_H = p.sc_H;
+    f.sc_W = p.sc_W;
     f.ldd = p.ldd;
     f.M = p.M;
     f.bn = p.bn;
@@ -1415,7 +1518,8 @@ static std::map<PlanKey, Plan> g_plan_cache;
 static std::mutex g_plan_mutex;
 
 static PlanKey plan_key(const GemmTcParams& p) {
-  return PlanKey(p.a_mode, p.b_mode, p.M, p.N, p.num_kb, p.bn, p.bk, p.n_tiles, p.cv_stride, p.mask_src ? 1 : 0);
+  return PlanKey(p.a_mode, p.b_mode, p.M, p.N, p.num_kb, p.bn, p.bk, p.n_tiles, p.cv_stride,
+                 (p.mask_src ? 1 : 0) | (p.add_src ? 2 : 0) | (p.sc_stride ? 4 : 0));
 }
 
 // Times the candidates of `p` (3 launches each, best of the last 2); returns the best time in ms, or a negative
@@ -1619,13 +1723,26 @@ int rb_gemm_tc(const void* A, int a_mn, long long lda, const void* B, int b_mn, 
   return launch(p, epi == EPI_F32_ATOMIC && split_k <= 0, split_k > 0 ? split_k : 0, !b_mn, stream);
 }
 
-// Convolution forward (also used for stride-1 data-grad with flipped filters).
-//   x   NHWC bf16 [N][H][W][Cp]      w  bf16 [Kout][R*S][Cp]     y  bf16 [N*P*Q][ldy]
-//   base pixel range: lower = -pad_lo, P/Q given by the caller.
-int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
-                     int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* bias, int relu,
-                     const void* mask_src, int n_valid, int n_store, float* ws, long long ws_bytes,
-                     unsigned int* status, cudaStream_t stream) {
+}  // extern "C"
+
+namespace rb {
+
+// What turns a forward convolution into (one output phase of) a data-gradient: filters read as they lie (B_DGRAD_MN),
+// rows scattered, an addend.
+struct DgradForm {
+  int packed;                              // the filters are transposed and flipped: [n_store][taps][Cp], K-major
+  int taps, base, du, dv;                  // filter taps of the layer, and which of them tap (u, v) is
+  int sc_stride, sc_a, sc_b, sc_H, sc_W;
+  const void* add;
+};
+
+// x NHWC bf16 [N][H][W][Cp]; w bf16 [Kout][R*S][Cp], or with `dg` the filters [k_rows][taps][n_store] of the layer whose
+// data-gradient this is (or their packed form); y bf16 [N*P*Q][ldy]. Base pixel range: lower = -pad, P / Q given by the
+// caller.
+static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
+                             int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* bias, int relu,
+                             const void* mask_src, int n_valid, int n_store, int k_rows, const DgradForm* dg, float* ws,
+                             long long ws_bytes, unsigned int* status, cudaStream_t stream) {
   int rc = ensure_driver_entry();
   if (rc) return rc;
   GemmTcParams p;
@@ -1646,12 +1763,25 @@ int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, 
   p.cv_cchunks = (Cp + p.bk - 1) / p.bk;
   p.num_kb = R * S * p.cv_cchunks;
   p.epi = EPI_BF16;
-  pick_bn(p, n_cols, 32, false, 1, true, [n_cols](GemmTcParams& q, int bn) {
-    q.bn = q.bn_load = bn;
+  p.a_mode = A_IM2COL_K;
+  const bool mn = dg && !dg->packed;
+  p.b_mode = mn ? B_DGRAD_MN : B_TILED_K3;
+  pick_bn(p, n_cols, 32, false, 1, true, [n_cols, mn](GemmTcParams& q, int bn) {
+    q.bn = bn;
+    q.bn_load = mn ? (bn + 63) / 64 * 64 : bn;
     q.n_tiles = (n_cols + bn - 1) / bn;
   });
-  p.a_mode = A_IM2COL_K;
-  p.b_mode = B_TILED_K3;
+  if (dg) {
+    p.dg_base = dg->base;
+    p.dg_du = dg->du;
+    p.dg_dv = dg->dv;
+    p.sc_stride = dg->sc_stride;
+    p.sc_a = dg->sc_a;
+    p.sc_b = dg->sc_b;
+    p.sc_H = dg->sc_H;
+    p.sc_W = dg->sc_W;
+    p.add_src = reinterpret_cast<const __nv_bfloat16*>(dg->add);
+  }
   p.cv_P = P;
   p.cv_Q = Q;
   p.cv_stride = stride;
@@ -1669,7 +1799,7 @@ int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, 
   // ---- halo mode (see the header comment): stride 1, more than one filter tap, image no wider than 128
   {
     const int force = g_opt.force_halo;   // 0 = never, 1 = whenever feasible
-    if (stride == 1 && R * S > 1 && Q <= 128 && force != 0) {
+    if (stride == 1 && R * S > 1 && Q <= 128 && force != 0 && !dg) {
       int pitch = 8;
       while (pitch < Q) pitch *= 2;
       const int rows = 128 / pitch;
@@ -1719,7 +1849,7 @@ int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, 
         if (rc) return rc;
         const long long work = (long long)N * groups * p.n_tiles;
         const int grid = work < g_num_sms ? (int)work : g_num_sms;
-        gemm_tc_kernel<false><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(p);
+        gemm_tc_kernel<false, false><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(p);
         return cudaGetLastError() == cudaSuccess ? 0 : -4;
       }
     }
@@ -1756,8 +1886,14 @@ int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, 
     if (e) return e;
     q.bn = q.bn_load = bn;
     q.n_tiles = (n_cols + bn - 1) / bn;
+    if (mn) {
+      q.bn_load = (bn + 63) / 64 * 64;
+      return make_map_3d(&q.tm_b, w, n_cols, dg->taps, k_rows, n_cols, (uint64_t)dg->taps * n_cols, 64, 1, q.bk,
+                         CU_TENSOR_MAP_SWIZZLE_128B);
+    }
     q.b_split = pairable_b_split(bn, q.bk);
-    return make_map_3d(&q.tm_b, w, Cp, (uint64_t)R * S, Kout, Cp, (uint64_t)R * S * Cp, q.bk, 1, bn / q.b_split, ksw);
+    const uint64_t taps = dg ? dg->taps : R * S;
+    return make_map_3d(&q.tm_b, w, Cp, taps, Kout, Cp, taps * Cp, q.bk, 1, bn / q.b_split, ksw);
   };
   // Candidates beside the default (im2col loads, tiles of at most 256 columns):
   //  * between 257 and 512 output columns, ONE tile as wide as the layer (two MMAs side by side, one accumulator
@@ -1802,6 +1938,85 @@ int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, 
   rc = configure(p, (use >> 16) & 1, use & 0xFFFF);
   if (rc) return rc;
   return launch(p, false, 1, true, stream);
+}
+
+}  // namespace rb
+
+extern "C" {
+
+// Convolution forward (also a stride-1 data-grad on flipped and transposed filters).
+//   x   NHWC bf16 [N][H][W][Cp]      w  bf16 [Kout][R*S][Cp]     y  bf16 [N*P*Q][ldy]
+//   base pixel range: lower = -pad_lo, P/Q given by the caller.
+int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
+                     int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* bias, int relu,
+                     const void* mask_src, int n_valid, int n_store, float* ws, long long ws_bytes,
+                     unsigned int* status, cudaStream_t stream) {
+  return conv_forward_form(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, bias, relu, mask_src, n_valid,
+                           n_store, 0, nullptr, ws, ws_bytes, status, stream);
+}
+
+// Convolution data-grad: dx[N][H][W][Cp] = mask(add + the gradient), from dy NHWC bf16 [N][P][Q][Kp] and the forward
+// filters w bf16 [Kout][R*S][Cp]. Channels >= c_valid of dx are written as zeros.
+//   stride 1: a forward convolution of dy, its filters read in place. stride s: s x s output phases; phase (a, b), the
+//   positions (s i + a, s j + b), is a stride-1 convolution of dy with every s-th filter tap, whose rows the epilogue
+//   scatters. A phase without taps gets mask(add), and nothing has to be done when add is dx itself and there is no mask.
+//   wt: null, or the filters transposed and flipped (rb_pack_dgrad_filters): then these are read, as a K-major operand.
+//   add, mask: optional, layout of dx; add may be dx. Returns -20 for a strided geometry with a phase of negative padding.
+int rb_conv_dgrad_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp, int c_valid,
+                     int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* add,
+                     const void* mask, float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
+  if (stride < 1 || Cp % 32 != 0) return -10;
+  struct Phase { int r0, c0, U, V, pt, pl, Hp, Wp; };
+  auto phase = [&](int a, int b) {
+    Phase f;
+    f.r0 = (a + pad_h) % stride;
+    f.c0 = (b + pad_w) % stride;
+    f.U = f.r0 < R ? (R - f.r0 + stride - 1) / stride : 0;
+    f.V = f.c0 < S ? (S - f.c0 + stride - 1) / stride : 0;
+    f.pt = f.U - 1 - (a + pad_h - f.r0) / stride;
+    f.pl = f.V - 1 - (b + pad_w - f.c0) / stride;
+    f.Hp = a < H ? (H - a + stride - 1) / stride : 0;
+    f.Wp = b < W ? (W - b + stride - 1) / stride : 0;
+    return f;
+  };
+  for (int a = 0; a < stride; ++a)
+    for (int b = 0; b < stride; ++b) {
+      const Phase f = phase(a, b);
+      if (stride > 1 && f.U > 0 && f.V > 0 && f.Hp > 0 && f.Wp > 0 && (f.pt < 0 || f.pl < 0)) return -20;
+    }
+  for (int a = 0; a < stride; ++a)
+    for (int b = 0; b < stride; ++b) {
+      const Phase f = phase(a, b);
+      if (f.Hp <= 0 || f.Wp <= 0) continue;
+      if (f.U == 0 || f.V == 0) {
+        if (add == dx && !mask) continue;
+        const int rc = fill_phase((const __nv_bfloat16*)add, (const __nv_bfloat16*)mask, (__nv_bfloat16*)dx, N, f.Hp, f.Wp,
+                                  stride, a, b, H, W, Cp, stream);
+        if (rc) return rc;
+        continue;
+      }
+      DgradForm dg;
+      dg.packed = wt != nullptr;
+      dg.taps = R * S;
+      dg.base = (f.r0 + stride * (f.U - 1)) * S + f.c0 + stride * (f.V - 1);
+      dg.du = -stride * S;
+      dg.dv = -stride;
+      if (wt) {   // tap t lies at R * S - 1 - t
+        dg.base = R * S - 1 - dg.base;
+        dg.du = -dg.du;
+        dg.dv = -dg.dv;
+      }
+      dg.sc_stride = stride > 1 ? stride : 0;
+      dg.sc_a = a;
+      dg.sc_b = b;
+      dg.sc_H = H;
+      dg.sc_W = W;
+      dg.add = add;
+      const int rc = conv_forward_form(dy, N, P, Q, Kp, wt ? wt : w, Cp, f.U, f.V, 1, f.pt, f.pl, f.Hp, f.Wp, dx, Cp, nullptr, 0,
+                                       mask, c_valid, Cp, Kout, &dg, ws, ws_bytes, status, stream);
+      if (rc) return rc;
+    }
+  return 0;
 }
 
 // Convolution weight-grad:  dw[Kout][R*S][Cp] (fp32) (+)= sum over pixels dy[pix][k] * x[pix shifted by tap][c].

@@ -2,7 +2,8 @@
 // kernel (gemm_tc.cu). One kernel, configured at run time, serves:
 //   conv fprop   A = im2col(X) K-major (TMA im2col)   B = filters K-major
 //                or, stride 1: A = column-shifted halo tiles of X (plain tiled TMA, A_HALO_K), see gemm_tc.cu
-//   conv dgrad   A = im2col(dY) K-major               B = flipped/transposed filters K-major
+//   conv dgrad   A = im2col(dY) K-major               B = the filters as they are, MN-major (TMA tiled, B_DGRAD_MN), or
+//                                                         transposed and flipped ones, K-major
 //   conv wgrad   A = dY^T MN-major (tiled)            B = im2col(X) MN-major (TMA im2col)
 //   affine fwd   A = X K-major                        B = W K-major
 //   affine dgrad A = dY K-major                       B = W MN-major
@@ -18,7 +19,7 @@
 namespace rb {
 
 enum : int { A_TILED_K = 0, A_IM2COL_K = 1, A_TILED_MN = 2, A_HALO_K = 3, A_BOX_K = 4 };
-enum : int { B_TILED_K = 0, B_TILED_MN = 1, B_IM2COL_MN = 2, B_TILED_K3 = 3 };
+enum : int { B_TILED_K = 0, B_TILED_MN = 1, B_IM2COL_MN = 2, B_TILED_K3 = 3, B_DGRAD_MN = 4 };
 enum : int { EPI_BF16 = 0, EPI_F32_STORE = 1, EPI_F32_ATOMIC = 2 };
 
 struct alignas(64) GemmTcParams {
@@ -66,6 +67,15 @@ struct alignas(64) GemmTcParams {
   // unit serves at the rate of tiled loads instead of the 2-3 times slower im2col mode
   int bx_rows;
   int bx_pad_h, bx_pad_w;
+  // data-gradient filters (B_DGRAD_MN): the reduction runs over (tap, output channel k), and for a fixed tap the filters
+  // [k][tap][c] are a k x c matrix with c contiguous, which is an MN-major B operand: they are read as they lie, no
+  // transposed and flipped copy is made. Tap (u, v) of the equivalent forward convolution is tap
+  // dg_base + u * dg_du + v * dg_dv of the filters in memory (dg_dv = 0: taps in order).
+  int dg_base, dg_du, dg_dv;
+  // Row scatter (EPI_BF16): row (n, i, j) of the cv_P x cv_Q grid is row (n, i * sc_stride + sc_a, j * sc_stride + sc_b) of
+  // the sc_H x sc_W image in D, the mask and the addend: one output phase of a strided data-gradient. 0 = rows of D.
+  int sc_stride, sc_a, sc_b, sc_H, sc_W;
+  const __nv_bfloat16* add_src;    // EPI_BF16, optional, same layout as D (may be D): added before ReLU and mask
   // epilogue
   int epi;
   int relu;            // EPI_BF16: clamp at zero after the bias
@@ -92,5 +102,12 @@ struct alignas(64) GemmTcParams {
   // and each SM reads only half of B from its shared memory.
   int pair;
 };
+
+// Row of D (and mask, addend) that row m of the product belongs to.
+__host__ __device__ inline long long scatter_row(int m, int P, int Q, int stride, int a, int b, int H, int W) {
+  const int n = m / (P * Q), r = m - n * (P * Q);
+  const int i = r / Q, j = r - i * Q;
+  return ((long long)n * H + i * stride + a) * W + j * stride + b;
+}
 
 }  // namespace rb

@@ -21,15 +21,9 @@ import os
 
 from ..ops import layout
 from ..ops import native_ops as K
-from ..ops.conv_strided import dgrad_strided_tc
+from ..ops.conv_grad import DgradPlan, conv_dgrad
 from ..ops.native_ops import pad_channels
 from . import config as C
-
-
-def _strided_dgrad_on_tensor_cores() -> bool:
-    """Strided data-grad by output phases on the tensor-core kernel (ops/conv_strided.py) instead of the CUDA-core
-    kernel; RB_STRIDED_DGRAD_TC=0 selects the latter."""
-    return os.environ.get("RB_STRIDED_DGRAD_TC", "1") == "1"
 
 
 class ParamSeg:
@@ -607,12 +601,10 @@ class Conv2dOp(Op):
         if getattr(cfg, "bias", True):
             self.seg_b = ParamSeg(self.name + ".b", (cfg.out_channels,))
             self.segs.append(self.seg_b)
-        self.wt16 = None
+        self.dgrad = None        # DgradPlan on a GPU
 
     def alloc(self):
         super().alloc()
-        if self.net.training_capable and self.wants_prev_delta() and self.cfg.conv_stride == 1:
-            self.wt16 = torch.zeros((self.cp, self.rs, self.out_cp), dtype=torch.bfloat16, device=self.net.device)
         if self.net.device.type == "cuda" and not self.direct:
             self._tune()
 
@@ -622,9 +614,9 @@ class Conv2dOp(Op):
         n, ko = self.net.batch, self.cfg.out_channels
         K.tune_conv(n, h, w, self.cp, ko, r, r, s, p, p, self.P, self.Q, self.out_cp, relu=self.has_relu,
                     has_bias=self.seg_b is not None, n_valid=ko, n_store=self.out_cp)
-        if self.wt16 is not None:
-            K.tune_conv(n, self.P, self.Q, self.out_cp, self.cp, r, r, 1, r - 1 - p, r - 1 - p, h, w, self.cp,
-                        has_mask=self.mask_src() is not None, n_valid=self.in_c, n_store=self.cp)
+        if self.net.training_capable and self.wants_prev_delta():
+            self.dgrad = DgradPlan(n, self.P, self.Q, self.out_cp, ko, self.cp, self.in_c, r, s, p, h, w,
+                                   [(False, self.mask_src() is not None)])
 
     # geometry the kernels see (the s2d form is a stride-1, pad-0 convolution on the rearranged input)
     def _geom(self):
@@ -642,11 +634,8 @@ class Conv2dOp(Op):
                               ko, self.out_cp, r, r, s, p, p, self.P, self.Q, self.has_relu)
             self._act_forward()
             return
-        if train and self.wt16 is not None:
-            # the data-grad reads the filters transposed and flipped; re-packing them depends on the weights alone,
-            # so it runs beside the forward pass
-            w16 = self.view(self.seg_w, "params16")
-            self.net.side(lambda: K.pack_dgrad_filters(w16, self.wt16, ko, self.out_cp, r * r, self.cp))
+        if train and self.dgrad:
+            self.dgrad.prepare(self.net, self.view(self.seg_w, "params16"))
         K.conv_fprop_tc(self.prev.out, self.net.batch, h, w, self.cp, self.view(self.seg_w, "params16"), ko, r, r, s,
                         p, p, self.P, self.Q, self.out, self.out_cp,
                         bias=self.view(self.seg_b) if self.seg_b else None, relu=self.has_relu, n_valid=ko,
@@ -676,20 +665,9 @@ class Conv2dOp(Op):
             if self.direct:
                 K.conv_direct_dgrad(self.dout, w16, self.prev.dout, mask, n, h, w, self.cp, ko, self.out_cp, r, r, s,
                                     p, p, self.P, self.Q)
-            elif s == 1:
-                K.conv_fprop_tc(self.dout, n, self.P, self.Q, self.out_cp, self.wt16, self.cp, r, r, 1, r - 1 - p,
-                                r - 1 - p, h, w, self.prev.dout, self.cp, mask_src=mask, n_valid=self.in_c,
-                                n_store=self.cp)
             else:
-                done = False
-                if _strided_dgrad_on_tensor_cores():
-                    if not hasattr(self, "_sd_cache"):
-                        self._sd_cache = {}
-                    done = dgrad_strided_tc(self.dout, n, self.P, self.Q, self.out_cp, w16, ko, self.cp, self.in_c, r, r,
-                                            s, p, h, w, self.prev.dout, mask, cache=self._sd_cache)
-                if not done:
-                    K.conv_direct_dgrad(self.dout, w16, self.prev.dout, mask, n, h, w, self.cp, ko, self.out_cp, r, r,
-                                        s, p, p, self.P, self.Q)
+                conv_dgrad(self.dout, n, self.P, self.Q, self.out_cp, w16, ko, self.cp, self.in_c, r, s, p, h, w,
+                           self.prev.dout, mask=mask, wt=self.dgrad.wt if self.dgrad else None)
 
     # ---- parameters in reference layout
     def _w_ref(self, w_int):

@@ -15,6 +15,7 @@ import torch.nn.functional as F
 
 from ..ops import layout
 from ..ops import native_ops as K
+from ..ops.conv_grad import DgradPlan, conv_dgrad
 from ..ops.native_ops import pad_channels
 from .operators import Op, ParamSeg, _draw, conv_out
 
@@ -41,6 +42,7 @@ class _BnConv:
             self.gk, self.gs, self.gp = r2, 1, 0
         else:
             self.gh, self.gw, self.gk, self.gs, self.gp = self.h, self.w, k, stride, pad
+        self.dgrad = None        # DgradPlan on a GPU
         n = op.name + "." + tag
         self.seg_w = ParamSeg(n + ".w", (out_c, self.gk * self.gk, in_cp))
         self.seg_g = ParamSeg(n + ".scale", (self.kp,), decay=False)
@@ -49,7 +51,8 @@ class _BnConv:
         self.seg_rv = ParamSeg(n + ".run_var", (self.kp,), decay=False, trainable=False)
         self.segs = [self.seg_w, self.seg_g, self.seg_b, self.seg_rm, self.seg_rv]
 
-    def alloc(self, need_dx_filters):
+    def alloc(self, dx_forms=()):
+        """`dx_forms`: the (addend, mask) combinations in which `backward` will be asked for the input's delta."""
         net = self.op.net
         dev, n = net.device, net.batch
         self.conv_out = torch.zeros((n, self.P, self.Q, self.kp), dtype=torch.bfloat16, device=dev)
@@ -57,18 +60,13 @@ class _BnConv:
         self.istd = torch.ones(self.kp, device=dev)
         self.sums = torch.zeros(4 * self.kp + K.BN_SCRATCH_TAIL, device=dev)
         self.dconv = torch.zeros_like(self.conv_out) if net.training_capable else None
-        self.wt16 = None
-        if net.training_capable and need_dx_filters and self.gs == 1:
-            self.wt16 = torch.zeros((self.cp, self.gk * self.gk, self.kp), dtype=torch.bfloat16, device=dev)
         if dev.type == "cuda":
             # tile plans of the forward and data-grad shapes, measured once on scratch operands
             K.tune_conv(n, self.gh, self.gw, self.cp, self.ko, self.gk, self.gk, self.gs, self.gp, self.gp, self.P,
                         self.Q, self.kp, n_valid=self.ko, n_store=self.kp)
-            if self.wt16 is not None:
-                for has_mask in (False, True):
-                    K.tune_conv(n, self.P, self.Q, self.kp, self.cp, self.gk, self.gk, 1, self.gk - 1 - self.gp,
-                                self.gk - 1 - self.gp, self.gh, self.gw, self.cp, has_mask=has_mask,
-                                n_valid=self.in_c, n_store=self.cp)
+            if net.training_capable and dx_forms:
+                self.dgrad = DgradPlan(n, self.P, self.Q, self.kp, self.ko, self.cp, self.in_c, self.k, self.s, self.p,
+                                       self.h, self.w, dx_forms)
 
     def v(self, seg, which="params"):
         return self.op.net.seg_view(seg, which)
@@ -76,6 +74,8 @@ class _BnConv:
     def forward(self, x, out, residual, relu, train, t):
         net = self.op.net
         n = net.batch
+        if train and self.dgrad:
+            self.dgrad.prepare(net, self.v(self.seg_w, "params16"))
         K.conv_fprop_tc(x, n, self.gh, self.gw, self.cp, self.v(self.seg_w, "params16"), self.ko, self.gk, self.gk,
                         self.gs, self.gp, self.gp, self.P, self.Q, self.conv_out, self.kp, n_valid=self.ko,
                         n_store=self.kp)
@@ -90,8 +90,8 @@ class _BnConv:
             K.bn_fwd_infer(self.conv_out, rows, self.kp, self.ko, self.eps, self.v(self.seg_rm), self.v(self.seg_rv),
                            self.istd, self.v(self.seg_g), self.v(self.seg_b), residual, out, relu)
 
-    def backward(self, x, dout, y_relu, dx, mask):
-        """dout: delta w.r.t. the normalised output (masked by `y_relu` here if given)."""
+    def backward(self, x, dout, y_relu, dx, mask, add=None):
+        """dout: delta w.r.t. the normalised output (masked by `y_relu` here if given); dx = mask(add + input delta)."""
         net = self.op.net
         n = net.batch
         rows = n * self.P * self.Q
@@ -106,25 +106,9 @@ class _BnConv:
         if dx is not None:
             if self.s2d is not None:
                 raise RuntimeError("a space-to-depth'd convolution is a first layer: it has no input delta")
-            w16 = self.v(self.seg_w, "params16")
-            if self.s == 1:
-                K.pack_dgrad_filters(w16, self.wt16, self.ko, self.kp, self.k * self.k, self.cp)
-                K.conv_fprop_tc(self.dconv, n, self.P, self.Q, self.kp, self.wt16, self.cp, self.k, self.k, 1,
-                                self.k - 1 - self.p, self.k - 1 - self.p, self.h, self.w, dx, self.cp, mask_src=mask,
-                                n_valid=self.in_c, n_store=self.cp)
-            else:
-                from .operators import _strided_dgrad_on_tensor_cores
-                from ..ops.conv_strided import dgrad_strided_tc
-                done = False
-                if _strided_dgrad_on_tensor_cores():
-                    if not hasattr(self, "_sd_cache"):
-                        self._sd_cache = {}
-                    done = dgrad_strided_tc(self.dconv, n, self.P, self.Q, self.kp, w16, self.ko, self.cp, self.in_c,
-                                            self.k, self.k, self.s, self.p, self.h, self.w, dx, mask,
-                                            cache=self._sd_cache)
-                if not done:
-                    K.conv_direct_dgrad(self.dconv, w16, dx, mask, n, self.h, self.w, self.cp, self.ko, self.kp, self.k,
-                                        self.k, self.s, self.p, self.p, self.P, self.Q)
+            conv_dgrad(self.dconv, n, self.P, self.Q, self.kp, self.v(self.seg_w, "params16"), self.ko, self.cp, self.in_c,
+                       self.k, self.s, self.p, self.h, self.w, dx, add=add, mask=mask,
+                       wt=self.dgrad.wt if self.dgrad else None)
 
     # ---- parameters
     def _w_int(self, w_oihw):
@@ -229,7 +213,7 @@ class BNormConv2dOp(_BlockBase):
 
     def alloc(self):
         super().alloc()
-        self.u.alloc(self.wants_prev_delta())
+        self.u.alloc([(False, self.mask_src() is not None)] if self.wants_prev_delta() else ())
 
     def forward(self, train, t):
         self.u.forward(self.prev.out, self.out, None, self.has_relu, train, t)
@@ -264,8 +248,8 @@ class StackResConv2dOp(_BlockBase):
 
     def alloc(self):
         super().alloc()
-        self.u1.alloc(self.wants_prev_delta())
-        self.u2.alloc(True)
+        self.u1.alloc([(True, self.prev.has_relu)] if self.wants_prev_delta() else ())
+        self.u2.alloc([(False, True)])
         self.a1 = torch.zeros_like(self.out)
         self.da1 = torch.zeros_like(self.out) if self.net.training_capable else None
 
@@ -278,10 +262,8 @@ class StackResConv2dOp(_BlockBase):
         x = self.prev.out
         self.u2.backward(self.a1, self.dout, None, self.da1, self.a1)
         if self.wants_prev_delta():
-            self.u1.backward(x, self.da1, None, self.prev.dout, None)
-            K.add_bf16(self.prev.dout, self.dout, self.dout.numel())
-            if self.prev.has_relu:
-                K.relu_mask(self.prev.dout, self.prev.out, self.dout.numel())
+            # the identity path's delta and the producer's ReLU ride in the epilogue of the convolution's data-gradient
+            self.u1.backward(x, self.da1, None, self.prev.dout, self.mask_src(), add=self.dout)
         else:
             self.u1.backward(x, self.da1, None, None, None)
 
@@ -318,14 +300,14 @@ class ProjStackResConv2dOp(_BlockBase):
     def alloc(self):
         super().alloc()
         need = self.wants_prev_delta()
-        self.u1.alloc(need)
-        self.u2.alloc(True)
-        self.u3.alloc(need)
+        masked = self.prev.has_relu
+        self.u1.alloc([(False, masked)] if need else ())
+        self.u2.alloc([(False, True)])
+        self.u3.alloc([(True, masked)] if need else ())
         self.a1 = torch.zeros_like(self.out)
         self.sc = torch.zeros_like(self.out)
         if self.net.training_capable:
             self.da1 = torch.zeros_like(self.out)
-            self.dx2 = torch.zeros_like(self.prev.out) if need else None
 
     def forward(self, train, t):
         x = self.prev.out
@@ -337,12 +319,11 @@ class ProjStackResConv2dOp(_BlockBase):
         x = self.prev.out
         need = self.wants_prev_delta()
         self.u2.backward(self.a1, self.dout, None, self.da1, self.a1)
-        self.u1.backward(x, self.da1, None, self.prev.dout if need else None, None)
-        self.u3.backward(x, self.dout, None, self.dx2 if need else None, None)
-        if need:
-            K.add_bf16(self.prev.dout, self.dx2, self.dx2.numel())
-            if self.prev.has_relu:
-                K.relu_mask(self.prev.dout, self.prev.out, self.dx2.numel())
+        # the projection adds its part to what the other path has written, at the positions that it reads; the mask of the
+        # producer's ReLU is the same for both and may be applied to each
+        dx, mask = (self.prev.dout, self.mask_src()) if need else (None, None)
+        self.u1.backward(x, self.da1, None, dx, mask)
+        self.u3.backward(x, self.dout, None, dx, mask, add=dx)
 
     def ref_forward(self, x, train, t):
         sc = self.u3.ref(x, None, False, train, t)

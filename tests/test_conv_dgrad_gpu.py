@@ -1,0 +1,67 @@
+"""The data-gradient that reads the filters in place or from their packed copy, and scatters the phases of a strided one,
+against fp64 autograd:
+channel counts below, at and off the 64-wide blocks of the operand, tiles wider than 256 columns, one and several taps,
+strides 1 to 3, an addend (its own tensor, or dx itself) with and without the producer's mask, every plan option."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from rembrandt_b200.ops import layout
+from rembrandt_b200.ops import native_ops as K
+from rembrandt_b200.ops.conv_grad import conv_dgrad
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+SHAPES = [  # N, C, Ko, H, k, stride, pad
+    (2, 16, 16, 8, 3, 1, 1), (2, 64, 64, 14, 3, 1, 1), (3, 96, 40, 9, 5, 1, 2), (2, 256, 96, 13, 3, 1, 1),
+    (1, 384, 64, 7, 3, 1, 1), (2, 512, 320, 6, 1, 1, 0), (1, 3, 64, 30, 3, 1, 1), (5, 128, 128, 19, 3, 1, 1),
+    (2, 64, 128, 14, 3, 2, 1), (2, 32, 64, 15, 3, 2, 1), (3, 64, 128, 14, 1, 2, 0), (2, 96, 48, 13, 1, 2, 0),
+    (1, 128, 256, 8, 5, 3, 2), (2, 48, 64, 11, 2, 2, 0), (33, 32, 16, 8, 3, 2, 1)]
+
+
+def _run(shape, add, masked, packed=False, **options):
+    N, C, Ko, H, k, s, p = shape
+    g = torch.Generator(device=DEV).manual_seed(sum(shape))
+    rnd = lambda *d: torch.randn(d, generator=g, device=DEV).bfloat16().float()
+    Cp, Kp = K.pad_channels(C), K.pad_channels(Ko)
+    P = (H + 2 * p - k) // s + 1
+    w, dy, extra, below = rnd(Ko, C, k, k), rnd(N, Ko, P, P), rnd(N, C, H, H), rnd(N, C, H, H).relu()
+    x = torch.zeros(N, C, H, H, device=DEV, requires_grad=True)
+    (want,) = torch.autograd.grad(F.conv2d(x.double(), w.double(), stride=s, padding=p), x, dy.double())
+    want = want.double()
+    want = (want + extra.double() if add else want) * (below > 0 if masked else 1)
+    dx = torch.full((N, H, H, Cp), float("nan"), device=DEV, dtype=torch.bfloat16)
+    src = None
+    if add == "own":
+        src = layout.to_nhwc_padded(extra, Cp)
+    elif add == "dx":
+        dx = src = layout.to_nhwc_padded(extra, Cp)
+    wi, wt = layout.conv_weight_to_internal(w, Cp).bfloat16(), None
+    if packed:
+        wt = torch.full((Cp, k * k, Kp), float("nan"), device=DEV, dtype=torch.bfloat16)
+        K.pack_dgrad_filters(wi, wt, Ko, Kp, k * k, Cp)
+    with K.gemm_options(**options):
+        conv_dgrad(layout.to_nhwc_padded(dy, Kp), N, P, P, Kp, wi, Ko, Cp, C, k, s, p, H, H, dx, add=src,
+                   mask=layout.to_nhwc_padded(below, Cp) if masked else None, wt=wt)
+    torch.cuda.synchronize()
+    assert K.read_status() == 0
+    got = layout.from_nhwc_padded(dx, C).double()
+    # fp32 sums of up to taps * Ko products of N(0, 1) pairs, rounded once to bf16
+    err = (got - want).abs() - want.abs() * 2 ** -8
+    assert float(err.max()) < 1e-3 * (1 + (k * k * Ko) ** 0.5)
+    assert Cp == C or bool((dx[..., C:] == 0).all())
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+@pytest.mark.parametrize("add,masked", [(None, False), (None, True), ("own", True), ("dx", False)])
+@pytest.mark.parametrize("packed", [False, True])
+def test_against_autograd(shape, add, masked, packed):
+    _run(shape, add, masked, packed)
+
+
+@pytest.mark.parametrize("shape", [SHAPES[1], SHAPES[4], SHAPES[7], SHAPES[8], SHAPES[9]])
+@pytest.mark.parametrize("options", [dict(force_mt=2), dict(force_resident=1), dict(force_box=1), dict(force_wide=1),
+                                     dict(force_pair=1), dict(force_tail=1), dict(deterministic=1)])
+def test_plans(shape, options):
+    _run(shape, "own", True, **options)
