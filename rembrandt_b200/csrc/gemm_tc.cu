@@ -127,6 +127,16 @@ __device__ __forceinline__ void pixel_coords(const GemmTcParams& p, int pix, int
   h = pp * p.cv_stride + p.cv_lower_h;
 }
 
+// first output row / column and image of weight-grad k-block `kb` (box mode)
+__device__ __forceinline__ void box_coords(const GemmTcParams& p, int kb, int& w, int& h, int& n) {
+  const int per = p.wb_groups * p.wb_pieces;
+  n = kb / per;
+  const int r = kb - n * per;
+  const int g = r / p.wb_pieces;
+  h = g * p.wb_rows;
+  w = (r - g * p.wb_pieces) * p.wb_w;
+}
+
 // One unit of a CTA's work list: tile (tm, tn) over k-blocks [kb0, kb1). `tail` >= 0 marks a part of a cut item of
 // the last wave (index among the cut items); its sums go to the fp32 workspace instead of D.
 struct WorkItem {
@@ -347,6 +357,14 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       tmem_relinquish();
     }
   }
+  if (p.a_mode == A_BOX_MN && p.wb_rows * p.wb_w < p.bk) {
+    // the k-block's rows that no box ever writes: zeros in every stage and both operands
+    const int first = p.wb_rows * p.wb_w * 8, per_block = p.bk * 8;        // in 16-byte units per 64-column block
+    const int blocks = stages * stage_bytes / (p.bk * 128);
+    for (int i = threadIdx.x; i < blocks * per_block; i += GEMM_THREADS)
+      if (i % per_block >= first) *reinterpret_cast<uint4*>(ring + (size_t)i * 16) = make_uint4(0u, 0u, 0u, 0u);
+    fence_proxy_async_smem();
+  }
   tc_fence_before();
   __syncthreads();
   if (pair) cluster_sync_all();   // the peer's barriers are initialised before anything of ours signals them
@@ -417,13 +435,16 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       // loads this warp issues per stage, one lane each
       int nload;
       const int a_split = p.a_split > 0 ? p.a_split : 1, b_split = p.b_split > 0 ? p.b_split : 1;
-      if (is_a) nload = box ? mt : (p.a_mode == A_TILED_MN ? 2 : a_split) * mt;
+      const bool a_mn_blocks = p.a_mode == A_TILED_MN || p.a_mode == A_BOX_MN;
+      if (is_a) nload = box ? mt : (a_mn_blocks ? 2 : a_split) * mt;
       else if (p.b_mode == B_TILED_MN || p.b_mode == B_DGRAD_MN) nload = p.bn_load / 64;
-      else if (p.b_mode == B_IM2COL_MN) nload = p.wg_taps > 1 ? p.wg_taps * (p.wg_cw / 64) : p.bn_load / 64;
+      else if (p.b_mode == B_IM2COL_MN || p.b_mode == B_BOX_MN)
+        nload = p.wg_taps > 1 ? p.wg_taps * (p.wg_cw / 64) : p.bn_load / 64;
       else nload = b_split;
       // a pair counts every load on the leader's `full` barriers
       const uint32_t full0_leader = pair ? mapa_shared(smem_u32(&ctl->full[0]), 0u) : 0u;
-      const uint32_t my_tx = !is_a ? (uint32_t)b_bytes
+      const uint32_t my_tx = p.a_mode == A_BOX_MN ? (uint32_t)(nload * p.wb_rows * p.wb_w * 128)
+                             : !is_a ? (uint32_t)b_bytes
                              : box ? (uint32_t)(mt * p.bx_rows * p.cv_Q * p.bk * 2)   // the boxes bring whole rows only
                                    : (uint32_t)(mt * a_bytes);
       for (int work = cta_id; work < num_work && ok; work += cta_step) {
@@ -433,8 +454,8 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
         const int m0 = tm * BM * mt;
         // geometry that is fixed for the work item (every lane keeps what its own load needs)
         // sub-tile of this lane's A load, and which of the sub-tile's boxes it is
-        const int aj = (p.a_mode == A_TILED_MN) ? (lane >> 1) : lane / a_split;
-        const int aq = (p.a_mode == A_TILED_MN) ? 0 : lane - aj * a_split;
+        const int aj = a_mn_blocks ? (lane >> 1) : lane / a_split;
+        const int aq = a_mn_blocks ? 0 : lane - aj * a_split;
         const int a_rows = BM / a_split;
         int a_w = 0, a_h = 0, a_n = 0;
         if (is_a && p.a_mode == A_IM2COL_K && lane < nload) pixel_coords(p, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
@@ -444,7 +465,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
         }
         int b_tap = 0, b_c0 = 0;
         const int n0 = tn * p.bn + (pair ? (int)cta_rank * p.bn_load : 0);   // a pair's CTA loads its half of the rows
-        if (p.b_mode == B_IM2COL_MN) {
+        if (p.wgrad) {
           if (p.wg_taps > 1) {
             b_tap = tn * p.wg_taps;
           } else {
@@ -509,6 +530,11 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                 const int r = tap / p.cv_S;
                 const int sx = tap - r * p.cv_S;
                 tma_load_im2col_4d(saj, &p.tm_a, bar, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
+              } else if (p.a_mode == A_BOX_MN) {
+                const int half = lane & 1;
+                int w, h, n_img;
+                box_coords(p, kb, w, h, n_img);
+                tma_load_4d(saj + half * p.bk * 128, &p.tm_a, bar, mj + 64 * half, w, h, n_img);
               } else {  // A_TILED_MN: two boxes of 64 rows(M) x bk per sub-tile
                 const int half = lane & 1;
                 tma_load_2d(saj + half * p.bk * 128, &p.tm_a, bar, mj + 64 * half, kb * p.bk);
@@ -527,6 +553,16 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                           (kb - tap * p.cv_cchunks) * p.bk);
             } else if (p.b_mode == B_TILED_MN) {
               tma_load_2d(sb + lane * p.bk * 128, &p.tm_b, bar, n0 + 64 * lane, kb * p.bk);
+            } else if (p.b_mode == B_BOX_MN) {
+              int w, h, n_img;
+              box_coords(p, kb, w, h, n_img);
+              const int apt = p.wg_taps > 1 ? p.wg_cw / 64 : 32;   // 64-column blocks per tap (one tap: all of them)
+              const int t = lane / apt;
+              const int tap = min(b_tap + t, p.wg_ntaps - 1);      // slots past the last tap reload it
+              const int r = tap / p.cv_S;
+              const int sx = tap - r * p.cv_S;
+              tma_load_4d(sb + lane * p.bk * 128, &p.tm_b, bar, b_c0 + 64 * (lane - t * apt), w + sx - p.wb_pad_w,
+                          h + r - p.wb_pad_h, n_img);
             } else {  // B_IM2COL_MN
               int w, h, n_img;
               pixel_coords(p, kb * p.bk, w, h, n_img);
@@ -575,8 +611,8 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
     if (lane == 0 && cta_rank == 0) {   // of a pair, only the leader issues
-      const bool a_mn = (p.a_mode == A_TILED_MN);
-      const bool b_mn = (p.b_mode == B_TILED_MN || p.b_mode == B_IM2COL_MN || p.b_mode == B_DGRAD_MN);
+      const bool a_mn = p.a_mode == A_TILED_MN || p.a_mode == A_BOX_MN;
+      const bool b_mn = p.b_mode != B_TILED_K && p.b_mode != B_TILED_K3;
       // a tile wider than 256 columns is two MMAs side by side (256 + the rest) that share the A descriptor
       const uint32_t idesc = make_idesc_bf16(pair ? 2 * BM : BM, (uint32_t)min(p.bn, 256), a_mn ? 1u : 0u, b_mn ? 1u : 0u);
       const uint32_t idesc2 = p.bn > 256 ? make_idesc_bf16(BM, (uint32_t)(p.bn - 256), a_mn ? 1u : 0u, b_mn ? 1u : 0u) : 0u;
@@ -709,10 +745,10 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       tc_fence_after();
       int col0;        // first column of D this tile writes
       int col_limit;   // tile-local bound on stored columns
-      if (p.b_mode == B_IM2COL_MN && p.wg_taps > 1) {
+      if (p.wgrad && p.wg_taps > 1) {
         col0 = 0;            // columns are mapped per 32-column chunk below
         col_limit = p.bn;
-      } else if (p.b_mode == B_IM2COL_MN) {
+      } else if (p.wgrad) {
         const int tap = tn / p.wg_ctiles;
         const int c0 = (tn - tap * p.wg_ctiles) * p.bn;
         col0 = tap * p.wg_cpad + c0;
@@ -912,7 +948,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
           tmem_ld_wait();
           if (!tail && c >= col_limit) continue;
           int gcol = tail ? c : col0 + c;
-          if (!tail && p.b_mode == B_IM2COL_MN && p.wg_taps > 1) {
+          if (!tail && p.wgrad && p.wg_taps > 1) {
             const int t = c / p.wg_cw, cc = c - t * p.wg_cw;
             const int tap = tn * p.wg_taps + t;
             if (tap >= p.wg_ntaps || cc >= p.wg_cpad) continue;
@@ -2080,20 +2116,60 @@ int rb_conv_wgrad_tc(const void* x, int N, int H, int W, int Cp, const void* dy,
   }
   if (best_bn == 0) return -3;
   setup(p, best_bn, best_taps);
-  p.a_mode = A_TILED_MN;
-  p.b_mode = B_IM2COL_MN;
+  p.wgrad = 1;
   p.cv_P = P;
   p.cv_Q = Q;
   p.cv_stride = stride;
   p.cv_lower_h = -pad_h;
   p.cv_lower_w = -pad_w;
   p.cv_S = S;
-  const int upper_h = (P - 1) * stride - pad_h - (H - 1);
-  const int upper_w = (Q - 1) * stride - pad_w - (W - 1);
-  rc = make_map_2d(&p.tm_a, dy, Kout, (uint64_t)pixels, lddy, 64, p.bk, CU_TENSOR_MAP_SWIZZLE_128B);
-  if (rc) return rc;
-  rc = make_map_im2col(&p.tm_b, x, N, H, W, Cp, -pad_h, -pad_w, upper_h, upper_w, stride, 64, p.bk,
-                       CU_TENSOR_MAP_SWIZZLE_128B);
+  // How the pixels of a k-block are loaded:
+  //  * a 1 x 1 convolution at stride 1 reads plain rows of both tensors (96 -> 96 on 64 x 54 x 54: 14.0 -> 13.1 us);
+  //  * at stride 1, boxes of whole output rows (or pieces of one) of one image where these fill the k-blocks to 95 %,
+  //    that is rows of 8, 16, 32 or a multiple of 64: an im2col load takes up to twice as long per pixel row (64 -> 128
+  //    on 64 x 128 x 128: 266 -> 218 us; 32 -> 32 on 128 x 32 x 32: 36 -> 31, 5 x 5 on 16 x 16: 29 -> 25);
+  //  * else the im2col map: what a box leaves empty is MMA work for nothing (19 x 19 boards, 0.80 full: 46 us from im2col
+  //    loads, 48 from boxes; 13 x 13, 0.66 full: 38 against 50).
+  const bool plain = taps == 1 && stride == 1 && pad_h == 0 && pad_w == 0 && P == H && Q == W;
+  int box_rows = 0, box_w = 0, box_pieces = 1, box_groups = 1;
+  if (!plain && stride == 1 && g_opt.force_box != 0) {
+    box_pieces = (Q + p.bk - 1) / p.bk;
+    box_w = (Q + box_pieces - 1) / box_pieces;
+    box_rows = box_pieces > 1 ? 1 : p.bk / Q;
+    if (box_rows > P) box_rows = P;
+    box_groups = (P + box_rows - 1) / box_rows;
+    const double util = (double)P * Q / ((double)box_groups * box_pieces * p.bk);
+    if (util < 0.95 && g_opt.force_box != 1) box_rows = 0;
+  }
+  if (plain) {
+    p.a_mode = A_TILED_MN;
+    p.b_mode = B_TILED_MN;
+    p.wgrad = 0;
+    rc = make_map_2d(&p.tm_a, dy, Kout, (uint64_t)pixels, lddy, 64, p.bk, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!rc) rc = make_map_2d(&p.tm_b, x, Cp, (uint64_t)pixels, Cp, 64, p.bk, CU_TENSOR_MAP_SWIZZLE_128B);
+  } else if (box_rows > 0) {
+    p.a_mode = A_BOX_MN;
+    p.b_mode = B_BOX_MN;
+    p.wb_rows = box_rows;
+    p.wb_w = box_w;
+    p.wb_pieces = box_pieces;
+    p.wb_groups = box_groups;
+    p.wb_pad_h = pad_h;
+    p.wb_pad_w = pad_w;
+    p.num_kb = N * box_groups * box_pieces;
+    if (split_k > p.num_kb) split_k = p.num_kb;
+    rc = make_map_nhwc(&p.tm_a, dy, Kout, Q, P, N, lddy, 64, box_w, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!rc) rc = make_map_nhwc(&p.tm_b, x, Cp, W, H, N, Cp, 64, box_w, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+  } else {
+    p.a_mode = A_TILED_MN;
+    p.b_mode = B_IM2COL_MN;
+    const int upper_h = (P - 1) * stride - pad_h - (H - 1);
+    const int upper_w = (Q - 1) * stride - pad_w - (W - 1);
+    rc = make_map_2d(&p.tm_a, dy, Kout, (uint64_t)pixels, lddy, 64, p.bk, CU_TENSOR_MAP_SWIZZLE_128B);
+    if (!rc)
+      rc = make_map_im2col(&p.tm_b, x, N, H, W, Cp, -pad_h, -pad_w, upper_h, upper_w, stride, 64, p.bk,
+                           CU_TENSOR_MAP_SWIZZLE_128B);
+  }
   if (rc) return rc;
   p.epi = EPI_F32_ATOMIC;
   p.n_valid = p.N;

@@ -4,7 +4,8 @@
 //                or, stride 1: A = column-shifted halo tiles of X (plain tiled TMA, A_HALO_K), see gemm_tc.cu
 //   conv dgrad   A = im2col(dY) K-major               B = the filters as they are, MN-major (TMA tiled, B_DGRAD_MN), or
 //                                                         transposed and flipped ones, K-major
-//   conv wgrad   A = dY^T MN-major (tiled)            B = im2col(X) MN-major (TMA im2col)
+//   conv wgrad   A = dY^T MN-major (tiled)            B = im2col(X) MN-major (TMA im2col; tiled boxes of whole output
+//                                                         rows for both operands, or plain rows, where that is cheaper)
 //   affine fwd   A = X K-major                        B = W K-major
 //   affine dgrad A = dY K-major                       B = W MN-major
 //   affine wgrad A = dY^T MN-major                    B = X^T MN-major
@@ -18,8 +19,8 @@
 
 namespace rb {
 
-enum : int { A_TILED_K = 0, A_IM2COL_K = 1, A_TILED_MN = 2, A_HALO_K = 3, A_BOX_K = 4 };
-enum : int { B_TILED_K = 0, B_TILED_MN = 1, B_IM2COL_MN = 2, B_TILED_K3 = 3, B_DGRAD_MN = 4 };
+enum : int { A_TILED_K = 0, A_IM2COL_K = 1, A_TILED_MN = 2, A_HALO_K = 3, A_BOX_K = 4, A_BOX_MN = 5 };
+enum : int { B_TILED_K = 0, B_TILED_MN = 1, B_IM2COL_MN = 2, B_TILED_K3 = 3, B_DGRAD_MN = 4, B_BOX_MN = 5 };
 enum : int { EPI_BF16 = 0, EPI_F32_STORE = 1, EPI_F32_ATOMIC = 2 };
 
 struct alignas(64) GemmTcParams {
@@ -51,6 +52,14 @@ struct alignas(64) GemmTcParams {
   int wg_ctiles;       // channel tiles of bn per tap (B_IM2COL_MN)
   int wg_cpad;         // padded input channels: column of D = tap*wg_cpad + channel
   int a_split, b_split; // K-major operands: TMA boxes (one issuing lane each) per 128-row A sub-tile / per B tile
+  // weight-grad from boxes (A_BOX_MN / B_BOX_MN, stride 1): a k-block is wb_rows output rows x wb_w columns of one image
+  // (wb_rows * wb_w <= bk pixels). A is that box of dY, B the same box of X shifted by the filter tap, both plain tiled
+  // loads with zero fill outside the image; the rows of the k-block past the box are zeros from the start of the kernel.
+  int wgrad;           // columns of D are (tap, channel), see wg_*
+  int wb_rows, wb_w;
+  int wb_groups;       // row groups per image
+  int wb_pieces;       // column pieces per row (output rows wider than bk)
+  int wb_pad_h, wb_pad_w;
   int n_tiles;         // tiles along N (taps*wg_ctiles for wgrad)
   // halo mode (A_HALO_K): a sub-tile is hl_rows output rows of one image at a row pitch of hl_pitch positions
   int hl_pitch;        // 8..128, a power of two >= Q; hl_rows * hl_pitch = 128
