@@ -172,6 +172,32 @@ __global__ void __launch_bounds__(256) pack_dgrad_filters_kernel(const bf16* __r
   }
 }
 
+// Columns of a first layer's filters in the order of the input operator's windows: wp[k][j] = w[k][index[j]] (0 where
+// index[j] < 0). w is [rows][row_len], wp [rows][cols].
+__global__ void gather_columns_kernel(const bf16* __restrict__ w, const int* __restrict__ index, bf16* __restrict__ wp,
+                                      int rows, int row_len, int cols) {
+  pdl_prolog();
+  const int total = rows * cols;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int k = i / cols, at = index[i - k * cols];
+    wp[i] = at >= 0 ? w[(long long)k * row_len + at] : f2bf(0.f);
+  }
+}
+
+// The way back for the gradient: g[k][index[j]] += gp[k][j], the column of ones (if any) into the bias gradient, and gp is
+// cleared for the next accumulation. No two columns share an index.
+__global__ void scatter_columns_kernel(float* __restrict__ gp, const int* __restrict__ index, float* __restrict__ g,
+                                       float* __restrict__ gbias, int rows, int row_len, int cols, int ones) {
+  pdl_prolog();
+  const int total = rows * cols;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int k = i / cols, j = i - k * cols, at = index[j];
+    if (at >= 0) g[(long long)k * row_len + at] += gp[i];
+    else if (gbias && j == ones) gbias[k] += gp[i];
+    gp[i] = 0.f;
+  }
+}
+
 // Zero the entries of a space-to-depth'd first-layer filter gradient that have no counterpart in the
 // original filter: taps (r,s) >= ksize and padded channels.  dw is [Kout][R2*S2][Cp], channel =
 // (dy*f + dx)*cin + ci, original row = R2idx*f + dy.
@@ -315,6 +341,21 @@ int rb_pack_dgrad_filters(const void* w, void* wt, int Kout, int Kp, int RS, int
   if (tiles >= 0x7FFFFFFFll) return -10;
   launch_pdl(pack_dgrad_filters_kernel, (int)(tiles < 148 * 8 ? tiles : 148 * 8), 256, 0, st, (const bf16*)w, (bf16*)wt, Kout,
              Kp, RS, Cp);
+  return RB_LAUNCH_OK();
+}
+
+int rb_gather_columns(const void* w, const int* index, void* wp, int rows, int row_len, int cols, cudaStream_t st) {
+  if ((long long)rows * cols >= 0x7FFFFFFFll) return -10;
+  launch_pdl(gather_columns_kernel, grid_for((long long)rows * cols, 256), 256, 0, st, (const bf16*)w, index, (bf16*)wp,
+             rows, row_len, cols);
+  return RB_LAUNCH_OK();
+}
+
+int rb_scatter_columns(float* gp, const int* index, float* g, float* gbias, int rows, int row_len, int cols, int ones,
+                       cudaStream_t st) {
+  if ((long long)rows * cols >= 0x7FFFFFFFll) return -10;
+  launch_pdl(scatter_columns_kernel, grid_for((long long)rows * cols, 256), 256, 0, st, gp, index, g, gbias, rows, row_len,
+             cols, ones);
   return RB_LAUNCH_OK();
 }
 

@@ -22,6 +22,7 @@ import os
 from ..ops import layout
 from ..ops import native_ops as K
 from ..ops.conv_grad import DgradPlan, conv_dgrad
+from ..ops.first_layer import WindowedFirstLayer
 from ..ops.native_ops import pad_channels
 from . import config as C
 
@@ -175,6 +176,8 @@ class DataOp(Op):
     `pad` pixels (zero fill), which gives the usual pad-and-crop augmentation.
     """
 
+    windows = None     # (size, stride, zero border, rows, columns, channel of ones): see request_windows
+
     def setup(self, net, prev):
         super().setup(net, prev)
         cfg: C.Data3dCfg = self.cfg
@@ -214,6 +217,15 @@ class DataOp(Op):
         self.s2d_hw = s2d_hw
         self.out_cp = pad_channels(f * f * c)
 
+    def request_windows(self, ksize, stride, conv_pad, P, Q, cp, ones):
+        """Write the whole receptive field of every output position of the first convolution instead. A convolution that
+        was to get its image space-to-depth'd goes on seeing what that form put into its padding (the image beyond the
+        crop window, where there is any); one on the plain image has zeros there."""
+        border = 0 if self.mode == "s2d" else conv_pad
+        self.extra_pad = conv_pad
+        self.windows = (ksize, stride, border, P, Q, ones)
+        self.out_cp = cp
+
     def request_flat(self):
         h, w, c = self.out_hwc
         self.mode, self.f = "flat", max(h, w)
@@ -221,6 +233,8 @@ class DataOp(Op):
 
     def out_buffer_shape(self):
         n = self.net.batch
+        if self.windows:
+            return (n, self.windows[3], self.windows[4], self.out_cp)
         if self.mode == "s2d":
             return (n, self.s2d_hw, self.s2d_hw, self.out_cp)
         if self.mode == "flat":
@@ -249,7 +263,11 @@ class DataOp(Op):
         h, w, c = self.src_hwc
         cfg = self.cfg
         n = self.net.batch
-        if self.mode == "nhwc":
+        form = {}
+        if self.windows:
+            f, stride, border, oh, ow, ones = self.windows
+            form = dict(stride=stride, border=border, ones=ones)
+        elif self.mode == "nhwc":
             oh, ow, f = self.crop_h, self.crop_w, 1
         elif self.mode == "s2d":
             oh = ow = self.s2d_hw
@@ -269,7 +287,7 @@ class DataOp(Op):
             sigma, pv, pe = self.pca.std, list(self.pca.eigenvalues), list(self.pca.eigenvectors)
         K.input_u8(self.stage, self.mean_dev, self.out, n, c, h, w, ch, cw, oh, ow, self.out_cp, f, lo_y, hi_y, lo_x,
                    hi_x, rnd_crop, train and self.flip, cfg.per_batch_draws, self.scale, self.mean_scale, sigma, pv,
-                   pe, self.net.data_seed, 0, self.net.step_counter)
+                   pe, self.net.data_seed, 0, self.net.step_counter, **form)
 
     def ref_forward(self, x, train, t):
         """x: [B,C,H,W] uint8 or float. Centre crop / no flip at inference, torch RNG draws when training."""
@@ -575,6 +593,7 @@ class Conv2dOp(Op):
     """Convolution + bias + optional ReLU (src/operator/mod.rs:1366-2003), on the tcgen05 implicit-GEMM kernel."""
 
     has_params = True
+    takes_windows = True     # as a first layer: reads whole receptive fields from the input operator where that pays
 
     def setup(self, net, prev):
         super().setup(net, prev)
@@ -602,10 +621,16 @@ class Conv2dOp(Op):
             self.seg_b = ParamSeg(self.name + ".b", (cfg.out_channels,))
             self.segs.append(self.seg_b)
         self.dgrad = None        # DgradPlan on a GPU
+        self.windowed = None
+        if self.takes_windows and not self.direct and type(prev) is DataOp and WindowedFirstLayer.fits(prev, k, c, net.device):
+            self.windowed = WindowedFirstLayer(prev, k, s, p, self.P, self.Q, cfg.out_channels, c, self.cp, rs * self.cp,
+                                               self.f if self.s2d else None)
 
     def alloc(self):
         super().alloc()
-        if self.net.device.type == "cuda" and not self.direct:
+        if self.windowed:
+            self.windowed.alloc(self.net.batch, self.net.device, self.out_cp, self.has_relu, self.seg_b is not None)
+        elif self.net.device.type == "cuda" and not self.direct:
             self._tune()
 
     def _tune(self):
@@ -634,6 +659,11 @@ class Conv2dOp(Op):
                               ko, self.out_cp, r, r, s, p, p, self.P, self.Q, self.has_relu)
             self._act_forward()
             return
+        if self.windowed:
+            self.windowed.forward(self.prev.out, self.view(self.seg_w, "params16"), self.out, self.out_cp,
+                                  self.view(self.seg_b) if self.seg_b else None, self.has_relu)
+            self._act_forward()
+            return
         if train and self.dgrad:
             self.dgrad.prepare(self.net, self.view(self.seg_w, "params16"))
         K.conv_fprop_tc(self.prev.out, self.net.batch, h, w, self.cp, self.view(self.seg_w, "params16"), ko, r, r, s,
@@ -647,10 +677,13 @@ class Conv2dOp(Op):
         n, ko = self.net.batch, self.cfg.out_channels
         rows = n * self.P * self.Q
         self._act_backward()
-        if self.seg_b:
-            gb = self.view(self.seg_b, "grads")
+        gb = self.view(self.seg_b, "grads") if self.seg_b else None
+        if self.seg_b and not (self.windowed and self.windowed.ones >= 0):
             self.net.side(lambda: K.colsum(self.dout, rows, self.out_cp, ko, gb))     # beside weight- and data-grad
         gw = self.view(self.seg_w, "grads")
+        if self.windowed:
+            self.windowed.backward(self.prev.out, self.dout, self.out_cp, gw, gb)
+            return
         if self.direct:
             K.conv_direct_wgrad(self.prev.out, self.dout, gw, n, h, w, self.cp, ko, self.out_cp, r, r, s, p, p, self.P,
                                 self.Q)
@@ -723,6 +756,8 @@ class ResConv2dOp(Conv2dOp):
     """out = act(conv(x) + b + x): a residual convolution without normalisation (ResidualConv2dLayer,
     src/layer_new.rs:1179-1418). The convolution and its gradients are those of `Conv2dOp`; the identity path is an
     elementwise add before the activation in forward and an add into the producer's delta in backward."""
+
+    takes_windows = False    # its identity path reads the input as an image
 
     def setup(self, net, prev):
         rc = self.cfg

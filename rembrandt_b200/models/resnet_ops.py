@@ -16,8 +16,9 @@ import torch.nn.functional as F
 from ..ops import layout
 from ..ops import native_ops as K
 from ..ops.conv_grad import DgradPlan, conv_dgrad
+from ..ops.first_layer import WindowedFirstLayer
 from ..ops.native_ops import pad_channels
-from .operators import Op, ParamSeg, _draw, conv_out
+from .operators import DataOp, Op, ParamSeg, _draw, conv_out
 
 
 class _BnConv:
@@ -43,6 +44,7 @@ class _BnConv:
         else:
             self.gh, self.gw, self.gk, self.gs, self.gp = self.h, self.w, k, stride, pad
         self.dgrad = None        # DgradPlan on a GPU
+        self.windowed = None     # a WindowedFirstLayer: the input operator writes whole receptive fields
         n = op.name + "." + tag
         self.seg_w = ParamSeg(n + ".w", (out_c, self.gk * self.gk, in_cp))
         self.seg_g = ParamSeg(n + ".scale", (self.kp,), decay=False)
@@ -60,7 +62,9 @@ class _BnConv:
         self.istd = torch.ones(self.kp, device=dev)
         self.sums = torch.zeros(4 * self.kp + K.BN_SCRATCH_TAIL, device=dev)
         self.dconv = torch.zeros_like(self.conv_out) if net.training_capable else None
-        if dev.type == "cuda":
+        if self.windowed:
+            self.windowed.alloc(n, dev, self.kp, False, False)
+        elif dev.type == "cuda":
             # tile plans of the forward and data-grad shapes, measured once on scratch operands
             K.tune_conv(n, self.gh, self.gw, self.cp, self.ko, self.gk, self.gk, self.gs, self.gp, self.gp, self.P,
                         self.Q, self.kp, n_valid=self.ko, n_store=self.kp)
@@ -74,11 +78,14 @@ class _BnConv:
     def forward(self, x, out, residual, relu, train, t):
         net = self.op.net
         n = net.batch
+        w16 = self.v(self.seg_w, "params16")
         if train and self.dgrad:
-            self.dgrad.prepare(net, self.v(self.seg_w, "params16"))
-        K.conv_fprop_tc(x, n, self.gh, self.gw, self.cp, self.v(self.seg_w, "params16"), self.ko, self.gk, self.gk,
-                        self.gs, self.gp, self.gp, self.P, self.Q, self.conv_out, self.kp, n_valid=self.ko,
-                        n_store=self.kp)
+            self.dgrad.prepare(net, w16)
+        if self.windowed:
+            self.windowed.forward(x, w16, self.conv_out, self.kp)
+        else:
+            K.conv_fprop_tc(x, n, self.gh, self.gw, self.cp, w16, self.ko, self.gk, self.gk, self.gs, self.gp, self.gp,
+                            self.P, self.Q, self.conv_out, self.kp, n_valid=self.ko, n_store=self.kp)
         rows = n * self.P * self.Q
         if train:
             # the factor comes from the device-side step counter, so that graph replays keep averaging correctly
@@ -98,6 +105,9 @@ class _BnConv:
         K.bn_bwd(self.conv_out, dout, y_relu, rows, self.kp, self.ko, self.sums, self.mean, self.istd,
                  self.v(self.seg_g), self.v(self.seg_g, "grads"), self.v(self.seg_b, "grads"), self.dconv)
         gw = self.v(self.seg_w, "grads")
+        if self.windowed:
+            self.windowed.backward(x, self.dconv, self.kp, gw)
+            return
         K.conv_wgrad_tc(x, n, self.gh, self.gw, self.cp, self.dconv, self.kp, self.ko, self.gk, self.gk, self.gs,
                         self.gp, self.gp, self.P, self.Q, gw)
         if self.s2d is not None:
@@ -195,7 +205,6 @@ class BNormConv2dOp(_BlockBase):
         cfg = self.cfg
         h, w, c = prev.out_hwc
         s2d = None
-        from .operators import DataOp
         if isinstance(prev, DataOp) and cfg.conv_stride > 1 and c <= 4 and h == w and prev.mode == "nhwc":
             # a strided first layer on a few channels (the 7 x 7 / 2 stem): the input operator writes the image
             # space-to-depth'd, and the convolution becomes stride 1 over f * f * c channels instead of a strided
@@ -205,6 +214,10 @@ class BNormConv2dOp(_BlockBase):
             s2d = (f, r2, s2d_hw)
         self.u = _BnConv(self, "conv", (h, w), c, prev.out_cp, cfg.out_channels, cfg.conv_size, cfg.conv_stride,
                          cfg.conv_pad, cfg.init_weights, cfg.bnorm_mov_avg, cfg.bnorm_epsilon, s2d=s2d)
+        if type(prev) is DataOp and WindowedFirstLayer.fits(prev, cfg.conv_size, c, net.device):
+            self.u.windowed = WindowedFirstLayer(prev, cfg.conv_size, cfg.conv_stride, cfg.conv_pad, self.u.P, self.u.Q,
+                                                 cfg.out_channels, c, self.u.cp, self.u.gk * self.u.gk * self.u.cp,
+                                                 self.u.f if s2d else None)
         self.units = (self.u,)
         self.segs = list(self.u.segs)
         self.out_hwc = (self.u.P, self.u.Q, cfg.out_channels)

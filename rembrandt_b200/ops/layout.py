@@ -66,6 +66,18 @@ def s2d_weight_from_internal(w_int: torch.Tensor, c: int, ksize: int, f: int) ->
     return wp[:, :, :ksize, :ksize].contiguous()
 
 
+def window_columns(ksize: int, c: int, cp: int, f: int | None = None) -> torch.Tensor:
+    """Where column (r * ksize + s) * c + ch of a first layer's whole receptive field lies in a row of its internal filters:
+    [R*S][cp], or the space-to-depth'd form of factor `f`."""
+    r, s, ch = torch.meshgrid(torch.arange(ksize), torch.arange(ksize), torch.arange(c), indexing="ij")
+    if f is None:
+        at = (r * ksize + s) * cp + ch
+    else:
+        r2 = (ksize + f - 1) // f
+        at = ((r // f) * r2 + s // f) * cp + ((r % f) * f + s % f) * c + ch
+    return at.reshape(-1).to(torch.int32)
+
+
 def s2d_input(x_nchw: torch.Tensor, f: int, out_hw: int, cp2: int, dtype=torch.bfloat16) -> torch.Tensor:
     """Space-to-depth of an NCHW tensor into NHWC with `out_hw` rows/cols (zero beyond the image)."""
     n, c, h, w = x_nchw.shape

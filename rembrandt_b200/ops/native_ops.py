@@ -199,6 +199,18 @@ def pack_dgrad_filters(w16, wt16, Kout, Kp, RS, Cp):
           "rb_pack_dgrad_filters")
 
 
+def gather_columns(w16, index, wp, rows, row_len, cols):
+    """wp[k][j] = w16[k][index[j]], 0 where the index is negative."""
+    check(_native.cuda().rb_gather_columns(ptr(w16), ptr(index), ptr(wp), rows, row_len, cols, stream_handle()),
+          "rb_gather_columns")
+
+
+def scatter_columns(gp, index, g, gbias, rows, row_len, cols, ones):
+    """g[k][index[j]] += gp[k][j]; gbias[k] += gp[k][ones] (gbias may be None); gp = 0."""
+    check(_native.cuda().rb_scatter_columns(ptr(gp), ptr(index), ptr(g), ptr(gbias), rows, row_len, cols, ones,
+                                            stream_handle()), "rb_scatter_columns")
+
+
 def zero_s2d_structural(dw, Kout, R2, Cp, f, cin, ksize):
     check(_native.cuda().rb_zero_s2d_structural(ptr(dw), Kout, R2, Cp, f, cin, ksize, stream_handle()),
           "rb_zero_s2d_structural")
