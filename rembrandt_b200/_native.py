@@ -59,6 +59,7 @@ _CUDA_SIGS = {
     "rb_pack_dgrad_filters": [vp, vp, i32, i32, i32, i32, vp],
     "rb_gather_columns": [vp, vp, vp, i32, i32, i32, vp],
     "rb_scatter_columns": [vp, vp, vp, vp, i32, i32, i32, i32, vp],
+    "rb_publish_stats": [vp, vp, vp, vp],
     "rb_zero_s2d_structural": [vp, i32, i32, i32, i32, i32, i32, vp],
     # activations.cu
     "rb_act_fwd": [vp, i64, i32, i32, i32, f32, vp],

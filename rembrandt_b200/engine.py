@@ -5,16 +5,17 @@ reference issues one H2D copy per image, synchronises the stream several times p
 kernel individually, the engine
 
 * stages batches through two pinned-to-device buffers on a copy stream, so the H2D copy of batch i+1 overlaps
-  the compute of batch i;
-* captures forward + backward (+ exchange + update when the backend's kernels can be captured) in one CUDA
-  graph and replays it per step;
-* returns loss / accuracy with a one-step lag through a pinned host mirror, so the host never blocks on the
-  step it has just launched.
+  the compute of batch i; the input and loss operators read the staging slot itself;
+* captures forward + backward (+ exchange + update when the backend's kernels can be captured) + the publication of
+  loss / accuracy in one CUDA graph per slot and replays it per step; an inference pass is a graph as well;
+* returns loss / accuracy with a one-step lag through a pinned host mirror that the last kernel of the step writes, so
+  the host never blocks on the step it has just launched.
 
 On CPU the same interface runs the reference path eagerly.
 """
 from __future__ import annotations
 
+import contextlib
 from typing import Optional, Tuple
 
 import torch
@@ -38,7 +39,9 @@ class StepEngine:
         self.accum = max(1, opt.minibatch_size // net.batch)   # batches per optimizer iteration
         self.lr = opt.step_size.at_iter(0)
         self.iter = 0
-        self._graphs = {}
+        self._graphs = {}          # (last of its iteration, learning rate, staging slot, mirror) -> captured step
+        self._ran = set()          # (last of its iteration, learning rate) that have run eagerly once
+        self._eval_graphs = {}     # what the loss operator reads -> captured inference pass (None: has run eagerly once)
         self._pending = None
         self._lag_stats = None
         self.launches_per_step = 0
@@ -55,7 +58,7 @@ class StepEngine:
             self._consumed = [torch.cuda.Event() for _ in range(2)]
             self._slot = 0
             self._stats_dev = torch.zeros(2, dtype=torch.float32, device=dev)
-            self._stats_host = [torch.zeros(2, dtype=torch.float32).pin_memory() for _ in range(2)]
+            self._stats_host = [torch.zeros(2, dtype=torch.float32).pin_memory() for _ in range(3)]   # [2]: inference
             self._stats_ready = [torch.cuda.Event() for _ in range(2)]
             self._lr_dev = None
             # optional timing of the host-to-device copies (`time_h2d(True)`): pairs of events around each copy
@@ -117,12 +120,49 @@ class StepEngine:
         return self._stage_imgs[0].numel() + self._stage_lbls[0].numel() * 4 + extra
 
     # ------------------------------------------------------------------ one batch
-    def _bind_inputs(self, slot):
-        """Point the input and loss operators at a staging slot (device-to-device, on the compute stream)."""
-        self.net.input_op.stage.copy_(self._stage_imgs[slot], non_blocking=True)
-        self.net.loss_op.labels.copy_(self._stage_lbls[slot], non_blocking=True)
+    @contextlib.contextmanager
+    def _reading(self, slot):
+        """While active the input and loss operators read this staging slot (their own buffers are left for `load_batch`)."""
+        io, lo = self.net.input_op, self.net.loss_op
+        saved = io.stage, lo.labels, getattr(io, "shapes", None)
+        io.stage, lo.labels = self._stage_imgs[slot], self._stage_lbls[slot]
         if self._stage_shapes is not None:
-            self.net.input_op.shapes.copy_(self._stage_shapes[slot], non_blocking=True)
+            io.shapes = self._stage_shapes[slot]
+        try:
+            yield
+        finally:
+            io.stage, lo.labels = saved[:2]
+            if self._stage_shapes is not None:
+                io.shapes = saved[2]
+
+    def _publish(self, mirror):
+        """Loss / correct accumulated since the last time into a pinned mirror; the accumulators start again."""
+        lo = self.net.loss_op
+        if self.net.device.type == "cuda":
+            K.publish_stats(lo.loss_sum, lo.correct, self._stats_host[mirror])
+            return
+        self._stats_dev[0:1].copy_(lo.loss_sum, non_blocking=True)
+        self._stats_dev[1:2].copy_(lo.correct, non_blocking=True)
+        self._stats_host[mirror].copy_(self._stats_dev, non_blocking=True)
+        lo.loss_sum.zero_()
+        lo.correct.zero_()
+
+    def _capture(self, fn):
+        """`fn`'s launches on the current stream as a graph."""
+        stream = torch.cuda.current_stream()
+        stream.synchronize()
+        g = torch.cuda.CUDAGraph()
+        if self.comm.num_workers() > 1:
+            with torch.cuda.graph(g, stream=stream):
+                fn()
+            return g
+        # nothing is allocated or exchanged inside: no need to empty the allocator's cache and collect garbage first
+        g.capture_begin(capture_error_mode="thread_local")
+        try:
+            fn()
+        finally:
+            g.capture_end()
+        return g
 
     def _fwd_bwd(self, train=True, hook=None):
         with span("forward"):
@@ -179,43 +219,37 @@ class StepEngine:
         c = self.comm
         return c.num_workers() <= 1 or getattr(c, "graph_safe", False)
 
-    def _run_step(self, last_of_iteration: bool):
-        """Forward + backward (+ update when this batch completes a minibatch) on the compute stream."""
-        key = (last_of_iteration, self.lr if last_of_iteration else 0.0)
+    def _run_step(self, slot: int, mirror: int, last_of_iteration: bool):
+        """Forward + backward (+ update when this batch completes a minibatch) of a staged batch on the compute stream."""
+        conf = (last_of_iteration, self.lr if last_of_iteration else 0.0)
+        key = conf + (slot, mirror)
         full = last_of_iteration and self._graph_safe_update()
         hook = None
         if last_of_iteration and self._overlapped():
             # the exchange of a gradient bucket starts from inside backward, as soon as the bucket is complete
             self.comm.prepare(self.stepper, self.lr)
             hook = self.comm.on_op_backward
-        if self.use_graph:
+
+        def body(update):
+            with self._reading(slot):
+                self._fwd_bwd(hook=hook)
+            if update:
+                self._update()
+            self._publish(mirror)
+
+        if self.use_graph and conf in self._ran:
             g = self._graphs.get(key)
             if g is None:
-                # first use of this configuration runs eagerly (allocations, lazy init); the second captures
-                before = K.LAUNCHES[0]
-                self._fwd_bwd(hook=hook)
-                if full:
-                    self._update()
-                self.launches_per_step = K.LAUNCHES[0] - before
-                self._graphs[key] = "warm"
-            else:
-                if g == "warm":
-                    torch.cuda.current_stream().synchronize()
-                    g = torch.cuda.CUDAGraph()
-                    with torch.cuda.graph(g, stream=torch.cuda.current_stream()):
-                        self._fwd_bwd(hook=hook)
-                        if full:
-                            self._update()
-                    self._graphs[key] = g
-                g.replay()
+                g = self._graphs[key] = self._capture(lambda: body(full))
+            g.replay()
             if last_of_iteration and not full:
                 self._update()
-        else:
-            before = K.LAUNCHES[0]
-            self._fwd_bwd(hook=hook)
-            if last_of_iteration:
-                self._update()
-            self.launches_per_step = K.LAUNCHES[0] - before
+            return
+        # without graphs, or the first use of this configuration (allocations, lazy initialisation)
+        before = K.LAUNCHES[0]
+        body(last_of_iteration)
+        self.launches_per_step = K.LAUNCHES[0] - before
+        self._ran.add(conf)
 
     def step(self) -> Optional[Tuple[float, int]]:
         """Run the queued batch. Returns (loss, correct) of the *previous* call on CUDA (one-step lag), of this
@@ -234,18 +268,10 @@ class StepEngine:
         cs = self.compute_stream
         with torch.cuda.stream(cs):
             cs.wait_event(self._copy_done[slot])
-            self._bind_inputs(slot)
-            self._consumed[slot].record(cs)
-            self._run_step(last)
-            # publish loss / correct through the pinned mirror, then clear the accumulators
-            lo = net.loss_op
-            self._stats_dev[0:1].copy_(lo.loss_sum, non_blocking=True)
-            self._stats_dev[1:2].copy_(lo.correct, non_blocking=True)
             i = net.t & 1
-            self._stats_host[i].copy_(self._stats_dev, non_blocking=True)
+            self._run_step(slot, i, last)
+            self._consumed[slot].record(cs)
             self._stats_ready[i].record(cs)
-            lo.loss_sum.zero_()
-            lo.correct.zero_()
         prev = None
         if self._lag_stats is not None:
             j = self._lag_stats
@@ -282,12 +308,32 @@ class StepEngine:
             net.forward(False)
             return net.read_stats()
         with torch.cuda.stream(self.compute_stream):
-            if self._stage_shapes is None:
-                images_u8 = images_u8.to(net.device, non_blocking=True)
-            net.load_batch(images_u8, labels.to(net.device, non_blocking=True).int())
-            net.forward(False)
+            net.load_batch(images_u8, labels.int())      # host batches go straight into the operators' own buffers
+            self._eval_forward()
+            self._publish(2)
         self.compute_stream.synchronize()
-        return net.read_stats()
+        return float(self._stats_host[2][0]), int(self._stats_host[2][1])
+
+    def _eval_forward(self):
+        """The inference pass over the loaded batch: eager the first time, then a graph. What may differ between two calls
+        is what the loss operator has been given and the planner's options; a graph belongs to one such state and keeps
+        the tensors that it reads."""
+        net, lo = self.net, self.net.loss_op
+        if not self.use_graph:
+            net.forward(False)
+            return
+        read = [getattr(lo, n, None) for n in ("weights", "mask", "soft", "probs", "cat_weights", "target_w")]
+        key = (K.OPTION_CHANGES[0], net.sample_weight,
+               tuple(None if t is None else (t.data_ptr(), tuple(t.shape)) for t in read))
+        if key not in self._eval_graphs:
+            if len(self._eval_graphs) >= 4:
+                self._eval_graphs.clear()
+            self._eval_graphs[key] = None
+            net.forward(False)
+            return
+        if self._eval_graphs[key] is None:
+            self._eval_graphs[key] = (self._capture(lambda: net.forward(False)), read)
+        self._eval_graphs[key][0].replay()
 
     def synchronize(self):
         if self.is_cuda:

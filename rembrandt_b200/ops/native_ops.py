@@ -59,11 +59,15 @@ def gemm_workspace() -> torch.Tensor:
     return ws
 
 
+OPTION_CHANGES = [0]   # how often the planner's options or cached plans have been changed in this process
+
+
 def gemm_set_option(name: str, value: int) -> None:
     """Planner switch of the tensor-core kernel by name (force_mt, force_resident, force_halo, force_taps, force_tail,
     force_wide, bk32, bn_cap, a_split, b_split, autotune, deterministic); initial values come from RB_GEMM_<NAME> at first use."""
     if _native.cuda().rb_gemm_set_option(name.encode(), int(value)) != 0:
         raise KeyError(name)
+    OPTION_CHANGES[0] += 1
 
 
 def gemm_get_option(name: str) -> int:
@@ -126,6 +130,7 @@ def gemm_last_launch() -> dict:
 
 
 def gemm_clear_plans() -> None:
+    OPTION_CHANGES[0] += 1
     _native.cuda().rb_gemm_clear_plans()
 
 
@@ -259,6 +264,11 @@ def count_above(x, threshold, out):
     """out[0] (int64, device) += number of elements of the bf16 / fp32 tensor `x` with |x| > threshold."""
     check(_native.cuda().rb_count_above(ptr(x), x.numel(), int(x.dtype == torch.float32), float(threshold), ptr(out),
                                         stream_handle()), "rb_count_above")
+
+
+def publish_stats(loss_sum, correct, host):
+    """host (pinned float32 [2]) = (loss_sum, correct); both accumulators are cleared."""
+    check(_native.cuda().rb_publish_stats(ptr(loss_sum), ptr(correct), ptr(host), stream_handle()), "rb_publish_stats")
 
 
 def add_bf16(a, b, n):

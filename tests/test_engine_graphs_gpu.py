@@ -1,0 +1,63 @@
+"""Steps and inference passes replayed from graphs against the same engine without graphs: alternating staging slots, an
+inference pass between feeding a batch and stepping on it, host batches of other label types, what the loss operator reads
+changing between two inference passes."""
+import pytest
+import torch
+
+from rembrandt_b200.api import build_replica
+
+pytestmark = pytest.mark.gpu
+
+
+def _batches(n, batch, seed=3):
+    g = torch.Generator().manual_seed(seed)
+    return [(torch.randint(0, 256, (batch, 1, 28, 28), dtype=torch.uint8, generator=g).pin_memory(),
+             torch.randint(0, 10, (batch,), dtype=torch.int32, generator=g).pin_memory()) for _ in range(n)]
+
+
+def _pair(batch):
+    return [build_replica("lenet", batch, use_graph=ug, seed=(5, 7)) for ug in (True, False)]
+
+
+def test_steps_and_inference_passes_agree_with_eager():
+    batch = 17
+    seen = []
+    for eng in _pair(batch):
+        out = []
+        for i, (x, y) in enumerate(_batches(9, batch)):
+            eng.feed(x, y)
+            if i % 3 == 1:                        # the staged batch must survive a validation pass
+                vx, vy = _batches(1, batch, seed=50 + i)[0]
+                out.append(eng.eval_batch(vx, vy.long() if i == 4 else vy))
+            s = eng.step()
+            if s is not None:
+                out.append(s)
+        out.append(eng.flush())
+        eng.synchronize()
+        seen.append((out, eng.net.params.clone()))
+    (a, pa), (b, pb) = seen
+    assert len(a) == len(b) == 12
+    for (la, ca), (lb, cb) in zip(a, b):
+        # the same kernels on the same data; sums of several CTAs may be added in another order
+        assert abs(la - lb) < 1e-3 * max(1.0, abs(lb)) and abs(ca - cb) <= 1
+    assert float((pa - pb).norm() / pb.norm()) < 1e-4
+
+
+def test_an_inference_graph_follows_what_the_loss_reads():
+    batch = 8
+    graphed, eager = _pair(batch)
+    (x, y), (x2, y2) = _batches(2, batch)
+    masks = [None, torch.ones(batch, 10, dtype=torch.uint8), None]
+    masks[1][:, ::2] = 0
+    on_device = (x2.cuda(), y2.cuda())
+    torch.cuda.synchronize()
+    for mask in masks:
+        for eng in (graphed, eager):
+            eng.net.loss_op.load_mask(mask)
+        for data in ((x, y), (x2, y2), (x, y), on_device, (x2.clone(), y2.clone())):
+            a, b = graphed.eval_batch(*data), eager.eval_batch(*data)
+            if mask is None:
+                assert abs(a[0] - b[0]) < 1e-3 * max(1.0, b[0]) and a[1] == b[1]
+            else:                                 # labels on masked categories make the loss infinite in both
+                assert a[1] == b[1] and (a[0] == b[0] or abs(a[0] - b[0]) < 1e-3 * abs(b[0]) or a[0] != a[0])
+    assert len(graphed._eval_graphs) == 2
