@@ -275,6 +275,47 @@ __device__ __forceinline__ bool issue_item(const IssueCtx& c, SharedCtl* ctl, un
   return true;
 }
 
+// The bf16 epilogue of 32 columns of one row without padded columns: packed fp32 adds for the bias, one conversion per pair,
+// ReLU and the mask of the previous layer's ReLU on the packed bf16 pair (rounding is monotone, so clamping after it gives
+// the same bits as clamping before), into 16-byte chunks of a 128-byte swizzled slab row (chunk index XOR row mod 8, the
+// layout the store's tensor map expects).
+// What a launch does not use is not there at all: two epilogue warps share a scheduler, and with the flags tested per
+// element a 32 x 64 slab took 2300 cycles, most of them branches.
+template <bool BIAS, bool RELU, bool MASK, bool ADD>
+__device__ __forceinline__ void epilogue_half(const uint32_t (&v)[32], uint8_t* row, int swz, int half, const float* bias,
+                                              const uint4* mask, const uint4* add) {
+  const __nv_bfloat162 zero2 = __floats2bfloat162_rn(0.f, 0.f);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    uint4 o;
+    uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
+    float4 bq[2];   // eight columns' worth at a time: all 32 would put the kernel over its register budget
+    if (BIAS) {
+      bq[0] = __ldg(reinterpret_cast<const float4*>(bias + q * 8));
+      bq[1] = __ldg(reinterpret_cast<const float4*>(bias + q * 8 + 4));
+    }
+    const float* bb = reinterpret_cast<const float*>(&bq[0]);
+    const uint4 av = ADD ? add[q] : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t* aw = reinterpret_cast<const uint32_t*>(&av);
+    const __nv_bfloat162* m2 = reinterpret_cast<const __nv_bfloat162*>(&mask[q]);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float x0 = __uint_as_float(v[q * 8 + 2 * e]), x1 = __uint_as_float(v[q * 8 + 2 * e + 1]);
+      if (BIAS) add2_f32(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1], bb[2 * e], bb[2 * e + 1], x0, x1);
+      if (ADD) {
+        x0 += __uint_as_float(aw[e] << 16);
+        x1 += __uint_as_float(aw[e] & 0xFFFF0000u);
+      }
+      __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
+      if (RELU) h = __hmax2(h, zero2);
+      uint32_t w = *reinterpret_cast<uint32_t*>(&h);
+      if (MASK) w &= __hgt2_mask(m2[e], zero2);
+      ow[e] = w;
+    }
+    *reinterpret_cast<uint4*>(row + ((half * 4 + q) ^ swz) * 16) = o;
+  }
+}
+
 // PAIR: the instantiation that runs as clusters of two CTAs (p.pair != 0). It is a kernel of its own because a
 // kernel that contains cta_group::2 instructions can only be launched with an even cluster size.
 // EXT: the instantiation whose bf16 epilogue can scatter rows and take an addend. The tests for these cost the epilogue of
@@ -725,10 +766,15 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
     const uint32_t set_cols = (uint32_t)(mt * p.acc_stride);
     const int col_half = (warp - 2) >> 2;        // which of the two warps of this lane quarter
     uint8_t* stg = staging + (warp - 2) * 4096;  // one 32-row x 128-byte slab buffer per warp
+    // a second one (bf16 epilogue, short main loops) lets a slab be worked on while the store of the one before it is
+    // still reading shared memory, which takes as long as the slab itself while the output is on its way to memory
+    const uint32_t flip_buf = p.epi_bufs == 2 ? (uint32_t)STAGING_BYTES : 0u;
+    uint32_t buf_off = 0u;
     const bool has_bias = p.bias != nullptr;
     uint64_t* mbar_m = &ctl->mask_bar[warp - 2];
     uint32_t mask_ph = 0;
     const float act_lo = p.relu ? 0.f : -INFINITY;
+    const int epi_kind = (has_bias ? 1 : 0) | (p.relu ? 2 : 0) | (p.mask_src ? 4 : 0);
     int acc = 0;
     uint32_t acc_ph = 0;
     bool ok = true;
@@ -793,8 +839,12 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
           // the two warps of a lane quarter alternate slabs, starting with the other warp on the second sub-tile, so
           // that a tile with an odd number of slabs (96 columns = a full and a half slab) splits evenly between them
           for (int c = ((col_half + j) & 1) * 64; c < p.bn && col0 + c < p.n_store; c += 128) {
-            uint8_t* buf = stg;
-            if (lane == 0) tma_store_wait_read<0>();   // the store that last used this buffer has read it
+            uint8_t* buf = stg - buf_off;
+            if (lane == 0) {   // the store that last used this buffer has read it
+              if (flip_buf) tma_store_wait_read<1>();
+              else tma_store_wait_read<0>();
+            }
+            buf_off ^= flip_buf;
             __syncwarp();
             const int gcol = col0 + c;
             uint4 mreg[8];
@@ -824,64 +874,59 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
               __syncwarp();
             }
             RB_PROF_T0(warp == 2);
+            uint8_t* const slab_row = buf + lane * 128;
+            const int swz = lane & 7;
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
               uint32_t v[32];
               const int nbase = gcol + half * 32;
               if (nbase >= p.n_store) continue;            // these columns do not exist in D: the store clips them
-              const bool fast = nbase + 32 <= p.n_valid;   // no padded column in this 32-column group
               tmem_ld_32x32(t_addr + (uint32_t)(c + half * 32), v);
               tmem_ld_wait();
-              const __nv_bfloat162 zero2 = __floats2bfloat162_rn(0.f, 0.f);
+              const float* bias = p.bias + nbase;
+              const uint4* m = &mreg[half * 4];
+              uint4 av[4];
+              if (addend) {
 #pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                uint4 o;
-                uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-                const uint4 mv = p.mask_src ? mreg[half * 4 + q] : make_uint4(0u, 0u, 0u, 0u);
-                const __nv_bfloat162* m2 = reinterpret_cast<const __nv_bfloat162*>(&mv);
-                uint4 av = make_uint4(0u, 0u, 0u, 0u);
-                if (addend && drow_of >= 0 && nbase + q * 8 < p.n_store)
-                  av = *reinterpret_cast<const uint4*>(p.add_src + drow_of * p.ldd + nbase + q * 8);
-                const uint32_t* aw = reinterpret_cast<const uint32_t*>(&av);
-                if (fast) {
-                  // Two epilogue warps share a scheduler, so this is bound by instruction count and dependent-issue
-                  // latency: packed fp32 adds for the bias, one conversion per pair, ReLU and the mask of the
-                  // previous layer's ReLU on the packed bf16 pair (rounding is monotone, so clamping after it gives
-                  // the same bits as clamping before).
-                  // (the bias is fetched eight columns at a time: holding all 32 columns' worth in registers put the
-                  // kernel over its register budget)
-                  float4 bq[2];
-                  if (has_bias) {
-                    bq[0] = __ldg(reinterpret_cast<const float4*>(p.bias + nbase + q * 8));
-                    bq[1] = __ldg(reinterpret_cast<const float4*>(p.bias + nbase + q * 8 + 4));
-                  }
-                  const float* bb = reinterpret_cast<const float*>(&bq[0]);
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    float x0 = __uint_as_float(v[q * 8 + 2 * e]), x1 = __uint_as_float(v[q * 8 + 2 * e + 1]);
-                    if (has_bias) add2_f32(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1], bb[2 * e], bb[2 * e + 1], x0, x1);
-                    if (addend) {
-                      x0 += __uint_as_float(aw[e] << 16);
-                      x1 += __uint_as_float(aw[e] & 0xFFFF0000u);
-                    }
-                    __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-                    if (p.relu) h = __hmax2(h, zero2);
-                    uint32_t w = *reinterpret_cast<uint32_t*>(&h);
-                    if (p.mask_src) w &= __hgt2_mask(m2[e], zero2);
-                    ow[e] = w;
-                  }
+                for (int q = 0; q < 4; ++q) {
+                  av[q] = make_uint4(0u, 0u, 0u, 0u);
+                  if (drow_of >= 0 && nbase + q * 8 < p.n_store)
+                    av[q] = *reinterpret_cast<const uint4*>(p.add_src + drow_of * p.ldd + nbase + q * 8);
+                }
+              }
+              if (nbase + 32 <= p.n_valid) {   // no padded column in this 32-column group
+                if (addend) {                  // data-gradients: no bias, no ReLU
+                  if (p.mask_src) epilogue_half<false, false, true, EXT>(v, slab_row, swz, half, bias, m, av);
+                  else epilogue_half<false, false, false, EXT>(v, slab_row, swz, half, bias, m, av);
                 } else {
+                  switch (epi_kind) {
+                    case 0: epilogue_half<false, false, false, false>(v, slab_row, swz, half, bias, m, av); break;
+                    case 1: epilogue_half<true, false, false, false>(v, slab_row, swz, half, bias, m, av); break;
+                    case 2: epilogue_half<false, true, false, false>(v, slab_row, swz, half, bias, m, av); break;
+                    case 3: epilogue_half<true, true, false, false>(v, slab_row, swz, half, bias, m, av); break;
+                    case 4: epilogue_half<false, false, true, false>(v, slab_row, swz, half, bias, m, av); break;
+                    case 5: epilogue_half<true, false, true, false>(v, slab_row, swz, half, bias, m, av); break;
+                    case 6: epilogue_half<false, true, true, false>(v, slab_row, swz, half, bias, m, av); break;
+                    default: epilogue_half<true, true, true, false>(v, slab_row, swz, half, bias, m, av); break;
+                  }
+                }
+              } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  const uint32_t* aw = reinterpret_cast<const uint32_t*>(&av[q]);
                   float f[8];
 #pragma unroll
                   for (int e = 0; e < 8; ++e) {
                     const int n = nbase + q * 8 + e;
                     float x = 0.f;
-                    const float extra = !addend ? 0.f : __uint_as_float((e & 1) ? (aw[e >> 1] & 0xFFFF0000u) : (aw[e >> 1] << 16));
+                    const float extra =
+                        !addend ? 0.f : __uint_as_float((e & 1) ? (aw[e >> 1] & 0xFFFF0000u) : (aw[e >> 1] << 16));
                     if (n < p.n_valid)
                       x = fmaxf(__uint_as_float(v[q * 8 + e]) + (has_bias ? __ldg(p.bias + n) : 0.f) + extra, act_lo);
                     f[e] = x;
                   }
                   if (p.mask_src) {
+                    const __nv_bfloat162* m2 = reinterpret_cast<const __nv_bfloat162*>(&m[q]);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                       const float2 mf = __bfloat1622float2(m2[e]);
@@ -889,13 +934,12 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                       if (!(mf.y > 0.f)) f[2 * e + 1] = 0.f;
                     }
                   }
+                  uint4 o;
                   __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
                   for (int e = 0; e < 4; ++e) o2[e] = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+                  *reinterpret_cast<uint4*>(slab_row + ((half * 4 + q) ^ swz) * 16) = o;
                 }
-                // 128-byte swizzle: 16-byte chunk index XOR (row mod 8), the layout the store's tensor map expects
-                const int chunk = (half * 4 + q) ^ (lane & 7);
-                *reinterpret_cast<uint4*>(buf + lane * 128 + chunk * 16) = o;
               }
             }
             RB_PROF_ADD(warp == 2, 7);
@@ -914,6 +958,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                       *reinterpret_cast<const uint4*>(buf + rr * 128 + ((ch ^ (rr & 7)) * 16));
               }
               __syncwarp();
+              if (lane == 0) tma_store_commit();   // every slab is one group, also an empty one (see the wait above)
               continue;
             }
             fence_proxy_async_smem();
@@ -930,9 +975,10 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                         *reinterpret_cast<const uint4*>(buf + lane * 128 + ((ch ^ (lane & 7)) * 16));
               }
               __syncwarp();
-            } else if (lane == 0 && (halo || row0 < p.M)) {
+              if (lane == 0) tma_store_commit();
+            } else if (lane == 0) {
               if (halo) tma_store_4d(&p.tm_d, buf, gcol, h_w, h_p, h_n);
-              else tma_store_2d(&p.tm_d, buf, gcol, row0);
+              else if (row0 < p.M) tma_store_2d(&p.tm_d, buf, gcol, row0);
               tma_store_commit();
             }
 #ifdef RB_GEMM_PROFILE
@@ -1343,6 +1389,16 @@ static int apply_plan(GemmTcParams& p, const Plan& pl) {
   const int stage = p.mt * a_bytes + (p.b_resident ? 0 : b_bytes);
   if (panel >= TILE_SMEM_BYTES) return 0;
   p.stages = (TILE_SMEM_BYTES - panel) / stage;
+  // Two slab buffers per epilogue warp where the main loop is too short to hide the epilogue and the stages that are left
+  // still cover a whole item or are four.
+  p.epi_bufs = 1;
+  if (p.epi == EPI_BF16 && p.num_kb <= 4 && TILE_SMEM_BYTES - STAGING_BYTES > panel) {
+    const int left = (TILE_SMEM_BYTES - STAGING_BYTES - panel) / stage;
+    if (left >= 4 || (left >= 2 && left >= p.num_kb)) {
+      p.epi_bufs = 2;
+      p.stages = left;
+    }
+  }
   if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
   if (p.stages < 2) return 0;
   if (p.mt == 2 && p.M <= BM) return 0;

@@ -86,6 +86,7 @@ struct alignas(64) GemmTcParams {
   int sc_stride, sc_a, sc_b, sc_H, sc_W;
   const __nv_bfloat16* add_src;    // EPI_BF16, optional, same layout as D (may be D): added before ReLU and mask
   // epilogue
+  int epi_bufs;        // EPI_BF16: slab buffers per epilogue warp (2: the second set lies at the end of the tile space)
   int epi;
   int relu;            // EPI_BF16: clamp at zero after the bias
   int n_valid;         // columns >= n_valid are written as zero (channel padding)
