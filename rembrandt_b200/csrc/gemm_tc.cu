@@ -1,7 +1,7 @@
 // Persistent, warp-specialised tcgen05 GEMM / implicit-GEMM convolution for sm_100a.
 //
 //   warp 0      A producer: TMA loads (tiled, im2col, or halo tiles) of the A operand, one lane per box
-//   warp 1      MMA issuer (one elected lane): tcgen05.mma, fp32 accumulators in TMEM; owns TMEM alloc/dealloc
+//   warp 1      MMA issuer (one elected lane issues): tcgen05.mma, fp32 accumulators in TMEM; owns TMEM alloc/dealloc
 //   warps 2..9  epilogue: tcgen05.ld -> bias / ReLU / mask -> swizzled smem -> TMA store (bf16), or fp32 TMA
 //               store / reduce-add (split-K, gradient accumulation). Two warps share each TMEM lane quarter and
 //               alternate column slabs: with one warp per scheduler the epilogue is bound by instruction latency.
@@ -84,6 +84,14 @@ __device__ __forceinline__ bool ctl_wait(SharedCtl* ctl, uint64_t* bar, uint32_t
   return false;
 }
 
+// The same for a whole converged warp: the result is the same in every lane.
+__device__ __forceinline__ bool ctl_wait_warp(SharedCtl* ctl, uint64_t* bar, uint32_t parity, unsigned int* status) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  int ok = 0;
+  if ((threadIdx.x & 31) == 0) ok = ctl_wait(ctl, bar, parity, status) ? 1 : 0;
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
 // Role profile (built only with -DRB_GEMM_PROFILE, see `python -m rembrandt_b200._build --profile`): cycles that the
 // roles of ONE CTA (block 3) spend waiting, summed over launches -- [0] A producer on a free stage, [1] B producer on
 // a free stage, [2] MMA issuer on a filled stage, [3] MMA issuer on a drained accumulator, [4] the CTA's whole run,
@@ -99,7 +107,18 @@ __device__ __forceinline__ bool ctl_wait_role(SharedCtl* ctl, uint64_t* bar, uin
   if (blockIdx.x == 3) atomicAdd(&g_role_cycles[slot], (unsigned long long)(clock64() - t0));
   return r;
 }
+__device__ __forceinline__ bool ctl_wait_warp_role(SharedCtl* ctl, uint64_t* bar, uint32_t parity, unsigned int* status,
+                                                   int slot) {
+  const long long t0 = clock64();
+  const bool r = ctl_wait_warp(ctl, bar, parity, status);
+  if (blockIdx.x == 3 && (threadIdx.x & 31) == 0) atomicAdd(&g_role_cycles[slot], (unsigned long long)(clock64() - t0));
+  return r;
+}
 #else
+__device__ __forceinline__ bool ctl_wait_warp_role(SharedCtl* ctl, uint64_t* bar, uint32_t parity, unsigned int* status,
+                                                   int) {
+  return ctl_wait_warp(ctl, bar, parity, status);
+}
 __device__ __forceinline__ bool ctl_wait_role(SharedCtl* ctl, uint64_t* bar, uint32_t parity, unsigned int* status,
                                               int) {
   return ctl_wait(ctl, bar, parity, status);
@@ -125,16 +144,6 @@ __device__ __forceinline__ void pixel_coords(const GemmTcParams& p, int pix, int
   const int qq = r2 - pp * p.cv_Q;
   w = qq * p.cv_stride + p.cv_lower_w;
   h = pp * p.cv_stride + p.cv_lower_h;
-}
-
-// first output row / column and image of weight-grad k-block `kb` (box mode)
-__device__ __forceinline__ void box_coords(const GemmTcParams& p, int kb, int& w, int& h, int& n) {
-  const int per = p.wb_groups * p.wb_pieces;
-  n = kb / per;
-  const int r = kb - n * per;
-  const int g = r / p.wb_pieces;
-  h = g * p.wb_rows;
-  w = (r - g * p.wb_pieces) * p.wb_w;
 }
 
 // One unit of a CTA's work list: tile (tm, tn) over k-blocks [kb0, kb1). `tail` >= 0 marks a part of a cut item of
@@ -173,8 +182,8 @@ __device__ __forceinline__ int dgrad_tap(const GemmTcParams& p, int tap) {
   return p.dg_base + u * p.dg_du + (tap - u * p.cv_S) * p.dg_dv;
 }
 
-__device__ __forceinline__ void load_b(const GemmTcParams& p, uint8_t* sb, uint64_t* bar, int kb, int n0, int b_tap,
-                                       int b_c0) {
+// One k-block of a resident B panel (weights: never a weight-grad's operand), by one thread.
+__device__ __forceinline__ void load_b(const GemmTcParams& p, uint8_t* sb, uint64_t* bar, int kb, int n0) {
   const int b_split = p.b_split > 0 ? p.b_split : 1;
   const int b_rows = p.bn_load / b_split;
   if (p.b_mode == B_TILED_K) {
@@ -192,31 +201,11 @@ __device__ __forceinline__ void load_b(const GemmTcParams& p, uint8_t* sb, uint6
       tma_load_3d(sb + j * p.bk * 128, &p.tm_b, bar, n0 + 64 * j, dgrad_tap(p, tap), cc * p.bk);
   } else if (p.b_mode == B_TILED_MN) {
     for (int j = 0; j < p.bn_load / 64; ++j) tma_load_2d(sb + j * p.bk * 128, &p.tm_b, bar, n0 + 64 * j, kb * p.bk);
-  } else {  // B_IM2COL_MN
-    int w, h, n_img;
-    pixel_coords(p, kb * p.bk, w, h, n_img);
-    if (p.wg_taps > 1) {
-      // several filter taps side by side in one column tile: they share the A (dY) stage
-      const int apt = p.wg_cw / 64;  // 64-column atoms per tap
-      for (int t = 0; t < p.wg_taps; ++t) {
-        const int tap = min(b_tap + t, p.wg_ntaps - 1);   // slots past the last tap reload it; the epilogue skips them
-        const int r = tap / p.cv_S;
-        const int sx = tap - r * p.cv_S;
-        for (int j = 0; j < apt; ++j)
-          tma_load_im2col_4d(sb + (t * apt + j) * p.bk * 128, &p.tm_b, bar, 64 * j, w, h, n_img, (uint16_t)sx,
-                             (uint16_t)r);
-      }
-    } else {
-      const int r = b_tap / p.cv_S;
-      const int sx = b_tap - r * p.cv_S;
-      for (int j = 0; j < p.bn_load / 64; ++j)
-        tma_load_im2col_4d(sb + j * p.bk * 128, &p.tm_b, bar, b_c0 + 64 * j, w, h, n_img, (uint16_t)sx, (uint16_t)r);
-    }
   }
 }
 
 // The MMAs of one k-block, fully unrolled: MT sub-tiles x KK 16-deep steps (x 2 for a tile wider than 256 columns).
-// The one issuing thread's instruction stream is what bounds the kernel when operands arrive in time (a single extra
+// The issuing warp's instruction stream is what bounds the kernel when operands arrive in time (a single extra
 // branch per MMA in this loop cost 44 % on a weight-grad launch), so nothing here is computed per MMA that can be
 // computed per k-block, and only the first MMA into an accumulator carries a predicate.
 template <int KK, int MT, bool WIDE, bool PAIR>
@@ -244,7 +233,7 @@ __device__ __forceinline__ void issue_kblock(uint32_t d_tmem, uint32_t acc_strid
   }
 }
 
-// What the issuing thread needs for the k-blocks of one work item, fixed for the launch.
+// What the issuing warp needs for the k-blocks of one work item, fixed for the launch.
 struct IssueCtx {
   uint32_t ring_u32, tiles_u32, stage_bytes, b_bytes, b_in_stage;   // b_in_stage: offset of B inside a stage
   uint32_t acc_stride, a_adv, b_adv, idesc, idesc2;
@@ -257,7 +246,7 @@ template <int KK, int MT, bool WIDE, bool PAIR>
 __device__ __forceinline__ bool issue_item(const IssueCtx& c, SharedCtl* ctl, unsigned int* status, uint32_t d_tmem,
                                            int kb0, int kb1, int& s, uint32_t& ph) {
   for (int kb = kb0; kb < kb1; ++kb) {
-    if (!ctl_wait_role(ctl, &ctl->full[s], ph, status, 2)) return false;
+    if (!ctl_wait_warp_role(ctl, &ctl->full[s], ph, status, 2)) return false;
     tc_fence_after();
     const uint32_t sa = c.ring_u32 + (uint32_t)s * c.stage_bytes;
     const uint32_t sb = c.b_resident ? c.tiles_u32 + (uint32_t)kb * c.b_bytes : sa + c.b_in_stage;
@@ -473,10 +462,13 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
         }
       }
     } else if (is_a || !p.b_resident) {
-      // loads this warp issues per stage, one lane each
-      int nload;
+      // Loads this warp issues per stage, one lane each. What a lane's load needs is worked out once per launch (where in a
+      // stage it goes) or per work item (its pixel, tap or column), and carried from k-block to k-block by additions: with
+      // the divisions by run-time values that the coordinates otherwise take, a k-block cost the warp ~1200 cycles.
       const int a_split = p.a_split > 0 ? p.a_split : 1, b_split = p.b_split > 0 ? p.b_split : 1;
       const bool a_mn_blocks = p.a_mode == A_TILED_MN || p.a_mode == A_BOX_MN;
+      const int mode = is_a ? p.a_mode : 8 + p.b_mode;
+      int nload;
       if (is_a) nload = box ? mt : (a_mn_blocks ? 2 : a_split) * mt;
       else if (p.b_mode == B_TILED_MN || p.b_mode == B_DGRAD_MN) nload = p.bn_load / 64;
       else if (p.b_mode == B_IM2COL_MN || p.b_mode == B_BOX_MN)
@@ -488,30 +480,63 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                              : !is_a ? (uint32_t)b_bytes
                              : box ? (uint32_t)(mt * p.bx_rows * p.cv_Q * p.bk * 2)   // the boxes bring whole rows only
                                    : (uint32_t)(mt * a_bytes);
+      // sub-tile of this lane's A load, and which of the sub-tile's boxes it is; where the load goes inside a stage
+      const int aj = a_mn_blocks ? (lane >> 1) : lane / a_split;
+      const int aq = a_mn_blocks ? (lane & 1) : lane - aj * a_split;
+      const int a_rows = BM / a_split, b_rows = p.bn_load / b_split;
+      int dst;
+      if (box && is_a) dst = lane * a_bytes;
+      else if (is_a) dst = aj * a_bytes + (a_mn_blocks ? aq * p.bk * 128 : aq * a_rows * p.bk * 2);
+      else dst = mt * a_bytes + lane * (p.b_mode == B_TILED_K || p.b_mode == B_TILED_K3 ? b_rows * p.bk * 2 : p.bk * 128);
+      // the taps of a convolution are walked in order; a weight-grad walks pixels, bk at a time
+      const int cchunks = p.cv_cchunks > 0 ? p.cv_cchunks : 1, taps_w = p.cv_S > 0 ? p.cv_S : 1;
+      int step_q = 0, step_p = 0, step_n = 0;
+      if (mode == 8 + B_IM2COL_MN) {
+        step_q = p.bk % p.cv_Q;
+        step_p = (p.bk / p.cv_Q) % p.cv_P;
+        step_n = p.bk / (p.cv_Q * p.cv_P);
+      }
+      const int wg_apt = p.wg_taps > 1 ? p.wg_cw / 64 : 32;     // 64-column blocks per tap of a tile (one tap: all of them)
+      const int wg_t = lane / wg_apt, wg_c = 64 * (lane - wg_t * wg_apt);
       for (int work = cta_id; work < num_work && ok; work += cta_step) {
         const WorkItem it = decode_work(p, work, m_items, direct, kb_per_split);
         const int tn = it.tn, kb0 = it.kb0, kb1 = it.kb1;
         const int tm = pair ? it.tm * 2 + (int)cta_rank : it.tm;
         const int m0 = tm * BM * mt;
-        // geometry that is fixed for the work item (every lane keeps what its own load needs)
-        // sub-tile of this lane's A load, and which of the sub-tile's boxes it is
-        const int aj = a_mn_blocks ? (lane >> 1) : lane / a_split;
-        const int aq = a_mn_blocks ? 0 : lane - aj * a_split;
-        const int a_rows = BM / a_split;
-        int a_w = 0, a_h = 0, a_n = 0;
-        if (is_a && p.a_mode == A_IM2COL_K && lane < nload) pixel_coords(p, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
-        if (is_a && box) {   // lane j loads sub-tile j: image a_n, first output row a_h
+        int a_w = 0, a_h = 0, a_n = 0;   // first pixel of this lane's A load
+        if (mode == A_IM2COL_K && lane < nload) pixel_coords(p, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
+        if (mode == A_BOX_K) {   // lane j loads sub-tile j: image a_n, first output row a_h
           a_n = tm / bx_groups;
           a_h = ((tm - a_n * bx_groups) * mt + lane) * p.bx_rows;
         }
-        int b_tap = 0, b_c0 = 0;
         const int n0 = tn * p.bn + (pair ? (int)cta_rank * p.bn_load : 0);   // a pair's CTA loads its half of the rows
+        // filter tap (r, sx), its number, and channel chunk of k-block kb
+        int tap = kb0 / cchunks;
+        int cc = kb0 - tap * cchunks;
+        int r = tap / taps_w;
+        int sx = tap - r * taps_w;
+        // weight-grad: this lane's tap and channel, and the k-block's first pixel (column, row, image) or box
+        int wg_r = 0, wg_s = 0, wg_c0 = wg_c, px = 0, py = 0, pn = 0;
         if (p.wgrad) {
+          int b_tap;
           if (p.wg_taps > 1) {
-            b_tap = tn * p.wg_taps;
+            b_tap = min(tn * p.wg_taps + wg_t, p.wg_ntaps - 1);   // slots past the last tap reload it; the epilogue skips them
           } else {
             b_tap = tn / p.wg_ctiles;
-            b_c0 = (tn - b_tap * p.wg_ctiles) * p.bn;
+            wg_c0 = (tn - b_tap * p.wg_ctiles) * p.bn + 64 * lane;
+          }
+          wg_r = b_tap / taps_w;
+          wg_s = b_tap - wg_r * taps_w;
+          if (mode == 8 + B_IM2COL_MN) {
+            const int pix = kb0 * p.bk, pq = p.cv_P * p.cv_Q;
+            pn = pix / pq;
+            py = (pix - pn * pq) / p.cv_Q;
+            px = pix - pn * pq - py * p.cv_Q;
+          } else if (p.a_mode == A_BOX_MN) {
+            const int per = p.wb_groups * p.wb_pieces;
+            pn = kb0 / per;
+            py = (kb0 - pn * per) / p.wb_pieces;       // row group
+            px = kb0 - pn * per - py * p.wb_pieces;    // piece of the row
           }
         }
         for (int kb = kb0; kb < kb1; ++kb) {
@@ -525,105 +550,74 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
           }
           w_ok = __shfl_sync(0xffffffffu, w_ok, 0);
           if (!w_ok) { ok = false; break; }
-          uint8_t* sa = ring + s * stage_bytes;
-          uint8_t* sb = sa + mt * a_bytes;
+          uint8_t* to = ring + s * stage_bytes + dst;
           uint64_t* bar = &ctl->full[s];
-          if (pair) {
-            // K-major A; K-major B or filters as they lie; the bytes are counted on the leader's barrier of this stage
-            const uint32_t bar2 = full0_leader + (uint32_t)s * 8u;
-            if (lane < nload) {
-              const int tap = p.cv_cchunks > 0 ? kb / p.cv_cchunks : 0;   // filter tap (convolution operands)
-              if (is_a) {
-                uint8_t* saj = sa + aj * a_bytes + aq * a_rows * p.bk * 2;
-                if (p.a_mode == A_TILED_K) {
-                  tma2_load_2d(saj, &p.tm_a, bar2, kb * p.bk, m0 + aj * BM + aq * a_rows);
-                } else {   // A_IM2COL_K
-                  const int cc = kb - tap * p.cv_cchunks;
-                  const int r = tap / p.cv_S;
-                  const int sx = tap - r * p.cv_S;
-                  tma2_load_im2col_4d(saj, &p.tm_a, bar2, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
-                }
-              } else if (p.b_mode == B_DGRAD_MN) {
-                tma2_load_3d(sb + lane * p.bk * 128, &p.tm_b, bar2, n0 + 64 * lane, dgrad_tap(p, tap),
-                             (kb - tap * p.cv_cchunks) * p.bk);
-              } else {
-                const int b_rows = p.bn_load / b_split;
-                uint8_t* sbq = sb + lane * b_rows * p.bk * 2;
-                if (p.b_mode == B_TILED_K) tma2_load_2d(sbq, &p.tm_b, bar2, kb * p.bk, n0 + lane * b_rows);
-                else tma2_load_3d(sbq, &p.tm_b, bar2, (kb - tap * p.cv_cchunks) * p.bk, dgrad_tap(p, tap), n0 + lane * b_rows);
-              }
-            }
-          } else if (lane < nload) {
-            if (is_a) {
-              uint8_t* saj = sa + aj * a_bytes + aq * a_rows * p.bk * 2;
-              const int mj = m0 + aj * BM + aq * a_rows;
-              if (p.a_mode == A_TILED_K) {
-                tma_load_2d(saj, &p.tm_a, bar, kb * p.bk, mj);
-              } else if (box) {
-                const int tap = kb / p.cv_cchunks;
-                const int cc = kb - tap * p.cv_cchunks;
-                const int r = tap / p.cv_S;
-                const int sx = tap - r * p.cv_S;
-                tma_load_4d(sa + lane * a_bytes, &p.tm_a, bar, cc * p.bk, sx - p.bx_pad_w, a_h + r - p.bx_pad_h, a_n);
-              } else if (p.a_mode == A_IM2COL_K) {
-                const int tap = kb / p.cv_cchunks;
-                const int cc = kb - tap * p.cv_cchunks;
-                const int r = tap / p.cv_S;
-                const int sx = tap - r * p.cv_S;
-                tma_load_im2col_4d(saj, &p.tm_a, bar, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
-              } else if (p.a_mode == A_BOX_MN) {
-                const int half = lane & 1;
-                int w, h, n_img;
-                box_coords(p, kb, w, h, n_img);
-                tma_load_4d(saj + half * p.bk * 128, &p.tm_a, bar, mj + 64 * half, w, h, n_img);
-              } else {  // A_TILED_MN: two boxes of 64 rows(M) x bk per sub-tile
-                const int half = lane & 1;
-                tma_load_2d(saj + half * p.bk * 128, &p.tm_a, bar, mj + 64 * half, kb * p.bk);
-              }
-            } else if (p.b_mode == B_TILED_K) {
-              const int b_rows = p.bn_load / b_split;
-              tma_load_2d(sb + lane * b_rows * p.bk * 2, &p.tm_b, bar, kb * p.bk, n0 + lane * b_rows);
-            } else if (p.b_mode == B_TILED_K3) {
-              const int tap = kb / p.cv_cchunks;
-              const int cc = kb - tap * p.cv_cchunks;
-              const int b_rows = p.bn_load / b_split;
-              tma_load_3d(sb + lane * b_rows * p.bk * 2, &p.tm_b, bar, cc * p.bk, dgrad_tap(p, tap), n0 + lane * b_rows);
-            } else if (p.b_mode == B_DGRAD_MN) {
-              const int tap = kb / p.cv_cchunks;
-              tma_load_3d(sb + lane * p.bk * 128, &p.tm_b, bar, n0 + 64 * lane, dgrad_tap(p, tap),
-                          (kb - tap * p.cv_cchunks) * p.bk);
-            } else if (p.b_mode == B_TILED_MN) {
-              tma_load_2d(sb + lane * p.bk * 128, &p.tm_b, bar, n0 + 64 * lane, kb * p.bk);
-            } else if (p.b_mode == B_BOX_MN) {
-              int w, h, n_img;
-              box_coords(p, kb, w, h, n_img);
-              const int apt = p.wg_taps > 1 ? p.wg_cw / 64 : 32;   // 64-column blocks per tap (one tap: all of them)
-              const int t = lane / apt;
-              const int tap = min(b_tap + t, p.wg_ntaps - 1);      // slots past the last tap reload it
-              const int r = tap / p.cv_S;
-              const int sx = tap - r * p.cv_S;
-              tma_load_4d(sb + lane * p.bk * 128, &p.tm_b, bar, b_c0 + 64 * (lane - t * apt), w + sx - p.wb_pad_w,
-                          h + r - p.wb_pad_h, n_img);
-            } else {  // B_IM2COL_MN
-              int w, h, n_img;
-              pixel_coords(p, kb * p.bk, w, h, n_img);
-              if (p.wg_taps > 1) {
-                // several filter taps side by side in one column tile: they share the A (dY) stage
-                const int apt = p.wg_cw / 64;  // 64-column atoms per tap
-                const int t = lane / apt, j = lane - t * apt;
-                const int tap = min(b_tap + t, p.wg_ntaps - 1);   // slots past the last tap reload it; the epilogue skips them
-                const int r = tap / p.cv_S;
-                const int sx = tap - r * p.cv_S;
-                tma_load_im2col_4d(sb + lane * p.bk * 128, &p.tm_b, bar, 64 * j, w, h, n_img, (uint16_t)sx, (uint16_t)r);
-              } else {
-                const int r = b_tap / p.cv_S;
-                const int sx = b_tap - r * p.cv_S;
-                tma_load_im2col_4d(sb + lane * p.bk * 128, &p.tm_b, bar, b_c0 + 64 * lane, w, h, n_img, (uint16_t)sx,
-                                   (uint16_t)r);
+          const uint32_t bar2 = full0_leader + (uint32_t)s * 8u;   // pairs: the leader's barrier of this stage
+          if (lane < nload) {
+            // pairs: K-major A; K-major B or filters as they lie
+            switch (mode) {
+              case A_TILED_K:
+                if (pair) tma2_load_2d(to, &p.tm_a, bar2, kb * p.bk, m0 + aj * BM + aq * a_rows);
+                else tma_load_2d(to, &p.tm_a, bar, kb * p.bk, m0 + aj * BM + aq * a_rows);
+                break;
+              case A_IM2COL_K:
+                if (pair) tma2_load_im2col_4d(to, &p.tm_a, bar2, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
+                else tma_load_im2col_4d(to, &p.tm_a, bar, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
+                break;
+              case A_TILED_MN:   // two boxes of 64 rows(M) x bk per sub-tile
+                if (!pair) tma_load_2d(to, &p.tm_a, bar, m0 + aj * BM + 64 * aq, kb * p.bk);
+                break;
+              case A_BOX_K:
+                if (!pair) tma_load_4d(to, &p.tm_a, bar, cc * p.bk, sx - p.bx_pad_w, a_h + r - p.bx_pad_h, a_n);
+                break;
+              case A_BOX_MN:
+                if (!pair) tma_load_4d(to, &p.tm_a, bar, m0 + aj * BM + 64 * aq, px * p.wb_w, py * p.wb_rows, pn);
+                break;
+              case 8 + B_TILED_K:
+                if (pair) tma2_load_2d(to, &p.tm_b, bar2, kb * p.bk, n0 + lane * b_rows);
+                else tma_load_2d(to, &p.tm_b, bar, kb * p.bk, n0 + lane * b_rows);
+                break;
+              case 8 + B_TILED_MN:
+                if (!pair) tma_load_2d(to, &p.tm_b, bar, n0 + 64 * lane, kb * p.bk);
+                break;
+              case 8 + B_IM2COL_MN:
+                if (!pair)
+                  tma_load_im2col_4d(to, &p.tm_b, bar, wg_c0, px * p.cv_stride + p.cv_lower_w,
+                                     py * p.cv_stride + p.cv_lower_h, pn, (uint16_t)wg_s, (uint16_t)wg_r);
+                break;
+              case 8 + B_BOX_MN:
+                if (!pair)
+                  tma_load_4d(to, &p.tm_b, bar, wg_c0, px * p.wb_w + wg_s - p.wb_pad_w, py * p.wb_rows + wg_r - p.wb_pad_h,
+                              pn);
+                break;
+              default: {   // B_TILED_K3, B_DGRAD_MN: tap of the filters in memory
+                const int wtap = p.dg_dv == 0 ? tap : p.dg_base + r * p.dg_du + sx * p.dg_dv;
+                const bool k3 = p.b_mode == B_TILED_K3;
+                const int c0 = k3 ? cc * p.bk : n0 + 64 * lane, c2 = k3 ? n0 + lane * b_rows : cc * p.bk;
+                if (pair) tma2_load_3d(to, &p.tm_b, bar2, c0, wtap, c2);
+                else tma_load_3d(to, &p.tm_b, bar, c0, wtap, c2);
+                break;
               }
             }
           }
           __syncwarp();
+          if (++cc == cchunks) {
+            cc = 0;
+            ++tap;
+            if (++sx == taps_w) { sx = 0; ++r; }
+          }
+          if (p.a_mode == A_BOX_MN) {
+            if (++px == p.wb_pieces) {
+              px = 0;
+              if (++py == p.wb_groups) { py = 0; ++pn; }
+            }
+          } else if (mode == 8 + B_IM2COL_MN) {
+            px += step_q;
+            py += step_p;
+            pn += step_n;
+            if (px >= p.cv_Q) { px -= p.cv_Q; ++py; }
+            if (py >= p.cv_P) { py -= p.cv_P; ++pn; }
+          }
           ++issued;
           if (++s == stages) { s = 0; ph ^= 1u; }
         }
@@ -646,12 +640,13 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       if (blockIdx.x < num_work) {
         if (lane == 0) mbar_expect_tx(&ctl->b_full, (uint32_t)panel_bytes);
         __syncwarp();
-        for (int kb = lane; kb < p.num_kb; kb += 32) load_b(p, tiles + kb * b_bytes, &ctl->b_full, kb, 0, 0, 0);
+        for (int kb = lane; kb < p.num_kb; kb += 32) load_b(p, tiles + kb * b_bytes, &ctl->b_full, kb, 0);
       }
     }
   } else if (warp == 1) {
     // ------------------------------ MMA issuer ------------------------------
-    if (lane == 0 && cta_rank == 0) {   // of a pair, only the leader issues
+    // the whole warp runs this, converged, and one elected thread issues (see tc_mma_f16)
+    if (cta_rank == 0) {   // of a pair, only the leader issues
       const bool a_mn = p.a_mode == A_TILED_MN || p.a_mode == A_BOX_MN;
       const bool b_mn = p.b_mode != B_TILED_K && p.b_mode != B_TILED_K3;
       // a tile wider than 256 columns is two MMAs side by side (256 + the rest) that share the A descriptor
@@ -677,23 +672,23 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       int acc = 0;
       uint32_t acc_ph = 0;
       bool ok = true;
-      if (p.b_resident && blockIdx.x < num_work) ok = ctl_wait(ctl, &ctl->b_full, 0u, p.status);
+      if (p.b_resident && blockIdx.x < num_work) ok = ctl_wait_warp(ctl, &ctl->b_full, 0u, p.status);
       if (halo) {
         int bs = 0, as = 0;
         uint32_t bph = 0, aph = 0;
         const uint32_t row_bytes = (uint32_t)p.bk * 2u;
         for (int work = cta_id; work < num_work && ok; work += cta_step) {
-          if (!ctl_wait(ctl, &ctl->acc_empty[acc], acc_ph ^ 1u, p.status)) { ok = false; break; }
+          if (!ctl_wait_warp(ctl, &ctl->acc_empty[acc], acc_ph ^ 1u, p.status)) { ok = false; break; }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)acc * set_cols;
           bool fresh = true;   // the first MMA into each accumulator overwrites it
           for (int sx = 0; sx < p.cv_S && ok; ++sx) {
             for (int cc = 0; cc < p.cv_cchunks && ok; ++cc) {
-              if (!ctl_wait(ctl, &ctl->a_full[as], aph, p.status)) { ok = false; break; }
+              if (!ctl_wait_warp(ctl, &ctl->a_full[as], aph, p.status)) { ok = false; break; }
               tc_fence_after();
               const uint32_t a_base = smem_u32(a_ring + as * p.hl_a_bytes);
               for (int r = 0; r < p.hl_R; ++r) {
-                if (!ctl_wait(ctl, &ctl->full[bs], bph, p.status)) { ok = false; break; }
+                if (!ctl_wait_warp(ctl, &ctl->full[bs], bph, p.status)) { ok = false; break; }
                 tc_fence_after();
                 const uint64_t db = make_smem_desc(smem_u32(b_ring + bs * b_bytes), b_lbo, b_sbo, b_lay);
                 for (int j = 0; j < mt; ++j) {
@@ -740,7 +735,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       const int issue_kind = (kk_steps == 4 ? 0 : 3) + (idesc2 ? 2 : (mt == 2 ? 1 : 0));
       for (int work = cta_id; work < num_work && ok && !halo; work += cta_step) {
         const WorkItem it = decode_work(p, work, m_items, direct, kb_per_split);
-        if (!ctl_wait_role(ctl, &ctl->acc_empty[acc], acc_ph ^ 1u, p.status, 3)) { ok = false; break; }
+        if (!ctl_wait_warp_role(ctl, &ctl->acc_empty[acc], acc_ph ^ 1u, p.status, 3)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * set_cols;
         switch (issue_kind) {
