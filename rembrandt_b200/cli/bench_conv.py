@@ -11,6 +11,7 @@ import json
 import torch
 
 from ..ops import native_ops as K
+from ..ops.conv_grad import DgradPlan, conv_dgrad
 from ..utils.timing import time_fn, time_graph
 
 SHAPES = {
@@ -55,13 +56,11 @@ def run(name, batch, passes, iters, warmup, tune=True, roles=False, eager=False)
     if tune:
         # what a network does when it is built: the tile plans of the two overwrite-mode passes are measured once
         K.tune_conv(batch, H, W, Cp, Ko, R, R, s, p, p, P, Q, Kp, relu=True, has_bias=True, n_valid=Ko, n_store=Kp)
-        if s == 1:
-            K.tune_conv(batch, P, Q, Kp, Cp, R, R, 1, R - 1 - p, R - 1 - p, H, W, Cp, has_mask=True, n_valid=C,
-                        n_store=Cp)
     x = torch.randn(batch, H, W, Cp, device=dev).bfloat16()
     w = (torch.randn(Ko, R * R, Cp, device=dev) * 0.05).bfloat16()
-    wt = torch.zeros(Cp, R * R, Kp, device=dev, dtype=torch.bfloat16)
-    K.pack_dgrad_filters(w, wt, Ko, Kp, R * R, Cp)
+    wt = DgradPlan(batch, P, Q, Kp, Ko, Cp, C, R, s, p, H, W, [(False, True)]).wt if tune else None
+    if wt is not None:
+        K.pack_dgrad_filters(w, wt, Ko, Kp, R * R, Cp)
     b = torch.zeros(Ko, device=dev)
     y = torch.zeros(batch, P, Q, Kp, device=dev, dtype=torch.bfloat16)
     dy = torch.randn(batch, P, Q, Kp, device=dev).bfloat16()
@@ -72,14 +71,11 @@ def run(name, batch, passes, iters, warmup, tune=True, roles=False, eager=False)
     fns = {
         "fprop": lambda: K.conv_fprop_tc(x, batch, H, W, Cp, w, Ko, R, R, s, p, p, P, Q, y, Kp, bias=b, relu=True,
                                          n_valid=Ko, n_store=Kp),
-        "dgrad": lambda: K.conv_fprop_tc(dy, batch, P, Q, Kp, wt, Cp, R, R, 1, R - 1 - p, R - 1 - p, H, W, dx, Cp,
-                                         mask_src=x, n_valid=C, n_store=Cp),
+        "dgrad": lambda: conv_dgrad(dy, batch, P, Q, Kp, w, Ko, Cp, C, R, s, p, H, W, dx, mask=x, wt=wt),
         "wgrad": lambda: K.conv_wgrad_tc(x, batch, H, W, Cp, dy, Kp, Ko, R, R, s, p, p, P, Q, dw),
     }
     for name_, fn in fns.items():
         if passes != "all" and passes != name_:
-            continue
-        if name_ == "dgrad" and s != 1:
             continue
         if roles:
             fn()

@@ -2,7 +2,7 @@
 
 Three-channel images leave most of a filter tap's padded channels empty, and an implicit-GEMM load per tap fetches them all
 the same: a 3 x 3 layer on 64 images of 256 x 256 x 3 took 604 us forward and 909 us for its weight gradient, for 0.8 GB of
-real traffic each. Here the input operator writes the whole receptive field of every output position, k * k * c values side
+real traffic each (this form: 206 and 160). Here the input operator writes the whole receptive field of every output position, k * k * c values side
 by side (27 of 32 channels: no more bytes than one padded pixel), and the convolution is a 1 x 1 one over them; the weight
 gradient is a product of two matrices as they lie. A spare column holds ones, whose weight-gradient column is the bias
 gradient. The parameters keep their layout: filters are gathered into window order before the forward pass, and the
