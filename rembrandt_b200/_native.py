@@ -43,8 +43,8 @@ _CUDA_SIGS = {
     "rb_conv_direct_dgrad": [vp, vp, vp, vp] + [i32] * 13 + [vp],
     "rb_conv_direct_wgrad": [vp, vp, vp] + [i32] * 13 + [vp],
     # pool.cu
-    "rb_pool_fwd": [vp, vp, vp] + [i32] * 11 + [vp],
-    "rb_pool_bwd": [vp, vp, vp, vp, vp] + [i32] * 10 + [vp],
+    "rb_pool_fwd": [vp, vp, vp] + [i32] * 12 + [vp],
+    "rb_pool_bwd": [vp, vp, vp, vp, vp] + [i32] * 11 + [vp],
     # lrn.cu
     "rb_lrn_fwd": [vp, vp, i64, i32, i32, f32, f32, f32, vp],
     "rb_lrn_bwd": [vp, vp, vp, vp, i64, i32, i32, f32, f32, f32, vp],

@@ -2,8 +2,9 @@
 // Output extent is given by the caller (floor or ceil rounding both occur in the reference:
 // src/operator/mod.rs:2022-2027 floor, src/layer.rs:1741-1747 ceil). Average pooling divides by the
 // full window size (padding counted), as cuDNN's AverageCountIncludingPadding does
-// (src/operator/mod.rs:2053-2066). Max pooling records the window offset of the (first) maximum in
-// one byte per output so that the backward pass is an exact gather with no atomics.
+// (src/operator/mod.rs:2053-2066). Max pooling records the window offset of the (first) maximum for
+// every output so that the backward pass is an exact gather with no atomics: in one byte, or in two where
+// a byte cannot hold every offset and the code that no offset has ("no gradient", all bits set).
 #include "launch.cuh"
 #include <cstdlib>
 
@@ -11,8 +12,9 @@
 
 namespace rb {
 
-template <typename IT>
-__global__ void maxpool_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, uint8_t* __restrict__ idx, int N,
+// CT: the type of a recorded offset, uint8_t or uint16_t.
+template <typename IT, typename CT>
+__global__ void maxpool_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict__ y, CT* __restrict__ idx, int N,
                                    int H, int W, int C, int P, int Q, int k, int stride, int pad, int relu) {
   pdl_prolog();
   const int cv = C / 8;
@@ -42,21 +44,24 @@ __global__ void maxpool_fwd_kernel(const bf16* __restrict__ x, bf16* __restrict_
       }
     }
     const long long o = (((long long)n * P + p) * Q + q) * C + c8 * 8;
-    uint32_t lo = 0, hi = 0;
+    constexpr int BITS = 8 * sizeof(CT), PER = 32 / BITS;   // codes per word
+    uint32_t words[8 / PER] = {};
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       if (best[j] == -INFINITY) best[j] = 0.f;
-      if (relu && !(best[j] > 0.f)) { best[j] = 0.f; bi[j] = 255; }  // 255: no gradient flows
-      if (j < 4) lo |= (uint32_t)(bi[j] & 255) << (8 * j); else hi |= (uint32_t)(bi[j] & 255) << (8 * (j - 4));
+      if (relu && !(best[j] > 0.f)) { best[j] = 0.f; bi[j] = -1; }  // no gradient flows
+      words[j / PER] |= (uint32_t)(CT)bi[j] << (BITS * (j % PER));
     }
     store8(y + o, best);
-    *reinterpret_cast<uint2*>(idx + o) = make_uint2(lo, hi);
+#pragma unroll
+    for (int j = 0; j < 8 / PER; j += 2)
+      *reinterpret_cast<uint2*>(idx + o + j * PER) = make_uint2(words[j], words[j + 1]);
   }
 }
 
 // dx[n,h,w,c] = sum over windows covering (h,w) whose recorded argmax is (h,w) of dy.
-template <typename IT>
-__global__ void maxpool_bwd_kernel(const bf16* __restrict__ dy, const uint8_t* __restrict__ idx, bf16* __restrict__ dx,
+template <typename IT, typename CT>
+__global__ void maxpool_bwd_kernel(const bf16* __restrict__ dy, const CT* __restrict__ idx, bf16* __restrict__ dx,
                                    const bf16* __restrict__ mask_src, int N, int H, int W, int C, int P, int Q,
                                    int k, int stride, int pad) {
   pdl_prolog();
@@ -82,15 +87,19 @@ __global__ void maxpool_bwd_kernel(const bf16* __restrict__ dy, const uint8_t* _
         const int s = w - (q * stride - pad);
         const int code = r * k + s;
         const long long o = (((long long)n * P + p) * Q + q) * C + c8 * 8;
-        const uint2 iv = *reinterpret_cast<const uint2*>(idx + o);
+        constexpr int BITS = 8 * sizeof(CT), PER = 32 / BITS;
+        uint32_t words[8 / PER];
+#pragma unroll
+        for (int j = 0; j < 8 / PER; j += 2) {
+          const uint2 iv = *reinterpret_cast<const uint2*>(idx + o + j * PER);
+          words[j] = iv.x;
+          words[j + 1] = iv.y;
+        }
         float g[8];
         load8(dy + o, g);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const uint32_t word = j < 4 ? iv.x : iv.y;
-          const int b = (word >> (8 * (j & 3))) & 255;
-          if (b == code) acc[j] += g[j];
-        }
+        for (int j = 0; j < 8; ++j)
+          if ((int)(CT)(words[j / PER] >> (BITS * (j % PER))) == code) acc[j] += g[j];
       }
     }
     const long long xi = (((long long)n * H + h) * W + w) * C + c8 * 8;
@@ -246,9 +255,9 @@ __device__ __forceinline__ uint32_t div_magic(uint32_t x, uint32_t magic) { retu
 __device__ __forceinline__ __nv_bfloat162 as_bf2(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
 __device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 
-template <int KK, int SS>
+template <int KK, int SS, typename CT = uint8_t>
 __global__ void __launch_bounds__(256) maxpool_fwd_rows_kernel(const bf16* __restrict__ x, bf16* __restrict__ y,
-                                                               uint8_t* __restrict__ idx, int H, int W, int C, int P,
+                                                               CT* __restrict__ idx, int H, int W, int C, int P,
                                                                int Q, int k_rt, int stride_rt, int pad, int relu,
                                                                uint32_t cv_magic) {
   pdl_prolog();
@@ -295,25 +304,28 @@ __global__ void __launch_bounds__(256) maxpool_fwd_rows_kernel(const bf16* __res
     }
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      // an empty window leaves -inf: output 0; with a fused ReLU non-positive maxima become 0 with code 255
+      // an empty window leaves -inf: output 0; with a fused ReLU non-positive maxima become 0 without a gradient
       uint32_t keep = ~__heq2_mask(as_bf2(best[e]), as_bf2(ninf2));
       if (relu) {
         const uint32_t pos = __hgt2_mask(as_bf2(best[e]), zero2);
-        bi[e] = (bi[e] & pos) | (0x00FF00FFu & ~pos);
+        bi[e] = (bi[e] & pos) | ~pos;
         keep &= pos;
       }
       best[e] &= keep;
     }
     const long long o = orow + (long long)j * 8;
     *reinterpret_cast<uint4*>(y + o) = make_uint4(best[0], best[1], best[2], best[3]);
-    // low bytes of the four 16-bit code pairs -> 8 code bytes
-    *reinterpret_cast<uint2*>(idx + o) = make_uint2(__byte_perm(bi[0], bi[1], 0x6420), __byte_perm(bi[2], bi[3], 0x6420));
+    if (sizeof(CT) == 2)
+      *reinterpret_cast<uint4*>(idx + o) = make_uint4(bi[0], bi[1], bi[2], bi[3]);
+    else   // low bytes of the four 16-bit code pairs -> 8 code bytes
+      *reinterpret_cast<uint2*>(idx + o) =
+          make_uint2(__byte_perm(bi[0], bi[1], 0x6420), __byte_perm(bi[2], bi[3], 0x6420));
   }
 }
 
-template <int KK, int SS>
+template <int KK, int SS, typename CT = uint8_t>
 __global__ void __launch_bounds__(256) maxpool_bwd_rows_kernel(const bf16* __restrict__ dy,
-                                                               const uint8_t* __restrict__ idx, bf16* __restrict__ dx,
+                                                               const CT* __restrict__ idx, bf16* __restrict__ dx,
                                                                const bf16* __restrict__ mask_src, int H, int W, int C,
                                                                int P, int Q, int k_rt, int stride_rt, int pad,
                                                                uint32_t cv_magic) {
@@ -326,7 +338,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_rows_kernel(const bf16* __res
   const int p_lo = max(0, (h + pad - k + stride) / stride), p_hi = min(P - 1, (h + pad) / stride);
   const long long xrow = ((long long)n * H + h) * W * C;
   const bf16* dyn = dy + (long long)n * P * Q * C;
-  const uint8_t* idn = idx + (long long)n * P * Q * C;
+  const CT* idn = idx + (long long)n * P * Q * C;
   const __nv_bfloat162 zero2 = as_bf2(0u);
   for (int j = threadIdx.x; j < W * cv; j += blockDim.x) {
     const int w = (int)div_magic((uint32_t)j, cv_magic), c8 = j - w * cv;
@@ -337,15 +349,30 @@ __global__ void __launch_bounds__(256) maxpool_bwd_rows_kernel(const bf16* __res
       for (int q = q_lo; q <= q_hi; ++q) {
         const int code = r * k + (w - (q * stride - pad));
         const int o = (p * Q + q) * C + c8 * 8;
-        const uint2 iv = *reinterpret_cast<const uint2*>(idn + o);
-        const uint32_t pat = (uint32_t)code * 0x01010101u;
-        const uint32_t mlo = __vcmpeq4(iv.x, pat), mhi = __vcmpeq4(iv.y, pat);   // 0xff where the code matches
-        if ((mlo | mhi) == 0u) continue;
+        uint32_t m[4];   // a channel pair's 16-bit halves: all ones where the code matches
+        if (sizeof(CT) == 2) {
+          const uint4 iv = *reinterpret_cast<const uint4*>(idn + o);
+          const uint32_t pat = (uint32_t)code * 0x00010001u;
+          m[0] = __vcmpeq2(iv.x, pat);
+          m[1] = __vcmpeq2(iv.y, pat);
+          m[2] = __vcmpeq2(iv.z, pat);
+          m[3] = __vcmpeq2(iv.w, pat);
+          if ((m[0] | m[1] | m[2] | m[3]) == 0u) continue;
+        } else {
+          const uint2 iv = *reinterpret_cast<const uint2*>(idn + o);
+          const uint32_t pat = (uint32_t)code * 0x01010101u;
+          const uint32_t mlo = __vcmpeq4(iv.x, pat), mhi = __vcmpeq4(iv.y, pat);   // 0xff where the code matches
+          if ((mlo | mhi) == 0u) continue;
+          m[0] = __byte_perm(mlo, 0u, 0x1100);
+          m[1] = __byte_perm(mlo, 0u, 0x3322);
+          m[2] = __byte_perm(mhi, 0u, 0x1100);
+          m[3] = __byte_perm(mhi, 0u, 0x3322);
+        }
         const uint4 g = *reinterpret_cast<const uint4*>(dyn + o);
-        acc[0] = __hadd2(acc[0], as_bf2(g.x & __byte_perm(mlo, 0u, 0x1100)));
-        acc[1] = __hadd2(acc[1], as_bf2(g.y & __byte_perm(mlo, 0u, 0x3322)));
-        acc[2] = __hadd2(acc[2], as_bf2(g.z & __byte_perm(mhi, 0u, 0x1100)));
-        acc[3] = __hadd2(acc[3], as_bf2(g.w & __byte_perm(mhi, 0u, 0x3322)));
+        acc[0] = __hadd2(acc[0], as_bf2(g.x & m[0]));
+        acc[1] = __hadd2(acc[1], as_bf2(g.y & m[1]));
+        acc[2] = __hadd2(acc[2], as_bf2(g.z & m[2]));
+        acc[3] = __hadd2(acc[3], as_bf2(g.w & m[3]));
       }
     }
     uint32_t out[4] = {as_u32(acc[0]), as_u32(acc[1]), as_u32(acc[2]), as_u32(acc[3])};
@@ -446,14 +473,19 @@ using namespace rb;
 
 extern "C" {
 
+// code_bytes: 1 or 2, the size of a recorded offset (max pooling). With `relu`, k * k has to be less than the code that
+// means "no gradient" (255 / 65535); the backward pass refuses windows with more offsets than codes.
 int rb_pool_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, int P, int Q, int k, int stride,
-                int pad, int is_max, int relu, cudaStream_t st) {
-  if (C % 8) return -10;
+                int pad, int is_max, int relu, int code_bytes, cudaStream_t st) {
+  if (C % 8 || (code_bytes != 1 && code_bytes != 2)) return -10;
   const long long total = (long long)N * P * Q * (C / 8);
   const bool small = (long long)N * (H > P ? H : P) * (W > Q ? W : Q) * C < 0x7FFFFFFFll;  // 32-bit index math
   // generic kernels with 32- or 64-bit index arithmetic
-  auto generic = [&](auto maxk, auto avgk) {
-    if (is_max)
+  auto generic = [&](auto maxk, auto maxk2, auto avgk) {
+    if (is_max && code_bytes == 2)
+      launch_pdl(maxk2, grid_for(total, 256), 256, 0, st, (const bf16*)x, (bf16*)y, (uint16_t*)idx, N, H, W, C, P, Q, k,
+                 stride, pad, relu);
+    else if (is_max)
       launch_pdl(maxk, grid_for(total, 256), 256, 0, st, (const bf16*)x, (bf16*)y, (uint8_t*)idx, N, H, W, C, P, Q, k,
                  stride, pad, relu);
     else
@@ -464,14 +496,14 @@ int rb_pool_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, i
   if (is_max && small && !getenv("RB_POOL_GENERIC") && Q * cv >= 64 && Q * cv < 65536 && (long long)N * P < 0x7FFFFFFF) {
     const int threads = Q * cv >= 256 ? 256 : (Q * cv + 31) / 32 * 32;
     const uint32_t magic = (uint32_t)((0x100000000ull + cv - 1) / cv);
-    auto rows = [&](auto kern) {
-      launch_pdl(kern, N * P, threads, 0, st, (const bf16*)x, (bf16*)y, (uint8_t*)idx, H, W, C, P, Q, k, stride, pad,
-                 relu, magic);
+    auto rows = [&](auto kern, auto* codes) {
+      launch_pdl(kern, N * P, threads, 0, st, (const bf16*)x, (bf16*)y, codes, H, W, C, P, Q, k, stride, pad, relu, magic);
     };
-    if (k == 3 && stride == 2) rows(maxpool_fwd_rows_kernel<3, 2>);
-    else if (k == 2 && stride == 2) rows(maxpool_fwd_rows_kernel<2, 2>);
-    else if (k == 3 && stride == 1) rows(maxpool_fwd_rows_kernel<3, 1>);
-    else rows(maxpool_fwd_rows_kernel<0, 0>);
+    if (code_bytes == 2) rows(maxpool_fwd_rows_kernel<0, 0, uint16_t>, (uint16_t*)idx);
+    else if (k == 3 && stride == 2) rows(maxpool_fwd_rows_kernel<3, 2>, (uint8_t*)idx);
+    else if (k == 2 && stride == 2) rows(maxpool_fwd_rows_kernel<2, 2>, (uint8_t*)idx);
+    else if (k == 3 && stride == 1) rows(maxpool_fwd_rows_kernel<3, 1>, (uint8_t*)idx);
+    else rows(maxpool_fwd_rows_kernel<0, 0>, (uint8_t*)idx);
     return RB_LAUNCH_OK();
   }
   // a block per window pays while one thread per output cannot fill the chip and the window is worth splitting
@@ -481,18 +513,25 @@ int rb_pool_fwd(const void* x, void* y, void* idx, int N, int H, int W, int C, i
                (const bf16*)x, (bf16*)y, H, W, C, P, Q, k, stride, pad, relu, gpb);
     return RB_LAUNCH_OK();
   }
-  if (small) generic(maxpool_fwd_kernel<unsigned int>, avgpool_fwd_kernel<unsigned int>);
-  else generic(maxpool_fwd_kernel<long long>, avgpool_fwd_kernel<long long>);
+  if (small)
+    generic(maxpool_fwd_kernel<unsigned int, uint8_t>, maxpool_fwd_kernel<unsigned int, uint16_t>,
+            avgpool_fwd_kernel<unsigned int>);
+  else
+    generic(maxpool_fwd_kernel<long long, uint8_t>, maxpool_fwd_kernel<long long, uint16_t>, avgpool_fwd_kernel<long long>);
   return RB_LAUNCH_OK();
 }
 
 int rb_pool_bwd(const void* dy, const void* idx, const void* y_relu, void* dx, const void* mask_src, int N, int H,
-                int W, int C, int P, int Q, int k, int stride, int pad, int is_max, cudaStream_t st) {
-  if (C % 8) return -10;
+                int W, int C, int P, int Q, int k, int stride, int pad, int is_max, int code_bytes, cudaStream_t st) {
+  if (C % 8 || (code_bytes != 1 && code_bytes != 2)) return -10;
+  if (is_max && (long long)k * k > (code_bytes == 2 ? 65535 : 256)) return -12;
   const long long total = (long long)N * H * W * (C / 8);
   const bool small = (long long)N * (H > P ? H : P) * (W > Q ? W : Q) * C < 0x7FFFFFFFll;
-  auto generic = [&](auto maxk, auto avgk) {
-    if (is_max)
+  auto generic = [&](auto maxk, auto maxk2, auto avgk) {
+    if (is_max && code_bytes == 2)
+      launch_pdl(maxk2, grid_for(total, 256), 256, 0, st, (const bf16*)dy, (const uint16_t*)idx, (bf16*)dx,
+                 (const bf16*)mask_src, N, H, W, C, P, Q, k, stride, pad);
+    else if (is_max)
       launch_pdl(maxk, grid_for(total, 256), 256, 0, st, (const bf16*)dy, (const uint8_t*)idx, (bf16*)dx,
                  (const bf16*)mask_src, N, H, W, C, P, Q, k, stride, pad);
     else
@@ -503,9 +542,9 @@ int rb_pool_bwd(const void* dy, const void* idx, const void* y_relu, void* dx, c
   if (is_max && small && !getenv("RB_POOL_GENERIC") && W * cv >= 64 && W * cv < 65536 && (long long)N * H < 0x7FFFFFFF) {
     const int threads = W * cv >= 256 ? 256 : (W * cv + 31) / 32 * 32;
     const uint32_t magic = (uint32_t)((0x100000000ull + cv - 1) / cv);
-    auto rows = [&](auto kern) {
-      launch_pdl(kern, N * H, threads, 0, st, (const bf16*)dy, (const uint8_t*)idx, (bf16*)dx, (const bf16*)mask_src,
-                 H, W, C, P, Q, k, stride, pad, magic);
+    auto rows = [&](auto kern, auto* codes) {
+      launch_pdl(kern, N * H, threads, 0, st, (const bf16*)dy, codes, (bf16*)dx, (const bf16*)mask_src, H, W, C, P, Q, k,
+                 stride, pad, magic);
     };
     const int I = (H + pad + 1) / 2, J = (W + pad + 1) / 2;
     auto blocks2 = [&](auto kern) {
@@ -513,14 +552,18 @@ int rb_pool_bwd(const void* dy, const void* idx, const void* y_relu, void* dx, c
       launch_pdl(kern, N * I, t2, 0, st, (const bf16*)dy, (const uint8_t*)idx, (bf16*)dx, (const bf16*)mask_src, H, W, C, P,
                  Q, pad, I, J, magic);
     };
-    if (k == 3 && stride == 2) blocks2(maxpool_bwd_s2_kernel<3>);
+    if (code_bytes == 2) rows(maxpool_bwd_rows_kernel<0, 0, uint16_t>, (const uint16_t*)idx);
+    else if (k == 3 && stride == 2) blocks2(maxpool_bwd_s2_kernel<3>);
     else if (k == 2 && stride == 2) blocks2(maxpool_bwd_s2_kernel<2>);
-    else if (k == 3 && stride == 1) rows(maxpool_bwd_rows_kernel<3, 1>);
-    else rows(maxpool_bwd_rows_kernel<0, 0>);
+    else if (k == 3 && stride == 1) rows(maxpool_bwd_rows_kernel<3, 1>, (const uint8_t*)idx);
+    else rows(maxpool_bwd_rows_kernel<0, 0>, (const uint8_t*)idx);
     return RB_LAUNCH_OK();
   }
-  if (small) generic(maxpool_bwd_kernel<unsigned int>, avgpool_bwd_kernel<unsigned int>);
-  else generic(maxpool_bwd_kernel<long long>, avgpool_bwd_kernel<long long>);
+  if (small)
+    generic(maxpool_bwd_kernel<unsigned int, uint8_t>, maxpool_bwd_kernel<unsigned int, uint16_t>,
+            avgpool_bwd_kernel<unsigned int>);
+  else
+    generic(maxpool_bwd_kernel<long long, uint8_t>, maxpool_bwd_kernel<long long, uint16_t>, avgpool_bwd_kernel<long long>);
   return RB_LAUNCH_OK();
 }
 

@@ -965,13 +965,14 @@ class Pool2dOp(Op):
     def alloc(self):
         super().alloc()
         if self.is_max:
-            self.idx = torch.zeros(self.out.shape, dtype=torch.uint8, device=self.net.device)
+            self.idx = torch.zeros(self.out.shape, dtype=K.pool_code_dtype(self.cfg.pool_size), device=self.net.device)
 
     def forward(self, train, t):
         h, w, _ = self.prev.out_hwc
         cfg = self.cfg
         # behind a ReLU a maximum is never negative, so clamping it changes nothing, but makes the kernel record "no
-        # gradient" for windows whose maximum is zero: what the mask of the producer's ReLU would remove in backward
+        # gradient" (a code that no window offset has, see `K.pool_code_dtype`) for windows whose maximum is zero: what the
+        # mask of the producer's ReLU would remove in backward
         K.pool_fwd(self.prev.out, self.out, self.idx, self.net.batch, h, w, self.out_cp, self.P, self.Q, cfg.pool_size,
                    cfg.pool_stride, cfg.pool_pad, self.is_max, self.fused_relu or (self.is_max and self.prev.has_relu))
 
@@ -982,9 +983,9 @@ class Pool2dOp(Op):
         cfg = self.cfg
         mask, y_relu = self.mask_src(), self.out if self.fused_relu else None
         if self.is_max:
-            # the recorded window offsets carry the mask (see forward): the producer's output, the largest tensor of
+            # the recorded window offsets carry both masks (see forward): the producer's output, the largest tensor of
             # the pass, is not read again (2 x 2 windows on 64 x 256 x 256 x 64: 1.28 GB of traffic become 0.74)
-            mask, y_relu = None, self.out if mask is not None else None
+            mask = y_relu = None
         K.pool_bwd(self.dout, self.idx, y_relu, self.prev.dout, mask, self.net.batch, h, w, self.out_cp, self.P, self.Q,
                    cfg.pool_size, cfg.pool_stride, cfg.pool_pad, self.is_max)
 

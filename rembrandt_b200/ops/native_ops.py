@@ -279,14 +279,21 @@ def f32_to_bf16(x, y, n):
     check(_native.cuda().rb_f32_to_bf16(ptr(x), ptr(y), n, stream_handle()), "rb_f32_to_bf16")
 
 
+def pool_code_dtype(k):
+    """What max pooling records the offsets of its k x k windows in: the smallest type with a code to spare (all bits set)
+    for windows that pass no gradient on. (`pool_fwd` also takes 16 x 16 windows in bytes, without `relu`.)"""
+    return torch.uint8 if k * k <= 255 else torch.int16
+
+
 def pool_fwd(x, y, idx, N, H, W, C, P, Q, k, stride, pad, is_max, relu):
     check(_native.cuda().rb_pool_fwd(ptr(x), ptr(y), ptr(idx), N, H, W, C, P, Q, k, stride, pad, int(is_max),
-                                     int(relu), stream_handle()), "rb_pool_fwd")
+                                     int(relu), 1 if idx is None else idx.element_size(), stream_handle()), "rb_pool_fwd")
 
 
 def pool_bwd(dy, idx, y_relu, dx, mask_src, N, H, W, C, P, Q, k, stride, pad, is_max):
     check(_native.cuda().rb_pool_bwd(ptr(dy), ptr(idx), ptr(y_relu), ptr(dx), ptr(mask_src), N, H, W, C, P, Q, k,
-                                     stride, pad, int(is_max), stream_handle()), "rb_pool_bwd")
+                                     stride, pad, int(is_max), 1 if idx is None else idx.element_size(), stream_handle()),
+          "rb_pool_bwd")
 
 
 def lrn_fwd(x, y, pixels, C, size, alpha_eff, beta, k):

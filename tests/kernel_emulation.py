@@ -186,7 +186,10 @@ def pool_fwd(x, y, idx, N, H, W, C, P, Q, k, stride, pad, is_max, relu):
         win = _windows(xi, k, stride, pad, P, Q, float("-inf"))
         best, arg = win.max(dim=4)
         if idx is not None:
-            idx.reshape(-1)[: N * P * Q * C].view(N, P, Q, C).copy_(arg.permute(0, 2, 3, 1).to(torch.uint8))
+            if relu:                             # no gradient: the code with all bits set
+                arg = torch.where(best > 0, arg, torch.full_like(arg, -1))
+            # wraps like the kernels' stores: only offsets that fit the codes' type can be told apart in backward
+            idx.reshape(-1)[: N * P * Q * C].view(N, P, Q, C).copy_(arg.permute(0, 2, 3, 1).to(idx.dtype))
     else:
         best = _windows(xi, k, stride, pad, P, Q, 0.0).sum(4) / (k * k)
     if relu:
@@ -196,11 +199,16 @@ def pool_fwd(x, y, idx, N, H, W, C, P, Q, k, stride, pad, is_max, relu):
 
 def pool_bwd(dy, idx, y_relu, dx, mask_src, N, H, W, C, P, Q, k, stride, pad, is_max):
     g = dy.reshape(-1)[: N * P * Q * C].view(N, P, Q, C).float()
-    if y_relu is not None:
+    if y_relu is not None and not is_max:        # max pooling: the recorded codes say it
         g = g * (y_relu.reshape(-1)[: N * P * Q * C].view(N, P, Q, C).float() > 0)
     need_h, need_w = (P - 1) * stride + k, (Q - 1) * stride + k
     grid = torch.zeros(N, max(need_h, pad + H), max(need_w, pad + W), C)
-    arg = idx.reshape(-1)[: N * P * Q * C].view(N, P, Q, C).long() if is_max else None
+    arg = None
+    if is_max:
+        bits = 8 * idx.element_size()
+        if k * k > (256 if bits == 8 else 65535):
+            raise RuntimeError("more window offsets than codes")
+        arg = idx.reshape(-1)[: N * P * Q * C].view(N, P, Q, C).long() & ((1 << bits) - 1)
     for r in range(k):
         for s in range(k):
             part = g * (arg == r * k + s) if is_max else g / (k * k)
@@ -498,6 +506,6 @@ def install(monkeypatch):
         if name in EMULATED:
             monkeypatch.setattr(K, name, EMULATED[name])
         elif isinstance(obj, types.FunctionType) and obj.__module__ == K.__name__ and \
-                name not in ("pad_channels", "status_word", "read_status"):
+                name not in ("pad_channels", "pool_code_dtype", "status_word", "read_status"):
             monkeypatch.setattr(K, name, _unsupported(name))
     monkeypatch.setattr(K, "read_status", lambda: 0)
