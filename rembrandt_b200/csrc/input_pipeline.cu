@@ -46,8 +46,9 @@ __device__ __forceinline__ void sample_draw(const InputArgs& a, int n, int& oy, 
     oy = a.lo_y + (int)(r[0] % (uint32_t)(a.hi_y - a.lo_y + 1));
     ox = a.lo_x + (int)(r[1] % (uint32_t)(a.hi_x - a.lo_x + 1));
   } else {
-    oy = (a.lo_y + a.hi_y) / 2;
-    ox = (a.lo_x + a.hi_x) / 2;
+    // rounded down: padding absorbed from the first layer lowers both ends and must not move the centre
+    oy = (a.lo_y + a.hi_y) >> 1;
+    ox = (a.lo_x + a.hi_x) >> 1;
   }
   flip = a.random_flip ? (int)(r[2] & 1u) : 0;
   shift[0] = shift[1] = shift[2] = 0.f;

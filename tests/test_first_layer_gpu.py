@@ -3,6 +3,7 @@ parameters. Plain and strided (space-to-depth'd) filters, with and without a spa
 smaller than the image, normalised layers, a layer too wide for it."""
 import pytest
 import torch
+import torch.nn.functional as F
 
 from rembrandt_b200.models.config import (Act, AffineCfg, BNormConv2dCfg, Conv2dCfg, Data3dCfg, ParamsInit, Preproc,
                                           SequentialOperatorConfig, SoftmaxKLLossCfg)
@@ -62,3 +63,30 @@ def test_against_the_host_path(hw, c, k, s, p, ko, bnorm, crop, windows):
         # bf16 activations and deltas (2^-9 each) against fp32, ReLU signs that flip at zero; a normalisation takes the
         # mean and the projection on its output out of the delta, so what is left carries two to three times the error
         assert float((a - b).norm()) < (9e-2 if bnorm else 3e-2) * float(b.norm()) + 1e-6, gs.name
+
+
+@pytest.mark.parametrize("hw,crop,k,s,p,bnorm", [
+    (15, 14, 3, 1, 1, False), (17, 14, 5, 1, 2, False), (16, 15, 3, 1, 1, False), (17, 14, 4, 1, 0, False),
+    (21, 20, 7, 2, 3, True), (24, 19, 5, 2, 2, False), (33, 32, 11, 4, 5, False)])
+def test_the_inference_crop_is_centred(hw, crop, k, s, p, bnorm):
+    """Margins that are odd and smaller than the layer's padding on both sides, in the windowed and the space-to-depth form:
+    the convolution of the crop that the host path takes. One pixel off changes noise images altogether."""
+    batch = 3
+    g, h = (Net(_cfg(hw, 3, k, s, p, 16, bnorm, crop), batch, device=d, seed=(3, 4)) for d in ("cuda", "cpu"))
+    gen = torch.Generator().manual_seed(hw + k)
+    x = torch.randint(0, 256, (batch, 3, hw, hw), dtype=torch.uint8, generator=gen)
+    g.load_batch(x, torch.zeros(batch, dtype=torch.int32))
+    g.forward(False)
+    torch.cuda.synchronize()
+    op = g.hidden_ops[0]
+    if bnorm:
+        w, got = op.u._w_ref(g.seg_view(op.u.seg_w).float().cpu()), op.u.conv_out
+    else:
+        w, got = op._w_ref(g.seg_view(op.seg_w).float().cpu()), op.out
+    want = F.conv2d(h.input_op.ref_forward(x, False, 0), w.bfloat16().float(), stride=s, padding=p)
+    if not bnorm:
+        want = want.relu()                       # the biases are zero at first
+    inner = slice(2, -2)                         # the space-to-depth form sees the image beyond the crop in its padding
+    a = got[..., :16].float().cpu().permute(0, 3, 1, 2)[..., inner, inner]
+    # bf16 pixels and one rounding of the result: 2^-9 each
+    assert float((a - want[..., inner, inner]).norm()) < 1e-2 * float(want[..., inner, inner].norm())

@@ -31,7 +31,7 @@ def test_windows(N, C, H, W, win, stride, pad, extra, border):
     K.input_u8(src, mean, dst, N, C, H, W, eh, ew, OH, OW, Cp, win, lo_y, hi_y, lo_x, hi_x, False, False, False, 0.5, 0.25,
                0.0, None, None, 1, 0, stride=stride, border=pad if border else 0, ones=ones)
     img = src.float() * 0.5 - 0.25 * mean
-    oy, ox = int((lo_y + hi_y) / 2), int((lo_x + hi_x) / 2)   # truncating, as the kernel centres its window
+    oy, ox = (H - ch) // 2 - pad, (W - cw) // 2 - pad         # centred on the crop, whatever padding surrounds it
     big = F.pad(img, (pad + ew, pad + ew, pad + eh, pad + eh))[:, :, pad + eh + oy: pad + 2 * eh + oy,
                                                              pad + ew + ox: pad + 2 * ew + ox].clone()
     if border and pad:
