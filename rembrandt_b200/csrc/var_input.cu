@@ -71,9 +71,9 @@ __global__ void __launch_bounds__(256) var_input_kernel(const __grid_constant__ 
     }
     int ox, oy;
     if (a.train && rw > a.crop_w) ox = (int)(r[0] % (uint32_t)(rw - a.crop_w + 1));
-    else ox = (rw - a.crop_w) / 2;
+    else ox = (rw - a.crop_w) >> 1;   // rounded down, also for images smaller than the window
     if (a.train && rh > a.crop_h) oy = (int)(r[1] % (uint32_t)(rh - a.crop_h + 1));
-    else oy = (rh - a.crop_h) / 2;
+    else oy = (rh - a.crop_h) >> 1;
     const int flip = (a.train && a.random_flip) ? (int)(r[2] & 1u) : 0;
     if (a.draws && x == 0 && y == 0) {
       a.draws[n * 4 + 0] = sdim; a.draws[n * 4 + 1] = ox; a.draws[n * 4 + 2] = oy; a.draws[n * 4 + 3] = flip;

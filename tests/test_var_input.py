@@ -120,6 +120,18 @@ def test_var_input_kernel_matches_restatement(train):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("scale", [27, 31])
+def test_var_input_centres_images_smaller_than_the_window(scale):
+    net, host = (Net(_var_cfg(32, scale, scale), 4, device=d) for d in ("cuda", "cpu"))
+    imgs = _batch(4)
+    net.load_batch(imgs, torch.zeros(4, dtype=torch.int32))
+    net.input_op.forward(False, 0)
+    torch.cuda.synchronize()
+    got = net.input_op.out[..., :3].float().cpu().permute(0, 3, 1, 2)
+    assert torch.allclose(got, host.input_op.ref_forward(imgs, False, 0), atol=6e-3, rtol=8e-3)
+
+
+@pytest.mark.gpu
 def test_var_input_space_to_depth_feeds_strided_conv():
     """A strided first convolution reads the space-to-depth form; logits must match the CPU reference path."""
     cfg = _var_cfg(35, 40, 40, flip=False, stride=2)
