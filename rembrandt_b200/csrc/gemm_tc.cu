@@ -1603,13 +1603,16 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
 // (sub-tiles per item, resident B, tail cut) choice on the given stream and caches the fastest. The cost model
 // alone mis-ranks them by up to 30 % (it knows rows filled, not how much of the epilogue is exposed). Outside
 // tuning mode a launch never times anything: it takes the cached plan, or the cost model's.
-typedef std::tuple<int, int, int, int, int, int, int, int, int, int> PlanKey;
+// Box plans depend on the extents of the output rows, not on their product alone: at odd sizes two phases of a strided
+// data-gradient have the same M, N and k-blocks with rows and columns exchanged.
+typedef std::tuple<int, int, int, int, int, int, int, int, int, int, int, int, int, int> PlanKey;
 static std::map<PlanKey, Plan> g_plan_cache;
 static std::mutex g_plan_mutex;
 
 static PlanKey plan_key(const GemmTcParams& p) {
   return PlanKey(p.a_mode, p.b_mode, p.M, p.N, p.num_kb, p.bn, p.bk, p.n_tiles, p.cv_stride,
-                 (p.mask_src ? 1 : 0) | (p.add_src ? 2 : 0) | (p.sc_stride ? 4 : 0));
+                 (p.mask_src ? 1 : 0) | (p.add_src ? 2 : 0) | (p.sc_stride ? 4 : 0), p.cv_P, p.cv_Q, p.cv_S,
+                 p.cv_cchunks);
 }
 
 // Times the candidates of `p` (3 launches each, best of the last 2); returns the best time in ms, or a negative
@@ -1690,13 +1693,13 @@ static int launch(GemmTcParams& p, bool allow_split, int fixed_split, bool b_is_
       if (g_opt.force_mt) break;
     }
   }
+  const Plan model = pl;
   if (p.epi == EPI_BF16 && !forced) {
     std::lock_guard<std::mutex> lock(g_plan_mutex);
     auto it = g_plan_cache.find(plan_key(p));
     if (it != g_plan_cache.end()) {
       Plan cached = it->second;
       if (cached.tail && (!p.ws || g_opt.deterministic)) cached.tail = 0;   // tuned with a workspace, launched without
-      if (cached.pair && !pair_ok(p)) cached = pl;
       pl = cached;
     } else if (tunable(p, stream)) {
       Plan best = pl;
@@ -1704,7 +1707,9 @@ static int launch(GemmTcParams& p, bool allow_split, int fixed_split, bool b_is_
       g_plan_cache[plan_key(p)] = pl;
     }
   }
-  return run_plan(p, pl, stream);
+  const int rc = run_plan(p, pl, stream);
+  // a plan from the cache that does not fit this launch (a smaller workspace, options changed since): the cost model's
+  return rc == -3 ? run_plan(p, model, stream) : rc;
 }
 
 static int round_bn(int n, int cap) {
@@ -2006,7 +2011,9 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
     if (g_opt.force_wide == 1 || g_opt.force_box == 1) {
       use = ((bn_wide && g_opt.force_wide == 1) ? bn_wide : bn_default) | ((box_ok && g_opt.force_box == 1) ? 1 << 16 : 0);
     } else if (it != g_bn_cache.end()) {
-      use = it->second;
+      use = it->second;   // as far as it still applies: the options may have changed since it was measured
+      if (!box_ok) use &= 0xFFFF;
+      if ((use & 0xFFFF) != bn_default && (use & 0xFFFF) != bn_wide) use = bn_default | (use & 1 << 16);
     } else if (tunable(p, stream)) {
       float best_ms = 1e30f;
       for (int box = 0; box <= (box_ok ? 1 : 0); ++box) {
