@@ -88,12 +88,16 @@ __device__ __forceinline__ bool ctl_wait(SharedCtl* ctl, uint64_t* bar, uint32_t
   return false;
 }
 
-// The same for a whole converged warp: the result is the same in every lane.
+// The same for a whole converged warp: the result is the same in every lane. Where lane 0 alone has seen the phase, the
+// barrier at the end orders the other lanes (one of which may be the elected one that issues) after what it acquired; the
+// shuffle alone orders no memory.
 __device__ __forceinline__ bool ctl_wait_warp(SharedCtl* ctl, uint64_t* bar, uint32_t parity, unsigned int* status) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   int ok = 0;
   if ((threadIdx.x & 31) == 0) ok = ctl_wait(ctl, bar, parity, status) ? 1 : 0;
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  __syncwarp();
+  return ok != 0;
 }
 
 // Role profile (built only with -DRB_GEMM_PROFILE, see `python -m rembrandt_b200._build --profile`): cycles that the
