@@ -82,7 +82,11 @@ class DgradPlan:
     """How one convolution's data-gradient reads its filters: in place, or from a transposed and flipped copy made once per
     step beside the forward pass. In place saves the copy; the copy is the K-major operand, with which the large shapes run
     10 % faster (64 x 64 x 64 x 256 -> 256: 274 against 243 us). Both are measured once per shape and process, on scratch
-    operands; the copy has to win by more than a launch costs and half of the time that making it takes."""
+    operands; the copy has to win by more than a launch costs and half of the time that making it takes. Where a sixth of the
+    time in place is less than that, no plans are searched for the copy: it was at most 13 % faster on every shape measured,
+    and the search is most of what building a small network costs."""
+
+    LAUNCH_MS, MOST_GAIN = 0.003, 1 / 6
 
     def __init__(self, n, P, Q, kp, ko, cp, in_c, k, stride, pad, H, W, forms):
         """`forms`: the (addend, mask) combinations that will be asked for."""
@@ -96,19 +100,22 @@ class DgradPlan:
         n, P, Q, kp, ko, cp, in_c, k, stride, pad, H, W = self.geom
         zeros = lambda *s: torch.zeros(s, dtype=torch.bfloat16, device="cuda")
         dy, w, wt, dx = zeros(n, P, Q, kp), zeros(ko, k * k, cp), zeros(cp, k * k, kp), zeros(n, H, W, cp)
-        gain = 0.0
-        for has_add, has_mask in forms:
-            extra = dict(add=torch.zeros_like(dx) if has_add else None, mask=torch.zeros_like(dx) if has_mask else None)
-            ms = []
-            for packed in (None, wt):
+
+        def mean_ms(packed):
+            total = 0.0
+            for has_add, has_mask in forms:
+                extra = dict(add=torch.zeros_like(dx) if has_add else None, mask=torch.zeros_like(dx) if has_mask else None)
                 run = lambda: conv_dgrad(dy, n, P, Q, kp, w, ko, cp, in_c, k, stride, pad, H, W, dx, wt=packed, **extra)
                 with K.gemm_tuning():
                     run()
-                ms.append(_device_ms(run))
-            gain += (ms[0] - ms[1]) / len(forms)
+                total += _device_ms(run)
+            return total / len(forms)
+
         pack = lambda: K.pack_dgrad_filters(w, wt, ko, kp, k * k, cp)
         pack()
-        better = gain > 0.003 + 0.5 * _device_ms(pack)
+        cost = self.LAUNCH_MS + 0.5 * _device_ms(pack)
+        in_place = mean_ms(None)
+        better = in_place * self.MOST_GAIN > cost and in_place - mean_ms(wt) > cost
         torch.cuda.current_stream().synchronize()
         return better
 

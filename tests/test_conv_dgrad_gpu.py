@@ -65,3 +65,16 @@ def test_against_autograd(shape, add, masked, packed):
                                      dict(force_pair=1), dict(force_tail=1), dict(deterministic=1)])
 def test_plans(shape, options):
     _run(shape, "own", True, **options)
+
+
+@pytest.mark.parametrize("shape,searched", [((32, 8, 8, 32, 32, 32, 32, 3, 1, 1, 8, 8), False),
+                                            ((32, 64, 64, 256, 256, 256, 256, 3, 1, 1, 64, 64), True)])
+def test_the_copy_is_measured_only_where_it_can_win(monkeypatch, shape, searched):
+    from rembrandt_b200.ops import conv_grad
+    seen, real = [], conv_grad.conv_dgrad
+    monkeypatch.setattr(conv_grad, "conv_dgrad", lambda *a, **k: (seen.append(k.get("wt") is not None), real(*a, **k)))
+    monkeypatch.setattr(conv_grad, "_measured", {})
+    plan = conv_grad.DgradPlan(*shape, [(False, True), (True, True)])
+    torch.cuda.synchronize()
+    assert K.read_status() == 0 and any(seen) == searched
+    assert searched or plan.wt is None
