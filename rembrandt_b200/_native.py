@@ -59,7 +59,7 @@ _CUDA_SIGS = {
     "rb_pack_dgrad_filters": [vp, vp, i32, i32, i32, i32, vp],
     "rb_gather_columns": [vp, vp, vp, i32, i32, i32, vp],
     "rb_scatter_columns": [vp, vp, vp, vp, i32, i32, i32, i32, vp],
-    "rb_publish_stats": [vp, vp, vp, vp],
+    "rb_publish_stats": [vp, vp, vp, vp, vp],
     "rb_zero_s2d_structural": [vp, i32, i32, i32, i32, i32, i32, vp],
     # activations.cu
     "rb_act_fwd": [vp, i64, i32, i32, i32, f32, vp],
@@ -71,8 +71,8 @@ _CUDA_SIGS = {
     "rb_categorical_loss": [vp, i32, i32, i32, vp, vp, f32, vp, vp, vp, vp, vp, vp, vp, i32, vp],
     "rb_softmax_ce": [vp, i32, i32, i32, i32, vp, vp, f32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp],
     # sgd_fused.cu
-    "rb_sgd_fused": [vp, vp, vp, vp, i64, f32, f32, f32, f32, i32, i32, vp],
-    "rb_sgd_fused_grid": [vp, vp, vp, vp, i64, f32, f32, f32, f32, i32, i32, i32, i32, vp],
+    "rb_sgd_fused": [vp, vp, vp, vp, i64, f32, vp, f32, f32, f32, i32, i32, vp],
+    "rb_sgd_fused_grid": [vp, vp, vp, vp, i64, f32, vp, f32, f32, f32, i32, i32, i32, i32, vp],
     "rb_axpy_shadow": [vp, vp, vp, i64, f32, vp],
     "rb_axpby": [vp, vp, i64, f32, f32, vp],
     # input_pipeline.cu

@@ -307,6 +307,7 @@ __global__ void __launch_bounds__(AR_THREADS, 6) allreduce_sgd_kernel(const __gr
         }
         if (a.zero_grads) *reinterpret_cast<float4*>(a.grads[a.rank] + e) = zero;
         SgdHyper h = a.h;
+        if (h.lr_dev) h.lr = *h.lr_dev;
         if (e >= a.decay_len) h.l2 = 0.f;
         float4 w = wa[u], v = va[u];
         sgd_elem(w.x, g.x, v.x, h);

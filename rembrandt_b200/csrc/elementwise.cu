@@ -222,9 +222,15 @@ __global__ void zero_s2d_structural_kernel(float* __restrict__ dw, int Kout, int
 }
 
 // Loss and number of correct samples of a step into page-locked host memory, and the accumulators cleared: the last launch
-// of a step, in place of two copies, a conversion, a copy to the host and two fills.
-__global__ void publish_stats_kernel(float* loss_sum, int* correct, volatile float* host) {
+// of a step, in place of two copies, a conversion, a copy to the host and two fills. With `turn` the two rows of `host` are
+// written in turn.
+__global__ void publish_stats_kernel(float* loss_sum, int* correct, volatile float* host, unsigned int* turn) {
   pdl_prolog();
+  if (turn) {
+    const unsigned int t = *turn;
+    host += 2 * (t & 1u);
+    *turn = t ^ 1u;
+  }
   host[0] = *loss_sum;
   host[1] = (float)*correct;
   *loss_sum = 0.f;
@@ -342,8 +348,8 @@ int rb_add_bf16(void* a, const void* b, long long n, cudaStream_t st) {
   return RB_LAUNCH_OK();
 }
 
-int rb_publish_stats(float* loss_sum, int* correct, float* host, cudaStream_t st) {
-  launch_pdl(publish_stats_kernel, 1, 1, 0, st, loss_sum, correct, (volatile float*)host);
+int rb_publish_stats(float* loss_sum, int* correct, float* host, unsigned int* turn, cudaStream_t st) {
+  launch_pdl(publish_stats_kernel, 1, 1, 0, st, loss_sum, correct, (volatile float*)host, turn);
   return RB_LAUNCH_OK();
 }
 

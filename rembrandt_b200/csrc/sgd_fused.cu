@@ -18,18 +18,20 @@ struct SgdArgs : SgdHyper {
   long long n;
 };
 
-__global__ void sgd_fused_kernel(SgdArgs a) {
+__global__ void sgd_fused_kernel(const SgdArgs a) {
   pdl_prolog();
+  SgdHyper h = a;
+  if (h.lr_dev) h.lr = *h.lr_dev;
   const long long n4 = a.n / 4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4;
        i += (long long)gridDim.x * blockDim.x) {
     float4 w = reinterpret_cast<float4*>(a.w)[i];
     float4 g = reinterpret_cast<float4*>(a.g)[i];
     float4 v = a.v ? reinterpret_cast<float4*>(a.v)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    sgd_elem(w.x, g.x, v.x, a);
-    sgd_elem(w.y, g.y, v.y, a);
-    sgd_elem(w.z, g.z, v.z, a);
-    sgd_elem(w.w, g.w, v.w, a);
+    sgd_elem(w.x, g.x, v.x, h);
+    sgd_elem(w.y, g.y, v.y, h);
+    sgd_elem(w.z, g.z, v.z, h);
+    sgd_elem(w.w, g.w, v.w, h);
     if (a.phase & 3) reinterpret_cast<float4*>(a.w)[i] = w;
     if (a.v && (a.phase & 1)) reinterpret_cast<float4*>(a.v)[i] = v;
     if ((a.phase & 4) || a.mode == 5) reinterpret_cast<float4*>(a.g)[i] = g;
@@ -45,7 +47,7 @@ __global__ void sgd_fused_kernel(SgdArgs a) {
   for (long long i = n4 * 4 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < a.n;
        i += (long long)gridDim.x * blockDim.x) {
     float w = a.w[i], g = a.g[i], v = a.v ? a.v[i] : 0.f;
-    sgd_elem(w, g, v, a);
+    sgd_elem(w, g, v, h);
     if (a.phase & 3) a.w[i] = w;
     if (a.v && (a.phase & 1)) a.v[i] = v;
     if ((a.phase & 4) || a.mode == 5) a.g[i] = g;
@@ -78,11 +80,12 @@ using namespace rb;
 
 extern "C" {
 
-int rb_sgd_fused(float* w, float* g, float* v, void* w16, long long n, float lr, float mu, float l2, float grad_scale,
-                 int mode, int phase, cudaStream_t st) {
+// lr_dev: null, or one float on the device that is used instead of `lr`.
+int rb_sgd_fused(float* w, float* g, float* v, void* w16, long long n, float lr, const float* lr_dev, float mu, float l2,
+                 float grad_scale, int mode, int phase, cudaStream_t st) {
   if (n <= 0) return 0;
   SgdArgs a;
-  a.lr = lr; a.mu = mu; a.l2 = l2; a.grad_scale = grad_scale; a.mode = mode; a.phase = phase;
+  a.lr = lr; a.lr_dev = lr_dev; a.mu = mu; a.l2 = l2; a.grad_scale = grad_scale; a.mode = mode; a.phase = phase;
   a.w = w; a.g = g; a.v = v; a.w16 = (bf16*)w16; a.n = n;
   long long blocks = (n / 4 + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
@@ -93,12 +96,12 @@ int rb_sgd_fused(float* w, float* g, float* v, void* w16, long long n, float lr,
 
 // Same kernel with a caller-chosen grid: blocks of 128 threads fit on an SM next to a resident GEMM CTA, which lets
 // the update of a finished gradient bucket run on a second stream while backward continues.
-int rb_sgd_fused_grid(float* w, float* g, float* v, void* w16, long long n, float lr, float mu, float l2,
-                      float grad_scale, int mode, int phase, int blocks, int threads, cudaStream_t st) {
+int rb_sgd_fused_grid(float* w, float* g, float* v, void* w16, long long n, float lr, const float* lr_dev, float mu,
+                      float l2, float grad_scale, int mode, int phase, int blocks, int threads, cudaStream_t st) {
   if (n <= 0) return 0;
   if (blocks < 1 || threads < 32 || threads > 1024 || (threads & 31)) return -10;
   SgdArgs a;
-  a.lr = lr; a.mu = mu; a.l2 = l2; a.grad_scale = grad_scale; a.mode = mode; a.phase = phase;
+  a.lr = lr; a.lr_dev = lr_dev; a.mu = mu; a.l2 = l2; a.grad_scale = grad_scale; a.mode = mode; a.phase = phase;
   a.w = w; a.g = g; a.v = v; a.w16 = (bf16*)w16; a.n = n;
   const long long need = (n / 4 + threads - 1) / threads;
   if (need < blocks) blocks = need < 1 ? 1 : (int)need;

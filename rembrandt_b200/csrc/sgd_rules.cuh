@@ -17,6 +17,8 @@ namespace rb {
 struct SgdHyper {
   float lr, mu, l2, grad_scale;
   int mode, phase;
+  const float* lr_dev;   // if given, the learning rate is read from here when the kernel runs: a captured step follows a
+                         // schedule without being captured again
 };
 
 __device__ __forceinline__ void sgd_elem(float& w, float& g, float& v, const SgdHyper& a) {

@@ -7,7 +7,8 @@ kernel individually, the engine
 * stages batches through two pinned-to-device buffers on a copy stream, so the H2D copy of batch i+1 overlaps
   the compute of batch i; the input and loss operators read the staging slot itself;
 * captures forward + backward (+ exchange + update when the backend's kernels can be captured) + the publication of
-  loss / accuracy in one CUDA graph per slot and replays it per step; an inference pass is a graph as well;
+  loss / accuracy in one CUDA graph per slot and replays it per step (the learning rate is read from device memory, so
+  a schedule captures nothing again); an inference pass is a graph as well;
 * returns loss / accuracy with a one-step lag through a pinned host mirror that the last kernel of the step writes, so
   the host never blocks on the step it has just launched.
 
@@ -39,8 +40,8 @@ class StepEngine:
         self.accum = max(1, opt.minibatch_size // net.batch)   # batches per optimizer iteration
         self.lr = opt.step_size.at_iter(0)
         self.iter = 0
-        self._graphs = {}          # (last of its iteration, learning rate, staging slot, mirror) -> captured step
-        self._ran = set()          # (last of its iteration, learning rate) that have run eagerly once
+        self._graphs = {}          # (last of its iteration, staging slot) -> captured step
+        self._ran = set()          # whether last of its iteration: forms of the step that have run eagerly once
         self._eval_graphs = {}     # what the loss operator reads -> captured inference pass (None: has run eagerly once)
         self._pending = None
         self._lag_stats = None
@@ -58,9 +59,12 @@ class StepEngine:
             self._consumed = [torch.cuda.Event() for _ in range(2)]
             self._slot = 0
             self._stats_dev = torch.zeros(2, dtype=torch.float32, device=dev)
-            self._stats_host = [torch.zeros(2, dtype=torch.float32).pin_memory() for _ in range(3)]   # [2]: inference
+            # rows 0 and 1: steps, written in turn (the device keeps count for graph replays); row 2: inference
+            self._stats_host = torch.zeros((3, 2), dtype=torch.float32).pin_memory()
             self._stats_ready = [torch.cuda.Event() for _ in range(2)]
-            self._lr_dev = None
+            self._turn, self._turn_dev = 0, torch.zeros(1, dtype=torch.int32, device=dev)
+            # the learning rate that captured steps read, and what was last written there
+            self._lr_dev, self._lr_written = torch.zeros(1, dtype=torch.float32, device=dev), None
             # optional timing of the host-to-device copies (`time_h2d(True)`): pairs of events around each copy
             self._h2d_timing = False
             self._h2d_events = []
@@ -135,15 +139,18 @@ class StepEngine:
             if self._stage_shapes is not None:
                 io.shapes = saved[2]
 
-    def _publish(self, mirror):
+    def _publish(self, inference=False):
         """Loss / correct accumulated since the last time into a pinned mirror; the accumulators start again."""
         lo = self.net.loss_op
         if self.net.device.type == "cuda":
-            K.publish_stats(lo.loss_sum, lo.correct, self._stats_host[mirror])
+            if inference:
+                K.publish_stats(lo.loss_sum, lo.correct, self._stats_host[2])
+            else:
+                K.publish_stats(lo.loss_sum, lo.correct, self._stats_host, turn=self._turn_dev)
             return
         self._stats_dev[0:1].copy_(lo.loss_sum, non_blocking=True)
         self._stats_dev[1:2].copy_(lo.correct, non_blocking=True)
-        self._stats_host[mirror].copy_(self._stats_dev, non_blocking=True)
+        self._stats_host[2 if inference else self._turn].copy_(self._stats_dev, non_blocking=True)
         lo.loss_sum.zero_()
         lo.correct.zero_()
 
@@ -173,15 +180,15 @@ class StepEngine:
         if self.is_cuda:
             self.net.step_counter.add_(1)
 
-    def _update(self):
-        """Exchange + optimizer step for one iteration, in the configured order."""
+    def _update(self, lr=None):
+        """Exchange + optimizer step for one iteration, in the configured order, with the engine's learning rate (or what is
+        given: a number, or one float on the device)."""
         # no_grad: on CPU the flat parameter vector is an autograd leaf, and the exchanges mix it in place
         with span("update"), torch.no_grad():
-            self._update_in_order()
+            self._update_in_order(self.lr if lr is None else lr)
 
-    def _update_in_order(self):
+    def _update_in_order(self, lr):
         o, c, st, net = self.opt, self.comm, self.stepper, self.net
-        lr = self.lr
         # the reference counts the iteration before it tests the interval (src/opt/sgd/new.rs:372,402): exchanges
         # happen at iterations k, 2k, ...
         communicate = c.num_workers() > 1 and ((self.iter + 1) % max(1, o.comm_interval) == 0)
@@ -219,25 +226,29 @@ class StepEngine:
         c = self.comm
         return c.num_workers() <= 1 or getattr(c, "graph_safe", False)
 
-    def _run_step(self, slot: int, mirror: int, last_of_iteration: bool):
+    def _run_step(self, slot: int, last_of_iteration: bool):
         """Forward + backward (+ update when this batch completes a minibatch) of a staged batch on the compute stream."""
-        conf = (last_of_iteration, self.lr if last_of_iteration else 0.0)
-        key = conf + (slot, mirror)
         full = last_of_iteration and self._graph_safe_update()
+        graphed = self.use_graph and last_of_iteration in self._ran
+        lr = self._lr_dev if graphed else self.lr
+        if graphed and last_of_iteration and self._lr_written != self.lr:
+            self._lr_dev.fill_(self.lr)
+            self._lr_written = self.lr
         hook = None
         if last_of_iteration and self._overlapped():
             # the exchange of a gradient bucket starts from inside backward, as soon as the bucket is complete
-            self.comm.prepare(self.stepper, self.lr)
+            self.comm.prepare(self.stepper, lr)
             hook = self.comm.on_op_backward
 
         def body(update):
             with self._reading(slot):
                 self._fwd_bwd(hook=hook)
             if update:
-                self._update()
-            self._publish(mirror)
+                self._update(lr)
+            self._publish()
 
-        if self.use_graph and conf in self._ran:
+        if graphed:
+            key = (last_of_iteration, slot)
             g = self._graphs.get(key)
             if g is None:
                 g = self._graphs[key] = self._capture(lambda: body(full))
@@ -245,11 +256,11 @@ class StepEngine:
             if last_of_iteration and not full:
                 self._update()
             return
-        # without graphs, or the first use of this configuration (allocations, lazy initialisation)
+        # without graphs, or the first use of this form (allocations, lazy initialisation)
         before = K.LAUNCHES[0]
         body(last_of_iteration)
         self.launches_per_step = K.LAUNCHES[0] - before
-        self._ran.add(conf)
+        self._ran.add(last_of_iteration)
 
     def step(self) -> Optional[Tuple[float, int]]:
         """Run the queued batch. Returns (loss, correct) of the *previous* call on CUDA (one-step lag), of this
@@ -268,8 +279,9 @@ class StepEngine:
         cs = self.compute_stream
         with torch.cuda.stream(cs):
             cs.wait_event(self._copy_done[slot])
-            i = net.t & 1
-            self._run_step(slot, i, last)
+            i = self._turn
+            self._run_step(slot, last)
+            self._turn ^= 1
             self._consumed[slot].record(cs)
             self._stats_ready[i].record(cs)
         prev = None
@@ -277,7 +289,7 @@ class StepEngine:
             j = self._lag_stats
             self._stats_ready[j].synchronize()
             prev = (float(self._stats_host[j][0]), int(self._stats_host[j][1]))
-        self._lag_stats = net.t & 1
+        self._lag_stats = i
         if last:
             self.iter += 1
             self.comm.next()
@@ -310,7 +322,7 @@ class StepEngine:
         with torch.cuda.stream(self.compute_stream):
             net.load_batch(images_u8, labels.int())      # host batches go straight into the operators' own buffers
             self._eval_forward()
-            self._publish(2)
+            self._publish(inference=True)
         self.compute_stream.synchronize()
         return float(self._stats_host[2][0]), int(self._stats_host[2][1])
 

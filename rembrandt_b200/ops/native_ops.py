@@ -266,9 +266,11 @@ def count_above(x, threshold, out):
                                         stream_handle()), "rb_count_above")
 
 
-def publish_stats(loss_sum, correct, host):
-    """host (pinned float32 [2]) = (loss_sum, correct); both accumulators are cleared."""
-    check(_native.cuda().rb_publish_stats(ptr(loss_sum), ptr(correct), ptr(host), stream_handle()), "rb_publish_stats")
+def publish_stats(loss_sum, correct, host, turn=None):
+    """host (pinned float32 [2]) = (loss_sum, correct); both accumulators are cleared. With `turn` (one integer on the device,
+    zero at first) host is [2, 2] and its rows are written in turn."""
+    check(_native.cuda().rb_publish_stats(ptr(loss_sum), ptr(correct), ptr(host), ptr(turn), stream_handle()),
+          "rb_publish_stats")
 
 
 def add_bf16(a, b, n):
@@ -344,14 +346,19 @@ def pointwise_loss(x, B, K, ld, target, weights, w_scalar, delta, loss_sum=None,
           "rb_pointwise_loss")
 
 
+def rate_args(lr):
+    """A learning rate as (value, address): a number, or one float32 on the device that the kernel reads when it runs."""
+    return (0.0, ptr(lr)) if torch.is_tensor(lr) else (float(lr), None)
+
+
 def sgd_fused(w, g, v, w16, n, lr, mu, l2, grad_scale, mode, phase=7):
-    check(_native.cuda().rb_sgd_fused(ptr(w), ptr(g), ptr(v), ptr(w16), n, lr, mu, l2, grad_scale, mode, phase,
+    check(_native.cuda().rb_sgd_fused(ptr(w), ptr(g), ptr(v), ptr(w16), n, *rate_args(lr), mu, l2, grad_scale, mode, phase,
                                       stream_handle()), "rb_sgd_fused")
 
 
 def sgd_fused_grid(w, g, v, w16, n, lr, mu, l2, grad_scale, mode, phase=7, blocks=296, threads=128):
     """The fused SGD sweep with an explicit grid (small blocks that co-reside with the GEMM CTAs)."""
-    check(_native.cuda().rb_sgd_fused_grid(ptr(w), ptr(g), ptr(v), ptr(w16), n, lr, mu, l2, grad_scale, mode, phase,
+    check(_native.cuda().rb_sgd_fused_grid(ptr(w), ptr(g), ptr(v), ptr(w16), n, *rate_args(lr), mu, l2, grad_scale, mode, phase,
                                            int(blocks), int(threads), stream_handle()), "rb_sgd_fused_grid")
 
 

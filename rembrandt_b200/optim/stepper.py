@@ -31,7 +31,8 @@ class SgdStepper:
         return out
 
     def step(self, lr: float, grad_scale: float = 1.0, phase: int = 7, lo: int = 0, hi: int = None, grid=None):
-        """`grid` = (blocks, threads) launches the sweep with small blocks (used when it runs beside backward)."""
+        """`lr`: a number, or one float on the device that the sweep reads when it runs. `grid` = (blocks, threads) launches
+        the sweep with small blocks (used when it runs beside backward)."""
         net = self.net
         hi = net.flat_len if hi is None else hi
         for a, b, l2 in self._ranges(lo, hi):

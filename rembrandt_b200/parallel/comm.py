@@ -209,7 +209,7 @@ class LocalOverlapComm(NullComm):
             self._by_trigger.setdefault(idx, []).append((off, n))
 
     def prepare(self, stepper, lr):
-        self._stepper, self._lr = stepper, float(lr)
+        self._stepper, self._lr = stepper, lr
         self._forked = False
 
     def on_op_backward(self, op_index):

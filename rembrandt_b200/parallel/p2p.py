@@ -270,7 +270,7 @@ class FusedAllreduceSgdComm(AllreduceComm, _P2PBase):
     # ---- per-step protocol driven by the engine
     def prepare(self, stepper, lr):
         self.kernel_launches_per_step = 0
-        self._hyper = (float(lr), stepper.mu, stepper.l2, 1.0 / self.world, stepper.mode)
+        self._hyper = (lr, stepper.mu, stepper.l2, 1.0 / self.world, stepper.mode)
 
     def on_op_backward(self, op_index):
         recs = self._by_trigger.get(op_index)
@@ -326,7 +326,8 @@ class FusedAllreduceSgdComm(AllreduceComm, _P2PBase):
         a.wait_ns = int(self.wait_ns)
         if op == 0:
             lr, mu, l2, gs, mode = self._hyper
-            a.h.lr, a.h.mu, a.h.l2, a.h.grad_scale, a.h.mode, a.h.phase = lr, mu, l2, gs, mode, 3
+            a.h.lr, a.h.lr_dev = K.rate_args(lr)
+            a.h.mu, a.h.l2, a.h.grad_scale, a.h.mode, a.h.phase = mu, l2, gs, mode, 3
         work = n if a.one_shot else (n + self.world - 1) // self.world
         blocks = max(1, min(self.blocks, (work // 8 + 127) // 128))
         streams = getattr(self, "comm_streams", None) or [self.comm_stream]

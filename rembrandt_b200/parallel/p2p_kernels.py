@@ -27,7 +27,8 @@ SIGS = {
 
 
 class SgdHyper(C.Structure):
-    _fields_ = [("lr", f32), ("mu", f32), ("l2", f32), ("grad_scale", f32), ("mode", i32), ("phase", i32)]
+    _fields_ = [("lr", f32), ("mu", f32), ("l2", f32), ("grad_scale", f32), ("mode", i32), ("phase", i32),
+                ("lr_dev", vp)]
 
 
 class ArSgdArgs(C.Structure):

@@ -506,6 +506,6 @@ def install(monkeypatch):
         if name in EMULATED:
             monkeypatch.setattr(K, name, EMULATED[name])
         elif isinstance(obj, types.FunctionType) and obj.__module__ == K.__name__ and \
-                name not in ("pad_channels", "pool_code_dtype", "status_word", "read_status"):
+                name not in ("pad_channels", "pool_code_dtype", "rate_args", "status_word", "read_status"):
             monkeypatch.setattr(K, name, _unsupported(name))
     monkeypatch.setattr(K, "read_status", lambda: 0)

@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from rembrandt_b200.api import build_replica
+from rembrandt_b200.optim.sgd import Momentum, SgdOptConfig, StepSizeSchedule
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +62,41 @@ def test_an_inference_graph_follows_what_the_loss_reads():
             else:                                 # labels on masked categories make the loss infinite in both
                 assert a[1] == b[1] and (a[0] == b[0] or abs(a[0] - b[0]) < 1e-3 * abs(b[0]) or a[0] != a[0])
     assert len(graphed._eval_graphs) == 2
+
+
+@pytest.mark.parametrize("accum", [1, 3])
+def test_a_changing_learning_rate_needs_no_further_capture(accum):
+    """The rate changes before most iterations: the same parameters and statistics as without graphs, from at most one graph
+    per staging slot and form of the step."""
+    # small enough that training does not amplify rounding: at ten times these rates its loss grows, and differences with it
+    batch, rates = 8, [2e-3, 2e-3, 1e-3, 4e-3, 4e-3, 5e-4, 0.0, 6e-3]
+    seen = []
+    for ug in (True, False):
+        opt = SgdOptConfig(minibatch_size=batch * accum, step_size=StepSizeSchedule.constant(rates[0]),
+                           momentum=Momentum.UPDATE_NESTEROV, mu=0.9, l2_reg_coef=1e-3, display_iters=0)
+        eng = build_replica("lenet", batch, use_graph=ug, seed=(5, 7), opt=opt)
+        assert eng.accum == accum
+        stats, params, captured = [], [], 0
+        for i, (x, y) in enumerate(_batches(len(rates) * accum, batch)):
+            if i % accum == 0:
+                eng.set_lr(rates[i // accum])
+            eng.feed(x, y)
+            s = eng.step()
+            stats += [s] if s is not None else []
+            captured = max(captured, len(eng._graphs))
+            if (i + 1) % accum == 0:
+                eng.synchronize()
+                params.append(eng.net.params.clone())
+        stats.append(eng.flush())
+        eng.synchronize()
+        assert captured <= (2 if accum == 1 else 4) and (captured > 0) == ug
+        seen.append((stats, params))
+    (a, pa), (b, pb) = seen
+    assert len(a) == len(b) == len(rates) * accum
+    for (la, ca), (lb, cb) in zip(a, b):
+        assert abs(la - lb) < 1e-3 * max(1.0, abs(lb)) and abs(ca - cb) <= 1
+    for i in range(1, len(rates)):
+        # The same kernels on the same data: what sums in another order leave is about a percent of an update. An update
+        # with the rate before it is off by (1 + mu) * (difference of the rates) * |g|, against an update of at most
+        # (1 + mu) * rate * |g| + mu^2 * |v| with |v| <= sum of mu^k * rate * |g|: a tenth and more wherever these rates change.
+        assert float((pa[i] - pb[i]).norm()) < 0.04 * float((pb[i] - pb[i - 1]).norm()), i
