@@ -471,12 +471,13 @@ int rb_bn_fwd_train(const void* x, long long rows, int C, int c_valid, float* su
   return RB_LAUNCH_OK();
 }
 
-// The same in two launches: `ws` is 4*C + 32 floats, on a 16-byte boundary, zero before their first use (BnScratch).
+// The same in two launches: `ws` is 4*C + 32 floats, on a 16-byte boundary, zero before their first use, and used for nothing
+// but calls of the two-launch forms with the same C: one buffer of sums is left as it is (BnScratch).
 int rb_bn_fwd_train_ws(const void* x, long long rows, int C, int c_valid, float* ws, float eps, float factor,
                        float* mean, float* istd, float* run_mean, float* run_var, const float* gamma,
                        const float* beta, const void* residual, void* y, int relu, int avg_kind,
                        const unsigned int* step_ptr, cudaStream_t st) {
-  if (C % 8) return -10;
+  if (C % 8 || ((uintptr_t)ws & 15u)) return -10;
   const BnStats stats = {mean, istd, run_mean, run_var, step_ptr, eps, factor, avg_kind};
   const BnScratch scr = bn_scratch(ws, C);
   launch_bn_reduce((const bf16*)x, nullptr, nullptr, nullptr, nullptr, rows, C, nullptr, 0, scr, st);
@@ -515,7 +516,7 @@ int rb_bn_bwd(const void* x, const void* dy, const void* y_relu, long long rows,
 int rb_bn_bwd_ws(const void* x, const void* dy, const void* y_relu, long long rows, int C, int c_valid, float* ws,
                  const float* mean, const float* istd, const float* gamma, float* dgamma, float* dbeta, void* dx,
                  cudaStream_t st) {
-  if (C % 8) return -10;
+  if (C % 8 || ((uintptr_t)ws & 15u)) return -10;
   const BnScratch scr = bn_scratch(ws, C);
   launch_bn_reduce((const bf16*)x, (const bf16*)dy, (const bf16*)y_relu, mean, istd, rows, C, nullptr, 1, scr, st);
   launch_bn_bwd_apply((const bf16*)x, (const bf16*)dy, (const bf16*)y_relu, mean, istd, gamma, nullptr, scr, dgamma, dbeta,

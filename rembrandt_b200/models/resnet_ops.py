@@ -60,7 +60,7 @@ class _BnConv:
         self.conv_out = torch.zeros((n, self.P, self.Q, self.kp), dtype=torch.bfloat16, device=dev)
         self.mean = torch.zeros(self.kp, device=dev)
         self.istd = torch.ones(self.kp, device=dev)
-        self.sums = torch.zeros(4 * self.kp + K.BN_SCRATCH_TAIL, device=dev)
+        self.sums = K.bn_scratch(self.kp, dev)
         self.dconv = torch.zeros_like(self.conv_out) if net.training_capable else None
         if self.windowed:
             self.windowed.alloc(n, dev, self.kp, False, False)
@@ -90,9 +90,9 @@ class _BnConv:
         if train:
             # the factor comes from the device-side step counter, so that graph replays keep averaging correctly
             kind = 1 if self.mov_avg.kind == "cumulative" else 2
-            K.bn_fwd_train(self.conv_out, rows, self.kp, self.ko, self.sums, self.eps, self.mov_avg.factor,
-                           self.mean, self.istd, self.v(self.seg_rm), self.v(self.seg_rv), self.v(self.seg_g),
-                           self.v(self.seg_b), residual, out, relu, avg_kind=kind, step_ptr=net.step_counter)
+            K.bn_fwd_train_ws(self.conv_out, rows, self.kp, self.ko, self.sums, self.eps, self.mov_avg.factor,
+                              self.mean, self.istd, self.v(self.seg_rm), self.v(self.seg_rv), self.v(self.seg_g),
+                              self.v(self.seg_b), residual, out, relu, avg_kind=kind, step_ptr=net.step_counter)
         else:
             K.bn_fwd_infer(self.conv_out, rows, self.kp, self.ko, self.eps, self.v(self.seg_rm), self.v(self.seg_rv),
                            self.istd, self.v(self.seg_g), self.v(self.seg_b), residual, out, relu)
@@ -102,8 +102,8 @@ class _BnConv:
         net = self.op.net
         n = net.batch
         rows = n * self.P * self.Q
-        K.bn_bwd(self.conv_out, dout, y_relu, rows, self.kp, self.ko, self.sums, self.mean, self.istd,
-                 self.v(self.seg_g), self.v(self.seg_g, "grads"), self.v(self.seg_b, "grads"), self.dconv)
+        K.bn_bwd_ws(self.conv_out, dout, y_relu, rows, self.kp, self.ko, self.sums, self.mean, self.istd,
+                    self.v(self.seg_g), self.v(self.seg_g, "grads"), self.v(self.seg_b, "grads"), self.dconv)
         gw = self.v(self.seg_w, "grads")
         if self.windowed:
             self.windowed.backward(x, self.dconv, self.kp, gw)

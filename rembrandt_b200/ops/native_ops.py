@@ -412,25 +412,41 @@ def synth_labels(labels, n, classes, seed, step):
                                          stream_handle()), "rb_synth_labels")
 
 
-# With 4 * C + BN_SCRATCH_TAIL floats of scratch (zeros at first) instead of 2 * C a normalisation takes two launches
-# instead of three: two buffers of sums, used in turn, and the two words that say which (kept on the device).
+# The two-launch forms of normalisation (`*_ws`) keep 4 * C + BN_SCRATCH_TAIL floats between calls: two buffers of sums, used
+# in turn, and the two words that say which (on the device).
 BN_SCRATCH_TAIL = 32
 
 
-def _bn_form(name, sums, C):
-    two = sums.numel() == 4 * C + BN_SCRATCH_TAIL and sums.data_ptr() % 16 == 0
-    return name + "_ws" if two else name
+def bn_scratch(C, device):
+    """Scratch of `bn_fwd_train_ws` and `bn_bwd_ws` for one layer of C channels."""
+    return torch.zeros(4 * C + BN_SCRATCH_TAIL, dtype=torch.float32, device=device)
+
+
+def _check_bn_scratch(ws, C):
+    if ws.numel() < 4 * C + BN_SCRATCH_TAIL or ws.data_ptr() % 16:
+        raise ValueError(f"normalisation of {C} channels in two launches takes {4 * C + BN_SCRATCH_TAIL} floats of scratch on a "
+                         f"16-byte boundary, not {ws.numel()} at {ws.data_ptr():#x}")
 
 
 def bn_fwd_train(x, rows, C, c_valid, sums, eps, factor, mean, istd, run_mean, run_var, gamma, beta, residual, y,
                  relu, avg_kind=0, step_ptr=None):
     """avg_kind 1 (cumulative) / 2 (exponential, 1 at step 0) derive the averaging factor from the device-side step
     counter `step_ptr`, so that a captured graph keeps averaging correctly; 0 uses `factor` as given.
-    `sums`: zeros, 2 * C floats, or 4 * C + BN_SCRATCH_TAIL for the form with one launch less."""
-    name = _bn_form("rb_bn_fwd_train", sums, C)
-    check(getattr(_native.cuda(), name)(ptr(x), rows, C, c_valid, ptr(sums), eps, factor, ptr(mean), ptr(istd),
-                                        ptr(run_mean), ptr(run_var), ptr(gamma), ptr(beta), ptr(residual), ptr(y),
-                                        int(relu), int(avg_kind), ptr(step_ptr), stream_handle()), name)
+    `sums`: at least 2 * C floats, zeros, which are zeros again afterwards: any layers may share them."""
+    check(_native.cuda().rb_bn_fwd_train(ptr(x), rows, C, c_valid, ptr(sums), eps, factor, ptr(mean), ptr(istd),
+                                         ptr(run_mean), ptr(run_var), ptr(gamma), ptr(beta), ptr(residual), ptr(y),
+                                         int(relu), int(avg_kind), ptr(step_ptr), stream_handle()), "rb_bn_fwd_train")
+
+
+def bn_fwd_train_ws(x, rows, C, c_valid, ws, eps, factor, mean, istd, run_mean, run_var, gamma, beta, residual, y,
+                    relu, avg_kind=0, step_ptr=None):
+    """`bn_fwd_train` in two launches instead of three. `ws`: `bn_scratch(C)`, which nothing but calls of the two-launch forms
+    with the same C may use."""
+    _check_bn_scratch(ws, C)
+    check(_native.cuda().rb_bn_fwd_train_ws(ptr(x), rows, C, c_valid, ptr(ws), eps, factor, ptr(mean), ptr(istd),
+                                            ptr(run_mean), ptr(run_var), ptr(gamma), ptr(beta), ptr(residual), ptr(y),
+                                            int(relu), int(avg_kind), ptr(step_ptr), stream_handle()),
+          "rb_bn_fwd_train_ws")
 
 
 def bn_fwd_infer(x, rows, C, c_valid, eps, run_mean, run_var, istd_tmp, gamma, beta, residual, y, relu):
@@ -440,6 +456,12 @@ def bn_fwd_infer(x, rows, C, c_valid, eps, run_mean, run_var, istd_tmp, gamma, b
 
 
 def bn_bwd(x, dy, y_relu, rows, C, c_valid, sums, mean, istd, gamma, dgamma, dbeta, dx):
-    name = _bn_form("rb_bn_bwd", sums, C)
-    check(getattr(_native.cuda(), name)(ptr(x), ptr(dy), ptr(y_relu), rows, C, c_valid, ptr(sums), ptr(mean), ptr(istd),
-                                        ptr(gamma), ptr(dgamma), ptr(dbeta), ptr(dx), stream_handle()), name)
+    check(_native.cuda().rb_bn_bwd(ptr(x), ptr(dy), ptr(y_relu), rows, C, c_valid, ptr(sums), ptr(mean), ptr(istd),
+                                   ptr(gamma), ptr(dgamma), ptr(dbeta), ptr(dx), stream_handle()), "rb_bn_bwd")
+
+
+def bn_bwd_ws(x, dy, y_relu, rows, C, c_valid, ws, mean, istd, gamma, dgamma, dbeta, dx):
+    """`bn_bwd` in two launches instead of three, with the scratch of `bn_fwd_train_ws`."""
+    _check_bn_scratch(ws, C)
+    check(_native.cuda().rb_bn_bwd_ws(ptr(x), ptr(dy), ptr(y_relu), rows, C, c_valid, ptr(ws), ptr(mean), ptr(istd),
+                                      ptr(gamma), ptr(dgamma), ptr(dbeta), ptr(dx), stream_handle()), "rb_bn_bwd_ws")

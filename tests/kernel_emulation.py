@@ -497,6 +497,7 @@ EMULATED = {f.__name__: f for f in (conv_fprop_tc, conv_wgrad_tc, conv_direct_fw
                                     softmax_ce, input_u8, sgd_fused, bn_fwd_train, bn_fwd_infer, bn_bwd,
                                     pointwise_loss, categorical_loss, lrn_fwd, lrn_bwd, dropout, var_input_u8, sgd_fused_grid,
                                     axpy_shadow, gemm_set_option)}
+EMULATED.update(bn_fwd_train_ws=bn_fwd_train, bn_bwd_ws=bn_bwd)
 
 
 def install(monkeypatch):
@@ -506,6 +507,6 @@ def install(monkeypatch):
         if name in EMULATED:
             monkeypatch.setattr(K, name, EMULATED[name])
         elif isinstance(obj, types.FunctionType) and obj.__module__ == K.__name__ and \
-                name not in ("pad_channels", "pool_code_dtype", "rate_args", "status_word", "read_status"):
+                name not in ("pad_channels", "pool_code_dtype", "bn_scratch", "rate_args", "status_word", "read_status"):
             monkeypatch.setattr(K, name, _unsupported(name))
     monkeypatch.setattr(K, "read_status", lambda: 0)

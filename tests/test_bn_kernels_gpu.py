@@ -1,7 +1,7 @@
 """The two-launch form of batch normalisation (statistics worked out by the kernel that applies them) against fp64 torch,
 at channel counts that do and do not divide a block, more channels than one block covers, padded channels, and row counts
-from one to several waves; every call runs three times on the same
-scratch, once without a backward pass between."""
+from one to several waves; every call runs three times on the same scratch, once without a backward pass between. And a scratch
+of the three-launch form that layers of several widths share, among them one whose two-launch scratch has its length."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -26,7 +26,7 @@ def test_two_launch_form(rows, C, valid):
     x[:, valid:] = 0
     res = rnd(rows, C).bfloat16()
     gamma, beta = rnd(C) * 0.1 + 1, rnd(C)
-    sums = torch.zeros(4 * C + K.BN_SCRATCH_TAIL, device=DEV)
+    sums = K.bn_scratch(C, DEV)
     mean, istd = torch.empty(C, device=DEV), torch.empty(C, device=DEV)
     y = torch.empty(rows, C, device=DEV, dtype=torch.bfloat16)
     dy = rnd(rows, C).bfloat16()
@@ -38,7 +38,7 @@ def test_two_launch_form(rows, C, valid):
     out = torch.relu(xh * gamma.double() + beta.double() + res.double())[:, :valid]
     for again in range(3):
         rm, rv = torch.zeros(C, device=DEV), torch.ones(C, device=DEV)
-        K.bn_fwd_train(x, rows, C, valid, sums, 1e-5, 0.25, mean, istd, rm, rv, gamma, beta, res, y, True)
+        K.bn_fwd_train_ws(x, rows, C, valid, sums, 1e-5, 0.25, mean, istd, rm, rv, gamma, beta, res, y, True)
         # means of `rows` fp32 sums against 64 bits: 1e-4 of the deviation covers 92416 summands many times over
         assert float(((mean.double() - m64) * s64)[:valid].abs().max()) < 1e-4
         if rows > 1:
@@ -51,7 +51,7 @@ def test_two_launch_form(rows, C, valid):
             continue
         dg, db = torch.ones(C, device=DEV), torch.ones(C, device=DEV)
         dx = torch.empty_like(x)
-        K.bn_bwd(x, dy, y, rows, C, valid, sums, mean, istd, gamma, dg, db, dx)
+        K.bn_bwd_ws(x, dy, y, rows, C, valid, sums, mean, istd, gamma, dg, db, dx)
         gm = dy.double() * (y.double() > 0)
         assert float((db.double() - 1 - gm.sum(0))[:valid].abs().max()) < 1e-4 * rows ** 0.5 * 10
         if rows > 1:
@@ -65,3 +65,23 @@ def test_two_launch_form(rows, C, valid):
     K.bn_fwd_infer(x, rows, C, valid, 1e-5, rm, rv, istd, gamma, beta, res, y, False)
     want = (xd - rm.double()) * torch.rsqrt(rv.double() + 1e-5) * gamma.double() + beta.double() + res.double()
     _close(y[:, :valid], want[:, :valid], 4e-3)
+
+
+def test_layers_share_a_scratch_of_the_three_launch_form():
+    widths = (32, 80, 32, 80)
+    sums = torch.zeros(2 * 80, device=DEV)           # 4 * 32 + 32 floats as well
+    assert sums.numel() == 4 * 32 + K.BN_SCRATCH_TAIL
+    g = torch.Generator(device=DEV).manual_seed(9)
+    rows = 500
+    for C in widths:
+        x = (torch.randn(rows, C, generator=g, device=DEV) * 2 + 1).bfloat16()
+        gamma, beta = torch.ones(C, device=DEV), torch.zeros(C, device=DEV)
+        mean, istd, dg, db = (torch.zeros(C, device=DEV) for _ in range(4))
+        y, dx = torch.empty_like(x), torch.empty_like(x)
+        K.bn_fwd_train(x, rows, C, C, sums, 1e-5, 1.0, mean, istd, None, None, gamma, beta, None, y, False)
+        K.bn_bwd(x, x, None, rows, C, C, sums, mean, istd, gamma, dg, db, dx)
+        m64 = x.double().mean(0)
+        assert float((mean.double() - m64).abs().max()) < 1e-4 and (sums == 0).all()
+        assert float((db.double() - x.double().sum(0)).abs().max()) < 1e-4 * rows ** 0.5 * 10
+    with pytest.raises(ValueError):
+        K.bn_bwd_ws(x, x, None, rows, 80, 80, sums, mean, istd, gamma, dg, db, dx)
