@@ -622,7 +622,8 @@ class Conv2dOp(Op):
             self.segs.append(self.seg_b)
         self.dgrad = None        # DgradPlan on a GPU
         self.windowed = None
-        if self.takes_windows and not self.direct and type(prev) is DataOp and WindowedFirstLayer.fits(prev, k, c, net.device):
+        if (self.takes_windows and not self.direct and type(prev) is DataOp and
+                WindowedFirstLayer.fits(prev, k, c, rs * self.cp, net.device)):
             self.windowed = WindowedFirstLayer(prev, k, s, p, self.P, self.Q, cfg.out_channels, c, self.cp, rs * self.cp,
                                                self.f if self.s2d else None)
 

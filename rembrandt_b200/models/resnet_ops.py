@@ -214,10 +214,10 @@ class BNormConv2dOp(_BlockBase):
             s2d = (f, r2, s2d_hw)
         self.u = _BnConv(self, "conv", (h, w), c, prev.out_cp, cfg.out_channels, cfg.conv_size, cfg.conv_stride,
                          cfg.conv_pad, cfg.init_weights, cfg.bnorm_mov_avg, cfg.bnorm_epsilon, s2d=s2d)
-        if type(prev) is DataOp and WindowedFirstLayer.fits(prev, cfg.conv_size, c, net.device):
+        row_len = self.u.gk * self.u.gk * self.u.cp
+        if type(prev) is DataOp and WindowedFirstLayer.fits(prev, cfg.conv_size, c, row_len, net.device):
             self.u.windowed = WindowedFirstLayer(prev, cfg.conv_size, cfg.conv_stride, cfg.conv_pad, self.u.P, self.u.Q,
-                                                 cfg.out_channels, c, self.u.cp, self.u.gk * self.u.gk * self.u.cp,
-                                                 self.u.f if s2d else None)
+                                                 cfg.out_channels, c, self.u.cp, row_len, self.u.f if s2d else None)
         self.units = (self.u,)
         self.segs = list(self.u.segs)
         self.out_hwc = (self.u.P, self.u.Q, cfg.out_channels)
