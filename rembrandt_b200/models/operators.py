@@ -642,7 +642,7 @@ class Conv2dOp(Op):
                     has_bias=self.seg_b is not None, n_valid=ko, n_store=self.out_cp)
         if self.net.training_capable and self.wants_prev_delta():
             self.dgrad = DgradPlan(n, self.P, self.Q, self.out_cp, ko, self.cp, self.in_c, r, s, p, h, w,
-                                   [(False, self.mask_src() is not None)])
+                                   [(False, self.mask_src() is not None)], self.net.device)
 
     # geometry the kernels see (the s2d form is a stride-1, pad-0 convolution on the rearranged input)
     def _geom(self):

@@ -70,7 +70,7 @@ class _BnConv:
                         self.Q, self.kp, n_valid=self.ko, n_store=self.kp)
             if net.training_capable and dx_forms:
                 self.dgrad = DgradPlan(n, self.P, self.Q, self.kp, self.ko, self.cp, self.in_c, self.k, self.s, self.p,
-                                       self.h, self.w, dx_forms)
+                                       self.h, self.w, dx_forms, dev)
 
     def v(self, seg, which="params"):
         return self.op.net.seg_view(seg, which)

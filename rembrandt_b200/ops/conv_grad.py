@@ -88,13 +88,14 @@ class DgradPlan:
 
     LAUNCH_MS, MOST_GAIN = 0.003, 1 / 6
 
-    def __init__(self, n, P, Q, kp, ko, cp, in_c, k, stride, pad, H, W, forms):
-        """`forms`: the (addend, mask) combinations that will be asked for."""
+    def __init__(self, n, P, Q, kp, ko, cp, in_c, k, stride, pad, H, W, forms, device="cuda"):
+        """`forms`: the (addend, mask) combinations that will be asked for; `device`: the network's, current or not."""
         self.geom = (n, P, Q, kp, ko, cp, in_c, k, stride, pad, H, W)
-        key = (torch.cuda.current_device(),) + self.geom + (tuple(forms),)
-        if key not in _measured:
-            _measured[key] = self._measure(forms)
-        self.wt = torch.zeros((cp, k * k, kp), dtype=torch.bfloat16, device="cuda") if _measured[key] else None
+        with torch.cuda.device(device):
+            key = (torch.cuda.current_device(),) + self.geom + (tuple(forms),)
+            if key not in _measured:
+                _measured[key] = self._measure(forms)
+        self.wt = torch.zeros((cp, k * k, kp), dtype=torch.bfloat16, device=device) if _measured[key] else None
 
     def _measure(self, forms) -> bool:
         n, P, Q, kp, ko, cp, in_c, k, stride, pad, H, W = self.geom
