@@ -61,6 +61,7 @@ class StepEngine:
             self._stats_dev = torch.zeros(2, dtype=torch.float32, device=dev)
             # rows 0 and 1: steps, written in turn (the device keeps count for graph replays); row 2: inference
             self._stats_host = torch.zeros((3, 2), dtype=torch.float32).pin_memory()
+            self._mirrors = list(self._stats_host)
             self._stats_ready = [torch.cuda.Event() for _ in range(2)]
             self._turn, self._turn_dev = 0, torch.zeros(1, dtype=torch.int32, device=dev)
             # the learning rate that captured steps read, and what was last written there
@@ -144,15 +145,19 @@ class StepEngine:
         lo = self.net.loss_op
         if self.net.device.type == "cuda":
             if inference:
-                K.publish_stats(lo.loss_sum, lo.correct, self._stats_host[2])
+                K.publish_stats(lo.loss_sum, lo.correct, self._mirrors[2])
             else:
                 K.publish_stats(lo.loss_sum, lo.correct, self._stats_host, turn=self._turn_dev)
             return
         self._stats_dev[0:1].copy_(lo.loss_sum, non_blocking=True)
         self._stats_dev[1:2].copy_(lo.correct, non_blocking=True)
-        self._stats_host[2 if inference else self._turn].copy_(self._stats_dev, non_blocking=True)
+        self._mirrors[2 if inference else self._turn].copy_(self._stats_dev, non_blocking=True)
         lo.loss_sum.zero_()
         lo.correct.zero_()
+
+    def _read(self, mirror) -> Tuple[float, int]:
+        loss, correct = self._mirrors[mirror].tolist()
+        return loss, int(correct)
 
     def _capture(self, fn):
         """`fn`'s launches on the current stream as a graph."""
@@ -288,7 +293,7 @@ class StepEngine:
         if self._lag_stats is not None:
             j = self._lag_stats
             self._stats_ready[j].synchronize()
-            prev = (float(self._stats_host[j][0]), int(self._stats_host[j][1]))
+            prev = self._read(j)
         self._lag_stats = i
         if last:
             self.iter += 1
@@ -303,7 +308,7 @@ class StepEngine:
         j = self._lag_stats
         self._stats_ready[j].synchronize()
         self._lag_stats = None
-        return float(self._stats_host[j][0]), int(self._stats_host[j][1])
+        return self._read(j)
 
     def d2h_bytes_per_step(self) -> int:
         return 8 if self.is_cuda else 0
@@ -324,7 +329,7 @@ class StepEngine:
             self._eval_forward()
             self._publish(inference=True)
         self.compute_stream.synchronize()
-        return float(self._stats_host[2][0]), int(self._stats_host[2][1])
+        return self._read(2)
 
     def _eval_forward(self):
         """The inference pass over the loaded batch: eager the first time, then a graph. What may differ between two calls
