@@ -250,9 +250,11 @@ __global__ void bn_finalize_kernel(float* __restrict__ sums, const bf16* __restr
 }
 
 // y = act(gamma * (x - mean) * istd + beta [+ residual]), with mean and istd from st.mean / st.istd (BN_GIVEN), from the
-// running statistics (BN_INFER) or from a reduction's sums (BN_SUMS: every block works them out for its own channels). Per row and thread: 16 bytes in (32 with a residual), 16 out, one subtract and one
-// fused multiply-add per channel; four rows in flight. A thread used to fetch all five values of all its eight channels
-// again for every row, and 64-bit divide to find them: 92416 x 128 took 22 us, now 11.
+// running statistics (BN_INFER) or from a reduction's sums (BN_SUMS: every block works them out for its own channels). Per row
+// and thread: 16 bytes in (32 with a residual), 16 out, one subtract and one fused multiply-add per channel; four rows in
+// flight. A thread used to fetch all five values of all its eight channels again for every row, and 64-bit divide to find
+// them: 92416 x 128 took 22 us, now 11 with given statistics or running ones. From sums it takes 13 (cold caches; 18 with
+// two divisions per channel and more blocks than fit at once).
 enum { BN_GIVEN = 0, BN_INFER = 1, BN_SUMS = 2 };
 template <int FROM, int RES>
 __global__ void __launch_bounds__(256) bn_apply_kernel(const bf16* __restrict__ x, const BnStats st, const BnScratch ws,
@@ -486,12 +488,11 @@ int rb_bn_fwd_train_ws(const void* x, long long rows, int C, int c_valid, float*
   return RB_LAUNCH_OK();
 }
 
-// One launch; `istd_tmp` is left over from when the inverse deviations were computed by a kernel of their own.
+// One launch, which works out the inverse deviations itself: the argument that once was scratch for them is not looked at.
 int rb_bn_fwd_infer(const void* x, long long rows, int C, int c_valid, float eps, const float* run_mean,
-                    const float* run_var, float* istd_tmp, const float* gamma, const float* beta, const void* residual,
-                    void* y, int relu, cudaStream_t st) {
+                    const float* run_var, float* /* scratch */, const float* gamma, const float* beta,
+                    const void* residual, void* y, int relu, cudaStream_t st) {
   if (C % 8) return -10;
-  (void)istd_tmp;
   const BnStats stats = {nullptr, nullptr, (float*)run_mean, (float*)run_var, nullptr, eps, 0.f, 0};
   launch_bn_apply<BN_INFER>((const bf16*)x, stats, BnScratch{}, gamma, beta, (const bf16*)residual, (bf16*)y, rows, C,
                             c_valid, relu, st);

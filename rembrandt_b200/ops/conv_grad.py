@@ -3,8 +3,9 @@
 On a GPU this is `rb_conv_dgrad_tc` (csrc/gemm_tc.cu): the filters are read as they lie (or from a transposed and flipped
 copy, `DgradPlan`), the output phases of a strided convolution are written straight to their places in dx, and the addend
 (the delta of an identity path, or the gradient of a parallel branch already in dx) and the mask of the producer's ReLU
-ride in the epilogue. Without a GPU the same result is put together from the kernel fronts of `native_ops`, which the CPU
-tests replace by plain torch.
+ride in the epilogue. Strided geometries that it does not take, and all with RB_STRIDED_DGRAD_TC=0, run on the CUDA-core
+kernel. Without a GPU the result is put together from the kernel fronts of `native_ops`, which the CPU tests replace by
+plain torch.
 """
 from __future__ import annotations
 
@@ -26,6 +27,8 @@ def _strided_on_cuda_cores(stride) -> bool:
 
 
 def _compose(dy, n, P, Q, kp, w16, ko, cp, in_c, k, stride, pad, H, W, dx, add, mask):
+    """The same from several launches. On a GPU only strided convolutions come here, without phases that the tensor-core
+    kernel could run."""
     out = torch.empty_like(dx) if add is not None and add.data_ptr() == dx.data_ptr() else dx
     late = mask if add is not None else None
     early = None if add is not None else mask
@@ -34,8 +37,8 @@ def _compose(dy, n, P, Q, kp, w16, ko, cp, in_c, k, stride, pad, H, W, dx, add, 
         K.pack_dgrad_filters(w16, wt, ko, kp, k * k, cp)
         K.conv_fprop_tc(dy, n, P, Q, kp, wt, cp, k, k, 1, k - 1 - pad, k - 1 - pad, H, W, out, cp, mask_src=early,
                         n_valid=in_c, n_store=cp)
-    elif _strided_on_cuda_cores(stride) or not dgrad_strided_tc(dy, n, P, Q, kp, w16, ko, cp, in_c, k, k, stride, pad, H, W,
-                                                                out, early):
+    elif dy.device.type == "cuda" or _strided_on_cuda_cores(stride) or not dgrad_strided_tc(
+            dy, n, P, Q, kp, w16, ko, cp, in_c, k, k, stride, pad, H, W, out, early):
         K.conv_direct_dgrad(dy, w16, out, early, n, H, W, cp, ko, kp, k, k, stride, pad, pad, P, Q)
     if add is not None:
         K.add_bf16(out, add, out.numel())

@@ -7,11 +7,13 @@ r = r0 + s u, c = c0 + s v with r0 = (a + pad) mod s, c0 = (b + pad) mod s, and
     qa = (a + pad - r0) / s,   qb = (b + pad - c0) / s
 
 which is a stride-1 convolution of dY with the flipped sub-filter, top / left padding (U - 1) - qa, (V - 1) - qb.
-Each of the s x s phases runs through the forward convolution path (`conv_fprop_tc`) into a compact tensor that is
-then interleaved into dX; phases with no tap (e.g. three of the four phases of a 1 x 1 stride-2 projection) are zero.
+Each of the s x s phases is a stride-1 convolution; phases with no tap (e.g. three of the four phases of a 1 x 1 stride-2
+projection) are zero. On a GPU training runs them through `rb_conv_dgrad_tc` (csrc/gemm_tc.cu), which reads the filters where
+they lie and scatters the phases' rows itself.
 
-`phase_plan` is pure arithmetic (tested on CPU against autograd through `dgrad_by_phases_reference`); the device
-path below only swaps the plain-torch convolution for the kernel.
+`phase_plan` is pure arithmetic (tested on CPU against autograd through `dgrad_by_phases_reference`); `dgrad_strided_tc` is
+the same on the forward kernel's front (`conv_fprop_tc`), one compact tensor per phase, interleaved afterwards: what
+`conv_grad.conv_dgrad` does without a GPU.
 """
 from __future__ import annotations
 
@@ -72,10 +74,10 @@ def dgrad_by_phases_reference(dy: torch.Tensor, w: torch.Tensor, H: int, W: int,
 
 
 def dgrad_strided_tc(dy, n, P, Q, kp, w16, ko, cp, in_c, R, S, stride, pad, H, W, dx, mask=None, cache=None):
-    """Device path. dy: bf16 [n, P, Q, kp]; w16: bf16 filters [ko][R*S][cp]; dx: bf16 [n, H, W, cp] (overwritten);
+    """dy: bf16 [n, P, Q, kp]; w16: bf16 filters [ko][R*S][cp]; dx: bf16 [n, H, W, cp] (overwritten);
     mask: optional bf16 [n, H, W, cp], dx is zeroed where mask <= 0. Returns False when a phase needs a negative
-    padding (the caller then uses the direct kernel). `cache` (a dict owned by the calling operator) keeps the
-    per-phase filter and output buffers between calls, so that a training step allocates nothing here."""
+    padding (the caller then uses the direct kernel). `cache` (a dict that the caller keeps) holds the per-phase
+    filter and output buffers between calls."""
     from . import native_ops as K
     plan = phase_plan(H, W, R, S, stride, pad)
     if any(ph.U and ph.V and (ph.pad_t < 0 or ph.pad_l < 0) for ph in plan):

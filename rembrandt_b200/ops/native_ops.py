@@ -450,6 +450,7 @@ def bn_fwd_train_ws(x, rows, C, c_valid, ws, eps, factor, mean, istd, run_mean, 
 
 
 def bn_fwd_infer(x, rows, C, c_valid, eps, run_mean, run_var, istd_tmp, gamma, beta, residual, y, relu):
+    """`istd_tmp` is not written: the inverse deviations stay in registers."""
     check(_native.cuda().rb_bn_fwd_infer(ptr(x), rows, C, c_valid, eps, ptr(run_mean), ptr(run_var), ptr(istd_tmp),
                                          ptr(gamma), ptr(beta), ptr(residual), ptr(y), int(relu), stream_handle()),
           "rb_bn_fwd_infer")

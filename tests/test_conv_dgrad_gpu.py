@@ -78,6 +78,12 @@ def test_oblong_images_and_measured_plans(shape, add, masked, packed, tuned):
     _run(shape, add, masked, packed, tuned)
 
 
+@pytest.mark.parametrize("shape", [(2, 32, 48, 9, 1, 2, 2, 12), (3, 64, 32, 11, 3, 3, 4)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_phases_of_negative_padding_run_on_cuda_cores(shape, masked):
+    _run(shape, None, masked)
+
+
 @pytest.mark.parametrize("shape", [SHAPES[1], SHAPES[4], SHAPES[7], SHAPES[8], SHAPES[9]])
 @pytest.mark.parametrize("options", [dict(force_mt=2), dict(force_resident=1), dict(force_box=1), dict(force_wide=1),
                                      dict(force_pair=1), dict(force_tail=1), dict(deterministic=1)])
