@@ -216,28 +216,20 @@ __device__ __forceinline__ void load_b(const GemmTcParams& p, uint8_t* sb, uint6
 // The issuing warp's instruction stream is what bounds the kernel when operands arrive in time (a single extra
 // branch per MMA in this loop cost 44 % on a weight-grad launch), so nothing here is computed per MMA that can be
 // computed per k-block, and only the first MMA into an accumulator carries a predicate.
+// The steps of one accumulator share an election and take one addition per operand each, and whether the next stage has
+// arrived is asked before the MMAs of this one are issued: a k-block cost the issuing warp ~100 cycles of waiting for its own
+// barrier and ~35 per MMA beyond what the tensor core needs (with the coordinates worked out before the dependency wait, see
+// `ahead_done`: 3 x 3, 64 -> 64 on 128 x 8 x 8: 8.8 -> 7.5 us; 128 -> 128 on 256 x 19 x 19, weight gradient: 33.6 -> 31.3).
 template <int KK, int MT, bool WIDE, bool PAIR>
-__device__ __forceinline__ void issue_kblock(uint32_t d_tmem, uint32_t acc_stride, uint64_t da, uint64_t a_sub,
-                                             uint64_t db, uint32_t a_adv, uint32_t b_adv, uint32_t idesc,
-                                             uint32_t idesc2, uint64_t b_wide_off, bool fresh) {
+__device__ __forceinline__ void issue_kblock(uint32_t d_tmem, uint32_t acc_stride, uint32_t a_lo, uint32_t a_hi, uint32_t a_sub,
+                                             uint32_t b_lo, uint32_t b_hi, uint32_t a_adv, uint32_t b_adv, uint32_t idesc,
+                                             uint32_t idesc2, uint32_t b_wide_off, bool fresh) {
 #pragma unroll
   for (int j = 0; j < MT; ++j) {
-    const uint32_t dj = d_tmem + (uint32_t)j * acc_stride;
-    const uint64_t daj = da + (uint64_t)j * a_sub;
-#pragma unroll
-    for (int kk = 0; kk < KK; ++kk) {
-      const uint64_t ak = daj + (uint64_t)(a_adv * kk), bk_ = db + (uint64_t)(b_adv * kk);
-      if (PAIR) {
-        if (kk == 0) tc_mma2_f16(dj, ak, bk_, idesc, fresh ? 0u : 1u);
-        else tc_mma2_f16_acc(dj, ak, bk_, idesc);
-      } else if (kk == 0) {
-        tc_mma_f16(dj, ak, bk_, idesc, fresh ? 0u : 1u);
-        if (WIDE) tc_mma_f16(dj + 256u, ak, bk_ + b_wide_off, idesc2, fresh ? 0u : 1u);
-      } else {
-        tc_mma_f16_acc(dj, ak, bk_, idesc);
-        if (WIDE) tc_mma_f16_acc(dj + 256u, ak, bk_ + b_wide_off, idesc2);
-      }
-    }
+    tc_mma_steps<KK, PAIR>(d_tmem + (uint32_t)j * acc_stride, a_lo + (uint32_t)j * a_sub, a_hi, b_lo, b_hi, a_adv, b_adv, idesc,
+                           fresh ? 0u : 1u);
+    if (WIDE)
+      tc_mma_steps<KK, false>(d_tmem + 256u, a_lo, a_hi, b_lo + b_wide_off, b_hi, a_adv, b_adv, idesc2, fresh ? 0u : 1u);
   }
 }
 
@@ -245,7 +237,7 @@ __device__ __forceinline__ void issue_kblock(uint32_t d_tmem, uint32_t acc_strid
 struct IssueCtx {
   uint32_t ring_u32, tiles_u32, stage_bytes, b_bytes, b_in_stage;   // b_in_stage: offset of B inside a stage
   uint32_t acc_stride, a_adv, b_adv, idesc, idesc2;
-  uint64_t a_desc0, b_desc0, a_sub, b_wide_off;
+  uint32_t a_desc0_lo, b_desc0_lo, a_hi, b_hi, a_sub, b_wide_off;   // descriptors: the address in the lower word is filled in
   int stages, b_resident;
 };
 
@@ -253,21 +245,22 @@ struct IssueCtx {
 template <int KK, int MT, bool WIDE, bool PAIR>
 __device__ __forceinline__ bool issue_item(const IssueCtx& c, SharedCtl* ctl, unsigned int* status, uint32_t d_tmem,
                                            int kb0, int kb1, int& s, uint32_t& ph) {
+  bool ready = mbar_test_wait(&ctl->full[s], ph);
   for (int kb = kb0; kb < kb1; ++kb) {
-    if (!ctl_wait_warp_role(ctl, &ctl->full[s], ph, status, 2)) return false;
+    if (!__all_sync(0xffffffffu, ready) && !ctl_wait_warp_role(ctl, &ctl->full[s], ph, status, 2)) return false;
     tc_fence_after();
     const uint32_t sa = c.ring_u32 + (uint32_t)s * c.stage_bytes;
     const uint32_t sb = c.b_resident ? c.tiles_u32 + (uint32_t)kb * c.b_bytes : sa + c.b_in_stage;
+    uint64_t* const done = &ctl->empty[s];
+    if (++s == c.stages) { s = 0; ph ^= 1u; }
+    ready = mbar_test_wait(&ctl->full[s], ph);      // the answer is under way while these are issued
     // descriptors differ from the templates only in the 14-bit start address (no carry out of it: shared memory
     // ends below 256 KB)
-    const uint64_t da = c.a_desc0 | (uint64_t)((sa >> 4) & 0x3FFFu);
-    const uint64_t db = c.b_desc0 | (uint64_t)((sb >> 4) & 0x3FFFu);
-    issue_kblock<KK, MT, WIDE, PAIR>(d_tmem, c.acc_stride, da, c.a_sub, db, c.a_adv, c.b_adv, c.idesc, c.idesc2,
-                                     c.b_wide_off, kb == kb0);
+    issue_kblock<KK, MT, WIDE, PAIR>(d_tmem, c.acc_stride, c.a_desc0_lo | (sa >> 4), c.a_hi, c.a_sub, c.b_desc0_lo | (sb >> 4),
+                                     c.b_hi, c.a_adv, c.b_adv, c.idesc, c.idesc2, c.b_wide_off, kb == kb0);
     // stage is free once these MMAs have read it (in both CTAs of a pair)
-    if (PAIR) tc_commit2_both(&ctl->empty[s]);
-    else tc_commit(&ctl->empty[s]);
-    if (++s == c.stages) { s = 0; ph ^= 1u; }
+    if (PAIR) tc_commit2_both(done);
+    else tc_commit(done);
   }
   return true;
 }
@@ -329,7 +322,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
   uint8_t* staging = tiles + TILE_SMEM_BYTES;
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(staging + STAGING_BYTES);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // known to be the same in all lanes
   const int lane = threadIdx.x & 31;
 
   // CTA pairs: rank of this CTA in its pair, and the persistent loop runs over pairs
@@ -407,12 +400,19 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
   __syncthreads();
   if (pair) cluster_sync_all();   // the peer's barriers are initialised before anything of ours signals them
   tc_fence_after();
-  // Programmatic dependent launch (option `pdl`): everything above touched only this CTA's own shared memory, TMEM
-  // and the launch parameters, so it may run while the kernels before this one on the stream are still finishing;
-  // nothing below (operands, bias, mask, output, workspace) is touched before they have completed and flushed.
-  // Without the launch attribute both instructions do nothing.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // Programmatic dependent launch (option `pdl`): what touches only this CTA's own shared memory, TMEM and the launch
+  // parameters may run while the kernels before this one on the stream are still finishing. Every warp that touches anything
+  // else (operands, bias, mask, output, workspace) calls `ahead_done` first, which returns when they have completed and
+  // flushed: the producers right before their first load, when its coordinates have been worked out and its stage claimed
+  // (1 - 2 us of integer divisions and first touches of code and parameters). Without the launch attribute the instructions
+  // do nothing.
+  bool ahead = true;
+  auto ahead_done = [&ahead]() {
+    if (!ahead) return;
+    ahead = false;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  };
   const uint32_t tmem_base = ctl->tmem_base;
 
   if (warp == 0 || warp == PRODUCER_B_WARP) {
@@ -430,6 +430,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       const int nst = is_a ? p.hl_a_stages : stages;
       uint64_t* fullb = is_a ? ctl->a_full : ctl->full;
       uint64_t* emptyb = is_a ? ctl->a_empty : ctl->empty;
+      ahead_done();
       if (lane == 0) {
         for (int work = cta_id; work < num_work && ok; work += cta_step) {
           const int tn = work / m_items;
@@ -560,6 +561,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
           uint8_t* to = ring + s * stage_bytes + dst;
           uint64_t* bar = &ctl->full[s];
           const uint32_t bar2 = full0_leader + (uint32_t)s * 8u;   // pairs: the leader's barrier of this stage
+          ahead_done();
           if (lane < nload) {
             // pairs: K-major A; K-major B or filters as they lie
             switch (mode) {
@@ -647,6 +649,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       if (blockIdx.x < num_work) {
         if (lane == 0) mbar_expect_tx(&ctl->b_full, (uint32_t)panel_bytes);
         __syncwarp();
+        ahead_done();
         for (int kb = lane; kb < p.num_kb; kb += 32) load_b(p, tiles + kb * b_bytes, &ctl->b_full, kb, 0);
       }
     }
@@ -659,7 +662,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       // a tile wider than 256 columns is two MMAs side by side (256 + the rest) that share the A descriptor
       const uint32_t idesc = make_idesc_bf16(pair ? 2 * BM : BM, (uint32_t)min(p.bn, 256), a_mn ? 1u : 0u, b_mn ? 1u : 0u);
       const uint32_t idesc2 = p.bn > 256 ? make_idesc_bf16(BM, (uint32_t)(p.bn - 256), a_mn ? 1u : 0u, b_mn ? 1u : 0u) : 0u;
-      const uint64_t b_wide_off = (uint64_t)((256u * (uint32_t)p.bk * 2u) >> 4);   // 256 rows (K-major) or 4 blocks on
+      const uint32_t b_wide_off = (256u * (uint32_t)p.bk * 2u) >> 4;   // 256 rows (K-major) or 4 blocks on
       // K-major: rows of bk*2 bytes, 8-row atoms -> SBO = 8*bk*2; swizzle 128B (bk=64) or 64B (bk=32)
       // MN-major: 64-element (128 B) rows per k, atoms of 8 k -> SBO = 1024, LBO = bk*128 between 64-wide blocks
       const uint32_t k_layout = (p.bk == 64) ? 2u : 4u;
@@ -702,10 +705,13 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                   // filter row r of sub-tile j: the same tile, (j * hl_rows + r) * hl_pitch rows further down
                   const uint32_t off = (uint32_t)((j * p.hl_rows + r) * p.hl_pitch) * row_bytes;
                   const uint64_t da = make_smem_desc(a_base + off, a_lbo, a_sbo, a_lay);
-                  for (int kk = 0; kk < kk_steps; ++kk) {
-                    tc_mma_f16(d_tmem + (uint32_t)(j * p.acc_stride), da + (uint64_t)(a_adv * kk),
-                               db + (uint64_t)(b_adv * kk), idesc, (!fresh || kk > 0) ? 1u : 0u);
-                  }
+                  const uint32_t dj = d_tmem + (uint32_t)(j * p.acc_stride);
+                  if (kk_steps == 4)
+                    tc_mma_steps<4, false>(dj, (uint32_t)da, (uint32_t)(da >> 32), (uint32_t)db, (uint32_t)(db >> 32), a_adv,
+                                           b_adv, idesc, fresh ? 0u : 1u);
+                  else
+                    tc_mma_steps<2, false>(dj, (uint32_t)da, (uint32_t)(da >> 32), (uint32_t)db, (uint32_t)(db >> 32), a_adv,
+                                           b_adv, idesc, fresh ? 0u : 1u);
                 }
                 fresh = false;
                 tc_commit(&ctl->empty[bs]);
@@ -733,9 +739,12 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       ic.b_adv = b_adv;
       ic.idesc = idesc;
       ic.idesc2 = idesc2;
-      ic.a_desc0 = make_smem_desc(0u, a_lbo, a_sbo, a_lay);
-      ic.b_desc0 = make_smem_desc(0u, b_lbo, b_sbo, b_lay);
-      ic.a_sub = (uint64_t)((uint32_t)a_bytes >> 4);     // next 128-row sub-tile of the stage
+      const uint64_t a_desc0 = make_smem_desc(0u, a_lbo, a_sbo, a_lay), b_desc0 = make_smem_desc(0u, b_lbo, b_sbo, b_lay);
+      ic.a_desc0_lo = (uint32_t)a_desc0;
+      ic.a_hi = (uint32_t)(a_desc0 >> 32);
+      ic.b_desc0_lo = (uint32_t)b_desc0;
+      ic.b_hi = (uint32_t)(b_desc0 >> 32);
+      ic.a_sub = (uint32_t)a_bytes >> 4;     // next 128-row sub-tile of the stage
       ic.b_wide_off = b_wide_off;
       ic.stages = stages;
       ic.b_resident = p.b_resident;
@@ -764,6 +773,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
     }
   } else if (warp < 2 + EPI_WARPS) {
     // ------------------------------ epilogue ------------------------------
+    ahead_done();
     const int lane_base = (warp & 3) * 32;  // TMEM lanes this warp may read
     const uint32_t set_cols = (uint32_t)(mt * p.acc_stride);
     const int col_half = (warp - 2) >> 2;        // which of the two warps of this lane quarter

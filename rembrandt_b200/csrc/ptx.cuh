@@ -52,6 +52,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// The same without waiting at all: `try_wait` may suspend the thread for microseconds where the phase is not over.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // Bounded wait: gives up after `limit_ns` and returns false. The caller then
 // raises the kernel's abort flag; nothing ever spins without a limit.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, uint64_t limit_ns) {
@@ -161,25 +173,39 @@ __device__ __forceinline__ void tc_fence_after() {
 // branch that one lane takes alone, the descriptors are that lane's values and have to be moved to uniform registers for
 // every instruction, ~200 cycles per MMA; in convergent code they are computed there.) The elected thread of a full warp is
 // always the same one, so commits cover the MMAs before them.
-__device__ __forceinline__ void tc_mma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                           uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, e;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// The same with the accumulate input always on: no predicate to compute in the issuing warp's instruction stream.
-__device__ __forceinline__ void tc_mma_f16_acc(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p, e;\n\t"
-      "setp.eq.u32 p, 1, 1;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc)
-      : "memory");
+// KK 16-deep MMA steps into one accumulator, `accumulate` for the first of them (the others add): descriptors in two words, of
+// which the lower one advances by a_adv / b_adv per step. One election per call, and what a step needs is one addition per
+// operand, so that the steps follow one another as fast as the tensor core takes them. PAIR: D of 256 rows, 128 TMEM lanes in
+// each CTA, A of 128 rows and B of N/2 rows per CTA; the leader's MMA warp only.
+template <int KK, bool PAIR>
+__device__ __forceinline__ void tc_mma_steps(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
+                                             uint32_t a_adv, uint32_t b_adv, uint32_t idesc, uint32_t accumulate) {
+#define RB_STEPS_HEAD(G)                                                        \
+  "{\n\t.reg .pred p, t, e;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"        \
+  "setp.ne.b32 p, %8, 0;\n\tsetp.eq.u32 t, 1, 1;\n\t"                         \
+  "elect.sync _|e, 0xffffffff;\n\t"                                            \
+  "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"                        \
+  "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], da, db, %7, p;\n\t"         \
+  "add.u32 x, %1, %5;\n\tadd.u32 y, %3, %6;\n\t"                              \
+  "mov.b64 da, {x, %2};\n\tmov.b64 db, {y, %4};\n\t"                          \
+  "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], da, db, %7, t;\n\t"
+#define RB_STEPS_NEXT(G)                                                        \
+  "add.u32 x, x, %5;\n\tadd.u32 y, y, %6;\n\t"                                \
+  "mov.b64 da, {x, %2};\n\tmov.b64 db, {y, %4};\n\t"                          \
+  "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], da, db, %7, t;\n\t"
+#define RB_STEPS_ARGS                                                                                                 \
+  ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(a_adv), "r"(b_adv), "r"(idesc), "r"(accumulate) : "memory"
+  static_assert(KK == 2 || KK == 4, "k-blocks are 32 or 64 deep");
+  if (PAIR) {
+    if (KK == 4) asm volatile(RB_STEPS_HEAD("2") RB_STEPS_NEXT("2") RB_STEPS_NEXT("2") "}" RB_STEPS_ARGS);
+    else asm volatile(RB_STEPS_HEAD("2") "}" RB_STEPS_ARGS);
+  } else {
+    if (KK == 4) asm volatile(RB_STEPS_HEAD("1") RB_STEPS_NEXT("1") RB_STEPS_NEXT("1") "}" RB_STEPS_ARGS);
+    else asm volatile(RB_STEPS_HEAD("1") "}" RB_STEPS_ARGS);
+  }
+#undef RB_STEPS_HEAD
+#undef RB_STEPS_NEXT
+#undef RB_STEPS_ARGS
 }
 // mbarrier arrives once every MMA issued so far by this warp has finished; called by the whole converged warp.
 __device__ __forceinline__ void tc_commit(uint64_t* bar) {
@@ -265,26 +291,6 @@ __device__ __forceinline__ void tmem_relinquish2() {
 }
 __device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// D (256 rows: 128 TMEM lanes in each CTA) (+)= A (128 rows per CTA) * B (N/2 rows per CTA); the leader's MMA warp only.
-__device__ __forceinline__ void tc_mma2_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, e;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void tc_mma2_f16_acc(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p, e;\n\t"
-      "setp.eq.u32 p, 1, 1;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc)
-      : "memory");
 }
 // The barrier at this shared-memory offset in BOTH CTAs of the pair arrives once the pair's MMAs issued so far
 // have finished (a commit, not a load: the only multicast in this library).
