@@ -1,6 +1,6 @@
 // Persistent, warp-specialised tcgen05 GEMM / implicit-GEMM convolution for sm_100a.
 //
-//   warp 0      A producer: TMA loads (tiled, im2col, or halo tiles) of the A operand, one lane per box
+//   warp 0      A producer: TMA loads (tiled, im2col, or whole image rows) of the A operand, one lane per box
 //   warp 1      MMA issuer (one elected lane issues): tcgen05.mma, fp32 accumulators in TMEM; owns TMEM alloc/dealloc
 //   warps 2..9  epilogue: tcgen05.ld -> bias / ReLU / mask -> swizzled smem -> TMA store (bf16), or fp32 TMA
 //               store / reduce-add (split-K, gradient accumulation). Two warps share each TMEM lane quarter and
@@ -23,14 +23,8 @@
 //     and stays resident (b_resident); split-K (fp32 reduce-add epilogue) spreads long reductions over all SMs;
 //   * which of these a forward / data-grad launch uses is decided by timing the candidates the first time a shape
 //     is seen (the launches are idempotent), see `launch`.
-//   * stride-1 convolutions can load A as column-shifted halo tiles (A_HALO_K): a sub-tile is hl_rows output rows
-//     of one image laid out at a row pitch of hl_pitch positions (128 rows of the MMA; positions past the image
-//     width or height are computed and dropped by the clipping TMA store). For filter column s the producer
-//     loads ONE tile of (mt * hl_rows + R - 1) input rows x hl_pitch columns starting at column s - pad (plain
-//     tiled TMA, zero fill outside the image); the R filter rows of that column are then descriptor offsets of
-//     r * hl_pitch rows into the same tile (multiples of the swizzle atom), so A is filled S times per item
-//     instead of R * S times. B streams through its own ring, one (r, s, channel chunk) tile per stage. Taken
-//     only when forced (RB_GEMM_FORCE_HALO=1): its padded tiles add MMA work, and MMA issue is what binds there.
+//   * stride-1 convolutions can load whole input rows once for all filter taps (A_FLAT_K, the comment at flat_geom):
+//     what binds the im2col form is that every tap brings the same pixels into shared memory again.
 // With two accumulator sets in TMEM the epilogue of work item i overlaps the main loop of item i+1; a
 // 256 x 256 item needs all 512 columns and runs without that overlap.
 //
@@ -43,9 +37,12 @@
 #include "launch.cuh"
 #include <ctype.h>
 #include <stdlib.h>
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
+#include <vector>
 
 namespace rb {
 
@@ -61,6 +58,7 @@ constexpr int GEMM_MAX_REGS = 144;
 constexpr int PRODUCER_B_WARP = 10;
 constexpr int EPI_WARPS = 8;
 constexpr int MAX_STAGES = 8;
+constexpr int MAX_A_STAGES = 3;   // flat mode
 constexpr int TILE_SMEM_BYTES = 192 * 1024;   // B panel (if resident) + stage ring
 constexpr int STAGING_BYTES = 32 * 1024;      // epilogue: 8 warps x one slab of 32 rows x 128 B
 constexpr int GEMM_SMEM_BYTES = TILE_SMEM_BYTES + STAGING_BYTES + 1024 /*align*/ + 512 /*barriers*/;
@@ -72,8 +70,8 @@ struct SharedCtl {
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t b_full;
-  uint64_t a_full[2];    // halo mode: the A ring has its own barriers
-  uint64_t a_empty[2];
+  uint64_t a_full[MAX_A_STAGES];    // flat mode: the A ring has its own barriers
+  uint64_t a_empty[MAX_A_STAGES];
   uint64_t mask_bar[EPI_WARPS];
   uint32_t tmem_base;
   volatile int abort_flag;
@@ -184,6 +182,16 @@ __device__ __forceinline__ WorkItem decode_work(const GemmTcParams& p, int work,
   return w;
 }
 
+// Flat mode: row of D (and mask, addend) that position `f` belongs to, -1 for the zero columns and rows between images.
+__device__ __forceinline__ long long flat_row(const GemmTcParams& p, int f) {
+  const int g = f / p.fl_pitch, q = f - g * p.fl_pitch;
+  const int n = g / p.fl_hp, i = g - n * p.fl_hp;
+  if (q >= p.cv_Q || i >= p.cv_P || n * p.cv_P * p.cv_Q >= p.M) return -1;
+  if (p.sc_stride)
+    return ((long long)n * p.sc_H + i * p.sc_stride + p.sc_a) * p.sc_W + q * p.sc_stride + p.sc_b;
+  return ((long long)n * p.cv_P + i) * p.cv_Q + q;
+}
+
 __device__ __forceinline__ int dgrad_tap(const GemmTcParams& p, int tap) {
   if (p.dg_dv == 0) return tap;
   const int u = tap / p.cv_S;
@@ -265,6 +273,57 @@ __device__ __forceinline__ bool issue_item(const IssueCtx& c, SharedCtl* ctl, un
   return true;
 }
 
+// Flat mode: the k-blocks of one work item, channel chunk by channel chunk. An A stage holds the chunk's input rows, so
+// filter tap (r, s) of sub-tile j is a descriptor offset of r * pitch + s positions into it: the swizzle is a function of
+// the address alone, so a tile may start at any of its rows.
+struct FlatCtx {
+  uint32_t a_ring_u32, b_ring_u32, a_stage_bytes, row_units;   // row_units: one position in 16-byte units
+  uint32_t lead_units, pitch_units, b_tap_units;               // b_tap_units: from tap to tap of the resident panel
+  int cchunks, R, S, a_stages, b_stages, b_resident;
+};
+template <int KK, int MT, bool PAIR>
+__device__ __forceinline__ bool issue_flat_item(const IssueCtx& c, const FlatCtx& f, SharedCtl* ctl, unsigned int* status,
+                                                uint32_t d_tmem, int& as, uint32_t& aph, int& bs, uint32_t& bph) {
+  bool fresh = true;
+  bool a_ready = mbar_test_wait(&ctl->a_full[as], aph);
+  bool b_ready = !f.b_resident && mbar_test_wait(&ctl->full[bs], bph);
+  for (int cc = 0; cc < f.cchunks; ++cc) {
+    if (!__all_sync(0xffffffffu, a_ready) && !ctl_wait_warp_role(ctl, &ctl->a_full[as], aph, status, 2)) return false;
+    uint32_t a_row = ((f.a_ring_u32 + (uint32_t)as * f.a_stage_bytes) >> 4) + f.lead_units;
+    uint32_t b_tap = (f.b_ring_u32 + (uint32_t)cc * c.b_bytes) >> 4;
+    uint64_t* const a_done = &ctl->a_empty[as];
+    if (++as == f.a_stages) { as = 0; aph ^= 1u; }
+    a_ready = mbar_test_wait(&ctl->a_full[as], aph);
+    for (int r = 0; r < f.R; ++r, a_row += f.pitch_units) {
+      uint32_t a_tap = a_row;
+      for (int sx = 0; sx < f.S; ++sx, a_tap += f.row_units) {
+        if (f.b_resident) {
+          tc_fence_after();
+          issue_kblock<KK, MT, false, PAIR>(d_tmem, c.acc_stride, c.a_desc0_lo | a_tap, c.a_hi, c.a_sub, c.b_desc0_lo | b_tap,
+                                            c.b_hi, c.a_adv, c.b_adv, c.idesc, c.idesc2, 0u, fresh);
+          b_tap += f.b_tap_units;
+        } else {
+          if (!__all_sync(0xffffffffu, b_ready) && !ctl_wait_warp_role(ctl, &ctl->full[bs], bph, status, 2)) return false;
+          tc_fence_after();
+          const uint32_t b_at = (f.b_ring_u32 + (uint32_t)bs * c.b_bytes) >> 4;
+          uint64_t* const done = &ctl->empty[bs];
+          if (++bs == f.b_stages) { bs = 0; bph ^= 1u; }
+          b_ready = mbar_test_wait(&ctl->full[bs], bph);
+          issue_kblock<KK, MT, false, PAIR>(d_tmem, c.acc_stride, c.a_desc0_lo | a_tap, c.a_hi, c.a_sub, c.b_desc0_lo | b_at,
+                                            c.b_hi, c.a_adv, c.b_adv, c.idesc, c.idesc2, 0u, fresh);
+          if (PAIR) tc_commit2_both(done);
+          else tc_commit(done);
+        }
+        fresh = false;
+      }
+    }
+    // every MMA that reads this A stage has been issued before this point
+    if (PAIR) tc_commit2_both(a_done);
+    else tc_commit(a_done);
+  }
+  return true;
+}
+
 // The bf16 epilogue of 32 columns of one row: packed fp32 adds for the bias, one conversion per pair,
 // ReLU and the mask of the previous layer's ReLU on the packed bf16 pair (rounding is monotone, so clamping after it gives
 // the same bits as clamping before), into 16-byte chunks of a 128-byte swizzled slab row (chunk index XOR row mod 8, the
@@ -339,7 +398,8 @@ __device__ __forceinline__ void epilogue_kinds(int kind, bool addend, const uint
 // EXT: the instantiation whose bf16 epilogue can scatter rows and take an addend. The tests for these cost the epilogue of
 // every other launch what they do not use: 1 x 1 layers, which are bound by it, ran 8 % slower with them (NIN's training
 // step at 64 images: 1255 instead of 1186 us).
-template <bool PAIR, bool EXT>
+// FLAT: the instantiation for A_FLAT_K, whose rows are always scattered (EXT).
+template <bool PAIR, bool EXT, bool FLAT>
 __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant__ GemmTcParams p) {
 #ifdef RB_GEMM_PROFILE
   const long long t_kernel0 = clock64();
@@ -367,26 +427,24 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
   uint8_t* ring = tiles + panel_bytes;
   const int stages = p.stages;
 
-  const bool halo = p.a_mode == A_HALO_K;
-  const bool box = p.a_mode == A_BOX_K;
+  const bool box = !FLAT && p.a_mode == A_BOX_K;
   const int bx_groups = box ? (p.cv_P + mt * p.bx_rows - 1) / (mt * p.bx_rows) : 1;   // work items per image
-  const int m_units = halo  ? (p.M / (p.cv_P * p.cv_Q)) * p.hl_groups
+  const int m_units = FLAT  ? (p.fl_units + mt - 1) / mt
                       : box ? (p.M / (p.cv_P * p.cv_Q)) * bx_groups
                             : (p.M + BM * mt - 1) / (BM * mt);
   const int m_items = pair ? (m_units + 1) >> 1 : m_units;   // a pair's item is two CTA-sized units
   const int n_tiles = p.n_tiles;
-  // whole items first, then the parts of the cut items of the last wave (tail cut; never in halo mode)
+  // whole items first, then the parts of the cut items of the last wave (tail cut; never in flat mode)
   const int direct = m_items * n_tiles - p.tail_items;
   const int num_work = p.tail_items > 0 ? direct + p.tail_items * p.tail_split : m_items * n_tiles * p.split_k;
-  // halo mode: [A ring: hl_a_stages x hl_a_bytes][B ring: stages x b_bytes]
-  uint8_t* a_ring = tiles;
-  uint8_t* b_ring = tiles + p.hl_a_stages * p.hl_a_bytes;
+  // flat mode: [A ring: fl_a_stages x fl_a_bytes][B ring: stages x b_bytes, or the resident panel]
+  uint8_t* const b_ring = FLAT ? tiles + p.fl_a_stages * p.fl_a_bytes : tiles;
   const int kb_per_split = (p.num_kb + p.split_k - 1) / p.split_k;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) {
       // one arrival per producer warp that fills it (a pair: both CTAs' producers arrive on the leader's barrier)
-      mbar_init(&ctl->full[s], pair ? 4 : ((halo || p.b_resident) ? 1 : 2));
+      mbar_init(&ctl->full[s], FLAT ? (pair ? 2 : 1) : pair ? 4 : (p.b_resident ? 1 : 2));
       mbar_init(&ctl->empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -394,8 +452,8 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       mbar_init(&ctl->acc_empty[a], pair ? 2 * EPI_WARPS : EPI_WARPS);
     }
     mbar_init(&ctl->b_full, 1);
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(&ctl->a_full[a], 1);
+    for (int a = 0; FLAT && a < MAX_A_STAGES; ++a) {
+      mbar_init(&ctl->a_full[a], pair ? 2 : 1);
       mbar_init(&ctl->a_empty[a], 1);
     }
     for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&ctl->mask_bar[w], 1);
@@ -453,51 +511,82 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
     int s = 0, issued = 0;
     uint32_t ph = 0;
     bool ok = true;
-    if (halo) {
-      const uint32_t a_tx = (uint32_t)(p.hl_rtot * p.hl_pitch * p.bk * 2);
-      const int nst = is_a ? p.hl_a_stages : stages;
-      uint64_t* fullb = is_a ? ctl->a_full : ctl->full;
-      uint64_t* emptyb = is_a ? ctl->a_empty : ctl->empty;
-      ahead_done();
-      if (lane == 0) {
-        for (int work = cta_id; work < num_work && ok; work += cta_step) {
-          const int tn = work / m_items;
-          const int tm = work - tn * m_items;
-          const int n_img = tm / p.hl_groups;
-          const int p0 = (tm - n_img * p.hl_groups) * mt * p.hl_rows;
-          const int n0 = tn * p.bn;
-          for (int sx = 0; sx < p.cv_S && ok; ++sx) {
-            for (int cc = 0; cc < p.cv_cchunks && ok; ++cc) {
-              if (is_a) {
-                if (!ctl_wait(ctl, &emptyb[s], ph ^ 1u, p.status)) { ok = false; break; }
-                mbar_expect_tx(&fullb[s], a_tx);
-                tma_load_4d(a_ring + s * p.hl_a_bytes, &p.tm_a, &fullb[s], cc * p.bk, sx - p.hl_pad_w,
-                            p0 - p.hl_pad_h, n_img);
-                ++issued;
-                if (++s == nst) { s = 0; ph ^= 1u; }
-              } else {
-                for (int r = 0; r < p.hl_R; ++r) {
-                  if (!ctl_wait(ctl, &emptyb[s], ph ^ 1u, p.status)) { ok = false; break; }
-                  mbar_expect_tx(&fullb[s], (uint32_t)b_bytes);
-                  tma_load_3d(b_ring + s * b_bytes, &p.tm_b, &fullb[s], cc * p.bk, r * p.cv_S + sx, n0);
-                  ++issued;
-                  if (++s == nst) { s = 0; ph ^= 1u; }
-                }
-              }
-            }
+    if (FLAT && (is_a || !p.b_resident)) {
+      // A: a stage is the fl_rows input rows of one channel chunk, one lane per row, every one fl_pitch positions of which
+      // those outside the image arrive as zeros. B: one (tap, channel chunk) tile per stage, one lane per box.
+      const int nst = is_a ? p.fl_a_stages : stages;
+      uint64_t* const fullb = is_a ? ctl->a_full : ctl->full;
+      uint64_t* const emptyb = is_a ? ctl->a_empty : ctl->empty;
+      const uint32_t full0_leader = pair ? mapa_shared(smem_u32(fullb), 0u) : 0u;
+      const int row_bytes = p.bk * 2;
+      const uint32_t tx = is_a ? (uint32_t)(p.fl_rows * p.fl_pitch * row_bytes) : (uint32_t)b_bytes;
+      const bool mn = p.b_mode == B_DGRAD_MN;
+      const int b_split = p.b_split > 0 ? p.b_split : 1, b_rows = p.bn_load / b_split;
+      const int nload = is_a ? p.fl_rows : (mn ? p.bn_load / 64 : b_split);
+      auto claim = [&]() -> bool {   // wait for a free stage and announce its bytes
+        int w_ok = 1;
+        if (lane == 0) {
+          w_ok = ctl_wait_role(ctl, &emptyb[s], ph ^ 1u, p.status, is_a ? 0 : 1) ? 1 : 0;
+          if (w_ok) {
+            if (pair) mbar_expect_tx_cluster(full0_leader + (uint32_t)s * 8u, tx);
+            else mbar_expect_tx(&fullb[s], tx);
           }
         }
-        if (!ok) {
-          // drain: wait (bounded) until the copies already issued have landed
-          const int back = min(issued, nst);
-          for (int i = 0; i < back; ++i) {
-            if (s == 0) { s = nst; ph ^= 1u; }
-            --s;
-            mbar_wait_bounded(&fullb[s], ph, 100000000ull);
+        return __shfl_sync(0xffffffffu, w_ok, 0) != 0;
+      };
+      for (int work = cta_id; work < num_work && ok; work += cta_step) {
+        const int tn = work / m_items;
+        const int tm = (work - tn * m_items) * (pair ? 2 : 1) + (int)cta_rank;
+        const int n0 = tn * p.bn + (pair ? (int)cta_rank * p.bn_load : 0);
+        const int f0 = tm * mt * p.fl_step;
+        const int g0 = f0 / p.fl_pitch;
+        // the item's first position always lies at fl_lead, whatever its column: both CTAs of a pair use one descriptor
+        uint8_t* const row0 = tiles + (p.fl_lead - (f0 - g0 * p.fl_pitch)) * row_bytes;
+        for (int cc = 0; cc < p.cv_cchunks && ok; ++cc) {
+          if (is_a) {
+            if (!claim()) { ok = false; break; }
+            ahead_done();
+            for (int i = lane; i < nload; i += 32) {
+              const int g = g0 + i, n = g / p.fl_hp, h = g - n * p.fl_hp - p.fl_pad_h;
+              uint8_t* to = row0 + s * p.fl_a_bytes + i * p.fl_pitch * row_bytes;
+              if (pair) tma2_load_4d(to, &p.tm_a, full0_leader + (uint32_t)s * 8u, cc * p.bk, -p.fl_pad_w, h, n);
+              else tma_load_4d(to, &p.tm_a, &fullb[s], cc * p.bk, -p.fl_pad_w, h, n);
+            }
+            __syncwarp();
+            ++issued;
+            if (++s == nst) { s = 0; ph ^= 1u; }
+            continue;
           }
+          for (int r = 0; r < p.fl_R && ok; ++r)
+            for (int sx = 0; sx < p.cv_S; ++sx) {
+              if (!claim()) { ok = false; break; }
+              ahead_done();
+              if (lane < nload) {
+                const int wtap = p.dg_dv == 0 ? r * p.cv_S + sx : p.dg_base + r * p.dg_du + sx * p.dg_dv;
+                const int c0 = mn ? n0 + 64 * lane : cc * p.bk, c2 = mn ? cc * p.bk : n0 + lane * b_rows;
+                uint8_t* to = b_ring + s * b_bytes + lane * (mn ? p.bk * 128 : b_rows * row_bytes);
+                if (pair) tma2_load_3d(to, &p.tm_b, full0_leader + (uint32_t)s * 8u, c0, wtap, c2);
+                else tma_load_3d(to, &p.tm_b, &fullb[s], c0, wtap, c2);
+              }
+              __syncwarp();
+              ++issued;
+              if (++s == nst) { s = 0; ph ^= 1u; }
+            }
         }
       }
-    } else if (is_a || !p.b_resident) {
+      if (!ok && lane == 0 && pair && cta_rank != 0) {
+        const uint64_t t0 = globaltimer_ns();   // as below
+        while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+      } else if (!ok && lane == 0) {
+        // drain: wait (bounded) until the copies already issued have landed
+        const int back = min(issued, nst);
+        for (int i = 0; i < back; ++i) {
+          if (s == 0) { s = nst; ph ^= 1u; }
+          --s;
+          mbar_wait_bounded(&fullb[s], ph, 100000000ull);
+        }
+      }
+    } else if (!FLAT && (is_a || !p.b_resident)) {
       // Loads this warp issues per stage, one lane each. What a lane's load needs is worked out once per launch (where in a
       // stage it goes) or per work item (its pixel, tap or column), and carried from k-block to k-block by additions: with
       // the divisions by run-time values that the coordinates otherwise take, a k-block cost the warp ~1200 cycles.
@@ -678,7 +767,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
         if (lane == 0) mbar_expect_tx(&ctl->b_full, (uint32_t)panel_bytes);
         __syncwarp();
         ahead_done();
-        for (int kb = lane; kb < p.num_kb; kb += 32) load_b(p, tiles + kb * b_bytes, &ctl->b_full, kb, 0);
+        for (int kb = lane; kb < p.num_kb; kb += 32) load_b(p, b_ring + kb * b_bytes, &ctl->b_full, kb, 0);
       }
     }
   } else if (warp == 1) {
@@ -711,50 +800,6 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       uint32_t acc_ph = 0;
       bool ok = true;
       if (p.b_resident && blockIdx.x < num_work) ok = ctl_wait_warp(ctl, &ctl->b_full, 0u, p.status);
-      if (halo) {
-        int bs = 0, as = 0;
-        uint32_t bph = 0, aph = 0;
-        const uint32_t row_bytes = (uint32_t)p.bk * 2u;
-        for (int work = cta_id; work < num_work && ok; work += cta_step) {
-          if (!ctl_wait_warp(ctl, &ctl->acc_empty[acc], acc_ph ^ 1u, p.status)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t d_tmem = tmem_base + (uint32_t)acc * set_cols;
-          bool fresh = true;   // the first MMA into each accumulator overwrites it
-          for (int sx = 0; sx < p.cv_S && ok; ++sx) {
-            for (int cc = 0; cc < p.cv_cchunks && ok; ++cc) {
-              if (!ctl_wait_warp(ctl, &ctl->a_full[as], aph, p.status)) { ok = false; break; }
-              tc_fence_after();
-              const uint32_t a_base = smem_u32(a_ring + as * p.hl_a_bytes);
-              for (int r = 0; r < p.hl_R; ++r) {
-                if (!ctl_wait_warp(ctl, &ctl->full[bs], bph, p.status)) { ok = false; break; }
-                tc_fence_after();
-                const uint64_t db = make_smem_desc(smem_u32(b_ring + bs * b_bytes), b_lbo, b_sbo, b_lay);
-                for (int j = 0; j < mt; ++j) {
-                  // filter row r of sub-tile j: the same tile, (j * hl_rows + r) * hl_pitch rows further down
-                  const uint32_t off = (uint32_t)((j * p.hl_rows + r) * p.hl_pitch) * row_bytes;
-                  const uint64_t da = make_smem_desc(a_base + off, a_lbo, a_sbo, a_lay);
-                  const uint32_t dj = d_tmem + (uint32_t)(j * p.acc_stride);
-                  if (kk_steps == 4)
-                    tc_mma_steps<4, false>(dj, (uint32_t)da, (uint32_t)(da >> 32), (uint32_t)db, (uint32_t)(db >> 32), a_adv,
-                                           b_adv, idesc, fresh ? 0u : 1u);
-                  else
-                    tc_mma_steps<2, false>(dj, (uint32_t)da, (uint32_t)(da >> 32), (uint32_t)db, (uint32_t)(db >> 32), a_adv,
-                                           b_adv, idesc, fresh ? 0u : 1u);
-                }
-                fresh = false;
-                tc_commit(&ctl->empty[bs]);
-                if (++bs == stages) { bs = 0; bph ^= 1u; }
-              }
-              if (!ok) break;
-              tc_commit(&ctl->a_empty[as]);   // every MMA that reads this A tile has been issued before this point
-              if (++as == p.hl_a_stages) { as = 0; aph ^= 1u; }
-            }
-          }
-          if (!ok) break;
-          tc_commit(&ctl->acc_full[acc]);
-          if (++acc == p.acc_bufs) { acc = 0; acc_ph ^= 1u; }
-        }
-      }
       // what the unrolled issue code needs, fixed for the launch
       IssueCtx ic;
       ic.ring_u32 = smem_u32(ring);
@@ -772,12 +817,50 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
       ic.a_hi = (uint32_t)(a_desc0 >> 32);
       ic.b_desc0_lo = (uint32_t)b_desc0;
       ic.b_hi = (uint32_t)(b_desc0 >> 32);
-      ic.a_sub = (uint32_t)a_bytes >> 4;     // next 128-row sub-tile of the stage
+      ic.a_sub = (uint32_t)(FLAT ? p.fl_step * p.bk * 2 : a_bytes) >> 4;     // next sub-tile of the stage
       ic.b_wide_off = b_wide_off;
       ic.stages = stages;
       ic.b_resident = p.b_resident;
+      if (FLAT) {
+        FlatCtx fc;
+        fc.a_ring_u32 = smem_u32(tiles);
+        fc.b_ring_u32 = smem_u32(b_ring);
+        fc.a_stage_bytes = (uint32_t)p.fl_a_bytes;
+        fc.row_units = (uint32_t)(p.bk * 2) >> 4;
+        fc.lead_units = (uint32_t)p.fl_lead * fc.row_units;
+        fc.pitch_units = (uint32_t)p.fl_pitch * fc.row_units;
+        fc.b_tap_units = (uint32_t)(p.cv_cchunks * b_bytes) >> 4;
+        fc.cchunks = p.cv_cchunks;
+        fc.R = p.fl_R;
+        fc.S = p.cv_S;
+        fc.a_stages = p.fl_a_stages;
+        fc.b_stages = stages;
+        fc.b_resident = p.b_resident;
+        int as = 0;
+        uint32_t aph = 0;
+        const int kind = (kk_steps == 4 ? 0 : 4) + mt;
+        for (int work = cta_id; work < num_work && ok; work += cta_step) {
+          if (!ctl_wait_warp_role(ctl, &ctl->acc_empty[acc], acc_ph ^ 1u, p.status, 3)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + (uint32_t)acc * set_cols;
+          switch (kind) {
+            case 1: ok = issue_flat_item<4, 1, PAIR>(ic, fc, ctl, p.status, d_tmem, as, aph, s, ph); break;
+            case 2: ok = issue_flat_item<4, 2, PAIR>(ic, fc, ctl, p.status, d_tmem, as, aph, s, ph); break;
+            case 3: ok = issue_flat_item<4, 3, PAIR>(ic, fc, ctl, p.status, d_tmem, as, aph, s, ph); break;
+            case 4: ok = issue_flat_item<4, 4, PAIR>(ic, fc, ctl, p.status, d_tmem, as, aph, s, ph); break;
+            case 5: ok = issue_flat_item<2, 1, PAIR>(ic, fc, ctl, p.status, d_tmem, as, aph, s, ph); break;
+            case 6: ok = issue_flat_item<2, 2, PAIR>(ic, fc, ctl, p.status, d_tmem, as, aph, s, ph); break;
+            case 7: ok = issue_flat_item<2, 3, PAIR>(ic, fc, ctl, p.status, d_tmem, as, aph, s, ph); break;
+            default: ok = issue_flat_item<2, 4, PAIR>(ic, fc, ctl, p.status, d_tmem, as, aph, s, ph); break;
+          }
+          if (!ok) break;
+          if (pair) tc_commit2_both(&ctl->acc_full[acc]);
+          else tc_commit(&ctl->acc_full[acc]);
+          if (++acc == p.acc_bufs) { acc = 0; acc_ph ^= 1u; }
+        }
+      }
       const int issue_kind = (kk_steps == 4 ? 0 : 3) + (idesc2 ? 2 : (mt == 2 ? 1 : 0));
-      for (int work = cta_id; work < num_work && ok && !halo; work += cta_step) {
+      for (int work = cta_id; work < num_work && ok && !FLAT; work += cta_step) {
         const WorkItem it = decode_work(p, work, m_items, direct, kb_per_split);
         if (!ctl_wait_warp_role(ctl, &ctl->acc_empty[acc], acc_ph ^ 1u, p.status, 3)) { ok = false; break; }
         tc_fence_after();
@@ -843,14 +926,6 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
         col_limit = min(p.bn, p.n_store - col0);
       }
       for (int j = 0; j < mt; ++j) {
-        // halo mode: this warp's 32-row band is (32 / pitch) output rows of one image, or a 32-wide piece of one
-        int h_n = 0, h_p = 0, h_w = 0;
-        if (halo) {
-          h_n = tm / p.hl_groups;
-          h_p = ((tm - h_n * p.hl_groups) * mt + j) * p.hl_rows + lane_base / p.hl_pitch;
-          h_w = lane_base % p.hl_pitch;
-          if (h_p >= p.cv_P || h_w >= p.cv_Q) continue;   // the whole band lies outside the image
-        }
         int row0 = tm * BM * mt + j * BM + lane_base;   // first row of this warp's 32-row band
         int band_rows = 32;                             // rows of the band that belong to this tile
         if (box) {
@@ -867,10 +942,11 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
             tmem_base + (uint32_t)acc * set_cols + (uint32_t)(j * p.acc_stride) + ((uint32_t)lane_base << 16);
         if (p.epi == EPI_BF16 && !tail) {
           // row of D that this lane's row belongs to (-1: none); only scattered rows and an addend need it
-          const bool scatter = EXT && p.sc_stride != 0;
+          const bool scatter = FLAT || (EXT && p.sc_stride != 0);
           const bool addend = EXT && p.add_src != nullptr;
           long long drow_of = -1;
-          if ((scatter || addend) && lane < band_rows && row0 + lane < p.M)
+          if (FLAT) drow_of = flat_row(p, (tm * mt + j) * p.fl_step + lane_base + lane);
+          else if ((scatter || addend) && lane < band_rows && row0 + lane < p.M)
             drow_of = scatter ? scatter_row(row0 + lane, p.cv_P, p.cv_Q, p.sc_stride, p.sc_a, p.sc_b, p.sc_H, p.sc_W)
                               : (long long)(row0 + lane);
           // 64-column slabs: TMEM -> registers -> bias / ReLU / mask -> swizzled shared memory -> TMA store.
@@ -899,8 +975,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
               // is copied to registers, and the buffer is then reused for the output
               if (lane == 0) {
                 mbar_expect_tx(mbar_m, 4096u);
-                if (halo) tma_load_4d(buf, &p.tm_mask, mbar_m, gcol, h_w, h_p, h_n);
-                else tma_load_2d(buf, &p.tm_mask, mbar_m, gcol, row0);
+                tma_load_2d(buf, &p.tm_mask, mbar_m, gcol, row0);
               }
               if (!mbar_wait_bounded(mbar_m, mask_ph, WAIT_LIMIT_NS)) {
                 ctl->abort_flag = 1;
@@ -972,8 +1047,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
               __syncwarp();
               if (lane == 0) tma_store_commit();
             } else if (lane == 0) {
-              if (halo) tma_store_4d(&p.tm_d, buf, gcol, h_w, h_p, h_n);
-              else if (row0 < p.M) tma_store_2d(&p.tm_d, buf, gcol, row0);
+              if (row0 < p.M) tma_store_2d(&p.tm_d, buf, gcol, row0);
               tma_store_commit();
             }
 #ifdef RB_GEMM_PROFILE
@@ -1075,8 +1149,9 @@ static int ensure_driver_entry() {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDriverGetVersion(&g_driver_version);
-  for (auto kern : {gemm_tc_kernel<false, false>, gemm_tc_kernel<true, false>, gemm_tc_kernel<false, true>,
-                    gemm_tc_kernel<true, true>})
+  for (auto kern : {gemm_tc_kernel<false, false, false>, gemm_tc_kernel<true, false, false>,
+                    gemm_tc_kernel<false, true, false>, gemm_tc_kernel<true, true, false>, gemm_tc_kernel<false, true, true>,
+                    gemm_tc_kernel<true, true, true>})
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) != cudaSuccess) return -2;
   {   // how many CTA pairs fit at once: the persistent loop of pair mode runs exactly that many clusters
     cudaLaunchConfig_t cfg;
@@ -1092,7 +1167,7 @@ static int ensure_driver_entry() {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, gemm_tc_kernel<true, true>, &cfg) != cudaSuccess) nc = 0;
+    if (cudaOccupancyMaxActiveClusters(&nc, gemm_tc_kernel<true, true, true>, &cfg) != cudaSuccess) nc = 0;
     cudaGetLastError();   // a refused query must not be taken for a failed launch later
     g_pair_clusters = nc > g_num_sms / 2 ? g_num_sms / 2 : nc;
   }
@@ -1180,7 +1255,7 @@ static int make_map_nhwc(CUtensorMap* m, const void* ptr, uint64_t C, uint64_t W
 struct GemmOptions {
   int force_mt = 0;          // RB_GEMM_FORCE_MT: 1 | 2 sub-tiles per item (0 = planner's choice)
   int force_resident = -1;   // RB_GEMM_FORCE_RESIDENT: 0 | 1
-  int force_halo = -1;       // RB_GEMM_FORCE_HALO: 0 = never, 1 = whenever feasible
+  int force_halo = -1;       // RB_GEMM_FORCE_HALO: whole input rows for all taps (flat mode): 0 = never, 1 = whenever feasible
   int force_taps = 0;        // RB_GEMM_FORCE_TAPS: filter taps per weight-grad tile
   int force_tail = -1;       // RB_GEMM_FORCE_TAIL: 0 = never cut the last wave, 1 = whenever feasible
   int force_wide = -1;       // RB_GEMM_FORCE_WIDE: 0 = tiles of at most 256 columns, 1 = one wide tile when N <= 512
@@ -1248,7 +1323,7 @@ struct Plan {
 // boxes of the B map (the map's box is bn / b_split rows, so b_split must be even), and more than one pair's rows.
 static bool pair_ok(const GemmTcParams& p) {
   if (g_opt.force_pair == 0 || g_pair_clusters <= 0) return false;
-  if (p.a_mode != A_TILED_K && p.a_mode != A_IM2COL_K) return false;
+  if (p.a_mode != A_TILED_K && p.a_mode != A_IM2COL_K && p.a_mode != A_FLAT_K) return false;
   if (p.b_mode == B_DGRAD_MN) {
     if (p.bn > 256 || p.bn % 128 != 0) return false;   // each CTA loads whole 64-column blocks
     return p.M > 2 * BM;
@@ -1286,7 +1361,7 @@ static int m_items_of(const GemmTcParams& p, int mt) {
     const int groups = (p.cv_P + mt * p.bx_rows - 1) / (mt * p.bx_rows);
     return (p.M / (p.cv_P * p.cv_Q)) * groups;
   }
-  const int units = (p.M + BM * mt - 1) / (BM * mt);
+  const int units = p.a_mode == A_FLAT_K ? (p.fl_units + mt - 1) / mt : (p.M + BM * mt - 1) / (BM * mt);
   return p.pair ? (units + 1) / 2 : units;
 }
 
@@ -1303,7 +1378,136 @@ static int tail_parts(long long items, int sms, int num_kb) {
   return s >= 2 ? s : 0;
 }
 
+// ---- flat mode -----------------------------------------------------------------------------------------------
+// A stride-1 convolution over rows of positions: every image row is fl_pitch positions long (the output row plus the zero
+// columns that the filter reaches, those at a row's end shared with the next row's beginning), every image fl_hp rows
+// (likewise), and all of them lie one after the other. Output position f then reads positions f + r * pitch + s, for every
+// filter tap (r, s) at the same distance, so one copy of the rows in shared memory serves all R * S taps of a channel chunk:
+// a tap is an offset in the A descriptor. What lies on zero columns and rows is computed and not stored (19 x 19: 11 %,
+// 13 x 13: 16 %, 32 x 32: 6 %, 56 x 56: 4 %).
+// Why: loaded tap by tap, a 128-row tile takes R * S x 16 KB per chunk from the L2, which delivers ~41 bytes per cycle and
+// SM: 128 -> 128 channels at two sub-tiles per item ask for 94, so the tensor pipe was 40 % busy; this asks for 25 to 41.
+// 96 -> 256 on 128 x 27 x 27, 5 x 5: data-gradient 115 -> 89 us; 256 -> 384 on 128 x 13 x 13: 42 -> 35; 16 -> 16 on
+// 128 x 32 x 32: 19.6 -> 16.2; 64 -> 128 on 64 x 128 x 128: data-gradient 205 -> 187.
+// Sub-tiles start 128 positions apart, or, on rows of at least 128 positions with at most 128 outputs, one row apart.
+static bool flat_geom(GemmTcParams& p, int N, int H, int W, int R, int S, int pad_h, int pad_w) {
+  const int P = p.cv_P, Q = p.cv_Q;
+  const int share_w = std::max(0, std::min({pad_w, S - 1, Q + S - 1 - pad_w - W}));
+  const int share_h = std::max(0, std::min({pad_h, R - 1, P + R - 1 - pad_h - H}));
+  p.fl_pitch = Q + S - 1 - share_w;
+  if (p.bk == 32) p.fl_pitch = (p.fl_pitch + 1) / 2 * 2;   // rows of 64-byte positions have to start on 128 bytes
+  if (p.fl_pitch > 112 && p.fl_pitch < BM) p.fl_pitch = BM;   // a sub-tile per row: whole-row items need no rows in between
+  p.fl_hp = P + R - 1 - share_h;
+  const bool by_rows = p.fl_pitch >= BM && Q <= BM;
+  p.fl_step = by_rows ? p.fl_pitch : BM;
+  const long long rows = (long long)N * p.fl_hp - (p.fl_hp - P);
+  const long long positions = rows * p.fl_pitch;
+  if (p.fl_pitch > 256 || pad_h < 0 || pad_w < 0 || positions > (1ll << 30)) return false;   // a box has at most 256 columns
+  p.fl_units = (int)(by_rows ? rows : (positions + BM - 1) / BM);
+  p.fl_R = R;
+  p.fl_pad_h = pad_h;
+  p.fl_pad_w = pad_w;
+  return true;
+}
+
+static int gcd_of(int a, int b) { return b == 0 ? a : gcd_of(b, a % b); }
+
+// Input rows and bytes of an A stage for `mt` sub-tiles per item.
+static void flat_stage(GemmTcParams& p, int mt) {
+  const int pitch = p.fl_pitch, row_bytes = p.bk * 2;
+  const bool by_rows = p.fl_step != BM, shared = pitch < p.cv_Q + p.cv_S - 1;
+  const int off_max = by_rows ? 0 : pitch - gcd_of(pitch, mt * p.fl_step);     // column of an item's first position
+  const int last = off_max + (mt - 1) * p.fl_step + (by_rows ? p.cv_Q : BM) - 1 + (shared ? p.cv_S - 1 : 0);
+  p.fl_rows = last / pitch + p.fl_R;
+  p.fl_lead = off_max;
+  const int loaded = p.fl_lead + p.fl_rows * pitch;
+  const int read = p.fl_lead + (mt - 1) * p.fl_step + BM + (p.fl_R - 1) * pitch + p.cv_S - 1;
+  p.fl_a_bytes = (std::max(loaded, read) * row_bytes + 1023) / 1024 * 1024;
+}
+
+// Fill in what follows from a plan; returns the grid size, or 0 when the plan does not fit.
+static int apply_flat_plan(GemmTcParams& p, const Plan& pl) {
+  if (pl.tail || pl.split != 1 || p.bn > 256 || pl.mt < 1 || pl.mt > 4) return 0;
+  if (p.fl_units < pl.mt) return 0;
+  p.mt = pl.mt;
+  p.split_k = 1;
+  p.b_resident = pl.resident;
+  if (pl.pair) {
+    if (!pair_ok(p) || pl.resident || p.fl_units <= pl.mt) return 0;
+    p.pair = 1;
+    p.bn_load = p.bn / 2;
+    if (p.b_mode != B_DGRAD_MN) p.b_split = p.b_split / 2;
+  }
+  p.acc_stride = 32;
+  while (p.acc_stride < p.bn) p.acc_stride *= 2;
+  if (p.mt * p.acc_stride > 512) return 0;
+  p.acc_bufs = 2 * p.mt * p.acc_stride <= 512 ? 2 : 1;
+  flat_stage(p, p.mt);
+  const int b_bytes = p.bn_load * p.bk * 2;
+  p.fl_a_stages = 2;
+  const int room = TILE_SMEM_BYTES - p.fl_a_stages * p.fl_a_bytes;
+  if (p.b_resident) {
+    if (p.n_tiles != 1 || room < p.num_kb * b_bytes) return 0;
+    p.stages = 2;                       // unused
+    if (room >= p.num_kb * b_bytes + p.fl_a_bytes) p.fl_a_stages = 3;
+  } else {
+    if (room < 2 * b_bytes) return 0;
+    p.stages = std::min(room / b_bytes, MAX_STAGES);
+  }
+  p.epi_bufs = 1;
+  p.tail_items = p.tail_split = 0;
+  const long long work = (long long)m_items_of(p, p.mt) * p.n_tiles;
+  if (p.pair) return 2 * (int)std::min<long long>(work, g_pair_clusters);
+  return (int)std::min<long long>(work, g_num_sms);
+}
+
+// Cycles of a launch, to rank plans by: MMA time (a 128 x N x 16 step takes N / 2 cycles, or what its operands take at 128
+// bytes per cycle from shared memory), L2 delivery (41 bytes per cycle and SM), ~150 cycles per k-block for the issuing warp,
+// an epilogue of ~900 cycles per 32 x 64 slab and warp, overlapped when there are two accumulator sets.
+static double flat_cost(const GemmTcParams& p, int grid) {
+  const double steps = (double)p.num_kb * (p.bk / 16) * p.mt;
+  const double step = std::max(p.bn / 2.0, 32.0 + (p.pair ? p.bn / 8.0 : p.bn / 4.0));
+  const double bytes = (double)p.cv_cchunks * p.fl_rows * p.fl_pitch * p.bk * 2 +
+                       (p.b_resident ? 0.0 : (double)p.num_kb * p.bn_load * p.bk * 2);
+  const double loop = std::max(steps * step, bytes / 41.0) + p.num_kb * (p.b_resident ? 60.0 : 150.0);
+  const double epi = p.mt * ((p.bn + 63) / 64) * 0.5 * 900.0;
+  const double item = p.acc_bufs == 2 ? std::max(loop, epi) + 200.0 : loop + epi + 600.0;
+  const long long work = (long long)m_items_of(p, p.mt) * p.n_tiles;
+  const long long ctas = p.pair ? grid / 2 : grid;
+  return (double)((work + ctas - 1) / ctas) * item + (p.acc_bufs == 2 ? epi : 0.0);
+}
+
+// The plans that fit, best first by flat_cost; returns how many.
+static int flat_plans(const GemmTcParams& p, Plan* out, int max_plans) {
+  int n = 0;
+  for (int pass = 0; pass < 2 && n == 0; ++pass)   // the force options restrict the search (ignored when infeasible)
+  for (int mt = 1; mt <= 4; ++mt) {
+    if (pass == 0 && g_opt.force_mt && mt != g_opt.force_mt) continue;
+    for (int kind = 0; kind < 3; ++kind) {
+      Plan pl{mt, 1, kind == 1, 0, 0.0};
+      pl.pair = kind == 2;
+      if (pass == 0 && g_opt.force_resident >= 0 && pl.resident != g_opt.force_resident) continue;
+      GemmTcParams q = p;
+      const int grid = apply_flat_plan(q, pl);
+      if (grid <= 0) continue;
+      pl.cost = flat_cost(q, grid);
+      int at = std::min(n, max_plans);
+      while (at > 0 && out[at - 1].cost > pl.cost) --at;
+      if (at == max_plans) continue;
+      n = std::min(n + 1, max_plans);
+      for (int i = n - 1; i > at; --i) out[i] = out[i - 1];
+      out[at] = pl;
+    }
+  }
+  return n;
+}
+
 static Plan plan_shape(const GemmTcParams& p, bool allow_split, int fixed_split, bool b_is_weights) {
+  if (p.a_mode == A_FLAT_K) {
+    Plan best{1, 1, 0, 0, 1e300};
+    flat_plans(p, &best, 1);
+    return best;
+  }
   if (g_opt.deterministic) {   // one CTA per output tile, its k-blocks in order
     allow_split = false;
     fixed_split = 1;
@@ -1367,6 +1571,7 @@ static Plan plan_shape(const GemmTcParams& p, bool allow_split, int fixed_split,
 
 // Fill in what follows from a plan; returns the grid size, or 0 when the plan does not fit.
 static int apply_plan(GemmTcParams& p, const Plan& pl) {
+  if (p.a_mode == A_FLAT_K) return apply_flat_plan(p, pl);
   p.mt = pl.mt;
   p.split_k = pl.split;
   p.b_resident = pl.resident;
@@ -1547,9 +1752,12 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
     cfg.attrs = n_at ? at : nullptr;
     cfg.numAttrs = (unsigned)n_at;
     const bool ext = p.sc_stride != 0 || p.add_src != nullptr;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, p.pair ? (ext ? gemm_tc_kernel<true, true> : gemm_tc_kernel<true, false>)
-                                                          : (ext ? gemm_tc_kernel<false, true> : gemm_tc_kernel<false, false>),
-                                             p);
+    const cudaError_t e = cudaLaunchKernelEx(
+        &cfg,
+        p.a_mode == A_FLAT_K ? (p.pair ? gemm_tc_kernel<true, true, true> : gemm_tc_kernel<false, true, true>)
+        : p.pair             ? (ext ? gemm_tc_kernel<true, true, false> : gemm_tc_kernel<true, false, false>)
+                             : (ext ? gemm_tc_kernel<false, true, false> : gemm_tc_kernel<false, false, false>),
+        p);
     if (e != cudaSuccess) {
       g_last_cuda_error = (int)e;
       cudaGetLastError();
@@ -1614,11 +1822,13 @@ static PlanKey plan_key(const GemmTcParams& p) {
 
 // Times the candidates of `p` (3 launches each, best of the last 2); returns the best time in ms, or a negative
 // value when nothing could be run.
-static float tune_plan(const GemmTcParams& p, bool b_is_weights, cudaStream_t stream, Plan* out) {
-  // the candidates: plain plans first (sub-tiles x resident B x tail cut), then CTA pairs
+static float tune_plan(const GemmTcParams& p, bool b_is_weights, cudaStream_t stream, Plan* out,
+                       const Plan* given = nullptr) {
+  // the candidates: the one given, or plain plans first (sub-tiles x resident B x tail cut), then CTA pairs
   Plan cands[12];
   int n_cands = 0;
-  for (int pr = 0; pr <= (pair_ok(p) ? 1 : 0); ++pr) {
+  if (given) cands[n_cands++] = *given;
+  for (int pr = 0; pr <= (pair_ok(p) ? 1 : 0) && !given; ++pr) {
     for (int mt = 1; mt <= 2; ++mt) {
       for (int res = 0; res <= (pr ? 0 : 1); ++res) {
         if (res && (!b_is_weights || p.n_tiles != 1)) continue;
@@ -1655,7 +1865,7 @@ static float tune_plan(const GemmTcParams& p, bool b_is_weights, cudaStream_t st
     }
     // pairs are timed after every plain plan and must win by 3 %: measured alone they tie to within 2 % on the
     // layers tried, and inside a training step (other kernels beside them) the plain plans did better
-    if (ok && ms < best_ms * (cands[c].pair ? 0.97f : 1.0f)) {
+    if (ok && ms < best_ms * (cands[c].pair && !given ? 0.97f : 1.0f)) {
       best_ms = ms;
       *out = cands[c];
     }
@@ -1888,64 +2098,6 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   p.bias = bias;
   p.mask_src = reinterpret_cast<const __nv_bfloat16*>(mask_src);
   p.status = status;
-  // ---- halo mode (see the header comment): stride 1, more than one filter tap, image no wider than 128
-  {
-    const int force = g_opt.force_halo;   // 0 = never, 1 = whenever feasible
-    if (stride == 1 && R * S > 1 && Q <= 128 && force != 0 && !dg) {
-      int pitch = 8;
-      while (pitch < Q) pitch *= 2;
-      const int rows = 128 / pitch;
-      const int mt = P > rows ? 2 : 1;
-      const int groups = (P + mt * rows - 1) / (mt * rows);
-      const double util = ((double)Q / pitch) * ((double)P / (groups * mt * rows));
-      // one column tile when it fits, else equal tiles of a multiple of 64 columns
-      const int nt = (n_cols + 255) / 256;
-      int bn = (n_cols + nt - 1) / nt;
-      bn = nt > 1 ? (bn + 63) / 64 * 64 : (bn + 31) / 32 * 32;
-      const int rtot = mt * rows + R - 1;
-      const int a_bytes = (rtot * pitch * p.bk * 2 + 1023) / 1024 * 1024;
-      const int b_bytes = bn * p.bk * 2;
-      int stages = (TILE_SMEM_BYTES - 2 * a_bytes) / b_bytes;
-      if (stages > MAX_STAGES) stages = MAX_STAGES;
-      (void)util;
-      // measured slower than the im2col path on every layer tried (0.239 vs 0.167 ms on AlexNet conv2), so the
-      // mode is only taken when forced; it stays for the tests and for further work
-      if (rtot <= 256 && bn <= 256 && stages >= 3 && force == 1) {
-        p.a_mode = A_HALO_K;
-        p.bn = p.bn_load = bn;
-        p.n_tiles = (n_cols + bn - 1) / bn;
-        p.hl_pitch = pitch;
-        p.hl_rows = rows;
-        p.hl_rtot = rtot;
-        p.hl_groups = groups;
-        p.hl_R = R;
-        p.hl_pad_h = pad_h;
-        p.hl_pad_w = pad_w;
-        p.hl_a_stages = 2;
-        p.hl_a_bytes = a_bytes;
-        p.mt = mt;
-        p.split_k = 1;
-        p.b_resident = 0;
-        p.acc_stride = bn > 128 ? 256 : 128;
-        p.acc_bufs = (2 * mt * p.acc_stride <= 512) ? 2 : 1;
-        p.stages = stages;
-        rc = make_map_nhwc(&p.tm_a, x, Cp, W, H, N, Cp, p.bk, pitch, rtot, ksw);
-        if (rc) return rc;
-        rc = make_map_3d(&p.tm_b, w, Cp, (uint64_t)R * S, Kout, Cp, (uint64_t)R * S * Cp, p.bk, 1, p.bn, ksw);
-        if (rc) return rc;
-        const uint32_t bw = pitch < 32 ? pitch : 32, bh = 32 / bw;
-        rc = make_map_nhwc(&p.tm_d, y, p.n_store, Q, P, N, ldy, 64, bw, bh, CU_TENSOR_MAP_SWIZZLE_128B);
-        if (rc) return rc;
-        if (mask_src)
-          rc = make_map_nhwc(&p.tm_mask, mask_src, p.n_store, Q, P, N, ldy, 64, bw, bh, CU_TENSOR_MAP_SWIZZLE_128B);
-        if (rc) return rc;
-        const long long work = (long long)N * groups * p.n_tiles;
-        const int grid = work < g_num_sms ? (int)work : g_num_sms;
-        gemm_tc_kernel<false, false><<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, stream>>>(p);
-        return cudaGetLastError() == cudaSuccess ? 0 : -4;
-      }
-    }
-  }
   // upper corner so that the base pixel takes exactly P x Q positions
   const int upper_h = (P - 1) * stride - pad_h - (H - 1);
   const int upper_w = (Q - 1) * stride - pad_w - (W - 1);
@@ -1955,11 +2107,17 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   if (rc) return rc;
   if (mask_src) rc = make_map_out(&p.tm_mask, const_cast<void*>(mask_src), p.n_store, p.M, ldy);
   if (rc) return rc;
-  // How the A operand is loaded (`box` = tap-shifted tiled boxes of whole output rows, else the im2col map, or plain
-  // tiled rows for a 1 x 1 convolution) and what depends on the tile width: column tiling, the filter map's box.
-  auto configure = [&](GemmTcParams& q, int box, int bn) -> int {
+  // How the A operand is loaded (`how`: LOAD_BOX = tap-shifted tiled boxes of whole output rows, LOAD_FLAT = whole input
+  // rows once for all taps, else the im2col map, or plain tiled rows for a 1 x 1 convolution) and what depends on the tile width: column tiling, the filter map's box.
+  enum { LOAD_BOX = 1, LOAD_FLAT = 2 };
+  auto configure = [&](GemmTcParams& q, int how, int bn) -> int {
     int e;
-    if (box) {
+    if (how == LOAD_FLAT) {
+      q.a_mode = A_FLAT_K;
+      q.a_split = 1;
+      if (!flat_geom(q, N, H, W, R, S, pad_h, pad_w)) return -3;
+      e = make_map_nhwc(&q.tm_a, x, Cp, W, H, N, Cp, q.bk, q.fl_pitch, 1, ksw);
+    } else if (how == LOAD_BOX) {
       q.a_mode = A_BOX_K;
       q.a_split = 1;
       q.bx_rows = BM / Q;
@@ -1993,43 +2151,78 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   //  * for stride-1 convolutions with more than one tap and output rows of at most 128 positions, box loads:
   //    cheaper per row for the TMA unit, at the price of tile rows that are computed and dropped when Q does not
   //    divide 128 (and when bx_rows does not divide P).
+  //  * for stride-1 convolutions with more than one tap, flat mode: the first few plans by its cost model, which is good
+  //    enough for these to hold the best.
   // Which is fastest is decided by measurement in tuning mode and remembered per shape; without a measurement the
   // default is taken.
   const int bn_default = p.bn;
   const int bn_wide = (n_cols > 256 && n_cols <= 512 && g_opt.force_wide != 0 && g_opt.bn_cap >= 256) ? n_cols : 0;
-  const bool box_ok = stride == 1 && R * S > 1 && Q <= BM && g_opt.force_box != 0 && g_opt.force_halo != 1;
-  int use = bn_default;   // low 16 bits: tile width; bit 16: box loads
-  if (bn_wide || box_ok) {
+  const bool box_ok = stride == 1 && R * S > 1 && Q <= BM && g_opt.force_box != 0;
+  // flat mode: the widths of one to four equal column tiles of at most 256 columns, 0 for those that are not
+  auto flat_bn = [n_cols](int nt) {
+    const int per = (n_cols + nt - 1) / nt, bn = nt == 1 ? (per + 31) / 32 * 32 : (per + 63) / 64 * 64;
+    return bn > 256 || bn * (nt - 1) >= n_cols ? 0 : bn;
+  };
+  bool flat_ok = stride == 1 && R * S > 1 && g_opt.force_halo != 0;
+  if (flat_ok) {
+    GemmTcParams q = p;
+    flat_ok = flat_geom(q, N, H, W, R, S, pad_h, pad_w);
+  }
+  auto flat_candidates = [&]() {      // (width, plan), best first
+    std::vector<std::pair<int, Plan>> all;
+    for (int nt = 1; nt <= 4 && flat_ok; ++nt) {
+      GemmTcParams q = p;
+      if (!flat_bn(nt) || configure(q, LOAD_FLAT, flat_bn(nt))) continue;
+      Plan plans[12];
+      const int n = flat_plans(q, plans, 12);
+      for (int i = 0; i < n; ++i) all.push_back({flat_bn(nt), plans[i]});
+    }
+    std::stable_sort(all.begin(), all.end(), [](const std::pair<int, Plan>& a, const std::pair<int, Plan>& b) {
+      return a.second.cost < b.second.cost;
+    });
+    return all;
+  };
+  int use = bn_default;   // low 16 bits: tile width; above: how A is loaded
+  if (bn_wide || box_ok || flat_ok) {
     p.bn = p.n_tiles = 0;
     p.a_mode = A_IM2COL_K;
     const PlanKey ckey = plan_key(p);
     std::lock_guard<std::mutex> lock(g_plan_mutex);   // released at the end of this block, before `launch` takes it
     auto it = g_bn_cache.find(ckey);
-    if (g_opt.force_wide == 1 || g_opt.force_box == 1) {
-      use = ((bn_wide && g_opt.force_wide == 1) ? bn_wide : bn_default) | ((box_ok && g_opt.force_box == 1) ? 1 << 16 : 0);
+    const auto forced = g_opt.force_halo == 1 ? flat_candidates() : std::vector<std::pair<int, Plan>>();
+    if (!forced.empty()) {
+      use = forced[0].first | (LOAD_FLAT << 16);
+    } else if (g_opt.force_wide == 1 || g_opt.force_box == 1) {
+      use = ((bn_wide && g_opt.force_wide == 1) ? bn_wide : bn_default) |
+            ((box_ok && g_opt.force_box == 1) ? LOAD_BOX << 16 : 0);
     } else if (it != g_bn_cache.end()) {
       use = it->second;   // as far as it still applies: the options may have changed since it was measured
-      if (!box_ok) use &= 0xFFFF;
-      if ((use & 0xFFFF) != bn_default && (use & 0xFFFF) != bn_wide) use = bn_default | (use & 1 << 16);
+      if ((use >> 16) == LOAD_FLAT && !flat_ok) use = bn_default;
+      if ((use >> 16) == LOAD_BOX && !box_ok) use &= 0xFFFF;
+      if ((use >> 16) != LOAD_FLAT && (use & 0xFFFF) != bn_default && (use & 0xFFFF) != bn_wide)
+        use = bn_default | (use & ~0xFFFF);
     } else if (tunable(p, stream)) {
       float best_ms = 1e30f;
-      for (int box = 0; box <= (box_ok ? 1 : 0); ++box) {
-        for (int bn : {bn_default, bn_wide}) {
-          if (bn == 0) continue;
-          GemmTcParams q = p;
-          if (configure(q, box, bn)) continue;
-          Plan pl{1, 1, 0, 0, 0.0};
-          const float ms = tune_plan(q, true, stream, &pl);
-          if (ms > 0.f) {
-            g_plan_cache[plan_key(q)] = pl;
-            if (ms < best_ms) { best_ms = ms; use = bn | (box << 16); }
-          }
+      auto measure = [&](int how, int bn, const Plan* given) {
+        GemmTcParams q = p;
+        if (configure(q, how, bn)) return;
+        Plan pl{1, 1, 0, 0, 0.0};
+        const float ms = tune_plan(q, true, stream, &pl, given);
+        if (ms > 0.f && ms < best_ms) {
+          best_ms = ms;
+          use = bn | (how << 16);
+          g_plan_cache[plan_key(q)] = pl;
         }
-      }
+      };
+      for (int how = 0; how <= (box_ok ? LOAD_BOX : 0); ++how)
+        for (int bn : {bn_default, bn_wide})
+          if (bn) measure(how, bn, nullptr);
+      const auto flat = flat_candidates();
+      for (size_t i = 0; i < flat.size() && i < 5; ++i) measure(LOAD_FLAT, flat[i].first, &flat[i].second);
       g_bn_cache[ckey] = use;
     }
   }
-  rc = configure(p, (use >> 16) & 1, use & 0xFFFF);
+  rc = configure(p, use >> 16, use & 0xFFFF);
   if (rc) return rc;
   return launch(p, false, 1, true, stream);
 }

@@ -1,7 +1,7 @@
 // Parameter block of the persistent tcgen05 GEMM / implicit-GEMM convolution
 // kernel (gemm_tc.cu). One kernel, configured at run time, serves:
 //   conv fprop   A = im2col(X) K-major (TMA im2col)   B = filters K-major
-//                or, stride 1: A = column-shifted halo tiles of X (plain tiled TMA, A_HALO_K), see gemm_tc.cu
+//                or, stride 1: A = whole input rows, loaded once for all filter taps (A_FLAT_K), see gemm_tc.cu
 //   conv dgrad   A = im2col(dY) K-major               B = the filters as they are, MN-major (TMA tiled, B_DGRAD_MN), or
 //                                                         transposed and flipped ones, K-major
 //   conv wgrad   A = dY^T MN-major (tiled)            B = im2col(X) MN-major (TMA im2col; tiled boxes of whole output
@@ -19,7 +19,7 @@
 
 namespace rb {
 
-enum : int { A_TILED_K = 0, A_IM2COL_K = 1, A_TILED_MN = 2, A_HALO_K = 3, A_BOX_K = 4, A_BOX_MN = 5 };
+enum : int { A_TILED_K = 0, A_IM2COL_K = 1, A_TILED_MN = 2, A_FLAT_K = 3, A_BOX_K = 4, A_BOX_MN = 5 };
 enum : int { B_TILED_K = 0, B_TILED_MN = 1, B_IM2COL_MN = 2, B_TILED_K3 = 3, B_DGRAD_MN = 4, B_BOX_MN = 5 };
 enum : int { EPI_BF16 = 0, EPI_F32_STORE = 1, EPI_F32_ATOMIC = 2 };
 
@@ -61,15 +61,17 @@ struct alignas(64) GemmTcParams {
   int wb_pieces;       // column pieces per row (output rows wider than bk)
   int wb_pad_h, wb_pad_w;
   int n_tiles;         // tiles along N (taps*wg_ctiles for wgrad)
-  // halo mode (A_HALO_K): a sub-tile is hl_rows output rows of one image at a row pitch of hl_pitch positions
-  int hl_pitch;        // 8..128, a power of two >= Q; hl_rows * hl_pitch = 128
-  int hl_rows;
-  int hl_rtot;         // input rows per A stage = mt * hl_rows + R - 1
-  int hl_groups;       // work items per image = ceil(P / (mt * hl_rows))
-  int hl_R;            // filter height
-  int hl_pad_h, hl_pad_w;
-  int hl_a_stages;     // A stages in shared memory (each hl_a_bytes apart)
-  int hl_a_bytes;
+  // flat mode (A_FLAT_K, stride-1 convolutions): see flat_geom in gemm_tc.cu
+  int fl_pitch;        // positions per output row, the row's zero columns included
+  int fl_hp;           // rows per image, its zero rows included
+  int fl_step;         // positions between the starts of neighbouring sub-tiles: 128, or one row (fl_pitch >= 128)
+  int fl_units;        // sub-tiles that cover every output row of every image
+  int fl_rows;         // input rows per A stage
+  int fl_lead;         // where in an A stage the first position of the work item lies
+  int fl_R;            // filter height
+  int fl_pad_h, fl_pad_w;
+  int fl_a_stages;     // A stages in shared memory (each fl_a_bytes apart)
+  int fl_a_bytes;
   // box mode (A_BOX_K, stride-1 convolutions): a sub-tile is bx_rows whole output rows of one image (bx_rows * Q <=
   // 128 positions, contiguous in the NHWC output); the A operand of filter tap (r, s) is ONE tiled 4-D box of
   // bx_rows x Q pixels x bk channels whose corner is shifted by the tap (zero fill outside the image), which the TMA
