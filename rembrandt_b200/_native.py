@@ -29,6 +29,8 @@ _CUDA_SIGS = {
     "rb_conv_fprop_tc": [vp, i32, i32, i32, i32, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, i64, vp, i32, vp,
                          i32, i32, vp, i64, vp, vp],
     "rb_conv_dgrad_tc": [vp, i32, i32, i32, i32, vp, vp] + [i32] * 10 + [vp, vp, vp, vp, i64, vp, vp],
+    "rb_conv_fprop_norm": [vp, i32, i32, i32, i32, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, i64, vp, vp, vp, i32, i32,
+                           i32, vp, i64, vp, vp],
     "rb_gemm_set_option": [vp, i32],
     "rb_gemm_get_option": [vp, vp],
     "rb_gemm_tune_mode": [i32],
@@ -85,6 +87,7 @@ _CUDA_SIGS = {
     "rb_bn_fwd_train_ws": [vp, i64, i32, i32, vp, f32, f32, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, vp, vp],
     "rb_bn_bwd_ws": [vp, vp, vp, i64, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp],
     "rb_bn_fwd_infer": [vp, i64, i32, i32, f32, vp, vp, vp, vp, vp, vp, vp, i32, vp],
+    "rb_bn_fold": [vp, vp, i32, vp, vp],
     "rb_bn_bwd": [vp, vp, vp, i64, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp],
 }
 

@@ -350,6 +350,27 @@ static void launch_bn_apply(const bf16* x, const BnStats& stats, const BnScratch
   else go(bn_apply_kernel<FROM, 0>);
 }
 
+// Scale and shift of normalisations by running statistics, for the epilogues of the convolutions before them
+// (rb_conv_fprop_norm): y = x * scale + shift. One block per layer; `units` holds per layer where gamma, beta, the running mean
+// and the running variance lie in `params` and where the layer's scale and shift go in `out`, its channels, padded and not, and
+// eps as a bit pattern.
+__global__ void __launch_bounds__(256) bn_fold_kernel(const float* __restrict__ params, const long long* __restrict__ units,
+                                                      float* __restrict__ out) {
+  pdl_prolog();
+  const long long* u = units + 8 * (long long)blockIdx.x;
+  const int C = (int)u[5], c_valid = (int)u[6];
+  const float eps = __int_as_float((int)u[7]);
+  for (int c = threadIdx.x; c < C; c += 256) {
+    float scale = 0.f, shift = 0.f;
+    if (c < c_valid) {
+      scale = params[u[0] + c] * rsqrtf(params[u[3] + c] + eps);
+      shift = params[u[1] + c] - params[u[2] + c] * scale;
+    }
+    out[u[4] + c] = scale;
+    out[u[4] + C + c] = shift;
+  }
+}
+
 // dx = gamma * istd * (dy - (dbeta + xhat * dgamma) / rows), with [dbeta | dgamma] of this batch from `plain` or from a
 // scratch; in the latter case they are also accumulated into the gradient buffers.
 template <int MASK>
@@ -496,6 +517,12 @@ int rb_bn_fwd_infer(const void* x, long long rows, int C, int c_valid, float eps
   const BnStats stats = {nullptr, nullptr, (float*)run_mean, (float*)run_var, nullptr, eps, 0.f, 0};
   launch_bn_apply<BN_INFER>((const bf16*)x, stats, BnScratch{}, gamma, beta, (const bf16*)residual, (bf16*)y, rows, C,
                             c_valid, relu, st);
+  return RB_LAUNCH_OK();
+}
+
+int rb_bn_fold(const float* params, const long long* units, int n_units, float* out, cudaStream_t st) {
+  if (n_units <= 0) return 0;
+  launch_pdl(bn_fold_kernel, dim3(n_units), dim3(256), 0, st, params, units, out);
   return RB_LAUNCH_OK();
 }
 

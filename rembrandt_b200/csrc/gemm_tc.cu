@@ -333,9 +333,9 @@ __device__ __forceinline__ bool issue_flat_item(const IssueCtx& c, const FlatCtx
 // PART: only the first `valid` of the 32 columns exist, the others are written as zeros (16 channels of 32: element by element
 // this took ~4000 cycles per 32 x 32 group and kept the issuing warp waiting for accumulators: ResNet-20's step at 128 images,
 // whose first stage has 16 channels: 1362 -> 1310 us).
-template <bool BIAS, bool RELU, bool MASK, bool ADD, bool PART>
+template <bool BIAS, bool RELU, bool MASK, bool ADD, bool PART, bool SCALE = false>
 __device__ __forceinline__ void epilogue_half(const uint32_t (&v)[32], uint8_t* row, int swz, int half, const float* bias,
-                                              const uint4* mask, const uint4* add, int valid) {
+                                              const uint4* mask, const uint4* add, int valid, const float* scale = nullptr) {
   const __nv_bfloat162 zero2 = __floats2bfloat162_rn(0.f, 0.f);
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -351,13 +351,23 @@ __device__ __forceinline__ void epilogue_half(const uint32_t (&v)[32], uint8_t* 
       for (int e = 0; e < 8; ++e) b1[e] = q * 8 + e < valid ? __ldg(bias + q * 8 + e) : 0.f;
     }
     const float* bb = reinterpret_cast<const float*>(&bq[0]);
+    float sc[8];
+    if (SCALE) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) sc[e] = !PART || q * 8 + e < valid ? __ldg(scale + q * 8 + e) : 0.f;
+    }
     const uint4 av = ADD ? add[q] : make_uint4(0u, 0u, 0u, 0u);
     const uint32_t* aw = reinterpret_cast<const uint32_t*>(&av);
     const __nv_bfloat162* m2 = reinterpret_cast<const __nv_bfloat162*>(&mask[q]);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       float x0 = __uint_as_float(v[q * 8 + 2 * e]), x1 = __uint_as_float(v[q * 8 + 2 * e + 1]);
-      if (BIAS) add2_f32(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1], bb[2 * e], bb[2 * e + 1], x0, x1);
+      if (SCALE) {
+        x0 = fmaf(x0, sc[2 * e], bb[2 * e]);
+        x1 = fmaf(x1, sc[2 * e + 1], bb[2 * e + 1]);
+      } else if (BIAS) {
+        add2_f32(v[q * 8 + 2 * e], v[q * 8 + 2 * e + 1], bb[2 * e], bb[2 * e + 1], x0, x1);
+      }
       if (ADD) {
         x0 += __uint_as_float(aw[e] << 16);
         x1 += __uint_as_float(aw[e] & 0xFFFF0000u);
@@ -393,13 +403,28 @@ __device__ __forceinline__ void epilogue_kinds(int kind, bool addend, const uint
   }
 }
 
+// The epilogue of a convolution whose normalisation is known beforehand (inference): scale, shift, residual and ReLU.
+template <bool PART>
+__device__ __forceinline__ void epilogue_norm(bool relu, bool addend, const uint32_t (&v)[32], uint8_t* row, int swz, int half,
+                                              const float* bias, const float* scale, const uint4* m, const uint4* av,
+                                              int valid) {
+  if (addend) {
+    if (relu) epilogue_half<true, true, false, true, PART, true>(v, row, swz, half, bias, m, av, valid, scale);
+    else epilogue_half<true, false, false, true, PART, true>(v, row, swz, half, bias, m, av, valid, scale);
+  } else {
+    if (relu) epilogue_half<true, true, false, false, PART, true>(v, row, swz, half, bias, m, av, valid, scale);
+    else epilogue_half<true, false, false, false, PART, true>(v, row, swz, half, bias, m, av, valid, scale);
+  }
+}
+
 // PAIR: the instantiation that runs as clusters of two CTAs (p.pair != 0). It is a kernel of its own because a
 // kernel that contains cta_group::2 instructions can only be launched with an even cluster size.
 // EXT: the instantiation whose bf16 epilogue can scatter rows and take an addend. The tests for these cost the epilogue of
 // every other launch what they do not use: 1 x 1 layers, which are bound by it, ran 8 % slower with them (NIN's training
 // step at 64 images: 1255 instead of 1186 us).
 // FLAT: the instantiation for A_FLAT_K, whose rows are always scattered (EXT).
-template <bool PAIR, bool EXT, bool FLAT>
+// NORM: the instantiation for launches with a scale (EXT).
+template <bool PAIR, bool EXT, bool FLAT, bool NORM>
 __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant__ GemmTcParams p) {
 #ifdef RB_GEMM_PROFILE
   const long long t_kernel0 = clock64();
@@ -1009,7 +1034,10 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
                 }
               }
               const int valid = p.n_valid - nbase;
-              if (valid >= 32) epilogue_kinds<EXT, false>(epi_kind, addend, v, slab_row, swz, half, bias, m, av, valid);
+              if (NORM) {
+                if (valid >= 32) epilogue_norm<false>(p.relu != 0, addend, v, slab_row, swz, half, bias, p.scale + nbase, m, av, valid);
+                else epilogue_norm<true>(p.relu != 0, addend, v, slab_row, swz, half, bias, p.scale + nbase, m, av, valid);
+              } else if (valid >= 32) epilogue_kinds<EXT, false>(epi_kind, addend, v, slab_row, swz, half, bias, m, av, valid);
               else epilogue_kinds<EXT, true>(epi_kind, addend, v, slab_row, swz, half, bias, m, av, valid);
             }
             RB_PROF_ADD(warp == 2, 7);
@@ -1117,6 +1145,14 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
 
 // =============================== host side ===============================
 
+typedef void (*Kernel)(GemmTcParams);
+static const Kernel KERNELS[] = {   // without and with CTA pairs
+    gemm_tc_kernel<false, false, false, false>, gemm_tc_kernel<true, false, false, false>,
+    gemm_tc_kernel<false, true, false, false>,  gemm_tc_kernel<true, true, false, false>,
+    gemm_tc_kernel<false, true, true, false>,   gemm_tc_kernel<true, true, true, false>,
+    gemm_tc_kernel<false, true, false, true>,   gemm_tc_kernel<true, true, false, true>,
+    gemm_tc_kernel<false, true, true, true>,    gemm_tc_kernel<true, true, true, true>};
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1149,9 +1185,7 @@ static int ensure_driver_entry() {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
   cudaDriverGetVersion(&g_driver_version);
-  for (auto kern : {gemm_tc_kernel<false, false, false>, gemm_tc_kernel<true, false, false>,
-                    gemm_tc_kernel<false, true, false>, gemm_tc_kernel<true, true, false>, gemm_tc_kernel<false, true, true>,
-                    gemm_tc_kernel<true, true, true>})
+  for (auto kern : KERNELS)
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) != cudaSuccess) return -2;
   {   // how many CTA pairs fit at once: the persistent loop of pair mode runs exactly that many clusters
     cudaLaunchConfig_t cfg;
@@ -1167,7 +1201,7 @@ static int ensure_driver_entry() {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, gemm_tc_kernel<true, true, true>, &cfg) != cudaSuccess) nc = 0;
+    if (cudaOccupancyMaxActiveClusters(&nc, gemm_tc_kernel<true, true, true, false>, &cfg) != cudaSuccess) nc = 0;
     cudaGetLastError();   // a refused query must not be taken for a failed launch later
     g_pair_clusters = nc > g_num_sms / 2 ? g_num_sms / 2 : nc;
   }
@@ -1637,6 +1671,7 @@ struct TailFixArgs {
   const __nv_bfloat16* mask;
   long long ldd;
   const __nv_bfloat16* add;
+  const float* scale;
   int M, bn, rows_per_item, m_items, direct, tail_items, n_valid, n_store, relu;
   int sc_stride, sc_a, sc_b, sc_H, sc_W;   // see GemmTcParams
   int box, P, Q, bx_rows, bx_groups, mt;   // box mode: rows of a sub-tile are whole output rows of one image
@@ -1676,6 +1711,7 @@ __global__ void tail_fix_kernel(const TailFixArgs a) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
       const int n = col + e;
+      if (a.scale && n < a.n_valid) f[e] *= __ldg(a.scale + n);
       f[e] = n < a.n_valid ? fmaxf(f[e] + (a.bias ? __ldg(a.bias + n) : 0.f) + extra[e], act_lo) : 0.f;
     }
     if (a.mask) {
@@ -1751,13 +1787,8 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
     }
     cfg.attrs = n_at ? at : nullptr;
     cfg.numAttrs = (unsigned)n_at;
-    const bool ext = p.sc_stride != 0 || p.add_src != nullptr;
-    const cudaError_t e = cudaLaunchKernelEx(
-        &cfg,
-        p.a_mode == A_FLAT_K ? (p.pair ? gemm_tc_kernel<true, true, true> : gemm_tc_kernel<false, true, true>)
-        : p.pair             ? (ext ? gemm_tc_kernel<true, true, false> : gemm_tc_kernel<true, false, false>)
-                             : (ext ? gemm_tc_kernel<false, true, false> : gemm_tc_kernel<false, false, false>),
-        p);
+    const int form = p.a_mode == A_FLAT_K ? 2 : p.scale || p.sc_stride != 0 || p.add_src != nullptr ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, KERNELS[(p.scale ? 2 * (form + 2) : 2 * form) + (p.pair ? 1 : 0)], p);
     if (e != cudaSuccess) {
       g_last_cuda_error = (int)e;
       cudaGetLastError();
@@ -1771,6 +1802,7 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
     f.bias = p.bias;
     f.mask = p.mask_src;
     f.add = p.add_src;
+    f.scale = p.scale;
     f.sc_stride = p.sc_stride;
     f.sc_a = p.sc_a;
     f.sc_b = p.sc_b;
@@ -1816,7 +1848,8 @@ static std::mutex g_plan_mutex;
 
 static PlanKey plan_key(const GemmTcParams& p) {
   return PlanKey(p.a_mode, p.b_mode, p.M, p.N, p.num_kb, p.bn, p.bk, p.n_tiles, p.cv_stride,
-                 (p.mask_src ? 1 : 0) | (p.add_src ? 2 : 0) | (p.sc_stride ? 4 : 0), p.cv_P, p.cv_Q, p.cv_S,
+                 // (a forward pass with its normalisation takes the plan of the one without)
+                 (p.mask_src ? 1 : 0) | (p.add_src && !p.scale ? 2 : 0) | (p.sc_stride ? 4 : 0), p.cv_P, p.cv_Q, p.cv_S,
                  p.cv_cchunks);
 }
 
@@ -2038,13 +2071,19 @@ struct DgradForm {
   const void* add;
 };
 
+// A normalisation in the epilogue of a forward pass, with an optional residual.
+struct NormForm {
+  const float* scale;
+  const void* residual;
+};
+
 // x NHWC bf16 [N][H][W][Cp]; w bf16 [Kout][R*S][Cp], or with `dg` the filters [k_rows][taps][n_store] of the layer whose
 // data-gradient this is (or their packed form); y bf16 [N*P*Q][ldy]. Base pixel range: lower = -pad, P / Q given by the
 // caller.
 static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
                              int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* bias, int relu,
-                             const void* mask_src, int n_valid, int n_store, int k_rows, const DgradForm* dg, float* ws,
-                             long long ws_bytes, unsigned int* status, cudaStream_t stream) {
+                             const void* mask_src, int n_valid, int n_store, int k_rows, const DgradForm* dg, const NormForm* norm,
+                             float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
   int rc = ensure_driver_entry();
   if (rc) return rc;
   GemmTcParams p;
@@ -2083,6 +2122,10 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
     p.sc_H = dg->sc_H;
     p.sc_W = dg->sc_W;
     p.add_src = reinterpret_cast<const __nv_bfloat16*>(dg->add);
+  }
+  if (norm) {
+    p.scale = norm->scale;
+    p.add_src = reinterpret_cast<const __nv_bfloat16*>(norm->residual);
   }
   p.cv_P = P;
   p.cv_Q = Q;
@@ -2239,7 +2282,20 @@ int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, 
                      const void* mask_src, int n_valid, int n_store, float* ws, long long ws_bytes,
                      unsigned int* status, cudaStream_t stream) {
   return conv_forward_form(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, bias, relu, mask_src, n_valid,
-                           n_store, 0, nullptr, ws, ws_bytes, status, stream);
+                           n_store, 0, nullptr, nullptr, ws, ws_bytes, status, stream);
+}
+
+// The same followed by a normalisation that is known beforehand, in the epilogue:
+// y = act(scale * conv(x) + shift [+ residual]), scale and shift (on a 16-byte boundary) per output column, residual laid out
+// like y.
+int rb_conv_fprop_norm(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
+                       int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* scale, const float* shift,
+                       const void* residual, int relu, int n_valid, int n_store, float* ws, long long ws_bytes,
+                       unsigned int* status, cudaStream_t stream) {
+  if (!scale || !shift || ((uintptr_t)shift & 15u)) return -10;
+  const NormForm form = {scale, residual};
+  return conv_forward_form(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, shift, relu, nullptr, n_valid,
+                           n_store, 0, nullptr, &form, ws, ws_bytes, status, stream);
 }
 
 // Convolution data-grad: dx[N][H][W][Cp] = mask(add + the gradient), from dy NHWC bf16 [N][P][Q][Kp] and the forward
@@ -2300,7 +2356,7 @@ int rb_conv_dgrad_tc(const void* dy, int N, int P, int Q, int Kp, const void* w,
       dg.sc_W = W;
       dg.add = add;
       const int rc = conv_forward_form(dy, N, P, Q, Kp, wt ? wt : w, Cp, f.U, f.V, 1, f.pt, f.pl, f.Hp, f.Wp, dx, Cp, nullptr, 0,
-                                       mask, c_valid, Cp, Kout, &dg, ws, ws_bytes, status, stream);
+                                       mask, c_valid, Cp, Kout, &dg, nullptr, ws, ws_bytes, status, stream);
       if (rc) return rc;
     }
   return 0;

@@ -96,6 +96,7 @@ struct alignas(64) GemmTcParams {
   long long ldd;       // row pitch of D in elements
   void* D;
   const float* bias;               // optional, indexed by column
+  const float* scale;              // EPI_BF16, optional, with bias: D = act(scale * product + bias + addend), no mask
   const __nv_bfloat16* mask_src;   // optional, same layout as D: D is zeroed where mask_src <= 0
   unsigned int* status;            // error bits (see ptx.cuh)
   // Tail cut (EPI_BF16, split_k = 1): the work items of the last, partly filled wave are cut along the reduction

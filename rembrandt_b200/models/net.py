@@ -143,6 +143,11 @@ class Net:
                 op.alloc()
         for op in self.ops:
             op.bind()
+        # normalisations that inference passes leave to the convolutions before them (None: there are none)
+        self.folded_norms = None
+        if self.device.type == "cuda":
+            from .resnet_ops import FoldedNorms
+            self.folded_norms = FoldedNorms.of(self)
         self._cpu_loss = None
         self._cpu_stats = [0.0, 0]
         self._cpu_batch = None
@@ -287,6 +292,8 @@ class Net:
         if self.is_cuda:
             if t is not None:
                 self.step_counter.fill_(int(t))
+            if not train and self.folded_norms is not None:
+                self.folded_norms.compute()
             for op in self.ops:
                 with span(op.name):
                     op.forward(train, self.t if t is None else t)

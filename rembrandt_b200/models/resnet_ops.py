@@ -21,6 +21,32 @@ from ..ops.native_ops import pad_channels
 from .operators import DataOp, Op, ParamSeg, _draw, conv_out
 
 
+class FoldedNorms:
+    """Scale and shift of every normalised convolution of a network by its running statistics, worked out by one launch at the
+    start of an inference pass; each convolution then normalises, adds the residual and applies the ReLU in its epilogue, which
+    saves a launch and two passes over the output (ResNet-18, 50 images: 904 -> 818 us a pass)."""
+
+    def __init__(self, net, units):
+        self.net, self.n = net, len(units)
+        rows, at = [], 0
+        for u in units:
+            eps = int(torch.tensor([u.eps], dtype=torch.float32).view(torch.int32))
+            rows.append([u.seg_g.offset, u.seg_b.offset, u.seg_rm.offset, u.seg_rv.offset, at, u.kp, u.ko, eps])
+            at += 2 * u.kp
+        self.table = torch.tensor(rows, dtype=torch.int64, device=net.device)
+        self.values = torch.zeros(at, dtype=torch.float32, device=net.device)
+        for u, row in zip(units, rows):
+            u.fold = (self.values[row[4]: row[4] + u.kp], self.values[row[4] + u.kp: row[4] + 2 * u.kp])
+
+    @staticmethod
+    def of(net):
+        units = [u for op in net.ops if isinstance(op, _BlockBase) for u in op.units]
+        return FoldedNorms(net, units) if units else None
+
+    def compute(self):
+        K.bn_fold(self.net.params, self.table, self.n, self.values)
+
+
 class _BnConv:
     """conv (no bias) -> batch norm [-> + residual] [-> ReLU], with its buffers and parameter segments."""
 
@@ -43,6 +69,7 @@ class _BnConv:
             self.gk, self.gs, self.gp = r2, 1, 0
         else:
             self.gh, self.gw, self.gk, self.gs, self.gp = self.h, self.w, k, stride, pad
+        self.fold = None         # (scale, shift) by the running statistics: a `FoldedNorms` computes them
         self.dgrad = None        # DgradPlan on a GPU
         self.windowed = None     # a WindowedFirstLayer: the input operator writes whole receptive fields
         n = op.name + "." + tag
@@ -81,6 +108,13 @@ class _BnConv:
         w16 = self.v(self.seg_w, "params16")
         if train and self.dgrad:
             self.dgrad.prepare(net, w16)
+        if not train and self.fold is not None:
+            if self.windowed:
+                self.windowed.forward_norm(x, w16, out, self.kp, *self.fold, residual, relu)
+            else:
+                K.conv_fprop_norm(x, n, self.gh, self.gw, self.cp, w16, self.ko, self.gk, self.gk, self.gs, self.gp, self.gp,
+                                  self.P, self.Q, out, self.kp, *self.fold, residual, relu, n_valid=self.ko, n_store=self.kp)
+            return
         if self.windowed:
             self.windowed.forward(x, w16, self.conv_out, self.kp)
         else:

@@ -153,6 +153,17 @@ def conv_fprop_tc(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, 
     check(rc, "rb_conv_fprop_tc")
 
 
+def conv_fprop_norm(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, scale, shift, residual=None, relu=False,
+                    n_valid=0, n_store=0):
+    """y = act(scale * conv(x) + shift [+ residual]): a convolution and a normalisation that is known beforehand (`bn_fold`) in
+    one launch."""
+    ws = gemm_workspace()
+    rc = _native.cuda().rb_conv_fprop_norm(ptr(x), N, H, W, Cp, ptr(w), Kout, R, S, stride, pad_h, pad_w, P, Q, ptr(y), ldy,
+                                           ptr(scale), ptr(shift), ptr(residual), int(relu), n_valid, n_store, ptr(ws),
+                                           ws.numel() * 4, ptr(status_word()), stream_handle())
+    check(rc, "rb_conv_fprop_norm")
+
+
 _tuned_convs: set = set()
 
 
@@ -454,6 +465,11 @@ def bn_fwd_infer(x, rows, C, c_valid, eps, run_mean, run_var, istd_tmp, gamma, b
     check(_native.cuda().rb_bn_fwd_infer(ptr(x), rows, C, c_valid, eps, ptr(run_mean), ptr(run_var), ptr(istd_tmp),
                                          ptr(gamma), ptr(beta), ptr(residual), ptr(y), int(relu), stream_handle()),
           "rb_bn_fwd_infer")
+
+
+def bn_fold(params, units, n_units, out):
+    """Scale and shift of `n_units` normalisations by running statistics; `units`: see `bn_fold_kernel` (csrc/bn.cu)."""
+    check(_native.cuda().rb_bn_fold(ptr(params), ptr(units), n_units, ptr(out), stream_handle()), "rb_bn_fold")
 
 
 def bn_bwd(x, dy, y_relu, rows, C, c_valid, sums, mean, istd, gamma, dgamma, dbeta, dx):
