@@ -22,7 +22,7 @@ from .operators import DataOp, Op, ParamSeg, _draw, conv_out
 
 
 class FoldedNorms:
-    """Scale and shift of every normalised convolution of a network by its running statistics, worked out by one launch at the
+    """Scale and shift of the normalised convolutions of a network (but first layers) by their running statistics, worked out by one launch at the
     start of an inference pass; each convolution then normalises, adds the residual and applies the ReLU in its epilogue, which
     saves a launch and two passes over the output (ResNet-18, 50 images: 904 -> 818 us a pass)."""
 
@@ -40,7 +40,8 @@ class FoldedNorms:
 
     @staticmethod
     def of(net):
-        units = [u for op in net.ops if isinstance(op, _BlockBase) for u in op.units]
+        # a first layer keeps its own launch: its plain output is what the input's window is checked by
+        units = [u for op in net.ops if isinstance(op, _BlockBase) for u in op.units if not u.windowed and u.s2d is None]
         return FoldedNorms(net, units) if units else None
 
     def compute(self):
@@ -109,11 +110,8 @@ class _BnConv:
         if train and self.dgrad:
             self.dgrad.prepare(net, w16)
         if not train and self.fold is not None:
-            if self.windowed:
-                self.windowed.forward_norm(x, w16, out, self.kp, *self.fold, residual, relu)
-            else:
-                K.conv_fprop_norm(x, n, self.gh, self.gw, self.cp, w16, self.ko, self.gk, self.gk, self.gs, self.gp, self.gp,
-                                  self.P, self.Q, out, self.kp, *self.fold, residual, relu, n_valid=self.ko, n_store=self.kp)
+            K.conv_fprop_norm(x, n, self.gh, self.gw, self.cp, w16, self.ko, self.gk, self.gk, self.gs, self.gp, self.gp, self.P,
+                              self.Q, out, self.kp, *self.fold, residual, relu, n_valid=self.ko, n_store=self.kp)
             return
         if self.windowed:
             self.windowed.forward(x, w16, self.conv_out, self.kp)

@@ -68,12 +68,6 @@ class WindowedFirstLayer:
         K.conv_fprop_tc(x, self.batch, self.P, self.Q, self.cols, self.w16, self.ko, 1, 1, 1, 0, 0, self.P, self.Q, y, ldy,
                         bias=bias, relu=relu, n_valid=self.ko, n_store=ldy)
 
-    def forward_norm(self, x, w16, y, ldy, scale, shift, residual, relu):
-        """The same with a normalisation in the epilogue (`native_ops.conv_fprop_norm`)."""
-        K.gather_columns(w16, self.index, self.w16, self.ko, self.row_len, self.cols)
-        K.conv_fprop_norm(x, self.batch, self.P, self.Q, self.cols, self.w16, self.ko, 1, 1, 1, 0, 0, self.P, self.Q, y, ldy,
-                          scale, shift, residual, relu, n_valid=self.ko, n_store=ldy)
-
     def backward(self, x, dy, ldy, gw, gbias=None):
         """Accumulates the filter gradient and, where there is a column of ones, the bias gradient."""
         K.gemm_tc(dy, 1, ldy, x, 1, self.cols, self.ko, self.cols, self.batch * self.P * self.Q, self.dw, self.cols,
