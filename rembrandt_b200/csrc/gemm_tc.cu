@@ -2265,9 +2265,13 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
       g_bn_cache[ckey] = use;
     }
   }
-  rc = configure(p, use >> 16, use & 0xFFFF);
-  if (rc) return rc;
-  return launch(p, false, 1, true, stream);
+  GemmTcParams q = p;
+  rc = configure(q, use >> 16, use & 0xFFFF);
+  if (rc == 0) rc = launch(q, false, 1, true, stream);
+  if (rc != -3 || (use >> 16) != LOAD_FLAT) return rc;
+  // nothing was launched: no flat plan fits this convolution, under these options, at the width that was measured
+  rc = configure(p, 0, bn_default);
+  return rc ? rc : launch(p, false, 1, true, stream);
 }
 
 }  // namespace rb

@@ -1,0 +1,88 @@
+// The planner of the tensor-core convolutions without a GPU: csrc/gemm_tc.cu compiled with the CUDA calls of its host code
+// replaced, so that a launch is only noted and a plan's time is what `fake_ms` says. Run with the name of a scenario
+// (test_conv_plans.py); says what is wrong and returns 1.
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdio.h>
+#include <string.h>
+
+static int g_launches = 0;
+static float fake_ms();
+#define cudaLaunchKernelEx(...) (++g_launches, cudaSuccess)
+#define cudaEventCreate(e) ((void)(e), cudaSuccess)
+#define cudaEventDestroy(e) ((void)(e), cudaSuccess)
+#define cudaEventRecord(e, s) ((void)(e), cudaSuccess)
+#define cudaEventSynchronize(e) ((void)(e), cudaSuccess)
+#define cudaEventElapsedTime(t, a, b) (*(t) = fake_ms(), cudaSuccess)
+#define cudaStreamIsCapturing(s, c) ((void)(s), (void)(c), cudaSuccess)
+#define cudaGetLastError() cudaSuccess
+#include "gemm_tc.cu"
+
+static CUresult no_tiled(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                         const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                         CUtensorMapFloatOOBfill) {
+  return CUDA_SUCCESS;
+}
+static CUresult no_im2col(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const int*,
+                          const int*, cuuint32_t, cuuint32_t, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                          CUtensorMapL2promotion, CUtensorMapFloatOOBfill) {
+  return CUDA_SUCCESS;
+}
+
+// {sub-tiles, split, resident, tail, pair, width, A load mode, ...} of the last launch
+enum { MT = 0, PAIR = 4, WIDTH = 5, MODE = 6 };
+static float (*g_time)(const int* launch) = nullptr;
+static float fake_ms() { return g_time ? g_time(g_last_launch) : 1.f; }
+static float flat_is_fastest(const int* l) { return l[MODE] == A_FLAT_K ? 1.f : 2.f; }
+static float flat_of_256_is_fastest(const int* l) { return l[MODE] == A_FLAT_K && l[WIDTH] == 256 ? 1.f : 2.f; }
+
+// A forward convolution, stride 1, on images of H x H.
+static int conv(int N, int C, int Ko, int H, int R, int pad) {
+  const int P = H + 2 * pad - R + 1;
+  void* const at = (void*)0x1000;   // never read: nothing is launched
+  return rb_conv_fprop_tc(at, N, H, H, C, at, Ko, R, R, 1, pad, pad, P, P, at, Ko, nullptr, 0, nullptr, Ko, Ko, nullptr, 0,
+                          nullptr, 0);
+}
+static void measure(float (*time)(const int*), int N, int C, int Ko, int H, int R, int pad) {
+  g_time = time;
+  g_tune_mode = 1;
+  conv(N, C, Ko, H, R, pad);
+  g_tune_mode = 0;
+}
+
+static int g_wrong = 0;
+static void expect(bool ok, const char* what) {
+  if (ok) return;
+  printf("wrong: %s (mode %d, width %d, sub-tiles %d, pair %d)\n", what, g_last_launch[MODE], g_last_launch[WIDTH],
+         g_last_launch[MT], g_last_launch[PAIR]);
+  g_wrong = 1;
+}
+
+// Flat mode is remembered, and no plan of it fits a later launch: other options, or other paddings of the same output
+// (3 x 3, 256 columns, rows of 111: padding 0 fits at a row pitch of 128, padding 1 does not at 112).
+static void remembered_flat_does_not_fit() {
+  measure(flat_is_fastest, 4, 64, 128, 108, 3, 1);
+  expect(conv(4, 64, 128, 108, 3, 1) == 0 && g_last_launch[MODE] == A_FLAT_K, "measured as flat");
+  g_opt.force_pair = 0;   // all plans of this one are CTA pairs
+  expect(conv(4, 64, 128, 108, 3, 1) == 0, "flat with pairs switched off since");
+  g_opt.force_pair = -1;
+  measure(flat_of_256_is_fastest, 4, 64, 256, 113, 3, 0);
+  expect(conv(4, 64, 256, 113, 3, 0) == 0 && g_last_launch[MODE] == A_FLAT_K, "measured as flat, padding 0");
+  expect(conv(4, 64, 256, 111, 3, 1) == 0, "the same output at padding 1");
+}
+
+int main(int argc, char** argv) {
+  const struct { const char* name; void (*run)(); } scenarios[] = {
+      {"remembered_flat_does_not_fit", remembered_flat_does_not_fit}};
+  g_encode_tiled = no_tiled;
+  g_encode_im2col = no_im2col;
+  g_num_sms = 148;
+  g_pair_clusters = 74;
+  for (auto& s : scenarios)
+    if (argc > 1 && strcmp(argv[1], s.name) == 0) {
+      s.run();
+      return g_wrong;
+    }
+  printf("no such scenario\n");
+  return 2;
+}
