@@ -1842,7 +1842,8 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
 // tuning mode a launch never times anything: it takes the cached plan, or the cost model's.
 // Box plans depend on the extents of the output rows, not on their product alone: at odd sizes two phases of a strided
 // data-gradient have the same M, N and k-blocks with rows and columns exchanged.
-typedef std::tuple<int, int, int, int, int, int, int, int, int, int, int, int, int, int> PlanKey;
+// Flat plans depend on the pitch and the rows per image, which follow from paddings and input extents as well.
+typedef std::tuple<int, int, int, int, int, int, int, int, int, int, int, int, int, int, int, int> PlanKey;
 static std::map<PlanKey, Plan> g_plan_cache;
 static std::mutex g_plan_mutex;
 
@@ -1850,7 +1851,7 @@ static PlanKey plan_key(const GemmTcParams& p) {
   return PlanKey(p.a_mode, p.b_mode, p.M, p.N, p.num_kb, p.bn, p.bk, p.n_tiles, p.cv_stride,
                  // (a forward pass with its normalisation takes the plan of the one without)
                  (p.mask_src ? 1 : 0) | (p.add_src && !p.scale ? 2 : 0) | (p.sc_stride ? 4 : 0), p.cv_P, p.cv_Q, p.cv_S,
-                 p.cv_cchunks);
+                 p.cv_cchunks, p.fl_pitch, p.fl_hp);
 }
 
 // Times the candidates of `p` (3 launches each, best of the last 2); returns the best time in ms, or a negative
@@ -2206,11 +2207,9 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
     const int per = (n_cols + nt - 1) / nt, bn = nt == 1 ? (per + 31) / 32 * 32 : (per + 63) / 64 * 64;
     return bn > 256 || bn * (nt - 1) >= n_cols ? 0 : bn;
   };
-  bool flat_ok = stride == 1 && R * S > 1 && g_opt.force_halo != 0;
-  if (flat_ok) {
-    GemmTcParams q = p;
-    flat_ok = flat_geom(q, N, H, W, R, S, pad_h, pad_w);
-  }
+  GemmTcParams key_p = p;
+  const bool flat_fits = stride == 1 && R * S > 1 && flat_geom(key_p, N, H, W, R, S, pad_h, pad_w);
+  const bool flat_ok = flat_fits && g_opt.force_halo != 0;
   auto flat_candidates = [&]() {      // (width, plan), best first
     std::vector<std::pair<int, Plan>> all;
     for (int nt = 1; nt <= 4 && flat_ok; ++nt) {
@@ -2227,9 +2226,8 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   };
   int use = bn_default;   // low 16 bits: tile width; above: how A is loaded
   if (bn_wide || box_ok || flat_ok) {
-    p.bn = p.n_tiles = 0;
-    p.a_mode = A_IM2COL_K;
-    const PlanKey ckey = plan_key(p);
+    key_p.bn = key_p.n_tiles = 0;
+    const PlanKey ckey = plan_key(key_p);
     std::lock_guard<std::mutex> lock(g_plan_mutex);   // released at the end of this block, before `launch` takes it
     auto it = g_bn_cache.find(ckey);
     const auto forced = g_opt.force_halo == 1 ? flat_candidates() : std::vector<std::pair<int, Plan>>();

@@ -71,9 +71,19 @@ static void remembered_flat_does_not_fit() {
   expect(conv(4, 64, 256, 111, 3, 1) == 0, "the same output at padding 1");
 }
 
+// What was measured for one row pitch says nothing about another: the same output at padding 1 (33) and 0 (34).
+static void paddings_are_measured_apart() {
+  measure(flat_is_fastest, 16, 64, 64, 32, 3, 1);
+  expect(conv(16, 64, 64, 32, 3, 1) == 0 && g_last_launch[MODE] == A_FLAT_K, "measured as flat");
+  expect(conv(16, 64, 64, 34, 3, 0) == 0 && g_last_launch[MODE] != A_FLAT_K, "not measured at padding 0");
+  measure(flat_is_fastest, 16, 64, 64, 34, 3, 0);
+  expect(conv(16, 64, 64, 34, 3, 0) == 0 && g_last_launch[MODE] == A_FLAT_K, "measured as flat at padding 0");
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
-      {"remembered_flat_does_not_fit", remembered_flat_does_not_fit}};
+      {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
+      {"paddings_are_measured_apart", paddings_are_measured_apart}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;
