@@ -1287,7 +1287,7 @@ static int make_map_nhwc(CUtensorMap* m, const void* ptr, uint64_t C, uint64_t W
 // Switches of the planner. Their initial values come from the environment (RB_GEMM_*), read once when the library
 // is first used; afterwards they change only through rb_gemm_set_option (tests, experiments).
 struct GemmOptions {
-  int force_mt = 0;          // RB_GEMM_FORCE_MT: 1 | 2 sub-tiles per item (0 = planner's choice)
+  int force_mt = 0;          // RB_GEMM_FORCE_MT: 1 | 2, flat mode up to 4, sub-tiles per item (0 = planner's choice)
   int force_resident = -1;   // RB_GEMM_FORCE_RESIDENT: 0 | 1
   int force_halo = -1;       // RB_GEMM_FORCE_HALO: whole input rows for all taps (flat mode): 0 = never, 1 = whenever feasible
   int force_taps = 0;        // RB_GEMM_FORCE_TAPS: filter taps per weight-grad tile
@@ -1606,6 +1606,7 @@ static Plan plan_shape(const GemmTcParams& p, bool allow_split, int fixed_split,
 // Fill in what follows from a plan; returns the grid size, or 0 when the plan does not fit.
 static int apply_plan(GemmTcParams& p, const Plan& pl) {
   if (p.a_mode == A_FLAT_K) return apply_flat_plan(p, pl);
+  if (pl.mt < 1 || pl.mt > 2) return 0;   // what issue_item is built for
   p.mt = pl.mt;
   p.split_k = pl.split;
   p.b_resident = pl.resident;
@@ -1922,7 +1923,8 @@ static int launch(GemmTcParams& p, bool allow_split, int fixed_split, bool b_is_
   if (pl.cost >= 1e299) return -3;
   bool forced = g_opt.force_mt || g_opt.force_resident >= 0 || g_opt.force_tail >= 0;
   if (g_opt.force_pair == 1 && pair_ok(p)) {   // pairs wherever they are feasible (tests, experiments)
-    for (int mt = g_opt.force_mt ? g_opt.force_mt : 2; mt >= 1; --mt) {
+    const int most = p.a_mode == A_FLAT_K ? 4 : 2;
+    for (int mt = g_opt.force_mt ? std::min(g_opt.force_mt, most) : 2; mt >= 1; --mt) {
       Plan pp{mt, pl.split, 0, 0, 0.0};
       pp.pair = 1;
       GemmTcParams q = p;

@@ -80,10 +80,28 @@ static void paddings_are_measured_apart() {
   expect(conv(16, 64, 64, 34, 3, 0) == 0 && g_last_launch[MODE] == A_FLAT_K, "measured as flat at padding 0");
 }
 
+// Three and four sub-tiles per item exist in flat mode only; a launch of another mode that is asked for them as CTA pairs must
+// not have accumulators that nothing computes.
+static void sub_tiles_of_other_modes() {
+  g_opt.force_pair = 1;
+  for (int mt = 1; mt <= 4; ++mt) {
+    g_opt.force_mt = mt;
+    expect(conv(16, 64, 64, 32, 3, 1) == 0 && g_last_launch[PAIR] == 1 && g_last_launch[MT] == (mt < 2 ? mt : 2), "im2col");
+    void* const at = (void*)0x1000;
+    expect(rb_gemm_tc(at, 0, 64, at, 0, 64, 4096, 64, 64, at, 64, 0, nullptr, 0, nullptr, 0, 0, 0, 0, nullptr, 0, nullptr, 0) == 0 &&
+               g_last_launch[PAIR] == 1 && g_last_launch[MT] == (mt < 2 ? mt : 2),
+           "matrix product");
+    g_opt.force_halo = 1;
+    expect(conv(16, 64, 64, 32, 3, 1) == 0 && g_last_launch[MODE] == A_FLAT_K && g_last_launch[MT] == mt, "flat");
+    g_opt.force_halo = -1;
+  }
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
       {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
-      {"paddings_are_measured_apart", paddings_are_measured_apart}};
+      {"paddings_are_measured_apart", paddings_are_measured_apart},
+      {"sub_tiles_of_other_modes", sub_tiles_of_other_modes}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;
