@@ -1305,7 +1305,8 @@ struct GemmOptions {
   int b_split = 1;
   int autotune = 1;          // RB_GEMM_AUTOTUNE: 0 = cost model only, even in tuning mode
   int deterministic = 0;     // RB_GEMM_DETERMINISTIC: 1 = no launch lets several CTAs add into the same output element
-                             // (no reduction split, no tail cut), so results are bit-identical from run to run
+                             // (no reduction split, no tail cut), so results are bit-identical from run to run, and the
+                             // order of additions does not depend on what is measured as the fastest (no flat mode)
 };
 static GemmOptions g_opt;
 static std::once_flag g_opt_once;
@@ -2211,7 +2212,8 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   };
   GemmTcParams key_p = p;
   const bool flat_fits = stride == 1 && R * S > 1 && flat_geom(key_p, N, H, W, R, S, pad_h, pad_w);
-  const bool flat_ok = flat_fits && g_opt.force_halo != 0;
+  // (flat mode adds the channel chunks outside the taps, all others inside: with `deterministic` timing must not choose the order)
+  const bool flat_ok = flat_fits && g_opt.force_halo != 0 && !g_opt.deterministic;
   auto flat_candidates = [&]() {      // (width, plan), best first
     std::vector<std::pair<int, Plan>> all;
     for (int nt = 1; nt <= 4 && flat_ok; ++nt) {

@@ -97,11 +97,28 @@ static void sub_tiles_of_other_modes() {
   }
 }
 
+// `deterministic`: every plan that timing may choose from adds the products of an output in one order. Flat mode has another
+// one (channel chunks outside, taps inside), so it is not among them, measured or forced.
+static void deterministic_keeps_one_order() {
+  measure(flat_is_fastest, 16, 128, 64, 32, 3, 1);
+  expect(conv(16, 128, 64, 32, 3, 1) == 0 && g_last_launch[MODE] == A_FLAT_K, "measured as flat");
+  g_opt.deterministic = 1;
+  expect(conv(16, 128, 64, 32, 3, 1) == 0 && g_last_launch[MODE] != A_FLAT_K, "measured before");
+  g_opt.force_halo = 1;
+  expect(conv(16, 128, 64, 32, 3, 1) == 0 && g_last_launch[MODE] != A_FLAT_K, "forced");
+  g_opt.force_halo = -1;
+  g_bn_cache.clear();
+  g_plan_cache.clear();
+  measure(flat_is_fastest, 16, 128, 64, 32, 3, 1);
+  expect(conv(16, 128, 64, 32, 3, 1) == 0 && g_last_launch[MODE] != A_FLAT_K, "measured under the option");
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
       {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
       {"paddings_are_measured_apart", paddings_are_measured_apart},
-      {"sub_tiles_of_other_modes", sub_tiles_of_other_modes}};
+      {"sub_tiles_of_other_modes", sub_tiles_of_other_modes},
+      {"deterministic_keeps_one_order", deterministic_keeps_one_order}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;
