@@ -1856,6 +1856,10 @@ static PlanKey plan_key(const GemmTcParams& p) {
                  p.cv_cchunks, p.fl_pitch, p.fl_hp);
 }
 
+// CTA pairs must win by 3 %: measured alone they tie to within 2 % on the layers tried, and inside a training step (other
+// kernels beside them) the plain plans did better.
+constexpr float PAIR_MARGIN = 0.97f;
+
 // Times the candidates of `p` (3 launches each, best of the last 2); returns the best time in ms, or a negative
 // value when nothing could be run.
 static float tune_plan(const GemmTcParams& p, bool b_is_weights, cudaStream_t stream, Plan* out,
@@ -1899,9 +1903,8 @@ static float tune_plan(const GemmTcParams& p, bool b_is_weights, cudaStream_t st
       if (ok) cudaEventElapsedTime(&t, e0, e1);
       if (ok && rep > 0 && t < ms) ms = t;   // the first run warms the caches
     }
-    // pairs are timed after every plain plan and must win by 3 %: measured alone they tie to within 2 % on the
-    // layers tried, and inside a training step (other kernels beside them) the plain plans did better
-    if (ok && ms < best_ms * (cands[c].pair && !given ? 0.97f : 1.0f)) {
+    // pairs are timed after every plain plan and must win by PAIR_MARGIN (a plan that is given: the caller's business)
+    if (ok && ms < best_ms * (cands[c].pair && !given ? PAIR_MARGIN : 1.0f)) {
       best_ms = ms;
       *out = cands[c];
     }
@@ -2253,7 +2256,7 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
         if (configure(q, how, bn)) return;
         Plan pl{1, 1, 0, 0, 0.0};
         const float ms = tune_plan(q, true, stream, &pl, given);
-        if (ms > 0.f && ms < best_ms) {
+        if (ms > 0.f && ms < best_ms * (given && given->pair ? PAIR_MARGIN : 1.0f)) {
           best_ms = ms;
           use = bn | (how << 16);
           g_plan_cache[plan_key(q)] = pl;
@@ -2263,7 +2266,9 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
         for (int bn : {bn_default, bn_wide})
           if (bn) measure(how, bn, nullptr);
       const auto flat = flat_candidates();
-      for (size_t i = 0; i < flat.size() && i < 5; ++i) measure(LOAD_FLAT, flat[i].first, &flat[i].second);
+      for (int pair = 0; pair <= 1; ++pair)
+        for (size_t i = 0; i < flat.size() && i < 5; ++i)
+          if (flat[i].second.pair == pair) measure(LOAD_FLAT, flat[i].first, &flat[i].second);
       g_bn_cache[ckey] = use;
     }
   }

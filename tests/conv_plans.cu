@@ -113,12 +113,29 @@ static void deterministic_keeps_one_order() {
   expect(conv(16, 128, 64, 32, 3, 1) == 0 && g_last_launch[MODE] != A_FLAT_K, "measured under the option");
 }
 
+// CTA pairs are taken where they win by 3 %, also in flat mode, whichever of the candidates is timed first.
+static float flat_pairs_win(const int* l, float by) { return l[MODE] != A_FLAT_K ? 2.f : l[PAIR] ? 1.f / by : 1.f; }
+static void pairs_win_by_a_margin() {
+  const struct { float (*time)(const int*); int pair; const char* what; } tries[] = {
+      {[](const int* l) { return flat_pairs_win(l, 1.02f); }, 0, "pairs 2 % faster"},
+      {[](const int* l) { return flat_pairs_win(l, 1.05f); }, 1, "pairs 5 % faster"},
+      {[](const int* l) { return flat_pairs_win(l, 0.99f); }, 0, "pairs slower"}};
+  for (auto& t : tries)
+    for (int Ko : {64, 128, 256, 384}) {
+      g_bn_cache.clear();
+      g_plan_cache.clear();
+      measure(t.time, 16, 128, Ko, 32, 3, 1);
+      expect(conv(16, 128, Ko, 32, 3, 1) == 0 && g_last_launch[MODE] == A_FLAT_K && g_last_launch[PAIR] == t.pair, t.what);
+    }
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
       {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
       {"paddings_are_measured_apart", paddings_are_measured_apart},
       {"sub_tiles_of_other_modes", sub_tiles_of_other_modes},
-      {"deterministic_keeps_one_order", deterministic_keeps_one_order}};
+      {"deterministic_keeps_one_order", deterministic_keeps_one_order},
+      {"pairs_win_by_a_margin", pairs_win_by_a_margin}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;
