@@ -2209,9 +2209,10 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   const int bn_wide = (n_cols > 256 && n_cols <= 512 && g_opt.force_wide != 0 && g_opt.bn_cap >= 256) ? n_cols : 0;
   const bool box_ok = stride == 1 && R * S > 1 && Q <= BM && g_opt.force_box != 0;
   // flat mode: the widths of one to four equal column tiles of at most 256 columns, 0 for those that are not
-  auto flat_bn = [n_cols](int nt) {
+  const int flat_cap = g_opt.bn_cap > 0 ? std::min(g_opt.bn_cap, 256) : 256;
+  auto flat_bn = [n_cols, flat_cap](int nt) {
     const int per = (n_cols + nt - 1) / nt, bn = nt == 1 ? (per + 31) / 32 * 32 : (per + 63) / 64 * 64;
-    return bn > 256 || bn * (nt - 1) >= n_cols ? 0 : bn;
+    return bn > flat_cap || bn * (nt - 1) >= n_cols ? 0 : bn;
   };
   GemmTcParams key_p = p;
   const bool flat_fits = stride == 1 && R * S > 1 && flat_geom(key_p, N, H, W, R, S, pad_h, pad_w);
@@ -2245,7 +2246,7 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
             ((box_ok && g_opt.force_box == 1) ? LOAD_BOX << 16 : 0);
     } else if (it != g_bn_cache.end()) {
       use = it->second;   // as far as it still applies: the options may have changed since it was measured
-      if ((use >> 16) == LOAD_FLAT && !flat_ok) use = bn_default;
+      if ((use >> 16) == LOAD_FLAT && (!flat_ok || (use & 0xFFFF) > flat_cap)) use = bn_default;
       if ((use >> 16) == LOAD_BOX && !box_ok) use &= 0xFFFF;
       if ((use >> 16) != LOAD_FLAT && (use & 0xFFFF) != bn_default && (use & 0xFFFF) != bn_wide)
         use = bn_default | (use & ~0xFFFF);

@@ -129,13 +129,30 @@ static void pairs_win_by_a_margin() {
     }
 }
 
+// `bn_cap` bounds the tile width of flat plans too, forced, measured, and measured before the option was set.
+static void flat_tiles_within_the_cap() {
+  g_opt.bn_cap = 128;
+  g_opt.force_halo = 1;
+  for (int Ko : {64, 128, 192, 256, 512}) expect(conv(16, 64, Ko, 32, 3, 1) == 0 && g_last_launch[WIDTH] <= 128, "forced");
+  g_opt.force_halo = -1;
+  measure(flat_is_fastest, 16, 64, 256, 32, 3, 1);
+  expect(conv(16, 64, 256, 32, 3, 1) == 0 && g_last_launch[MODE] == A_FLAT_K && g_last_launch[WIDTH] <= 128, "measured");
+  g_opt.bn_cap = 256;
+  g_bn_cache.clear();
+  measure(flat_of_256_is_fastest, 16, 64, 256, 32, 3, 1);
+  expect(conv(16, 64, 256, 32, 3, 1) == 0 && g_last_launch[MODE] == A_FLAT_K && g_last_launch[WIDTH] == 256, "measured at 256");
+  g_opt.bn_cap = 128;
+  expect(conv(16, 64, 256, 32, 3, 1) == 0 && g_last_launch[WIDTH] <= 128, "the cap came later");
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
       {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
       {"paddings_are_measured_apart", paddings_are_measured_apart},
       {"sub_tiles_of_other_modes", sub_tiles_of_other_modes},
       {"deterministic_keeps_one_order", deterministic_keeps_one_order},
-      {"pairs_win_by_a_margin", pairs_win_by_a_margin}};
+      {"pairs_win_by_a_margin", pairs_win_by_a_margin},
+      {"flat_tiles_within_the_cap", flat_tiles_within_the_cap}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;
