@@ -2298,13 +2298,13 @@ int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, 
 }
 
 // The same followed by a normalisation that is known beforehand, in the epilogue:
-// y = act(scale * conv(x) + shift [+ residual]), scale and shift (on a 16-byte boundary) per output column, residual laid out
-// like y.
+// y = act(scale * conv(x) + shift [+ residual]), scale and shift per output column, residual laid out like y; shift and residual
+// on a 16-byte boundary.
 int rb_conv_fprop_norm(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
                        int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* scale, const float* shift,
                        const void* residual, int relu, int n_valid, int n_store, float* ws, long long ws_bytes,
                        unsigned int* status, cudaStream_t stream) {
-  if (!scale || !shift || ((uintptr_t)shift & 15u)) return -10;
+  if (!scale || !shift || ((uintptr_t)shift & 15u) || ((uintptr_t)residual & 15u)) return -10;
   const NormForm form = {scale, residual};
   return conv_forward_form(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, shift, relu, nullptr, n_valid,
                            n_store, 0, nullptr, &form, ws, ws_bytes, status, stream);
@@ -2316,11 +2316,12 @@ int rb_conv_fprop_norm(const void* x, int N, int H, int W, int Cp, const void* w
 //   positions (s i + a, s j + b), is a stride-1 convolution of dy with every s-th filter tap, whose rows the epilogue
 //   scatters. A phase without taps gets mask(add), and nothing has to be done when add is dx itself and there is no mask.
 //   wt: null, or the filters transposed and flipped (rb_pack_dgrad_filters): then these are read, as a K-major operand.
-//   add, mask: optional, layout of dx; add may be dx. Returns -20 for a strided geometry with a phase of negative padding.
+//   add, mask: optional, layout of dx, add on a 16-byte boundary; add may be dx. Returns -20 for a strided geometry with a
+//   phase of negative padding.
 int rb_conv_dgrad_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp, int c_valid,
                      int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* add,
                      const void* mask, float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
-  if (stride < 1 || Cp % 32 != 0) return -10;
+  if (stride < 1 || Cp % 32 != 0 || ((uintptr_t)add & 15u)) return -10;
   struct Phase { int r0, c0, U, V, pt, pl, Hp, Wp; };
   auto phase = [&](int a, int b) {
     Phase f;

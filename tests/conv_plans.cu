@@ -145,6 +145,23 @@ static void flat_tiles_within_the_cap() {
   expect(conv(16, 64, 256, 32, 3, 1) == 0 && g_last_launch[WIDTH] <= 128, "the cap came later");
 }
 
+// The epilogue reads a residual (inference) or an addend (data-gradients) in 16-byte pieces: another alignment is an error.
+static void addends_are_aligned() {
+  for (int off = 0; off < 32; off += 2) {
+    const int want = off % 16 == 0 ? 0 : -10;
+    void *const at = (void*)0x1000, *const add = (void*)(0x2000 + (size_t)off);
+    for (int R : {1, 3}) {
+      const int pad = R / 2, before = g_launches;
+      expect(rb_conv_fprop_norm(at, 2, 8, 8, 32, at, 32, R, R, 1, pad, pad, 8, 8, at, 32, (const float*)at, (const float*)at, add,
+                                1, 32, 32, nullptr, 0, nullptr, 0) == want, "residual");
+      expect((g_launches != before) == (want == 0), "residual: launched");
+      for (int stride : {1, 2})
+        expect(rb_conv_dgrad_tc(at, 2, 8 / stride, 8 / stride, 32, at, nullptr, 32, 32, 32, R, R, stride, pad, pad, 8, 8, at, add,
+                                nullptr, nullptr, 0, nullptr, 0) == want, "addend");
+    }
+  }
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
       {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
@@ -152,7 +169,8 @@ int main(int argc, char** argv) {
       {"sub_tiles_of_other_modes", sub_tiles_of_other_modes},
       {"deterministic_keeps_one_order", deterministic_keeps_one_order},
       {"pairs_win_by_a_margin", pairs_win_by_a_margin},
-      {"flat_tiles_within_the_cap", flat_tiles_within_the_cap}};
+      {"flat_tiles_within_the_cap", flat_tiles_within_the_cap},
+      {"addends_are_aligned", addends_are_aligned}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;
