@@ -145,7 +145,7 @@ class Net:
             op.bind()
         # normalisations that inference passes leave to the convolutions before them (None: there are none)
         self.folded_norms = None
-        if self.device.type == "cuda":
+        if self.is_cuda:
             from .resnet_ops import FoldedNorms
             self.folded_norms = FoldedNorms.of(self)
         self._cpu_loss = None

@@ -423,6 +423,27 @@ def bn_fwd_infer(x, rows, C, c_valid, eps, run_mean, run_var, istd_tmp, gamma, b
               residual, y, relu)
 
 
+def bn_fold(params, units, n_units, out):
+    for g, b, rm, rv, at, C, c_valid, eps in units[:n_units].tolist():
+        eps = torch.tensor([eps], dtype=torch.int32).view(torch.float32)
+        vec = lambda o: params[o: o + c_valid]
+        scale = vec(g) * torch.rsqrt(vec(rv) + eps)
+        out[at: at + 2 * C] = 0
+        out[at: at + c_valid] = scale
+        out[at + C: at + C + c_valid] = vec(b) - vec(rm) * scale
+
+
+def conv_fprop_norm(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, scale, shift, residual=None, relu=False,
+                    n_valid=0, n_store=0):
+    acc = torch.zeros(N * P * Q, ldy)
+    conv_fprop_tc(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, acc, ldy, n_valid=n_valid, n_store=n_store)
+    live = n_valid or Kout
+    acc[:, :live] = acc[:, :live] * scale[:live] + shift[:live]
+    if residual is not None:
+        acc[:, :live] += _rows(residual, N * P * Q, ldy)[:, :live].float()
+    _finish(acc[:, :live], y, N * P * Q, ldy, None, relu, None, live, n_store or Kout)
+
+
 def bn_bwd(x, dy, y_relu, rows, C, c_valid, sums, mean, istd, gamma, dgamma, dbeta, dx):
     g = _rows(dy, rows, C)[:, :c_valid].float()
     if y_relu is not None:
@@ -494,8 +515,8 @@ def _unsupported(name):
 EMULATED = {f.__name__: f for f in (conv_fprop_tc, conv_wgrad_tc, conv_direct_fwd, conv_direct_wgrad,
                                     conv_direct_dgrad, pack_dgrad_filters, zero_s2d_structural, gemm_tc, bias_act,
                                     colsum, relu_mask, add_bf16, f32_to_bf16, act_fwd, act_bwd, pool_fwd, pool_bwd,
-                                    softmax_ce, input_u8, sgd_fused, bn_fwd_train, bn_fwd_infer, bn_bwd,
-                                    pointwise_loss, categorical_loss, lrn_fwd, lrn_bwd, dropout, var_input_u8, sgd_fused_grid,
+                                    softmax_ce, input_u8, sgd_fused, bn_fwd_train, bn_fwd_infer, bn_bwd, bn_fold,
+                                    conv_fprop_norm, pointwise_loss, categorical_loss, lrn_fwd, lrn_bwd, dropout, var_input_u8, sgd_fused_grid,
                                     axpy_shadow, gemm_set_option)}
 EMULATED.update(bn_fwd_train_ws=bn_fwd_train, bn_bwd_ws=bn_bwd)
 
