@@ -1,10 +1,13 @@
 """The form of the tensor-core convolution that keeps whole input rows in shared memory for all filter taps, against fp64: rows
 of one position to the longest that a load takes (and one longer, which another form runs), rows around 128 outputs, where
 sub-tiles change from 128 positions to one row, paddings of zero, of more than the filter reaches and on one side only, images
-of one row, filters of one row or column, several channel chunks, every number of sub-tiles per item, resident filters, pairs."""
+of one row, filters of one row or column, several channel chunks, every number of sub-tiles per item, resident filters, pairs;
+several items per CTA; data-gradients from filters read in place and packed, their strided phases, addends and masks."""
 import pytest
 import torch
 import torch.nn.functional as F
+
+from test_conv_dgrad_gpu import _run as data_gradient
 
 from rembrandt_b200.ops import layout
 from rembrandt_b200.ops import native_ops as K
@@ -47,3 +50,34 @@ def test_flat_convolution(case, options):
     ref = ref.permute(0, 2, 3, 1) * (m > 0)
     # operands are exact in bf16, sums are fp32: the rounding of the result, and the order of the additions of terms of size 1
     assert ((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1e-4).all()
+
+
+# several work items per CTA: rings of operands and both accumulator sets go on from item to item
+MANY = [(1200, 64, 13, 13, 64, 3, 3, 1, 1, 0, 0), (700, 160, 13, 12, 96, 3, 3, 1, 1, 0, 0), (500, 32, 13, 13, 320, 3, 3, 0, 1, 0, 0),
+        (160, 64, 8, 126, 64, 3, 3, 1, 1, 0, 0)]
+
+
+@pytest.mark.parametrize("options", [dict(force_mt=1), dict(force_mt=2), dict(force_mt=3), dict(force_mt=4),
+                                     dict(force_resident=1), dict(force_resident=0, force_pair=0), dict(force_pair=1)])
+@pytest.mark.parametrize("case", MANY)
+def test_many_items(case, options):
+    test_flat_convolution(case, options)
+    plan, (N, C, H, W, Ko, R, S, ph, pw) = K.gemm_last_launch(), case[:9]
+    # not less than: positions without the zero columns and rows, in whole items, by column tiles
+    items = N * (H + 2 * ph - R + 1) * (W + 2 * pw - S + 1) // (128 * plan["sub_tiles"]) * -(-Ko // plan["tile_width"])
+    assert items > plan["grid"]
+
+
+DGRADS = [  # N, C, Ko, H, k, stride, pad [, W]; the last phase of the strided ones has several taps
+    (5, 128, 128, 19, 3, 1, 1), (2, 256, 96, 13, 5, 1, 2), (3, 16, 40, 9, 3, 1, 1, 14), (900, 64, 64, 13, 3, 1, 1),
+    (37, 64, 32, 73, 3, 2, 1, 19), (2, 32, 64, 15, 3, 2, 1, 6), (1, 128, 256, 8, 5, 3, 2, 17), (300, 96, 64, 25, 3, 2, 1)]
+
+
+@pytest.mark.parametrize("options", [dict(), dict(force_mt=1), dict(force_mt=2), dict(force_mt=3), dict(force_mt=4),
+                                     dict(force_resident=1), dict(force_pair=1)])
+@pytest.mark.parametrize("add,masked", [(None, False), (None, True), ("own", True), ("dx", False), ("dx", True)])
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("shape", DGRADS)
+def test_flat_data_gradient(shape, packed, add, masked, options):
+    data_gradient(shape, add, masked, packed, force_halo=1, **options)
+    assert K.gemm_last_launch()["a_mode"] == FLAT
