@@ -30,7 +30,8 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=default",
 ]
 # --use_fast_math (approximate division / square root, flush-to-zero) only where no statistic, normaliser or loss is
-# computed: the tensor-core kernel's epilogue, pooling, data movement. Softmax / cross-entropy, LRN, batch-norm, the
+# computed: the tensor-core kernel's epilogue (it applies a normaliser that bn.cu has computed, by one fma), pooling, data
+# movement. Softmax / cross-entropy, LRN, batch-norm, the
 # optimizer and the exchange kernels that apply it are compiled with IEEE division and square root; where they call
 # an intrinsic such as __expf they do so explicitly.
 PRECISE_SOURCES = {"softmax_ce.cu", "lrn.cu", "bn.cu", "sgd_fused.cu", "comm_p2p.cu"}

@@ -18,7 +18,8 @@
 //     row's bytes: rows are kept 128 bytes wide (64 channels) even when that means a half-empty, zero-filled chunk;
 //   * the L2 delivers 10-12 TB/s into the shared memories, which is what binds layers of 64 and more channels; tiles are
 //     as wide as the layer allows (N <= 256);
-//   * a work item may cover two 128-row sub-tiles (mt = 2) that share one B stage and use two accumulators; when
+//   * a work item may cover two 128-row sub-tiles (mt = 2; up to four in flat mode) that share one B stage and use an
+//     accumulator each; when
 //     the whole B panel fits in shared memory and the CTA only ever needs that one panel, it is loaded once per CTA
 //     and stays resident (b_resident); split-K (fp32 reduce-add epilogue) spreads long reductions over all SMs;
 //   * which of these a forward / data-grad launch uses is decided by timing the candidates the first time a shape
@@ -516,7 +517,9 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
   // else (operands, bias, mask, output, workspace) calls `ahead_done` first, which returns when they have completed and
   // flushed: the producers right before their first load, when its coordinates have been worked out and its stage claimed
   // (1 - 2 us of integer divisions and first touches of code and parameters). Without the launch attribute the instructions
-  // do nothing.
+  // do nothing. The issuing warp does not call it: it waits for the first stage meanwhile, so the time that the kernels before
+  // this one still take after its blocks are resident counts against its wait limit (WAIT_LIMIT_NS; those that release their
+  // dependents early take a few milliseconds at most).
   bool ahead = true;
   auto ahead_done = [&ahead]() {
     if (!ahead) return;
@@ -1424,7 +1427,12 @@ static int tail_parts(long long items, int sms, int num_kb) {
 // SM: 128 -> 128 channels at two sub-tiles per item ask for 94, so the tensor pipe was 40 % busy; this asks for 25 to 41.
 // 96 -> 256 on 128 x 27 x 27, 5 x 5: data-gradient 115 -> 89 us; 256 -> 384 on 128 x 13 x 13: 42 -> 35; 16 -> 16 on
 // 128 x 32 x 32: 19.6 -> 16.2; 64 -> 128 on 64 x 128 x 128: data-gradient 205 -> 187.
+// Counted on 32 images of the first of these: 604 -> 198 MB into shared memory, 62 -> 55 us.
 // Sub-tiles start 128 positions apart, or, on rows of at least 128 positions with at most 128 outputs, one row apart.
+// Rows of 113 to 127 positions are made 128 long for that: 3 x 3, 64 -> 64 / 128 / 256, 16 images of 112 x 112, as they are
+// 44 / 58 / 107 us, 128 long 34 / 41 / 59 (tap by tap: 34 / 36 / 54); from 124 on they do not fit as they are. Shorter rows
+// would gain too (111: 44 / 47 / 81 against 32 / 38 / 56; 99: 29 / 39 / 60 against 30 / 37 / 52), but there the tap-by-tap plans
+// are as fast or faster (32 / 38 / 54; 29 / 32 / 48) and the measurement takes those.
 static bool flat_geom(GemmTcParams& p, int N, int H, int W, int R, int S, int pad_h, int pad_w) {
   const int P = p.cv_P, Q = p.cv_Q;
   const int share_w = std::max(0, std::min({pad_w, S - 1, Q + S - 1 - pad_w - W}));
@@ -1851,7 +1859,8 @@ static std::mutex g_plan_mutex;
 
 static PlanKey plan_key(const GemmTcParams& p) {
   return PlanKey(p.a_mode, p.b_mode, p.M, p.N, p.num_kb, p.bn, p.bk, p.n_tiles, p.cv_stride,
-                 // (a forward pass with its normalisation takes the plan of the one without)
+                 // (a forward pass with its normalisation takes the plan that was measured for the one without: it is not timed
+                 // by itself)
                  (p.mask_src ? 1 : 0) | (p.add_src && !p.scale ? 2 : 0) | (p.sc_stride ? 4 : 0), p.cv_P, p.cv_Q, p.cv_S,
                  p.cv_cchunks, p.fl_pitch, p.fl_hp);
 }
@@ -2158,7 +2167,8 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   if (mask_src) rc = make_map_out(&p.tm_mask, const_cast<void*>(mask_src), p.n_store, p.M, ldy);
   if (rc) return rc;
   // How the A operand is loaded (`how`: LOAD_BOX = tap-shifted tiled boxes of whole output rows, LOAD_FLAT = whole input
-  // rows once for all taps, else the im2col map, or plain tiled rows for a 1 x 1 convolution) and what depends on the tile width: column tiling, the filter map's box.
+  // rows once for all taps, else the im2col map, or plain tiled rows for a 1 x 1 convolution) and what depends on the tile
+  // width: column tiling, the filter map's box.
   enum { LOAD_BOX = 1, LOAD_FLAT = 2 };
   auto configure = [&](GemmTcParams& q, int how, int bn) -> int {
     int e;
@@ -2201,8 +2211,9 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   //  * for stride-1 convolutions with more than one tap and output rows of at most 128 positions, box loads:
   //    cheaper per row for the TMA unit, at the price of tile rows that are computed and dropped when Q does not
   //    divide 128 (and when bx_rows does not divide P).
-  //  * for stride-1 convolutions with more than one tap, flat mode: the first few plans by its cost model, which is good
-  //    enough for these to hold the best.
+  //  * for stride-1 convolutions with more than one tap, flat mode: the first five plans by its cost model. On 76 layers and
+  //    directions of this framework's networks these held the best plan that beat the other modes in all but one, which
+  //    loses 3 %.
   // Which is fastest is decided by measurement in tuning mode and remembered per shape; without a measurement the
   // default is taken.
   const int bn_default = p.bn;

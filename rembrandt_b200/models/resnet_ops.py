@@ -3,7 +3,8 @@
 Counterparts of the reference's ``BNormConv2dOperator`` (src/operator/conv.rs:52-912),
 ``StackResConv2dOperator`` (:914-2182, identity shortcut) and ``ProjStackResConv2dOperator`` (:2184-3852,
 1x1 strided projection shortcut). Convolutions run on the tcgen05 implicit-GEMM kernel without bias;
-normalisation, the residual add and the ReLU are one apply kernel after a statistics pass. Parameters per
+in training, normalisation, the residual add and the ReLU are one apply kernel after a statistics pass; at inference
+they are the convolution's epilogue (`FoldedNorms`; first layers of the special forms keep their own apply kernel). Parameters per
 normalised convolution: filter, scale, bias, running mean, running variance, in that order in the blob
 (conv.rs:379-406); only filter, scale and bias receive gradients; none of the normalisation parameters is
 L2-regularised (conv.rs:637-651).
@@ -22,9 +23,9 @@ from .operators import DataOp, Op, ParamSeg, _draw, conv_out
 
 
 class FoldedNorms:
-    """Scale and shift of the normalised convolutions of a network (but first layers) by their running statistics, worked out by one launch at the
-    start of an inference pass; each convolution then normalises, adds the residual and applies the ReLU in its epilogue, which
-    saves a launch and two passes over the output (ResNet-18, 50 images: 904 -> 843 us a pass)."""
+    """Scale and shift of the normalised convolutions of a network (but first layers) by their running statistics, worked out by
+    one launch at the start of an inference pass; each convolution then normalises, adds the residual and applies the ReLU in its
+    epilogue, which saves a launch and two passes over the output (ResNet-18, 50 images: 904 -> 843 us a pass)."""
 
     def __init__(self, net, units):
         self.net, self.n = net, len(units)
@@ -40,7 +41,8 @@ class FoldedNorms:
 
     @staticmethod
     def of(net):
-        # a first layer keeps its own launch: its plain output is what the input's window is checked by
+        # a first layer that reads whole windows or a space-to-depth image keeps its own launch: its plain output is what the
+        # input's window is checked by
         units = [u for op in net.ops if isinstance(op, _BlockBase) for u in op.units if not u.windowed and u.s2d is None]
         return FoldedNorms(net, units) if units else None
 

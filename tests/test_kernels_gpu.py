@@ -116,8 +116,8 @@ CONV_CASES = [
     (130, 32, 8, 8, 32, 5, 1, 2),
     (2, 64, 14, 14, 96, 3, 1, 1),     # data-grad reduces over 96 channels: a half-empty 64-channel chunk
     (2, 160, 9, 9, 64, 3, 1, 1),
-    (1, 32, 40, 40, 64, 3, 1, 1),     # halo mode: row pitch 64 (two output rows per sub-tile)
-    (1, 32, 70, 66, 32, 3, 1, 1),     # halo mode: row pitch 128, non-square
+    (1, 32, 40, 40, 64, 3, 1, 1),     # whole rows in shared memory: 41 positions a row, three rows and a bit per sub-tile
+    (1, 32, 70, 66, 32, 3, 1, 1),     # the same at 67 positions a row, non-square
     (128, 64, 13, 13, 64, 3, 1, 1),   # 169 row tiles on 148 SMs: the 21 of the last wave are cut along the reduction
     (128, 32, 13, 13, 320, 3, 1, 1),  # the same with one 320-column tile (two MMAs side by side)
     (40, 64, 27, 27, 64, 5, 1, 2),    # box loads: 4 output rows per sub-tile, 280 tiles, ragged last band of each tile
@@ -140,7 +140,7 @@ def _conv_setup(N, C, H, W, Ko, R, stride, pad, seed=0):
                         "wide", "wide_tail", "box", "box_mt2", "box_tail", "box_wide", "pair", "pair_mt1", "tuned"])
 def tile_mode(request):
     """Force the kernel's tile-shape planner through each of its modes (two sub-tiles per item, resident B,
-    column-shifted halo tiles for stride-1 convolutions, the last wave cut along the reduction, one tile as wide as
+    whole input rows in shared memory for stride-1 convolutions ("halo"), the last wave cut along the reduction, one tile as wide as
     the layer, tap-shifted box loads of whole output rows, CTA pairs issuing 256-row MMAs, plans chosen by
     measurement)."""
     mode = request.param
