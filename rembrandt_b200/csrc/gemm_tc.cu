@@ -61,6 +61,12 @@ constexpr int EPI_WARPS = 8;
 constexpr int MAX_STAGES = 8;
 constexpr int MAX_A_STAGES = 3;   // flat mode
 constexpr int TILE_SMEM_BYTES = 192 * 1024;   // B panel (if resident) + stage ring
+// The lean instantiation (weight-gradients that run beside other kernels of the step): what it leaves of an SM's shared memory
+// holds a block of the normalisation kernels (17 KB), and its registers leave room for one (20 - 26 K of 34.8 K). With 96 KB
+// a 256-column tile has two stages instead of three: Go network's step at 256 boards 1567 us, with 144 KB 1529, with all of
+// the shared memory (nothing beside it) 1650.
+constexpr int LEAN_TILE_BYTES = 144 * 1024;
+constexpr int LEAN_MAX_REGS = 80;
 constexpr int STAGING_BYTES = 32 * 1024;      // epilogue: 8 warps x one slab of 32 rows x 128 B
 constexpr int GEMM_SMEM_BYTES = TILE_SMEM_BYTES + STAGING_BYTES + 1024 /*align*/ + 512 /*barriers*/;
 constexpr uint64_t WAIT_LIMIT_NS = 2000000000ull;  // 2 s
@@ -425,15 +431,17 @@ __device__ __forceinline__ void epilogue_norm(bool relu, bool addend, const uint
 // step at 64 images: 1255 instead of 1186 us).
 // FLAT: the instantiation for A_FLAT_K, whose rows are always scattered (EXT).
 // NORM: the instantiation for launches with a scale (EXT).
-template <bool PAIR, bool EXT, bool FLAT, bool NORM>
-__global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant__ GemmTcParams p) {
+// LEAN: the instantiation for fp32 output with fewer registers (74: the bf16 epilogues are what takes 138) and less shared
+// memory, for launches beside which others are to run.
+template <bool PAIR, bool EXT, bool FLAT, bool NORM, bool LEAN>
+__global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant__ GemmTcParams p) {
 #ifdef RB_GEMM_PROFILE
   const long long t_kernel0 = clock64();
 #endif
   extern __shared__ uint8_t smem_raw[];
   // tiles start on a 1024-byte boundary (swizzle atoms); control block follows the tiles
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* staging = tiles + TILE_SMEM_BYTES;
+  uint8_t* staging = tiles + (LEAN ? LEAN_TILE_BYTES : TILE_SMEM_BYTES);
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(staging + STAGING_BYTES);
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);   // known to be the same in all lanes
@@ -968,7 +976,7 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
         }
         const uint32_t t_addr =
             tmem_base + (uint32_t)acc * set_cols + (uint32_t)(j * p.acc_stride) + ((uint32_t)lane_base << 16);
-        if (p.epi == EPI_BF16 && !tail) {
+        if (!LEAN && p.epi == EPI_BF16 && !tail) {
           // row of D that this lane's row belongs to (-1: none); only scattered rows and an addend need it
           const bool scatter = FLAT || (EXT && p.sc_stride != 0);
           const bool addend = EXT && p.add_src != nullptr;
@@ -1150,11 +1158,14 @@ __global__ void __maxnreg__(GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant_
 
 typedef void (*Kernel)(GemmTcParams);
 static const Kernel KERNELS[] = {   // without and with CTA pairs
-    gemm_tc_kernel<false, false, false, false>, gemm_tc_kernel<true, false, false, false>,
-    gemm_tc_kernel<false, true, false, false>,  gemm_tc_kernel<true, true, false, false>,
-    gemm_tc_kernel<false, true, true, false>,   gemm_tc_kernel<true, true, true, false>,
-    gemm_tc_kernel<false, true, false, true>,   gemm_tc_kernel<true, true, false, true>,
-    gemm_tc_kernel<false, true, true, true>,    gemm_tc_kernel<true, true, true, true>};
+    gemm_tc_kernel<false, false, false, false, false>, gemm_tc_kernel<true, false, false, false, false>,
+    gemm_tc_kernel<false, true, false, false, false>,  gemm_tc_kernel<true, true, false, false, false>,
+    gemm_tc_kernel<false, true, true, false, false>,   gemm_tc_kernel<true, true, true, false, false>,
+    gemm_tc_kernel<false, true, false, true, false>,   gemm_tc_kernel<true, true, false, true, false>,
+    gemm_tc_kernel<false, true, true, true, false>,    gemm_tc_kernel<true, true, true, true, false>,
+    gemm_tc_kernel<false, false, false, false, true>};
+constexpr int LEAN_KERNEL = 10;
+static int tile_bytes(const GemmTcParams& p) { return p.lean ? LEAN_TILE_BYTES : TILE_SMEM_BYTES; }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -1204,7 +1215,7 @@ static int ensure_driver_entry() {
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     int nc = 0;
-    if (cudaOccupancyMaxActiveClusters(&nc, gemm_tc_kernel<true, true, true, false>, &cfg) != cudaSuccess) nc = 0;
+    if (cudaOccupancyMaxActiveClusters(&nc, gemm_tc_kernel<true, true, true, false, false>, &cfg) != cudaSuccess) nc = 0;
     cudaGetLastError();   // a refused query must not be taken for a failed launch later
     g_pair_clusters = nc > g_num_sms / 2 ? g_num_sms / 2 : nc;
   }
@@ -1580,8 +1591,8 @@ static Plan plan_shape(const GemmTcParams& p, bool allow_split, int fixed_split,
         const long long panel = (long long)p.num_kb * b_bytes;
         if (res) {
           if (!b_is_weights || p.n_tiles != 1 || s != 1 || panel > 112 * 1024) continue;
-          if ((TILE_SMEM_BYTES - panel) / (mt * a_bytes) < 3) continue;
-        } else if (TILE_SMEM_BYTES / (mt * a_bytes + b_bytes) < 2) {
+          if ((tile_bytes(p) - panel) / (mt * a_bytes) < 3) continue;
+        } else if (tile_bytes(p) / (mt * a_bytes + b_bytes) < 2) {
           continue;
         }
         const int kbs = (p.num_kb + s - 1) / s;
@@ -1631,8 +1642,8 @@ static int apply_plan(GemmTcParams& p, const Plan& pl) {
   const int a_bytes = BM * p.bk * 2, b_bytes = p.bn_load * p.bk * 2;
   const int panel = p.b_resident ? p.num_kb * b_bytes : 0;
   const int stage = p.mt * a_bytes + (p.b_resident ? 0 : b_bytes);
-  if (panel >= TILE_SMEM_BYTES) return 0;
-  p.stages = (TILE_SMEM_BYTES - panel) / stage;
+  if (panel >= tile_bytes(p)) return 0;
+  p.stages = (tile_bytes(p) - panel) / stage;
   // Two slab buffers per epilogue warp where the main loop is too short to hide the epilogue and the stages that are left
   // still cover a whole item or are four.
   p.epi_bufs = 1;
@@ -1779,7 +1790,7 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
     memset(&cfg, 0, sizeof(cfg));
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = GEMM_SMEM_BYTES;
+    cfg.dynamicSmemBytes = (size_t)(GEMM_SMEM_BYTES - TILE_SMEM_BYTES + tile_bytes(p));
     cfg.stream = stream;
     cudaLaunchAttribute at[2];
     int n_at = 0;
@@ -1798,7 +1809,8 @@ static int run_plan(GemmTcParams p, const Plan& pl, cudaStream_t stream) {
     cfg.attrs = n_at ? at : nullptr;
     cfg.numAttrs = (unsigned)n_at;
     const int form = p.a_mode == A_FLAT_K ? 2 : p.scale || p.sc_stride != 0 || p.add_src != nullptr ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, KERNELS[(p.scale ? 2 * (form + 2) : 2 * form) + (p.pair ? 1 : 0)], p);
+    const int which = p.lean ? LEAN_KERNEL : (p.scale ? 2 * (form + 2) : 2 * form) + (p.pair ? 1 : 0);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, KERNELS[which], p);
     if (e != cudaSuccess) {
       g_last_cuda_error = (int)e;
       cudaGetLastError();
@@ -2388,14 +2400,16 @@ int rb_conv_dgrad_tc(const void* dy, int N, int P, int Q, int Kp, const void* w,
 
 // Convolution weight-grad:  dw[Kout][R*S][Cp] (fp32) (+)= sum over pixels dy[pix][k] * x[pix shifted by tap][c].
 //   The result is always accumulated into dw (red.add), so dw holds zeros or the running gradient on entry.
+//   beside: the launch is to leave room on the SMs for kernels that run at the same time (the lean instantiation).
 int rb_conv_wgrad_tc(const void* x, int N, int H, int W, int Cp, const void* dy, long long lddy, int Kout, int R,
-                     int S, int stride, int pad_h, int pad_w, int P, int Q, float* dw, int split_k,
+                     int S, int stride, int pad_h, int pad_w, int P, int Q, float* dw, int split_k, int beside,
                      unsigned int* status, cudaStream_t stream) {
   int rc = ensure_driver_entry();
   if (rc) return rc;
   GemmTcParams p;
   memset(&p, 0, sizeof(p));
   p.bk = 64;
+  p.lean = beside ? 1 : 0;
   p.M = Kout;
   p.N = R * S * Cp;
   const long long pixels = (long long)N * P * Q;

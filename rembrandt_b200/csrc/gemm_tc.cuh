@@ -114,6 +114,7 @@ struct alignas(64) GemmTcParams {
   // own TMEM. The even CTA issues one 256 x bn x 16 MMA where two CTAs alone would issue two 128 x bn x 16 ones,
   // and each SM reads only half of B from its shared memory.
   int pair;
+  int lean;            // fp32 output: the instantiation with less shared memory and fewer registers
 };
 
 // Row of D (and mask, addend) that row m of the product belongs to.

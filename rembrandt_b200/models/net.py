@@ -135,6 +135,7 @@ class Net:
         # DRAM and most of the register file idle; `side` forks, `join_side` joins (both are captured into graphs).
         self._side = None
         self._side_dirty = False
+        self._collected = False  # backward hands every operator's gradients on as soon as they are there
         if self.device.type == "cuda":
             self._side = torch.cuda.Stream(self.device)
             self._side_fork, self._side_join = torch.cuda.Event(), torch.cuda.Event()
@@ -270,6 +271,15 @@ class Net:
             fn()
         self._side_dirty = True
 
+    def beside(self, fn):
+        """Run `fn` (launches of a weight-gradient) beside what backward goes on with: on the side stream, as `fn(beside=True)`,
+        while a step is captured; here and now, as `fn()`, where a hook would wait for it at once, or where the events cost
+        the host more than they save (eager steps)."""
+        if self._side is None or self._collected or not torch.cuda.is_current_stream_capturing():
+            fn()
+        else:
+            self.side(lambda: fn(beside=True))
+
     def join_side(self):
         """Make the current stream wait for everything issued on the side stream."""
         if self._side is not None and self._side_dirty:
@@ -323,6 +333,7 @@ class Net:
         """Backward in reverse operator order. `hook(i)` is called after operator i has produced its parameter
         gradients (the communication backends start a bucket's exchange from it)."""
         if self.is_cuda:
+            self._collected = hook is not None
             for i in range(len(self.ops) - 2, 0, -1):
                 with span(self.ops[i].name):
                     self.ops[i].backward()

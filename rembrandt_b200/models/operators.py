@@ -594,6 +594,7 @@ class Conv2dOp(Op):
 
     has_params = True
     takes_windows = True     # as a first layer: reads whole receptive fields from the input operator where that pays
+    SMALL_WGRAD_FLOPS = 0.5e9
 
     def setup(self, net, prev):
         super().setup(net, prev)
@@ -689,9 +690,20 @@ class Conv2dOp(Op):
             K.conv_direct_wgrad(self.prev.out, self.dout, gw, n, h, w, self.cp, ko, self.out_cp, r, r, s, p, p, self.P,
                                 self.Q)
         else:
-            K.conv_wgrad_tc(self.prev.out, n, h, w, self.cp, self.dout, self.out_cp, ko, r, r, s, p, p, self.P,
-                            self.Q, gw)
-        if self.s2d:
+            def wgrad(beside=False):
+                K.conv_wgrad_tc(self.prev.out, n, h, w, self.cp, self.dout, self.out_cp, ko, r, r, s, p, p, self.P,
+                                self.Q, gw)
+                if self.s2d:
+                    K.zero_s2d_structural(gw, ko, self.r2, self.cp, self.f, self.in_c, self.cfg.conv_size)
+
+            # A small one is all latency, and the data-gradient, which does not depend on it, runs in the same time (LeNet's
+            # step at 64 images 127 -> 113 us, affine layers included). One that fills the SMs only gets into the way of the
+            # data-gradient's blocks (NIN at 64 images: 897 us as it is, 938 with all of them beside).
+            if 2.0 * rows * r * r * self.cp * self.out_cp < self.SMALL_WGRAD_FLOPS:
+                self.net.beside(wgrad)
+            else:
+                wgrad()
+        if self.direct and self.s2d:
             K.zero_s2d_structural(gw, ko, self.r2, self.cp, self.f, self.in_c, self.cfg.conv_size)
         if self.wants_prev_delta():
             mask = self.mask_src()
@@ -878,8 +890,10 @@ class AffineOp(Op):
         # dW[out][in] += dY^T X : both operands are read "MN-major" straight from their row-major buffers
         # one pass over the batch: overwrite when this is the only micro-batch of the iteration, else accumulate
         epi = K.EPI_F32_ATOMIC if self.net.accumulate else K.EPI_F32_STORE
-        K.gemm_tc(self.dout, 1, self.out_cp, self.prev.out, 1, self.k_in, ko, self.k_in, n,
-                  self.view(self.seg_w, "grads"), self.k_in, epi=epi, n_store=self.k_in, split_k=1)
+        gw = self.view(self.seg_w, "grads")
+        # beside the data-gradient: both are bound by the memory their weights or gradients take, or by latency
+        self.net.beside(lambda beside=False: K.gemm_tc(self.dout, 1, self.out_cp, self.prev.out, 1, self.k_in, ko, self.k_in, n,
+                                                       gw, self.k_in, epi=epi, n_store=self.k_in, split_k=1))
         if self.wants_prev_delta():
             K.gemm_tc(self.dout, 0, self.out_cp, self.view(self.seg_w, "params16"), 1, self.k_in, n, self.k_in,
                       ko, self.ws_in, self.k_in, epi=K.EPI_F32_ATOMIC, n_store=self.k_in, split_k=0,

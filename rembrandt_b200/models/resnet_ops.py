@@ -142,11 +142,16 @@ class _BnConv:
         if self.windowed:
             self.windowed.backward(x, self.dconv, self.kp, gw)
             return
-        K.conv_wgrad_tc(x, n, self.gh, self.gw, self.cp, self.dconv, self.kp, self.ko, self.gk, self.gk, self.gs,
-                        self.gp, self.gp, self.P, self.Q, gw)
-        if self.s2d is not None:
-            # entries of the rearranged filter that no tap of the original filter maps to stay zero
-            K.zero_s2d_structural(gw, self.ko, self.gk, self.cp, self.f, self.in_c, self.k)
+
+        def wgrad(**kw):
+            K.conv_wgrad_tc(x, n, self.gh, self.gw, self.cp, self.dconv, self.kp, self.ko, self.gk, self.gk, self.gs,
+                            self.gp, self.gp, self.P, self.Q, gw, **kw)
+            if self.s2d is not None:
+                # entries of the rearranged filter that no tap of the original filter maps to stay zero
+                K.zero_s2d_structural(gw, self.ko, self.gk, self.cp, self.f, self.in_c, self.k)
+
+        # the normalisations that come next leave the tensor cores idle: the weight-gradient runs there meanwhile
+        net.beside(wgrad)
         if dx is not None:
             if self.s2d is not None:
                 raise RuntimeError("a space-to-depth'd convolution is a first layer: it has no input delta")

@@ -189,9 +189,10 @@ def tune_conv(N, H, W, Cp, Kout, R, S, stride, pad_h, pad_w, P, Q, ldy, relu=Fal
     torch.cuda.current_stream().synchronize()
 
 
-def conv_wgrad_tc(x, N, H, W, Cp, dy, lddy, Kout, R, S, stride, pad_h, pad_w, P, Q, dw, split_k=0):
+def conv_wgrad_tc(x, N, H, W, Cp, dy, lddy, Kout, R, S, stride, pad_h, pad_w, P, Q, dw, split_k=0, beside=False):
+    """`beside`: leave room on the SMs for kernels that run at the same time."""
     rc = _native.cuda().rb_conv_wgrad_tc(ptr(x), N, H, W, Cp, ptr(dy), lddy, Kout, R, S, stride, pad_h, pad_w, P, Q,
-                                         ptr(dw), split_k, ptr(status_word()), stream_handle())
+                                         ptr(dw), split_k, int(beside), ptr(status_word()), stream_handle())
     check(rc, "rb_conv_wgrad_tc")
 
 
