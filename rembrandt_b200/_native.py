@@ -29,6 +29,7 @@ _CUDA_SIGS = {
     "rb_conv_fprop_tc": [vp, i32, i32, i32, i32, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, i64, vp, i32, vp,
                          i32, i32, vp, i64, vp, vp],
     "rb_conv_dgrad_tc": [vp, i32, i32, i32, i32, vp, vp] + [i32] * 10 + [vp, vp, vp, vp, i64, vp, vp],
+    "rb_conv_dgrad_onto_tc": [vp, i32, i32, i32, i32, vp, vp] + [i32] * 10 + [vp, vp, vp, i64, vp, vp],
     "rb_conv_fprop_norm": [vp, i32, i32, i32, i32, vp, i32, i32, i32, i32, i32, i32, i32, i32, vp, i64, vp, vp, vp, i32, i32,
                            i32, vp, i64, vp, vp],
     "rb_gemm_set_option": [vp, i32],

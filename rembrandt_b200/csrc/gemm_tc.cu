@@ -42,6 +42,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -148,27 +149,42 @@ __device__ __forceinline__ bool ctl_wait_role(SharedCtl* ctl, uint64_t* bar, uin
 #define RB_PROF_ADD(cond, slot)
 #endif
 
-// base pixel (w, h, n) of output position `pix` for the im2col tensor maps
-__device__ __forceinline__ void pixel_coords(const GemmTcParams& p, int pix, int& w, int& h, int& n) {
-  const int pq = p.cv_P * p.cv_Q;
+// base pixel (w, h, n) of output position `pix` of a P x Q grid for the im2col tensor maps
+__device__ __forceinline__ void pixel_coords(int P, int Q, int stride, int lower_h, int lower_w, int pix, int& w, int& h, int& n) {
+  const int pq = P * Q;
   n = pix / pq;
   const int r2 = pix - n * pq;
-  const int pp = r2 / p.cv_Q;
-  const int qq = r2 - pp * p.cv_Q;
-  w = qq * p.cv_stride + p.cv_lower_w;
-  h = pp * p.cv_stride + p.cv_lower_h;
+  const int pp = r2 / Q;
+  const int qq = r2 - pp * Q;
+  w = qq * stride + lower_w;
+  h = pp * stride + lower_h;
 }
 
 // One unit of a CTA's work list: tile (tm, tn) over k-blocks [kb0, kb1). `tail` >= 0 marks a part of a cut item of
 // the last wave (index among the cut items); its sums go to the fp32 workspace instead of D.
 struct WorkItem {
-  int tm, tn, kb0, kb1, tail;
+  int tm, tn, kb0, kb1, tail, phase;
 };
-__device__ __forceinline__ WorkItem decode_work(const GemmTcParams& p, int work, int m_items, int direct,
-                                                int kb_per_split) {
+__device__ __forceinline__ const GemmPhase& phase_of(const GemmPhasesParams& p, int k) { return p.ph[k]; }
+__device__ __forceinline__ const GemmPhase& phase_of(const GemmTcParams& p, int) {      // never looked at
+  return *reinterpret_cast<const GemmPhase*>(&p);
+}
+__device__ __forceinline__ int phases_of(const GemmPhasesParams& p) { return p.phases; }
+__device__ __forceinline__ int phases_of(const GemmTcParams&) { return 0; }
+template <bool PHASES, class Params>
+__device__ __forceinline__ WorkItem decode_work(const Params& p, int work, int m_items, int direct, int kb_per_split) {
   WorkItem w;
   int rem;
-  if (p.tail_items > 0 && work >= direct) {
+  w.phase = 0;
+  if (PHASES) {
+    for (int k = 1; k < phases_of(p); ++k) w.phase = work >= phase_of(p, k).work0 ? k : w.phase;
+    const GemmPhase& ph = phase_of(p, w.phase);
+    rem = work - ph.work0;
+    m_items = ph.m_items;
+    w.kb0 = 0;
+    w.kb1 = ph.num_kb;
+    w.tail = -1;
+  } else if (p.tail_items > 0 && work >= direct) {
     const int w2 = work - direct;
     const int part = w2 / p.tail_items;
     w.tail = w2 - part * p.tail_items;
@@ -431,10 +447,12 @@ __device__ __forceinline__ void epilogue_norm(bool relu, bool addend, const uint
 // step at 64 images: 1255 instead of 1186 us).
 // FLAT: the instantiation for A_FLAT_K, whose rows are always scattered (EXT).
 // NORM: the instantiation for launches with a scale (EXT).
+// PHASES: the instantiation for several output phases of a strided data-gradient (EXT).
 // LEAN: the instantiation for fp32 output with fewer registers (74: the bf16 epilogues are what takes 138) and less shared
 // memory, for launches beside which others are to run.
-template <bool PAIR, bool EXT, bool FLAT, bool NORM, bool LEAN>
-__global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel(const __grid_constant__ GemmTcParams p) {
+template <bool PAIR, bool EXT, bool FLAT, bool NORM, bool LEAN, bool PHASES = false>
+__global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel(
+    const __grid_constant__ std::conditional_t<PHASES, GemmPhasesParams, GemmTcParams> p) {
 #ifdef RB_GEMM_PROFILE
   const long long t_kernel0 = clock64();
 #endif
@@ -470,7 +488,8 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
   const int n_tiles = p.n_tiles;
   // whole items first, then the parts of the cut items of the last wave (tail cut; never in flat mode)
   const int direct = m_items * n_tiles - p.tail_items;
-  const int num_work = p.tail_items > 0 ? direct + p.tail_items * p.tail_split : m_items * n_tiles * p.split_k;
+  const int num_work = PHASES ? phase_of(p, phases_of(p) - 1).work0 + phase_of(p, phases_of(p) - 1).m_items * n_tiles
+                     : p.tail_items > 0 ? direct + p.tail_items * p.tail_split : m_items * n_tiles * p.split_k;
   // flat mode: [A ring: fl_a_stages x fl_a_bytes][B ring: stages x b_bytes, or the resident panel]
   uint8_t* const b_ring = FLAT ? tiles + p.fl_a_stages * p.fl_a_bytes : tiles;
   const int kb_per_split = (p.num_kb + p.split_k - 1) / p.split_k;
@@ -493,10 +512,13 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
     for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&ctl->mask_bar[w], 1);
     ctl->abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&p.tm_a);
+    if (PHASES)
+      for (int k = 0; k < phases_of(p); ++k) tma_prefetch_desc(&phase_of(p, k).tm_a);
+    else
+      tma_prefetch_desc(&p.tm_a);
     tma_prefetch_desc(&p.tm_b);
-    tma_prefetch_desc(&p.tm_d);
-    if (p.epi == EPI_BF16 && p.mask_src) tma_prefetch_desc(&p.tm_mask);
+    if (!PHASES) tma_prefetch_desc(&p.tm_d);
+    if (!PHASES && p.epi == EPI_BF16 && p.mask_src) tma_prefetch_desc(&p.tm_mask);
     if (p.tail_items > 0) tma_prefetch_desc(&p.tm_ws);
   }
   if (warp == 1) {
@@ -650,7 +672,9 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
       else if (is_a) dst = aj * a_bytes + (a_mn_blocks ? aq * p.bk * 128 : aq * a_rows * p.bk * 2);
       else dst = mt * a_bytes + lane * (p.b_mode == B_TILED_K || p.b_mode == B_TILED_K3 ? b_rows * p.bk * 2 : p.bk * 128);
       // the taps of a convolution are walked in order; a weight-grad walks pixels, bk at a time
-      const int cchunks = p.cv_cchunks > 0 ? p.cv_cchunks : 1, taps_w = p.cv_S > 0 ? p.cv_S : 1;
+      const int cchunks = p.cv_cchunks > 0 ? p.cv_cchunks : 1;
+      int taps_w = p.cv_S > 0 ? p.cv_S : 1, dg_base = p.dg_base;
+      const CUtensorMap* map_a = &p.tm_a;
       int step_q = 0, step_p = 0, step_n = 0;
       if (mode == 8 + B_IM2COL_MN) {
         step_q = p.bk % p.cv_Q;
@@ -660,12 +684,21 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
       const int wg_apt = p.wg_taps > 1 ? p.wg_cw / 64 : 32;     // 64-column blocks per tap of a tile (one tap: all of them)
       const int wg_t = lane / wg_apt, wg_c = 64 * (lane - wg_t * wg_apt);
       for (int work = cta_id; work < num_work && ok; work += cta_step) {
-        const WorkItem it = decode_work(p, work, m_items, direct, kb_per_split);
+        const WorkItem it = decode_work<PHASES>(p, work, m_items, direct, kb_per_split);
+        const GemmPhase& phase = phase_of(p, it.phase);
+        if (PHASES) {
+          taps_w = phase.S;
+          dg_base = phase.dg_base;
+          map_a = &phase.tm_a;
+        }
         const int tn = it.tn, kb0 = it.kb0, kb1 = it.kb1;
         const int tm = pair ? it.tm * 2 + (int)cta_rank : it.tm;
         const int m0 = tm * BM * mt;
         int a_w = 0, a_h = 0, a_n = 0;   // first pixel of this lane's A load
-        if (mode == A_IM2COL_K && lane < nload) pixel_coords(p, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
+        if (mode == A_IM2COL_K && lane < nload) {
+          if (PHASES) pixel_coords(phase.P, phase.Q, 1, phase.lower_h, phase.lower_w, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
+          else pixel_coords(p.cv_P, p.cv_Q, p.cv_stride, p.cv_lower_h, p.cv_lower_w, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
+        }
         if (mode == A_BOX_K) {   // lane j loads sub-tile j: image a_n, first output row a_h
           a_n = tm / bx_groups;
           a_h = ((tm - a_n * bx_groups) * mt + lane) * p.bx_rows;
@@ -724,7 +757,7 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
                 break;
               case A_IM2COL_K:
                 if (pair) tma2_load_im2col_4d(to, &p.tm_a, bar2, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
-                else tma_load_im2col_4d(to, &p.tm_a, bar, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
+                else tma_load_im2col_4d(to, map_a, bar, cc * p.bk, a_w, a_h, a_n, (uint16_t)sx, (uint16_t)r);
                 break;
               case A_TILED_MN:   // two boxes of 64 rows(M) x bk per sub-tile
                 if (!pair) tma_load_2d(to, &p.tm_a, bar, m0 + aj * BM + 64 * aq, kb * p.bk);
@@ -753,7 +786,7 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
                               pn);
                 break;
               default: {   // B_TILED_K3, B_DGRAD_MN: tap of the filters in memory
-                const int wtap = p.dg_dv == 0 ? tap : p.dg_base + r * p.dg_du + sx * p.dg_dv;
+                const int wtap = p.dg_dv == 0 ? tap : dg_base + r * p.dg_du + sx * p.dg_dv;
                 const bool k3 = p.b_mode == B_TILED_K3;
                 const int c0 = k3 ? cc * p.bk : n0 + 64 * lane, c2 = k3 ? n0 + lane * b_rows : cc * p.bk;
                 if (pair) tma2_load_3d(to, &p.tm_b, bar2, c0, wtap, c2);
@@ -897,7 +930,7 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
       }
       const int issue_kind = (kk_steps == 4 ? 0 : 3) + (idesc2 ? 2 : (mt == 2 ? 1 : 0));
       for (int work = cta_id; work < num_work && ok && !FLAT; work += cta_step) {
-        const WorkItem it = decode_work(p, work, m_items, direct, kb_per_split);
+        const WorkItem it = decode_work<PHASES>(p, work, m_items, direct, kb_per_split);
         if (!ctl_wait_warp_role(ctl, &ctl->acc_empty[acc], acc_ph ^ 1u, p.status, 3)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)acc * set_cols;
@@ -937,7 +970,9 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
     uint32_t acc_ph = 0;
     bool ok = true;
     for (int work = cta_id; work < num_work && ok; work += cta_step) {
-      const WorkItem it = decode_work(p, work, m_items, direct, kb_per_split);
+      const WorkItem it = decode_work<PHASES>(p, work, m_items, direct, kb_per_split);
+      const GemmPhase& phase = phase_of(p, it.phase);
+      const int rows_d = PHASES ? phase.M : p.M;
       const int tn = it.tn;
       const int tm = pair ? it.tm * 2 + (int)cta_rank : it.tm;
       const bool tail = it.tail >= 0;
@@ -978,11 +1013,14 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
             tmem_base + (uint32_t)acc * set_cols + (uint32_t)(j * p.acc_stride) + ((uint32_t)lane_base << 16);
         if (!LEAN && p.epi == EPI_BF16 && !tail) {
           // row of D that this lane's row belongs to (-1: none); only scattered rows and an addend need it
-          const bool scatter = FLAT || (EXT && p.sc_stride != 0);
+          const bool scatter = FLAT || PHASES || (EXT && p.sc_stride != 0);
           const bool addend = EXT && p.add_src != nullptr;
           long long drow_of = -1;
           if (FLAT) drow_of = flat_row(p, (tm * mt + j) * p.fl_step + lane_base + lane);
-          else if ((scatter || addend) && lane < band_rows && row0 + lane < p.M)
+          else if (PHASES) {
+            if (row0 + lane < rows_d)
+              drow_of = scatter_row(row0 + lane, phase.P, phase.Q, p.sc_stride, phase.sc_a, phase.sc_b, p.sc_H, p.sc_W);
+          } else if ((scatter || addend) && lane < band_rows && row0 + lane < p.M)
             drow_of = scatter ? scatter_row(row0 + lane, p.cv_P, p.cv_Q, p.sc_stride, p.sc_a, p.sc_b, p.sc_H, p.sc_W)
                               : (long long)(row0 + lane);
           // 64-column slabs: TMEM -> registers -> bias / ReLU / mask -> swizzled shared memory -> TMA store.
@@ -1165,6 +1203,7 @@ static const Kernel KERNELS[] = {   // without and with CTA pairs
     gemm_tc_kernel<false, true, true, true, false>,    gemm_tc_kernel<true, true, true, true, false>,
     gemm_tc_kernel<false, false, false, false, true>};
 constexpr int LEAN_KERNEL = 10;
+static void (*const PHASES_KERNEL)(GemmPhasesParams) = gemm_tc_kernel<false, true, false, false, false, true>;
 static int tile_bytes(const GemmTcParams& p) { return p.lean ? LEAN_TILE_BYTES : TILE_SMEM_BYTES; }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1201,6 +1240,7 @@ static int ensure_driver_entry() {
   cudaDriverGetVersion(&g_driver_version);
   for (auto kern : KERNELS)
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) != cudaSuccess) return -2;
+  if (cudaFuncSetAttribute(PHASES_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) != cudaSuccess) return -2;
   {   // how many CTA pairs fit at once: the persistent loop of pair mode runs exactly that many clusters
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -2305,6 +2345,255 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   return rc ? rc : launch(p, false, 1, true, stream);
 }
 
+// The output phases of a strided data-gradient (conv_dgrad below) that have filter taps.
+struct DgradPhase {
+  int a, b;                    // positions (s i + a, s j + b)
+  int r0, c0, U, V, pt, pl;    // first tap, taps, padding of the stride-1 convolution that the phase is
+  int Hp, Wp;                  // positions
+};
+
+// All of them in ONE launch (GemmPhasesParams). Launched one by one, a phase's work of a few us lies between the set-up and the
+// drain of its own launch, and leaves SMs idle at its end. 3 x 3 / 2, us for four launches and for one, on a replayed graph:
+// 64 <- 128 channels on 32 x 64 x 64: 41.8, 20.9; 256 <- 512 on 32 x 16 x 16: 52.6, 17.8; 32 <- 64 on 128 x 16 x 16: 24.3, 7.8;
+// 32 <- 32 on 512 x 32 x 32: 68.6, 47.2. The filters are read in place or from their packed copy, the phases with more taps come
+// first, and tile width and sub-tiles per item are common to all.
+static int run_phases(GemmPhasesParams p, int bn, int mt, int n_cols, cudaStream_t stream) {
+  p.bn = bn;
+  p.bn_load = p.b_mode == B_DGRAD_MN ? (bn + 63) / 64 * 64 : bn;
+  p.n_tiles = (n_cols + bn - 1) / bn;
+  p.mt = mt;
+  p.acc_stride = acc_stride_for(bn);
+  p.acc_bufs = 2 * mt * p.acc_stride <= 512 ? 2 : 1;
+  if (bn > 256 || mt * p.acc_stride > 512) return -3;
+  p.stages = std::min(TILE_SMEM_BYTES / (mt * BM * p.bk * 2 + p.bn_load * p.bk * 2), MAX_STAGES);
+  if (p.stages < 2) return -3;
+  int work = 0;
+  for (int k = 0; k < p.phases; ++k) {
+    p.ph[k].work0 = work;
+    p.ph[k].m_items = (p.ph[k].M + BM * mt - 1) / (BM * mt);
+    work += p.ph[k].m_items * p.n_tiles;
+  }
+  const int grid = std::min(work, g_num_sms);
+  const int last[9] = {mt, 1, 0, 0, 0, bn, p.a_mode, p.stages, grid};
+  memcpy(g_last_launch, last, sizeof(last));
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = GEMM_SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = g_opt.pdl >= 1 ? 1u : 0u;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, PHASES_KERNEL, p);
+  if (e == cudaSuccess) return 0;
+  g_last_cuda_error = (int)e;
+  cudaGetLastError();
+  return -4;
+}
+
+typedef std::tuple<int, int, int, int, int, int, int, int, int, int, int, int, int, int> PhasesKey;
+static std::map<PhasesKey, std::pair<int, int>> g_phases_cache;      // tile width (0: one launch per phase) and sub-tiles
+
+// `separate`: runs the phases one by one. Returns -3 when that is what is to be done and nothing has been launched.
+template <class Separate>
+static int dgrad_phases(const void* dy, int N, int P, int Q, int Kp, const void* w, bool packed, int Kout, int Cp, int c_valid,
+                        int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* add, const void* mask,
+                        const DgradPhase* phases, int n_phases, unsigned int* status, cudaStream_t stream, Separate separate) {
+  int rc = ensure_driver_entry();
+  if (rc) return rc;
+  GemmPhasesParams p;
+  memset(&p, 0, sizeof(p));
+  p.bk = (Kp % 64 == 0 || (Kp > 64 && g_opt.bk32 != 1)) ? 64 : 32;
+  if (Kp % 32 != 0) return -10;
+  const CUtensorMapSwizzle ksw = p.bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+  p.N = Cp;
+  p.a_mode = A_IM2COL_K;
+  p.b_mode = packed ? B_TILED_K3 : B_DGRAD_MN;
+  p.cv_cchunks = (Kp + p.bk - 1) / p.bk;
+  p.cv_stride = 1;
+  p.a_split = pick_box_split(g_opt.a_split, BM, p.bk);
+  p.split_k = 1;
+  p.epi = EPI_BF16;
+  p.epi_bufs = 1;
+  p.n_valid = c_valid;
+  p.n_store = Cp;
+  p.ldd = Cp;
+  p.D = dx;
+  p.add_src = reinterpret_cast<const __nv_bfloat16*>(add);
+  p.mask_src = reinterpret_cast<const __nv_bfloat16*>(mask);
+  p.status = status;
+  p.sc_stride = stride;
+  p.sc_H = H;
+  p.sc_W = W;
+  p.dg_du = packed ? stride * S : -stride * S;
+  p.dg_dv = packed ? stride : -stride;
+  p.phases = n_phases;
+  int order[MAX_PHASES];
+  for (int k = 0; k < n_phases; ++k) order[k] = k;
+  std::stable_sort(order, order + n_phases, [&](int x, int y) { return phases[x].U * phases[x].V > phases[y].U * phases[y].V; });
+  double rows_kb = 0.0;      // 128-row tiles x k-blocks of the launch
+  for (int k = 0; k < n_phases; ++k) {
+    const DgradPhase& f = phases[order[k]];
+    GemmPhase& g = p.ph[k];
+    g.M = N * f.Hp * f.Wp;
+    g.num_kb = f.U * f.V * p.cv_cchunks;
+    g.P = f.Hp;
+    g.Q = f.Wp;
+    g.lower_h = -f.pt;
+    g.lower_w = -f.pl;
+    g.S = f.V;
+    g.dg_base = (f.r0 + stride * (f.U - 1)) * S + f.c0 + stride * (f.V - 1);
+    if (packed) g.dg_base = R * S - 1 - g.dg_base;      // tap t lies at R * S - 1 - t
+    g.sc_a = f.a;
+    g.sc_b = f.b;
+    p.M = std::max(p.M, g.M);
+    p.num_kb = std::max(p.num_kb, g.num_kb);
+    rows_kb += (double)((g.M + BM - 1) / BM) * g.num_kb;
+    rc = make_map_im2col(&g.tm_a, dy, N, P, Q, Kp, -f.pt, -f.pl, f.Hp - f.pt - P, f.Wp - f.pl - Q, 1, p.bk, BM / p.a_split, ksw);
+    if (rc) return rc;
+  }
+  auto with_b = [&](GemmPhasesParams& q, int bn) -> int {      // the filters' map, whose box depends on the tile width
+    const uint64_t taps = (uint64_t)R * S;
+    if (!packed)
+      return make_map_3d(&q.tm_b, w, Cp, taps, Kout, Cp, taps * Cp, 64, 1, q.bk, CU_TENSOR_MAP_SWIZZLE_128B);
+    q.b_split = pick_box_split(g_opt.b_split, bn, q.bk);
+    return make_map_3d(&q.tm_b, w, Kp, taps, Cp, Kp, taps * Kp, q.bk, 1, bn / q.b_split, ksw);
+  };
+  // Candidates: one to four equal column tiles, one or two sub-tiles. The model ranks them by rows filled per SM (see Plan) plus
+  // what is left when the longest item ends last.
+  std::pair<int, int> cands[8], best(0, 0);
+  int n_cands = 0;
+  double best_cost = 1e300;
+  const int cap = g_opt.bn_cap > 0 ? std::min(g_opt.bn_cap, 256) : 256;
+  for (int nt = 1; nt <= 4; ++nt) {
+    const int per = (Cp + nt - 1) / nt, bn = nt == 1 ? (per + 31) / 32 * 32 : (per + 63) / 64 * 64;
+    if (bn > cap || bn * (nt - 1) >= Cp) continue;
+    for (int mt = 1; mt <= 2; ++mt) {
+      if (g_opt.force_mt && mt != std::min(g_opt.force_mt, 2)) continue;
+      if (mt == 2 && p.M <= BM) continue;
+      const double item = p.num_kb * (mt * BM + bn) * (p.bk / 64.0) + 0.3 * mt * bn;
+      const double cost = rows_kb / mt * nt * (mt * BM + bn) * (p.bk / 64.0) / g_num_sms + 0.5 * item;
+      cands[n_cands++] = {bn, mt};
+      if (std::max(cost, item) < best_cost) {
+        best_cost = std::max(cost, item);
+        best = cands[n_cands - 1];
+      }
+    }
+  }
+  if (n_cands == 0) return -3;
+  {
+    const PhasesKey key(N, P, Q, Kp, Cp, H, W, R, S, stride, pad_h, pad_w, packed ? 1 : 0, (mask ? 1 : 0) | (add ? 2 : 0));
+    std::unique_lock<std::mutex> lock(g_plan_mutex);
+    auto it = g_phases_cache.find(key);
+    if (it != g_phases_cache.end()) {
+      if (!g_opt.force_mt && it->second.first <= cap) best = it->second;
+    } else if (tunable(p, stream)) {
+      cudaEvent_t e0, e1;
+      cudaEventCreate(&e0);
+      cudaEventCreate(&e1);
+      float best_ms = 1e30f;
+      auto measure = [&](std::pair<int, int> cand, float margin, auto run) {
+        float ms = 1e30f;
+        bool ok = true;
+        for (int rep = 0; rep < 3 && ok; ++rep) {
+          cudaEventRecord(e0, stream);
+          ok = run() == 0;
+          cudaEventRecord(e1, stream);
+          ok = ok && cudaEventSynchronize(e1) == cudaSuccess;
+          float t = 0.f;
+          if (ok) cudaEventElapsedTime(&t, e0, e1);
+          if (ok && rep > 0 && t < ms) ms = t;
+        }
+        if (ok && ms < best_ms * margin) {
+          best_ms = ms;
+          best = cand;
+        }
+      };
+      for (int i = 0; i < n_cands; ++i) {
+        GemmPhasesParams q = p;
+        if (with_b(q, cands[i].first) == 0)
+          measure(cands[i], 1.0f, [&]() { return run_phases(q, cands[i].first, cands[i].second, Cp, stream); });
+      }
+      lock.unlock();      // launches of their own, which look their plans up
+      measure({0, 0}, 0.95f, separate);
+      lock.lock();
+      g_phases_cache[key] = best;
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+    }
+  }
+  if (best.first == 0) return -3;
+  rc = with_b(p, best.first);
+  return rc ? rc : run_phases(p, best.first, best.second, Cp, stream);
+}
+
+// See rb_conv_dgrad_tc; `add_masked`: add is zero already where the mask is.
+static int conv_dgrad(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp, int c_valid,
+                      int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* add,
+                     const void* mask, int add_masked, float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
+  if (stride < 1 || Cp % 32 != 0 || ((uintptr_t)add & 15u)) return -10;
+  std::vector<DgradPhase> all, with_taps;
+  for (int a = 0; a < stride; ++a)
+    for (int b = 0; b < stride; ++b) {
+      DgradPhase f;
+      f.a = a;
+      f.b = b;
+      f.r0 = (a + pad_h) % stride;
+      f.c0 = (b + pad_w) % stride;
+      f.U = f.r0 < R ? (R - f.r0 + stride - 1) / stride : 0;
+      f.V = f.c0 < S ? (S - f.c0 + stride - 1) / stride : 0;
+      f.pt = f.U - 1 - (a + pad_h - f.r0) / stride;
+      f.pl = f.V - 1 - (b + pad_w - f.c0) / stride;
+      f.Hp = a < H ? (H - a + stride - 1) / stride : 0;
+      f.Wp = b < W ? (W - b + stride - 1) / stride : 0;
+      if (f.Hp <= 0 || f.Wp <= 0) continue;
+      const bool taps = f.U > 0 && f.V > 0;
+      if (stride > 1 && taps && (f.pt < 0 || f.pl < 0)) return -20;
+      all.push_back(f);
+      if (taps) with_taps.push_back(f);
+    }
+  for (const DgradPhase& f : all) {
+    if ((f.U > 0 && f.V > 0) || (add == dx && (!mask || add_masked))) continue;
+    const int rc = fill_phase((const __nv_bfloat16*)add, (const __nv_bfloat16*)mask, (__nv_bfloat16*)dx, N, f.Hp, f.Wp, stride, f.a,
+                              f.b, H, W, Cp, stream);
+    if (rc) return rc;
+  }
+  auto separate = [&]() -> int {
+    for (const DgradPhase& f : with_taps) {
+      DgradForm dg;
+      dg.packed = wt != nullptr;
+      dg.taps = R * S;
+      dg.base = (f.r0 + stride * (f.U - 1)) * S + f.c0 + stride * (f.V - 1);
+      dg.du = -stride * S;
+      dg.dv = -stride;
+      if (wt) {   // tap t lies at R * S - 1 - t
+        dg.base = R * S - 1 - dg.base;
+        dg.du = -dg.du;
+        dg.dv = -dg.dv;
+      }
+      dg.sc_stride = stride > 1 ? stride : 0;
+      dg.sc_a = f.a;
+      dg.sc_b = f.b;
+      dg.sc_H = H;
+      dg.sc_W = W;
+      dg.add = add;
+      const int rc = conv_forward_form(dy, N, P, Q, Kp, wt ? wt : w, Cp, f.U, f.V, 1, f.pt, f.pl, f.Hp, f.Wp, dx, Cp, nullptr, 0,
+                                       mask, c_valid, Cp, Kout, &dg, nullptr, ws, ws_bytes, status, stream);
+      if (rc) return rc;
+    }
+    return 0;
+  };
+  if (with_taps.size() >= 2 && with_taps.size() <= MAX_PHASES) {
+    const int rc = dgrad_phases(dy, N, P, Q, Kp, wt ? wt : w, wt != nullptr, Kout, Cp, c_valid, R, S, stride, pad_h, pad_w, H, W, dx,
+                                add, mask, with_taps.data(), (int)with_taps.size(), status, stream, separate);
+    if (rc != -3) return rc;
+  }
+  return separate();
+}
+
 }  // namespace rb
 
 extern "C" {
@@ -2344,58 +2633,17 @@ int rb_conv_fprop_norm(const void* x, int N, int H, int W, int Cp, const void* w
 int rb_conv_dgrad_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp, int c_valid,
                      int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* add,
                      const void* mask, float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
-  if (stride < 1 || Cp % 32 != 0 || ((uintptr_t)add & 15u)) return -10;
-  struct Phase { int r0, c0, U, V, pt, pl, Hp, Wp; };
-  auto phase = [&](int a, int b) {
-    Phase f;
-    f.r0 = (a + pad_h) % stride;
-    f.c0 = (b + pad_w) % stride;
-    f.U = f.r0 < R ? (R - f.r0 + stride - 1) / stride : 0;
-    f.V = f.c0 < S ? (S - f.c0 + stride - 1) / stride : 0;
-    f.pt = f.U - 1 - (a + pad_h - f.r0) / stride;
-    f.pl = f.V - 1 - (b + pad_w - f.c0) / stride;
-    f.Hp = a < H ? (H - a + stride - 1) / stride : 0;
-    f.Wp = b < W ? (W - b + stride - 1) / stride : 0;
-    return f;
-  };
-  for (int a = 0; a < stride; ++a)
-    for (int b = 0; b < stride; ++b) {
-      const Phase f = phase(a, b);
-      if (stride > 1 && f.U > 0 && f.V > 0 && f.Hp > 0 && f.Wp > 0 && (f.pt < 0 || f.pl < 0)) return -20;
-    }
-  for (int a = 0; a < stride; ++a)
-    for (int b = 0; b < stride; ++b) {
-      const Phase f = phase(a, b);
-      if (f.Hp <= 0 || f.Wp <= 0) continue;
-      if (f.U == 0 || f.V == 0) {
-        if (add == dx && !mask) continue;
-        const int rc = fill_phase((const __nv_bfloat16*)add, (const __nv_bfloat16*)mask, (__nv_bfloat16*)dx, N, f.Hp, f.Wp,
-                                  stride, a, b, H, W, Cp, stream);
-        if (rc) return rc;
-        continue;
-      }
-      DgradForm dg;
-      dg.packed = wt != nullptr;
-      dg.taps = R * S;
-      dg.base = (f.r0 + stride * (f.U - 1)) * S + f.c0 + stride * (f.V - 1);
-      dg.du = -stride * S;
-      dg.dv = -stride;
-      if (wt) {   // tap t lies at R * S - 1 - t
-        dg.base = R * S - 1 - dg.base;
-        dg.du = -dg.du;
-        dg.dv = -dg.dv;
-      }
-      dg.sc_stride = stride > 1 ? stride : 0;
-      dg.sc_a = a;
-      dg.sc_b = b;
-      dg.sc_H = H;
-      dg.sc_W = W;
-      dg.add = add;
-      const int rc = conv_forward_form(dy, N, P, Q, Kp, wt ? wt : w, Cp, f.U, f.V, 1, f.pt, f.pl, f.Hp, f.Wp, dx, Cp, nullptr, 0,
-                                       mask, c_valid, Cp, Kout, &dg, nullptr, ws, ws_bytes, status, stream);
-      if (rc) return rc;
-    }
-  return 0;
+  return conv_dgrad(dy, N, P, Q, Kp, w, wt, Kout, Cp, c_valid, R, S, stride, pad_h, pad_w, H, W, dx, add, mask, 0, ws, ws_bytes,
+                    status, stream);
+}
+
+// dx += mask(the gradient) where dx is zero already at the places that the mask zeroes: positions that no filter tap reaches
+// stay as they are, without a launch that would write them again.
+int rb_conv_dgrad_onto_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp,
+                          int c_valid, int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* mask,
+                          float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
+  return conv_dgrad(dy, N, P, Q, Kp, w, wt, Kout, Cp, c_valid, R, S, stride, pad_h, pad_w, H, W, dx, dx, mask, 1, ws, ws_bytes,
+                    status, stream);
 }
 
 // Convolution weight-grad:  dw[Kout][R*S][Cp] (fp32) (+)= sum over pixels dy[pix][k] * x[pix shifted by tap][c].
@@ -2557,6 +2805,7 @@ int rb_gemm_clear_plans() {
   std::lock_guard<std::mutex> lock(g_plan_mutex);
   g_plan_cache.clear();
   g_bn_cache.clear();
+  g_phases_cache.clear();
   return 0;
 }
 

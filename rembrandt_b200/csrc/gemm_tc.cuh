@@ -117,6 +117,25 @@ struct alignas(64) GemmTcParams {
   int lean;            // fp32 output: the instantiation with less shared memory and fewer registers
 };
 
+// One output phase of a strided data-gradient in a launch that runs several: what takes the place of the fields of the same
+// meaning in GemmTcParams.
+struct alignas(64) GemmPhase {
+  CUtensorMap tm_a;
+  int work0;           // first work item
+  int M, m_items, num_kb;
+  int P, Q, lower_h, lower_w, S;
+  int dg_base;
+  int sc_a, sc_b;
+};
+constexpr int MAX_PHASES = 4;
+
+// Phases of one strided data-gradient that share a launch (EPI_BF16, rows scattered, im2col loads, no tail cut, no pairs): its
+// work items are those of the phases one after the other.
+struct alignas(64) GemmPhasesParams : GemmTcParams {
+  int phases;
+  GemmPhase ph[MAX_PHASES];
+};
+
 // Row of D (and mask, addend) that row m of the product belongs to.
 __host__ __device__ inline long long scatter_row(int m, int P, int Q, int stride, int a, int b, int H, int W) {
   const int n = m / (P * Q), r = m - n * (P * Q);

@@ -131,8 +131,9 @@ class _BnConv:
             K.bn_fwd_infer(self.conv_out, rows, self.kp, self.ko, self.eps, self.v(self.seg_rm), self.v(self.seg_rv),
                            self.istd, self.v(self.seg_g), self.v(self.seg_b), residual, out, relu)
 
-    def backward(self, x, dout, y_relu, dx, mask, add=None):
-        """dout: delta w.r.t. the normalised output (masked by `y_relu` here if given); dx = mask(add + input delta)."""
+    def backward(self, x, dout, y_relu, dx, mask, add=None, add_masked=False):
+        """dout: delta w.r.t. the normalised output (masked by `y_relu` here if given); dx = mask(add + input delta);
+        add_masked: add is zero already where the mask is."""
         net = self.op.net
         n = net.batch
         rows = n * self.P * self.Q
@@ -156,7 +157,7 @@ class _BnConv:
             if self.s2d is not None:
                 raise RuntimeError("a space-to-depth'd convolution is a first layer: it has no input delta")
             conv_dgrad(self.dconv, n, self.P, self.Q, self.kp, self.v(self.seg_w, "params16"), self.ko, self.cp, self.in_c,
-                       self.k, self.s, self.p, self.h, self.w, dx, add=add, mask=mask,
+                       self.k, self.s, self.p, self.h, self.w, dx, add=add, mask=mask, add_masked=add_masked,
                        wt=self.dgrad.wt if self.dgrad else None)
 
     # ---- parameters
@@ -375,7 +376,7 @@ class ProjStackResConv2dOp(_BlockBase):
         # producer's ReLU is the same for both and may be applied to each
         dx, mask = (self.prev.dout, self.mask_src()) if need else (None, None)
         self.u1.backward(x, self.da1, None, dx, mask)
-        self.u3.backward(x, self.dout, None, dx, mask, add=dx)
+        self.u3.backward(x, self.dout, None, dx, mask, add=dx, add_masked=True)
 
     def ref_forward(self, x, train, t):
         sc = self.u3.ref(x, None, False, train, t)

@@ -1,7 +1,8 @@
 """Data-gradient of a convolution, any stride, as one call: dx = mask(add + gradient).
 
 On a GPU this is `rb_conv_dgrad_tc` (csrc/gemm_tc.cu): the filters are read as they lie (or from a transposed and flipped
-copy, `DgradPlan`), the output phases of a strided convolution are written straight to their places in dx, and the addend
+copy, `DgradPlan`), the output phases of a strided convolution share a launch and are written straight to their places in dx, and
+the addend
 (the delta of an identity path, or the gradient of a parallel branch already in dx) and the mask of the producer's ReLU
 ride in the epilogue. Strided geometries that it does not take, and all with RB_STRIDED_DGRAD_TC=0, run on the CUDA-core
 kernel. Without a GPU the result is put together from the kernel fronts of `native_ops`, which the CPU tests replace by
@@ -48,17 +49,20 @@ def _compose(dy, n, P, Q, kp, w16, ko, cp, in_c, k, stride, pad, H, W, dx, add, 
             dx.copy_(out)
 
 
-def conv_dgrad(dy, n, P, Q, kp, w16, ko, cp, in_c, k, stride, pad, H, W, dx, add=None, mask=None, wt=None):
+def conv_dgrad(dy, n, P, Q, kp, w16, ko, cp, in_c, k, stride, pad, H, W, dx, add=None, mask=None, wt=None, add_masked=False):
     """dy: bf16 [n, P, Q, kp]; w16: bf16 filters [ko][k * k][cp]; dx: bf16 [n, H, W, cp], overwritten; add, mask: optional,
     shaped like dx (add may be dx); dx is zero where mask <= 0 and in channels >= in_c. wt: the filters as
-    `native_ops.pack_dgrad_filters` writes them, to be read instead of w16."""
+    `native_ops.pack_dgrad_filters` writes them, to be read instead of w16. add_masked: add is zero already where the mask is."""
     if dy.device.type != "cuda" or _strided_on_cuda_cores(stride):
         _compose(dy, n, P, Q, kp, w16, ko, cp, in_c, k, stride, pad, H, W, dx, add, mask)
         return
     ws = K.gemm_workspace()
-    rc = _native.cuda().rb_conv_dgrad_tc(ptr(dy), n, P, Q, kp, ptr(w16), ptr(wt), ko, cp, in_c, k, k, stride, pad, pad, H, W,
-                                         ptr(dx), ptr(add), ptr(mask), ptr(ws), ws.numel() * 4, ptr(K.status_word()),
-                                         stream_handle())
+    geom = (ptr(dy), n, P, Q, kp, ptr(w16), ptr(wt), ko, cp, in_c, k, k, stride, pad, pad, H, W, ptr(dx))
+    tail = (ptr(mask), ptr(ws), ws.numel() * 4, ptr(K.status_word()), stream_handle())
+    if add_masked and add is not None and add.data_ptr() == dx.data_ptr():
+        rc = _native.cuda().rb_conv_dgrad_onto_tc(*geom, *tail)
+    else:
+        rc = _native.cuda().rb_conv_dgrad_tc(*geom, ptr(add), *tail)
     if rc == NEGATIVE_PADDING:      # e.g. a padding larger than the filter: the CUDA-core kernel takes any geometry
         _compose(dy, n, P, Q, kp, w16, ko, cp, in_c, k, stride, pad, H, W, dx, add, mask)
         return
