@@ -37,6 +37,7 @@ _CUDA_SIGS = {
     "rb_gemm_tune_mode": [i32],
     "rb_gemm_clear_plans": [],
     "rb_conv_wgrad_tc": [vp, i32, i32, i32, i32, vp, i64, i32, i32, i32, i32, i32, i32, i32, i32, vp, i32, i32, vp, vp],
+    "rb_conv_wgrad_tune": [vp, i32, i32, i32, i32, vp, i64, i32, i32, i32, i32, i32, i32, i32, vp, i32, vp, vp],
     "rb_num_sms": [],
     "rb_gemm_role_profile": [vp],
     "rb_gemm_last_launch": [vp],

@@ -1192,6 +1192,8 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
   }
 }
 
+#include "wgrad_rows.cuh"
+
 // =============================== host side ===============================
 
 typedef void (*Kernel)(GemmTcParams);
@@ -1240,6 +1242,7 @@ static int ensure_driver_entry() {
   cudaDriverGetVersion(&g_driver_version);
   for (auto kern : KERNELS)
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) != cudaSuccess) return -2;
+  if (cudaFuncSetAttribute(wgrad_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) != cudaSuccess) return -2;
   if (cudaFuncSetAttribute(PHASES_KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM_BYTES) != cudaSuccess) return -2;
   {   // how many CTA pairs fit at once: the persistent loop of pair mode runs exactly that many clusters
     cudaLaunchConfig_t cfg;
@@ -1357,6 +1360,7 @@ struct GemmOptions {
   int bn_cap = 256;          // RB_GEMM_BN_CAP: upper bound on the tile width chosen by the planner
   int a_split = 1;           // RB_GEMM_A_SPLIT / RB_GEMM_B_SPLIT: TMA boxes per K-major tile
   int b_split = 1;
+  int force_rows = -1;       // RB_GEMM_FORCE_ROWS: weight-gradients from whole rows: 0 = never, n = the n-th plan wherever there is one
   int autotune = 1;          // RB_GEMM_AUTOTUNE: 0 = cost model only, even in tuning mode
   int deterministic = 0;     // RB_GEMM_DETERMINISTIC: 1 = no launch lets several CTAs add into the same output element
                              // (no reduction split, no tail cut), so results are bit-identical from run to run, and the
@@ -1370,7 +1374,7 @@ static int* option_slot(const char* name) {
   struct { const char* name; int* slot; } table[] = {
       {"force_mt", &g_opt.force_mt}, {"force_resident", &g_opt.force_resident}, {"force_halo", &g_opt.force_halo},
       {"force_taps", &g_opt.force_taps}, {"force_tail", &g_opt.force_tail}, {"force_wide", &g_opt.force_wide},
-      {"force_box", &g_opt.force_box}, {"force_pair", &g_opt.force_pair}, {"pdl", &g_opt.pdl},
+      {"force_box", &g_opt.force_box}, {"force_pair", &g_opt.force_pair}, {"force_rows", &g_opt.force_rows}, {"pdl", &g_opt.pdl},
       {"bk32", &g_opt.bk32}, {"bn_cap", &g_opt.bn_cap}, {"a_split", &g_opt.a_split}, {"b_split", &g_opt.b_split},
       {"autotune", &g_opt.autotune}, {"deterministic", &g_opt.deterministic}};
   for (auto& t : table)
@@ -1380,7 +1384,7 @@ static int* option_slot(const char* name) {
 static void options_from_env() {
   std::call_once(g_opt_once, [] {
     const char* names[] = {"force_mt", "force_resident", "force_halo", "force_taps", "force_tail", "force_wide", "force_box",
-                           "force_pair", "pdl", "bk32", "bn_cap", "a_split", "b_split", "autotune", "deterministic"};
+                           "force_pair", "force_rows", "pdl", "bk32", "bn_cap", "a_split", "b_split", "autotune", "deterministic"};
     for (const char* n : names) {
       char env[64] = "RB_GEMM_";
       size_t k = strlen(env);
@@ -1921,6 +1925,30 @@ static PlanKey plan_key(const GemmTcParams& p) {
 // kernels beside them) the plain plans did better.
 constexpr float PAIR_MARGIN = 0.97f;
 
+// Times a launch (the best of two after a first one); true, with its time in *best_ms, when it beats `margin` times *best_ms.
+template <class Run>
+static bool time_launches(cudaStream_t stream, Run run, float* best_ms, float margin = 1.0f) {
+  cudaEvent_t e0, e1;
+  cudaEventCreate(&e0);
+  cudaEventCreate(&e1);
+  float ms = 1e30f;
+  bool ok = true;
+  for (int rep = 0; rep < 3 && ok; ++rep) {
+    cudaEventRecord(e0, stream);
+    ok = run() == 0;
+    cudaEventRecord(e1, stream);
+    ok = ok && cudaEventSynchronize(e1) == cudaSuccess;
+    float t = 0.f;
+    if (ok) cudaEventElapsedTime(&t, e0, e1);
+    if (ok && rep > 0 && t < ms) ms = t;   // the first run warms the caches
+  }
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  if (!ok || ms >= *best_ms * margin) return false;
+  *best_ms = ms;
+  return true;
+}
+
 // Times the candidates of `p` (3 launches each, best of the last 2); returns the best time in ms, or a negative
 // value when nothing could be run.
 static float tune_plan(const GemmTcParams& p, bool b_is_weights, cudaStream_t stream, Plan* out,
@@ -1948,30 +1976,12 @@ static float tune_plan(const GemmTcParams& p, bool b_is_weights, cudaStream_t st
       }
     }
   }
-  cudaEvent_t e0, e1;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
   float best_ms = 1e30f;
-  for (int c = 0; c < n_cands; ++c) {
-    float ms = 1e30f;
-    bool ok = true;
-    for (int rep = 0; rep < 3 && ok; ++rep) {
-      cudaEventRecord(e0, stream);
-      ok = run_plan(p, cands[c], stream) == 0;
-      cudaEventRecord(e1, stream);
-      ok = ok && cudaEventSynchronize(e1) == cudaSuccess;
-      float t = 0.f;
-      if (ok) cudaEventElapsedTime(&t, e0, e1);
-      if (ok && rep > 0 && t < ms) ms = t;   // the first run warms the caches
-    }
-    // pairs are timed after every plain plan and must win by PAIR_MARGIN (a plan that is given: the caller's business)
-    if (ok && ms < best_ms * (cands[c].pair && !given ? PAIR_MARGIN : 1.0f)) {
-      best_ms = ms;
+  // pairs are timed after every plain plan and must win by PAIR_MARGIN (a plan that is given: the caller's business)
+  for (int c = 0; c < n_cands; ++c)
+    if (time_launches(stream, [&]() { return run_plan(p, cands[c], stream); }, &best_ms,
+                      cands[c].pair && !given ? PAIR_MARGIN : 1.0f))
       *out = cands[c];
-    }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
   return best_ms < 1e29f ? best_ms : -1.f;
 }
 
@@ -2345,6 +2355,143 @@ static int conv_forward_form(const void* x, int N, int H, int W, int Cp, const v
   return rc ? rc : launch(p, false, 1, true, stream);
 }
 
+// ---- weight-gradients from whole rows (wgrad_rows.cuh) ------------------------------------------------------------------
+// The cheapest plan for each division of a shape into items (filter rows, channel blocks, how positions line up), cheapest first.
+// Modelled in cycles: MMAs (a 128 x N x 16 step takes N / 2, at least 49), L2 delivery (41 bytes per cycle and SM), a fixed part
+// per chunk, the additions into dw (19 bytes per cycle and SM).
+static std::vector<WgradRowsParams> rows_plans(int N, int H, int W, int Cp, int Kout, int R, int S, int pad_h, int pad_w, int P,
+                                               int Q, int tile) {
+  std::vector<std::pair<double, WgradRowsParams>> all;
+  if (S > 8 || R * S < 2 || pad_h < 0 || pad_w < 0 || Cp % 32 != 0) return {};
+  const int sms = g_num_sms > 0 ? g_num_sms : 148;
+  WgradRowsParams p;
+  memset(&p, 0, sizeof(p));
+  p.R = R;
+  p.S = S;
+  p.pad_h = pad_h;
+  p.pad_w = pad_w;
+  p.Cp = Cp;
+  p.Kout = Kout;
+  p.xw = Cp % 64 == 0 || Cp > 128 ? 64 : 32;      // 32 and 96 channels without empty halves
+  p.dyw = Kout > 32 ? 64 : 32;
+  p.cblocks = (Cp + p.xw - 1) / p.xw;
+  p.dy_blocks = Kout > 64 ? 2 : 1;
+  p.m_tiles = (Kout + BM - 1) / BM;
+  p.tile_bytes = tile;
+  const int most = 256 / p.xw, pieces = (S + most - 1) / most, xpos = p.xw * 2, dypos = p.dyw * 2;
+  const int per_mma = p.per_mma = (S + pieces - 1) / pieces;
+  const int share = std::max(0, std::min({pad_w, S - 1, Q + S - 1 - pad_w - W}));
+  auto kb = [](long long bytes) { return (int)((bytes + 1023) / 1024 * 1024); };
+  for (int nr : {1, R}) {
+    for (int ncb = 1; ncb <= std::min(4, p.cblocks); ++ncb) {
+      if (nr * ncb * S * p.xw > 512 || nr * ncb * pieces > 4 || (nr == R && R == 1)) continue;
+      for (int run = 0; run <= 1; ++run) {
+        const int wdy = run ? Q + S - 1 - share : (Q + 15) / 16 * 16, wx = run ? wdy : wdy + S - 1;
+        if (wx > 256) continue;
+        double best_cost = -1.0;
+        WgradRowsParams best;
+        for (int rows = 1; rows <= std::min(P, 256 - nr + 1); ++rows) {
+          for (int images = 1; images <= (rows == P && nr == 1 ? std::min(N, 16) : 1); ++images) {
+            WgradRowsParams q = p;
+            q.nr = nr;
+            q.ncb = ncb;
+            q.rows = rows;
+            q.images = images;
+            const long long dy_pos = (long long)rows * images * wdy, x_pos = (long long)(rows + nr - 1) * images * wx;
+            q.segs = run ? 1 : rows * images;
+            q.steps = (int)(run ? (dy_pos + 15) / 16 : wdy / 16);
+            q.dy_seg = wdy * dypos >> 4;
+            q.x_seg = wx * xpos >> 4;
+            q.x_row = wx * xpos >> 4;
+            q.dy_bytes = (int)(dy_pos * dypos);
+            q.x_bytes = (int)(x_pos * xpos);
+            q.dy_block = kb((run ? q.steps * 16ll : dy_pos) * dypos);
+            q.x_block = kb((run ? x_pos + 16 + S : x_pos) * xpos);
+            q.clear = run;
+            const long long stage = (long long)q.dy_blocks * q.dy_block + (long long)ncb * q.x_block;
+            if (stage * 2 > tile) break;
+            q.stages = (int)std::min<long long>(tile / stage, MAX_STAGES);
+            q.row_groups = (P + rows - 1) / rows;
+            q.chunks = (N + images - 1) / images * q.row_groups;
+            q.groups_r = R / nr;
+            q.groups_c = (p.cblocks + ncb - 1) / ncb;
+            const int per = q.groups_r * q.groups_c * q.m_tiles;
+            q.splits = std::max(1, std::min(q.chunks, sms / per));
+            q.work = per * q.splits;
+            double mma = 0.0;
+            for (int s0 = 0; s0 < S; s0 += per_mma) mma += std::max(49.0, 0.5 * p.xw * std::min(per_mma, S - s0));
+            mma *= (double)nr * ncb * q.segs * q.steps;
+            // (a position of 64 bytes takes the TMA unit as long as one of 128: ~2.3 cycles)
+            const double load = std::max(((double)q.dy_blocks * q.dy_bytes + (double)ncb * q.x_bytes) / 41.0,
+                                         2.3 * ((double)q.dy_blocks * dy_pos + (double)ncb * x_pos));
+            const double chunk = std::max(mma, load) + (q.stages == 2 ? 0.15 * load + 200.0 : 120.0);
+            const double epilogue = (double)nr * ncb * S * p.xw * (std::min(Kout, BM) + 31) / 32 * 32 * 4 / 19.0 + 2500.0;
+            const double cost = ((q.work + sms - 1) / sms) * ((double)((q.chunks + q.splits - 1) / q.splits) * chunk + epilogue);
+            if (best_cost < 0.0 || cost < best_cost) {
+              best_cost = cost;
+              best = q;
+            }
+          }
+        }
+        if (best_cost >= 0.0) all.push_back({best_cost, best});
+      }
+    }
+  }
+  std::stable_sort(all.begin(), all.end(), [](const std::pair<double, WgradRowsParams>& a, const std::pair<double, WgradRowsParams>& b) {
+    return a.first < b.first;
+  });
+  std::vector<WgradRowsParams> plans;
+  for (const auto& a : all) plans.push_back(a.second);
+  return plans;
+}
+
+// What was measured as the fastest for a weight-gradient: a plan, or none of them (`rows` = 0: gemm_tc_kernel).
+typedef std::tuple<int, int, int, int, int, int, int, int, int, int, int, int> RowsKey;
+static std::map<RowsKey, WgradRowsParams> g_rows_cache;
+
+static int run_rows(WgradRowsParams p, const void* x, int N, int H, int W, const void* dy, long long lddy, int P, int Q, float* dw,
+                    unsigned int* status, cudaStream_t stream) {
+  p.status = status;
+  const int wdy = p.dy_seg * 16 / (p.dyw * 2), wx = p.x_seg * 16 / (p.xw * 2);
+  cuuint64_t dims_dy[4] = {(cuuint64_t)p.Kout, (cuuint64_t)Q, (cuuint64_t)P, (cuuint64_t)N};
+  cuuint64_t dims_x[4] = {(cuuint64_t)p.Cp, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
+  cuuint64_t str_dy[3] = {(cuuint64_t)lddy * 2, (cuuint64_t)lddy * Q * 2, (cuuint64_t)lddy * Q * P * 2};
+  cuuint64_t str_x[3] = {(cuuint64_t)p.Cp * 2, (cuuint64_t)p.Cp * W * 2, (cuuint64_t)p.Cp * W * H * 2};
+  cuuint32_t box_dy[4] = {(cuuint32_t)p.dyw, (cuuint32_t)wdy, (cuuint32_t)p.rows, (cuuint32_t)p.images};
+  cuuint32_t box_x[4] = {(cuuint32_t)p.xw, (cuuint32_t)wx, (cuuint32_t)(p.rows + p.nr - 1), (cuuint32_t)p.images};
+  cuuint32_t es[4] = {1, 1, 1, 1};
+  CUresult r = g_encode_tiled(&p.tm_dy, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(dy), dims_dy, str_dy, box_dy, es,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, p.dyw == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r == CUDA_SUCCESS)
+    r = g_encode_tiled(&p.tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(x), dims_x, str_x, box_x, es,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, p.xw == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return -(400 + (int)r);
+  const long long ldd = (long long)p.R * p.S * p.Cp;
+  const int rc = make_map_out_f32(&p.tm_dw, dw, ldd, p.Kout, ldd);
+  if (rc) return rc;
+  const int grid = std::min(p.work, g_num_sms);
+  const int last[9] = {p.nr, p.splits, p.ncb, p.rows, p.images, p.clear ? 0 : p.segs, A_ROWS, p.stages, grid};
+  memcpy(g_last_launch, last, sizeof(last));
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = (size_t)(GEMM_SMEM_BYTES - TILE_SMEM_BYTES + p.tile_bytes);
+  cfg.stream = stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = g_opt.pdl >= 1 ? 1u : 0u;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, wgrad_rows_kernel, p);
+  if (e == cudaSuccess) return 0;
+  g_last_cuda_error = (int)e;
+  cudaGetLastError();
+  return -4;
+}
+
 // The output phases of a strided data-gradient (conv_dgrad below) that have filter taps.
 struct DgradPhase {
   int a, b;                    // positions (s i + a, s j + b)
@@ -2491,38 +2638,17 @@ static int dgrad_phases(const void* dy, int N, int P, int Q, int Kp, const void*
     if (it != g_phases_cache.end()) {
       if (!g_opt.force_mt && it->second.first <= cap) best = it->second;
     } else if (tunable(p, stream)) {
-      cudaEvent_t e0, e1;
-      cudaEventCreate(&e0);
-      cudaEventCreate(&e1);
       float best_ms = 1e30f;
-      auto measure = [&](std::pair<int, int> cand, float margin, auto run) {
-        float ms = 1e30f;
-        bool ok = true;
-        for (int rep = 0; rep < 3 && ok; ++rep) {
-          cudaEventRecord(e0, stream);
-          ok = run() == 0;
-          cudaEventRecord(e1, stream);
-          ok = ok && cudaEventSynchronize(e1) == cudaSuccess;
-          float t = 0.f;
-          if (ok) cudaEventElapsedTime(&t, e0, e1);
-          if (ok && rep > 0 && t < ms) ms = t;
-        }
-        if (ok && ms < best_ms * margin) {
-          best_ms = ms;
-          best = cand;
-        }
-      };
       for (int i = 0; i < n_cands; ++i) {
         GemmPhasesParams q = p;
-        if (with_b(q, cands[i].first) == 0)
-          measure(cands[i], 1.0f, [&]() { return run_phases(q, cands[i].first, cands[i].second, Cp, stream); });
+        if (with_b(q, cands[i].first) == 0 &&
+            time_launches(stream, [&]() { return run_phases(q, cands[i].first, cands[i].second, Cp, stream); }, &best_ms))
+          best = cands[i];
       }
       lock.unlock();      // launches of their own, which look their plans up
-      measure({0, 0}, 0.95f, separate);
+      if (time_launches(stream, separate, &best_ms, 0.95f)) best = {0, 0};
       lock.lock();
       g_phases_cache[key] = best;
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
     }
   }
   if (best.first == 0) return -3;
@@ -2594,66 +2720,11 @@ static int conv_dgrad(const void* dy, int N, int P, int Q, int Kp, const void* w
   return separate();
 }
 
-}  // namespace rb
-
-extern "C" {
-
-// Convolution forward (also a stride-1 data-grad on flipped and transposed filters).
-//   x   NHWC bf16 [N][H][W][Cp]      w  bf16 [Kout][R*S][Cp]     y  bf16 [N*P*Q][ldy]
-//   base pixel range: lower = -pad_lo, P/Q given by the caller.
-int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
-                     int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* bias, int relu,
-                     const void* mask_src, int n_valid, int n_store, float* ws, long long ws_bytes,
-                     unsigned int* status, cudaStream_t stream) {
-  return conv_forward_form(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, bias, relu, mask_src, n_valid,
-                           n_store, 0, nullptr, nullptr, ws, ws_bytes, status, stream);
-}
-
-// The same followed by a normalisation that is known beforehand, in the epilogue:
-// y = act(scale * conv(x) + shift [+ residual]), scale and shift per output column, residual laid out like y; shift and residual
-// on a 16-byte boundary.
-int rb_conv_fprop_norm(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
-                       int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* scale, const float* shift,
-                       const void* residual, int relu, int n_valid, int n_store, float* ws, long long ws_bytes,
-                       unsigned int* status, cudaStream_t stream) {
-  if (!scale || !shift || ((uintptr_t)shift & 15u) || ((uintptr_t)residual & 15u)) return -10;
-  const NormForm form = {scale, residual};
-  return conv_forward_form(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, shift, relu, nullptr, n_valid,
-                           n_store, 0, nullptr, &form, ws, ws_bytes, status, stream);
-}
-
-// Convolution data-grad: dx[N][H][W][Cp] = mask(add + the gradient), from dy NHWC bf16 [N][P][Q][Kp] and the forward
-// filters w bf16 [Kout][R*S][Cp]. Channels >= c_valid of dx are written as zeros.
-//   stride 1: a forward convolution of dy, its filters read in place. stride s: s x s output phases; phase (a, b), the
-//   positions (s i + a, s j + b), is a stride-1 convolution of dy with every s-th filter tap, whose rows the epilogue
-//   scatters. A phase without taps gets mask(add), and nothing has to be done when add is dx itself and there is no mask.
-//   wt: null, or the filters transposed and flipped (rb_pack_dgrad_filters): then these are read, as a K-major operand.
-//   add, mask: optional, layout of dx, add on a 16-byte boundary; add may be dx. Returns -20 for a strided geometry with a
-//   phase of negative padding.
-int rb_conv_dgrad_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp, int c_valid,
-                     int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* add,
-                     const void* mask, float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
-  return conv_dgrad(dy, N, P, Q, Kp, w, wt, Kout, Cp, c_valid, R, S, stride, pad_h, pad_w, H, W, dx, add, mask, 0, ws, ws_bytes,
-                    status, stream);
-}
-
-// dx += mask(the gradient) where dx is zero already at the places that the mask zeroes: positions that no filter tap reaches
-// stay as they are, without a launch that would write them again.
-int rb_conv_dgrad_onto_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp,
-                          int c_valid, int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* mask,
-                          float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
-  return conv_dgrad(dy, N, P, Q, Kp, w, wt, Kout, Cp, c_valid, R, S, stride, pad_h, pad_w, H, W, dx, dx, mask, 1, ws, ws_bytes,
-                    status, stream);
-}
-
-// Convolution weight-grad:  dw[Kout][R*S][Cp] (fp32) (+)= sum over pixels dy[pix][k] * x[pix shifted by tap][c].
-//   The result is always accumulated into dw (red.add), so dw holds zeros or the running gradient on entry.
-//   beside: the launch is to leave room on the SMs for kernels that run at the same time (the lean instantiation).
-int rb_conv_wgrad_tc(const void* x, int N, int H, int W, int Cp, const void* dy, long long lddy, int Kout, int R,
-                     int S, int stride, int pad_h, int pad_w, int P, int Q, float* dw, int split_k, int beside,
-                     unsigned int* status, cudaStream_t stream) {
-  int rc = ensure_driver_entry();
-  if (rc) return rc;
+// See rb_conv_wgrad_tc: by gemm_tc_kernel.
+static int conv_wgrad(const void* x, int N, int H, int W, int Cp, const void* dy, long long lddy, int Kout, int R,
+                      int S, int stride, int pad_h, int pad_w, int P, int Q, float* dw, int split_k, int beside,
+                      unsigned int* status, cudaStream_t stream) {
+  int rc = 0;
   GemmTcParams p;
   memset(&p, 0, sizeof(p));
   p.bk = 64;
@@ -2777,6 +2848,125 @@ int rb_conv_wgrad_tc(const void* x, int N, int H, int W, int Cp, const void* dy,
   return launch(p, split_k <= 0, split_k > 0 ? split_k : 0, false, stream);
 }
 
+// See rb_conv_wgrad_tc and rb_conv_wgrad_tune.
+static int wgrad_by_plan(const void* x, int N, int H, int W, int Cp, const void* dy, long long lddy, int Kout, int R, int S,
+                         int stride, int pad_h, int pad_w, int P, int Q, float* dw, int split_k, int beside, bool measure,
+                         unsigned int* status, cudaStream_t stream) {
+  const int rc = ensure_driver_entry();
+  if (rc) return rc;
+  auto plain = [&]() {
+    return conv_wgrad(x, N, H, W, Cp, dy, lddy, Kout, R, S, stride, pad_h, pad_w, P, Q, dw, split_k, beside, status, stream);
+  };
+  const bool forced = g_opt.force_mt || g_opt.force_taps || g_opt.force_box >= 0;      // options of the other kernel
+  if (stride != 1 || R * S < 2 || split_k > 0 || g_opt.deterministic || g_opt.force_rows == 0 || forced || N < 1 || P < 1 || Q < 1)
+    return measure ? 0 : plain();
+  auto run = [&](const WgradRowsParams& p) { return run_rows(p, x, N, H, W, dy, lddy, P, Q, dw, status, stream); };
+  auto plans = [&]() {
+    return rows_plans(N, H, W, Cp, Kout, R, S, pad_h, pad_w, P, Q, beside ? LEAN_TILE_BYTES : TILE_SMEM_BYTES);
+  };
+  if (g_opt.force_rows > 0) {
+    const auto all = plans();
+    if (measure) return 0;
+    return all.empty() ? plain() : run(all[std::min<size_t>((size_t)g_opt.force_rows, all.size()) - 1]);
+  }
+  const RowsKey key(N, H, W, Cp, Kout, R, S, pad_h, pad_w, P, Q, beside ? 1 : 0);
+  std::unique_lock<std::mutex> lock(g_plan_mutex);
+  const auto it = g_rows_cache.find(key);
+  if (it != g_rows_cache.end()) {
+    const WgradRowsParams p = it->second;
+    lock.unlock();
+    return measure ? 0 : p.rows ? run(p) : plain();
+  }
+  if (!measure) {
+    lock.unlock();
+    return plain();
+  }
+  WgradRowsParams best;
+  memset(&best, 0, sizeof(best));
+  float best_ms = 1e30f;
+  lock.unlock();      // launches of their own, which look their plans up
+  time_launches(stream, plain, &best_ms);
+  const auto all = plans();
+  for (size_t i = 0; i < all.size() && i < 4; ++i)
+    if (time_launches(stream, [&]() { return run(all[i]); }, &best_ms)) best = all[i];
+  lock.lock();
+  g_rows_cache[key] = best;
+  return 0;
+}
+
+}  // namespace rb
+
+extern "C" {
+
+// Convolution forward (also a stride-1 data-grad on flipped and transposed filters).
+//   x   NHWC bf16 [N][H][W][Cp]      w  bf16 [Kout][R*S][Cp]     y  bf16 [N*P*Q][ldy]
+//   base pixel range: lower = -pad_lo, P/Q given by the caller.
+int rb_conv_fprop_tc(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
+                     int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* bias, int relu,
+                     const void* mask_src, int n_valid, int n_store, float* ws, long long ws_bytes,
+                     unsigned int* status, cudaStream_t stream) {
+  return conv_forward_form(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, bias, relu, mask_src, n_valid,
+                           n_store, 0, nullptr, nullptr, ws, ws_bytes, status, stream);
+}
+
+// The same followed by a normalisation that is known beforehand, in the epilogue:
+// y = act(scale * conv(x) + shift [+ residual]), scale and shift per output column, residual laid out like y; shift and residual
+// on a 16-byte boundary.
+int rb_conv_fprop_norm(const void* x, int N, int H, int W, int Cp, const void* w, int Kout, int R, int S, int stride,
+                       int pad_h, int pad_w, int P, int Q, void* y, long long ldy, const float* scale, const float* shift,
+                       const void* residual, int relu, int n_valid, int n_store, float* ws, long long ws_bytes,
+                       unsigned int* status, cudaStream_t stream) {
+  if (!scale || !shift || ((uintptr_t)shift & 15u) || ((uintptr_t)residual & 15u)) return -10;
+  const NormForm form = {scale, residual};
+  return conv_forward_form(x, N, H, W, Cp, w, Kout, R, S, stride, pad_h, pad_w, P, Q, y, ldy, shift, relu, nullptr, n_valid,
+                           n_store, 0, nullptr, &form, ws, ws_bytes, status, stream);
+}
+
+// Convolution data-grad: dx[N][H][W][Cp] = mask(add + the gradient), from dy NHWC bf16 [N][P][Q][Kp] and the forward
+// filters w bf16 [Kout][R*S][Cp]. Channels >= c_valid of dx are written as zeros.
+//   stride 1: a forward convolution of dy, its filters read in place. stride s: s x s output phases; phase (a, b), the
+//   positions (s i + a, s j + b), is a stride-1 convolution of dy with every s-th filter tap, whose rows the epilogue
+//   scatters. A phase without taps gets mask(add), and nothing has to be done when add is dx itself and there is no mask.
+//   wt: null, or the filters transposed and flipped (rb_pack_dgrad_filters): then these are read, as a K-major operand.
+//   add, mask: optional, layout of dx, add on a 16-byte boundary; add may be dx. Returns -20 for a strided geometry with a
+//   phase of negative padding.
+int rb_conv_dgrad_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp, int c_valid,
+                     int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* add,
+                     const void* mask, float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
+  return conv_dgrad(dy, N, P, Q, Kp, w, wt, Kout, Cp, c_valid, R, S, stride, pad_h, pad_w, H, W, dx, add, mask, 0, ws, ws_bytes,
+                    status, stream);
+}
+
+// dx += mask(the gradient) where dx is zero already at the places that the mask zeroes: positions that no filter tap reaches
+// stay as they are, without a launch that would write them again.
+int rb_conv_dgrad_onto_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp,
+                          int c_valid, int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* mask,
+                          float* ws, long long ws_bytes, unsigned int* status, cudaStream_t stream) {
+  return conv_dgrad(dy, N, P, Q, Kp, w, wt, Kout, Cp, c_valid, R, S, stride, pad_h, pad_w, H, W, dx, dx, mask, 1, ws, ws_bytes,
+                    status, stream);
+}
+
+// Convolution weight-grad:  dw[Kout][R*S][Cp] (fp32) (+)= sum over pixels dy[pix][k] * x[pix shifted by tap][c].
+//   The result is always accumulated into dw (red.add), so dw holds zeros or the running gradient on entry.
+//   beside: the launch is to leave room on the SMs for kernels that run at the same time (the lean instantiation, or less
+//   shared memory).
+//   Which kernel runs is what rb_conv_wgrad_tune has measured for the shape; without a measurement, with an explicit split and
+//   with `deterministic` (measurements must not choose the order of additions), gemm_tc_kernel.
+int rb_conv_wgrad_tc(const void* x, int N, int H, int W, int Cp, const void* dy, long long lddy, int Kout, int R,
+                     int S, int stride, int pad_h, int pad_w, int P, int Q, float* dw, int split_k, int beside,
+                     unsigned int* status, cudaStream_t stream) {
+  return wgrad_by_plan(x, N, H, W, Cp, dy, lddy, Kout, R, S, stride, pad_h, pad_w, P, Q, dw, split_k, beside, false, status, stream);
+}
+
+// Times gemm_tc_kernel and the first four plans of wgrad_rows_kernel by its model on these operands, which are scratch (dw is
+// added into many times), and remembers which was the fastest. Synchronises the stream: never inside a capture. Does nothing for
+// a shape that has been measured, or that has no such plans.
+int rb_conv_wgrad_tune(const void* x, int N, int H, int W, int Cp, const void* dy, long long lddy, int Kout, int R, int S,
+                       int pad_h, int pad_w, int P, int Q, float* dw, int beside, unsigned int* status, cudaStream_t stream) {
+  if (!g_opt.autotune) return 0;
+  return wgrad_by_plan(x, N, H, W, Cp, dy, lddy, Kout, R, S, 1, pad_h, pad_w, P, Q, dw, 0, beside, true, status, stream);
+}
+
 // Planner options by name (see GemmOptions); returns 0, or -1 for an unknown name.
 int rb_gemm_set_option(const char* name, int value) {
   options_from_env();
@@ -2806,6 +2996,7 @@ int rb_gemm_clear_plans() {
   g_plan_cache.clear();
   g_bn_cache.clear();
   g_phases_cache.clear();
+  g_rows_cache.clear();
   return 0;
 }
 

@@ -19,7 +19,7 @@
 
 namespace rb {
 
-enum : int { A_TILED_K = 0, A_IM2COL_K = 1, A_TILED_MN = 2, A_FLAT_K = 3, A_BOX_K = 4, A_BOX_MN = 5 };
+enum : int { A_TILED_K = 0, A_IM2COL_K = 1, A_TILED_MN = 2, A_FLAT_K = 3, A_BOX_K = 4, A_BOX_MN = 5, A_ROWS = 6 };   // A_ROWS: wgrad_rows.cuh
 enum : int { B_TILED_K = 0, B_TILED_MN = 1, B_IM2COL_MN = 2, B_TILED_K3 = 3, B_DGRAD_MN = 4, B_BOX_MN = 5 };
 enum : int { EPI_BF16 = 0, EPI_F32_STORE = 1, EPI_F32_ATOMIC = 2 };
 

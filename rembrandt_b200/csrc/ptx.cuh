@@ -190,8 +190,17 @@ __device__ __forceinline__ void tc_mma_steps(uint32_t tmem_d, uint32_t a_lo, uin
   "@e tcgen05.mma.cta_group::" G ".kind::f16 [%0], da, db, %7, t;\n\t"
 #define RB_STEPS_ARGS                                                                                                 \
   ::"r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(a_adv), "r"(b_adv), "r"(idesc), "r"(accumulate) : "memory"
-  static_assert(KK == 2 || KK == 4, "k-blocks are 32 or 64 deep");
-  if (PAIR) {
+  static_assert(KK == 1 || KK == 2 || KK == 4, "k-blocks are 16, 32 or 64 deep");
+  if (KK == 1) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\t"
+        "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(tmem_d),
+        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+  } else if (PAIR) {
     if (KK == 4) asm volatile(RB_STEPS_HEAD("2") RB_STEPS_NEXT("2") RB_STEPS_NEXT("2") "}" RB_STEPS_ARGS);
     else asm volatile(RB_STEPS_HEAD("2") "}" RB_STEPS_ARGS);
   } else {

@@ -641,6 +641,8 @@ class Conv2dOp(Op):
         n, ko = self.net.batch, self.cfg.out_channels
         K.tune_conv(n, h, w, self.cp, ko, r, r, s, p, p, self.P, self.Q, self.out_cp, relu=self.has_relu,
                     has_bias=self.seg_b is not None, n_valid=ko, n_store=self.out_cp)
+        if self.net.training_capable:
+            K.tune_wgrad(n, h, w, self.cp, ko, self.out_cp, r, r, s, p, p, self.P, self.Q)
         if self.net.training_capable and self.wants_prev_delta():
             self.dgrad = DgradPlan(n, self.P, self.Q, self.out_cp, ko, self.cp, self.in_c, r, s, p, h, w,
                                    [(False, self.mask_src() is not None)], self.net.device)

@@ -98,6 +98,9 @@ class _BnConv:
             # tile plans of the forward and data-grad shapes, measured once on scratch operands
             K.tune_conv(n, self.gh, self.gw, self.cp, self.ko, self.gk, self.gk, self.gs, self.gp, self.gp, self.P,
                         self.Q, self.kp, n_valid=self.ko, n_store=self.kp)
+            if net.training_capable:
+                K.tune_wgrad(n, self.gh, self.gw, self.cp, self.ko, self.kp, self.gk, self.gk, self.gs, self.gp, self.gp, self.P,
+                             self.Q, beside=(False, True))
             if net.training_capable and dx_forms:
                 self.dgrad = DgradPlan(n, self.P, self.Q, self.kp, self.ko, self.cp, self.in_c, self.k, self.s, self.p,
                                        self.h, self.w, dx_forms, dev)

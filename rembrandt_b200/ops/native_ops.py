@@ -64,7 +64,7 @@ OPTION_CHANGES = [0]   # how often the planner's options or cached plans have be
 
 def gemm_set_option(name: str, value: int) -> None:
     """Planner switch of the tensor-core kernel by name (force_mt, force_resident, force_halo, force_taps, force_tail,
-    force_wide, bk32, bn_cap, a_split, b_split, autotune, deterministic); initial values come from RB_GEMM_<NAME> at first use."""
+    force_wide, force_rows, bk32, bn_cap, a_split, b_split, autotune, deterministic); initial values come from RB_GEMM_<NAME> at first use."""
     if _native.cuda().rb_gemm_set_option(name.encode(), int(value)) != 0:
         raise KeyError(name)
     OPTION_CHANGES[0] += 1
@@ -194,6 +194,23 @@ def conv_wgrad_tc(x, N, H, W, Cp, dy, lddy, Kout, R, S, stride, pad_h, pad_w, P,
     rc = _native.cuda().rb_conv_wgrad_tc(ptr(x), N, H, W, Cp, ptr(dy), lddy, Kout, R, S, stride, pad_h, pad_w, P, Q,
                                          ptr(dw), split_k, int(beside), ptr(status_word()), stream_handle())
     check(rc, "rb_conv_wgrad_tc")
+
+
+def tune_wgrad(N, H, W, Cp, Kout, Kp, R, S, stride, pad_h, pad_w, P, Q, beside=(False,)):
+    """Measure which kernel and plan one weight-gradient takes, on scratch operands; `beside`: the forms that will be asked for.
+    Idempotent per shape and process."""
+    forms = [b for b in beside if ("wgrad", torch.cuda.current_device(), N, H, W, Cp, Kout, Kp, R, S, stride, pad_h, pad_w, P, Q, b)
+             not in _tuned_convs]
+    if stride != 1 or R * S < 2 or not forms:
+        return
+    x = torch.zeros((N, H, W, Cp), dtype=torch.bfloat16, device="cuda")
+    dy = torch.zeros((N, P, Q, Kp), dtype=torch.bfloat16, device="cuda")
+    dw = torch.zeros((Kout, R * S, Cp), dtype=torch.float32, device="cuda")
+    for b in forms:
+        _tuned_convs.add(("wgrad", torch.cuda.current_device(), N, H, W, Cp, Kout, Kp, R, S, stride, pad_h, pad_w, P, Q, b))
+        check(_native.cuda().rb_conv_wgrad_tune(ptr(x), N, H, W, Cp, ptr(dy), Kp, Kout, R, S, pad_h, pad_w, P, Q, ptr(dw), int(b),
+                                                ptr(status_word()), stream_handle()), "rb_conv_wgrad_tune")
+    torch.cuda.current_stream().synchronize()
 
 
 def conv_direct_fwd(x, w, bias, y, N, H, W, Cp, Kout, Kp, R, S, stride, pad_h, pad_w, P, Q, relu):
