@@ -39,9 +39,13 @@ struct InputArgs {
 };
 
 __device__ __forceinline__ void sample_draw(const InputArgs& a, int n, int& oy, int& ox, int& flip, float (&shift)[3]) {
-  uint32_t r[4];
-  const uint32_t step = a.step + (a.step_ptr ? *a.step_ptr : 0u);
-  Philox::gen(a.seed, a.per_batch ? 0ull : (uint64_t)n, step, r);
+  uint32_t r[4] = {0u, 0u, 0u, 0u};
+  const bool lighting = a.pca_sigma > 0.f && a.C == 3;
+  uint32_t step = a.step;
+  if (a.random_crop || a.random_flip || lighting) {      // (nothing to draw: inference, and networks without augmentation)
+    if (a.step_ptr) step += *a.step_ptr;
+    Philox::gen(a.seed, a.per_batch ? 0ull : (uint64_t)n, step, r);
+  }
   if (a.random_crop) {
     oy = a.lo_y + (int)(r[0] % (uint32_t)(a.hi_y - a.lo_y + 1));
     ox = a.lo_x + (int)(r[1] % (uint32_t)(a.hi_x - a.lo_x + 1));
@@ -52,7 +56,7 @@ __device__ __forceinline__ void sample_draw(const InputArgs& a, int n, int& oy, 
   }
   flip = a.random_flip ? (int)(r[2] & 1u) : 0;
   shift[0] = shift[1] = shift[2] = 0.f;
-  if (a.pca_sigma > 0.f && a.C == 3) {
+  if (lighting) {
     uint32_t q[4];
     Philox::gen(a.seed ^ 0x5bd1e995ull, (uint64_t)n, step, q);
     // Box-Muller: three normals from four uniforms
@@ -122,9 +126,11 @@ __device__ __forceinline__ uint32_t fast_div(uint32_t e, const Divider& v) { ret
 // time (two aligned words, shifted), several loads in flight per thread, converted (scale, mean, lighting shift, crop /
 // flip / zero padding) and kept in shared memory as bf16 planes [row][channel][pitch]; then every thread writes 16-byte
 // channel groups. A thread keeps the same channel group throughout, so where its eight values lie relative to a pixel is
-// worked out once, in registers. A block moves a few KB: latency and instruction count are what it costs, not bandwidth.
-// The kernel before this one read single bytes, looked the eight offsets up in shared memory per group, and walked the
-// lines of more than four channels one after the other with as many threads as a row has pixels.
+// worked out once, in registers. A block moves a few KB: latency and instruction count are what it costs, not bandwidth: which
+// of four pixels exist is worked out for all four at once, pixels beyond an edge are loaded and dropped, and nothing is drawn where
+// nothing is random. With the four tested one by one, and tiles small enough for eight blocks per SM (of which four fit), us for
+// LeNet's input at 64 images, the CIFAR network's at 128, AlexNet's at 128, ResNet-18's at 32, VGG-A's at 64: 13.1, 22.8, 54.7, 52.1,
+// 72.3; now 5.8, 10.6, 46.8, 40.7, 60.1.
 __global__ void __launch_bounds__(256) input_tile_kernel(InputArgs a, int rows, int pitch, Divider by_q, Divider by_c,
                                                          Divider by_ow) {
   pdl_prolog();
@@ -174,34 +180,35 @@ __global__ void __launch_bounds__(256) input_tile_kernel(InputArgs a, int rows, 
       if (y < a.border || y >= a.crop_h - a.border || sy < 0 || sy >= a.H) continue;
       // source column of position x0 (not flipped) or x0 + 3 (flipped): the lowest of the four
       const int sx = ox + (flip ? a.crop_w - 4 - x0 : x0);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int x = x0 + k, sk = sx + (flip ? 3 - k : k);
-        if (x >= a.border && x < a.crop_w - a.border && sk >= 0 && sk < a.W) ok[u] |= 1u << k;
-      }
-      if (!ok[u]) continue;
+      // which of the four lie in the window and in the image: k0 .. k1 - 1
+      const int k0 = max(max(a.border - x0, flip ? sx + 4 - a.W : -sx), 0);
+      const int k1 = min(min(a.crop_w - a.border - x0, flip ? sx + 4 : a.W - sx), 4);
+      if (k0 >= k1) continue;
+      ok[u] = (1u << k1) - (1u << k0);
       idx[u] = (c * a.H + sy) * a.W + sx;
       const uint8_t* px = img + idx[u];
       const int off = (int)(reinterpret_cast<uintptr_t>(px) & 3u);
       const uint8_t* w = px - off;
-      if (ok[u] == 15u && w >= a.src && w + 8 <= src_end) {
+      if (w >= a.src && w + 8 <= src_end) {      // (pixels of other rows may come along: they are dropped below)
         lo[u] = *reinterpret_cast<const uint32_t*>(w);
         hi[u] = *reinterpret_cast<const uint32_t*>(w + 4);
         sh[u] = off * 8;
-      } else {   // at an edge
-#pragma unroll
+      } else {   // the first or last of the batch
+#pragma unroll 1
         for (int k = 0; k < 4; ++k)
           if (ok[u] & (1u << (flip ? 3 - k : k))) lo[u] |= (uint32_t)px[k] << (8 * k);
       }
     }
     float mu[U][4];
+    if (a.mean) {
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        mu[u][k] = 0.f;
-        if (a.mean && (ok[u] & (1u << k))) mu[u][k] = a.mean[idx[u] + (flip ? 3 - k : k)];
-      }
+        for (int k = 0; k < 4; ++k) {
+          mu[u][k] = 0.f;
+          if (ok[u] & (1u << k)) mu[u][k] = a.mean[idx[u] + (flip ? 3 - k : k)];
+        }
+    }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (at[u] < 0) continue;
@@ -211,9 +218,13 @@ __global__ void __launch_bounds__(256) input_tile_kernel(InputArgs a, int rows, 
       float v[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        v[k] = (float)((px >> (8 * k)) & 255u) * a.scale - a.mean_scale * mu[u][k] + shift;
-        if (!(ok[u] & (1u << k))) v[k] = 0.f;
+        v[k] = (float)((px >> (8 * k)) & 255u) * a.scale;
+        if (a.mean) v[k] -= a.mean_scale * mu[u][k];
+        v[k] += shift;
       }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (!(ok[u] & (1u << k))) v[k] = 0.f;
       __nv_bfloat162 two[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
       *reinterpret_cast<uint2*>(st + at[u]) = *reinterpret_cast<uint2*>(two);
     }
@@ -300,19 +311,20 @@ int rb_input_u8(const void* src, const float* mean, void* dst, int N, int C, int
   for (int i = 0; i < 3; ++i) a.pca_vals[i] = pca_vals ? pca_vals[i] : 0.f;
   for (int i = 0; i < 9; ++i) a.pca_vecs[i] = pca_vecs ? pca_vecs[i] : 0.f;
   a.seed = seed; a.step = step; a.step_ptr = step_ptr;
-  // Output rows per block: as many as leave every SM eight blocks and the planes in 32 KB (fewer rows are staged twice
-  // when windows overlap, and a block's fixed cost is shared by more of them).
+  // Output rows per block: as many as leave every SM two blocks and the planes in 32 KB (fewer rows are staged twice
+  // when windows overlap, and a block's fixed cost, 3 - 4 us, is shared by more of them: with 4 blocks per SM 8.5 instead of 6.2 us
+  // for LeNet's input, 14.4 instead of 11.3 for the CIFAR network's; the larger ones are as fast from 2 to 4).
   const int seg_w = (OW - 1) * stride + f;
   const int quads = (seg_w + 3) / 4;
   const int pitch = 4 * (quads | 1);
   int rows = 0;
-  for (int r = 8; r >= 1; r >>= 1) {
+  for (int r = 16; r >= 1; r >>= 1) {
     const long long lines = ((long long)(r - 1) * stride + f) * C;
     const long long smem = (8 + lines * pitch) * 2;
     if (smem > (r == 1 ? 40 * 1024 : 32 * 1024)) continue;
     if (lines * quads * quads >= 0xFFFFFFFFll || (long long)r * OW * OW >= 0xFFFFFFFFll) continue;   // see Divider
     rows = r;
-    if ((long long)N * ((OH + r - 1) / r) >= 148 * 8) break;
+    if ((long long)N * ((OH + r - 1) / r) >= 148 * 2) break;
   }
   if (rows > 0 && Cp <= 2048 && N <= 65535 && (long long)C * H * W < 0x7FFFFFFF) {
     const size_t smem = (8 + (size_t)((rows - 1) * stride + f) * C * pitch) * 2;
