@@ -176,14 +176,14 @@ class StepEngine:
             g.capture_end()
         return g
 
-    def _fwd_bwd(self, train=True, hook=None):
+    def _fwd_bwd(self, train=True, hook=None, after_forward=None):
         with span("forward"):
             self.net.forward(train, None)
+        if after_forward is not None:
+            after_forward()
         if train:
             with span("backward"):
                 self.net.backward(hook)
-        if self.is_cuda:
-            self.net.step_counter.add_(1)
 
     def _update(self, lr=None):
         """Exchange + optimizer step for one iteration, in the configured order, with the engine's learning rate (or what is
@@ -246,11 +246,22 @@ class StepEngine:
             hook = self.comm.on_op_backward
 
         def body(update):
+            # What nothing in the rest of the step waits for is captured beside it: loss and accuracy beside backward, the count
+            # of steps (which dropout's backward pass still reads) beside the update.
+            net, aside = self.net, self.net.capturing()
             with self._reading(slot):
-                self._fwd_bwd(hook=hook)
+                self._fwd_bwd(hook=hook, after_forward=(lambda: net.side(self._publish)) if aside else None)
+            count = lambda: net.step_counter.add_(1)
+            if aside:
+                net.side(count)
+            else:
+                count()
             if update:
                 self._update(lr)
-            self._publish()
+            if aside:
+                net.join_side()
+            else:
+                self._publish()
 
         if graphed:
             key = (last_of_iteration, slot)

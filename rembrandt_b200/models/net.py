@@ -271,11 +271,15 @@ class Net:
             fn()
         self._side_dirty = True
 
+    def capturing(self) -> bool:
+        """Whether what is launched now becomes part of a graph."""
+        return self._side is not None and torch.cuda.is_current_stream_capturing()
+
     def beside(self, fn):
         """Run `fn` (launches of a weight-gradient) beside what backward goes on with: on the side stream, as `fn(beside=True)`,
         while a step is captured; here and now, as `fn()`, where a hook would wait for it at once, or where the events cost
         the host more than they save (eager steps)."""
-        if self._side is None or self._collected or not torch.cuda.is_current_stream_capturing():
+        if self._collected or not self.capturing():
             fn()
         else:
             self.side(lambda: fn(beside=True))
