@@ -189,7 +189,9 @@ __global__ void __launch_bounds__(256) bn_reduce_kernel(const bf16* __restrict__
 
 static void launch_bn_reduce(const bf16* x, const bf16* dy, const bf16* y, const float* mean, const float* istd,
                              long long rows, int C, float* plain, int backward, const BnScratch& ws, cudaStream_t st) {
-  const dim3 grid = row_grid(rows, C, 8, 148 * 4);
+  // Two blocks per SM: every block adds 2 * C sums to the same addresses, and in the backward pass the weight-gradient beside it
+  // leaves room for one or two. With four, the Go network's step at 256 boards took 1511 us, with two 1457, with one 1515.
+  const dim3 grid = row_grid(rows, C, 8, 148 * 2);
   auto go = [&](auto kern) { launch_pdl(kern, grid, dim3(256), 0, st, x, dy, y, mean, istd, rows, C, plain, ws); };
   if (!backward) go(bn_reduce_kernel<0, 0>);
   else if (y) go(bn_reduce_kernel<1, 1>);
@@ -450,7 +452,9 @@ __global__ void __launch_bounds__(256) bn_bwd_apply_kernel(const bf16* __restric
 static void launch_bn_bwd_apply(const bf16* x, const bf16* dy, const bf16* y, const float* mean, const float* istd,
                                 const float* gamma, const float* plain, const BnScratch& ws, float* dgamma,
                                 float* dbeta, bf16* dx, long long rows, int C, int c_valid, cudaStream_t st) {
-  dim3 grid = row_grid(rows, C, 4, 148 * 8);
+  // (no more blocks than find room beside the weight-gradient: with eight per SM the Go network's step took 1436 us, now 1420;
+  // ResNet-18's at 32 images 1465, now 1451)
+  dim3 grid = row_grid(rows, C, 4, 148 * 2);
   if (ws.sums) ++grid.x;   // the blocks that store what exists once per channel
   auto go = [&](auto kern) {
     launch_pdl(kern, grid, dim3(256), 0, st, x, dy, y, mean, istd, gamma, plain, ws, dgamma, dbeta, dx, rows, C, c_valid);
