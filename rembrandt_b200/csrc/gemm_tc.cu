@@ -2712,7 +2712,10 @@ static int conv_dgrad(const void* dy, int N, int P, int Q, int Kp, const void* w
     }
     return 0;
   };
-  if (with_taps.size() >= 2 && with_taps.size() <= MAX_PHASES) {
+  // an option that forces a form the one launch does not have is for the launches of the phases
+  const bool forced = g_opt.force_halo == 1 || g_opt.force_box == 1 || g_opt.force_wide == 1 || g_opt.force_pair == 1 ||
+                      g_opt.force_tail == 1 || g_opt.force_resident >= 0;
+  if (with_taps.size() >= 2 && with_taps.size() <= MAX_PHASES && !forced) {
     const int rc = dgrad_phases(dy, N, P, Q, Kp, wt ? wt : w, wt != nullptr, Kout, Cp, c_valid, R, S, stride, pad_h, pad_w, H, W, dx,
                                 add, mask, with_taps.data(), (int)with_taps.size(), status, stream, separate);
     if (rc != -3) return rc;
