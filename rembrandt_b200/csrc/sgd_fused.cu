@@ -90,7 +90,7 @@ int rb_sgd_fused(float* w, float* g, float* v, void* w16, long long n, float lr,
   a.w = w; a.g = g; a.v = v; a.w16 = (bf16*)w16; a.n = n;
   // One block for every 256 x 4 values, whatever their number: blocks that start in order keep the seven streams of a sweep
   // within a few MB of one another, where 1184 blocks that step through the whole range spread them over all of it.
-  // 62.4 M parameters: 279 -> 244 us (30 bytes each; 7.7 TB/s), 11.7 M: 55 -> 51 us, 1 M: 10 us both.
+  // 62.4 M parameters: 279 -> 244 us (26 bytes each: 6.65 TB/s), 11.7 M: 55 -> 51 us, 1 M: 10 us both.
   const int blocks = (int)std::min(std::max(1ll, (n / 4 + 255) / 256), 1ll << 30);
   launch_streaming(sgd_fused_kernel, blocks, 256, 0, st, a);
   return RB_LAUNCH_OK();

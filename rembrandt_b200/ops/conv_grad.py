@@ -2,8 +2,7 @@
 
 On a GPU this is `rb_conv_dgrad_tc` (csrc/gemm_tc.cu): the filters are read as they lie (or from a transposed and flipped
 copy, `DgradPlan`), the output phases of a strided convolution share a launch and are written straight to their places in dx, and
-the addend
-(the delta of an identity path, or the gradient of a parallel branch already in dx) and the mask of the producer's ReLU
+the addend (the delta of an identity path, or the gradient of a parallel branch already in dx) and the mask of the producer's ReLU
 ride in the epilogue. Strided geometries that it does not take, and all with RB_STRIDED_DGRAD_TC=0, run on the CUDA-core
 kernel. Without a GPU the result is put together from the kernel fronts of `native_ops`, which the CPU tests replace by
 plain torch.
