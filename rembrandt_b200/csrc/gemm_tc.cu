@@ -2860,7 +2860,9 @@ static int wgrad_by_plan(const void* x, int N, int H, int W, int Cp, const void*
   auto plain = [&]() {
     return conv_wgrad(x, N, H, W, Cp, dy, lddy, Kout, R, S, stride, pad_h, pad_w, P, Q, dw, split_k, beside, status, stream);
   };
-  const bool forced = g_opt.force_mt || g_opt.force_taps || g_opt.force_box >= 0;      // options of the other kernel
+  // options of the other kernel
+  const bool forced = g_opt.force_mt || g_opt.force_taps || g_opt.force_box >= 0 || g_opt.force_resident >= 0 ||
+                      (g_opt.bn_cap > 0 && g_opt.bn_cap < 256);
   if (stride != 1 || R * S < 2 || split_k > 0 || g_opt.deterministic || g_opt.force_rows == 0 || forced || N < 1 || P < 1 || Q < 1)
     return measure ? 0 : plain();
   auto run = [&](const WgradRowsParams& p) { return run_rows(p, x, N, H, W, dy, lddy, P, Q, dw, status, stream); };

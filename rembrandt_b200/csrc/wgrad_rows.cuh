@@ -21,6 +21,8 @@
 //             end shared with the next row's beginning), and the whole chunk is one reduction: what bounds small images, whose
 //             rows are no multiple of 16 (13 x 13: 192 positions for 169 outputs instead of 208). Positions behind the boxes are
 //             zeros from the start of the kernel, in both operands.
+// Either way zero columns of one operand meet pixels of the other: finite ones add nothing, an infinity or a NaN makes the sums
+// that it meets NaN, also those of taps at a border that tap by tap would not have met it.
 //
 // A work item is 128 output channels x (filter rows x blocks of channels) of at most 512 accumulator columns over a range of
 // chunks; items that share a range run at the same time. The sums are added into dw by TMA.

@@ -60,6 +60,34 @@ def test_every_plan_against_autograd(shape, beside):
     assert len(seen) > 1
 
 
+ODD = [  # N, C, Ko, H, W, R, S, pad_h, pad_w, more rows and columns of the output, more channels per row of dy
+    (3, 64, 96, 9, 13, 1, 5, 0, 2, 0, 0, 0), (2, 32, 64, 13, 9, 5, 1, 2, 0, 0, 0, 64), (2, 64, 64, 8, 10, 3, 2, 1, 0, 0, 1, 0),
+    (2, 96, 32, 7, 11, 2, 3, 0, 2, 1, -1, 32), (3, 64, 160, 10, 10, 3, 3, 1, 1, -3, -2, 0), (2, 128, 64, 6, 17, 3, 3, 4, 3, 0, 0, 0),
+    (2, 64, 64, 11, 6, 4, 3, 0, 1, 2, 2, 0), (1, 32, 32, 3, 3, 3, 3, 0, 0, 0, 0, 0)]
+
+
+@pytest.mark.parametrize("shape", ODD)
+def test_unequal_sides_and_outputs_cut_or_grown(shape):
+    N, C, Ko, H, W, R, S, ph, pw, dh, dw_, more = shape
+    torch.manual_seed(sum(shape))
+    P, Q, ld = H + 2 * ph - R + 1 + dh, W + 2 * pw - S + 1 + dw_, K.pad_channels(Ko) + more
+    x, dy = (torch.randn(N, C, H, W, device=DEV).bfloat16().float(), torch.randn(N, Ko, P, Q, device=DEV).bfloat16().float())
+    w = torch.zeros(Ko, C, R, S, device=DEV, dtype=torch.float64, requires_grad=True)
+    y = F.conv2d(F.pad(x.double(), (pw, pw + max(dw_, 0), ph, ph + max(dh, 0))), w)[:, :, :P, :Q]
+    (want,) = torch.autograd.grad(y, w, dy.double())
+    rows = torch.full((N, P, Q, ld), float("nan"), device=DEV, dtype=torch.bfloat16)      # what lies behind Ko is not read
+    rows[..., :Ko] = dy.permute(0, 2, 3, 1)
+    xh = layout.to_nhwc_padded(x, C)
+    for beside in (False, True):
+        for nth in range(1, 9):
+            out = torch.zeros((Ko, R * S, C), device=DEV)
+            with K.gemm_options(force_rows=nth):
+                K.conv_wgrad_tc(xh, N, H, W, C, rows, ld, Ko, R, S, 1, ph, pw, P, Q, out, beside=beside)
+            assert K.read_status() == 0 and (K.gemm_last_launch()["a_mode"] == ROWS) == (R > 1)      # no plans for one row of taps
+            got = out.view(Ko, R, S, C).permute(0, 3, 1, 2).double()
+            assert float((got - want).abs().max()) < 4e-6 * (N * P * Q) ** 0.5 * 4 + 2e-6      # as above
+
+
 @pytest.mark.parametrize("shape", [SHAPES[0], SHAPES[1], SHAPES[12]])
 def test_what_was_measured_is_what_runs(shape):
     args, check = _case(shape)
