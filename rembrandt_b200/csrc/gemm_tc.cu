@@ -2448,6 +2448,10 @@ static std::vector<WgradRowsParams> rows_plans(int N, int H, int W, int Cp, int 
 // What was measured as the fastest for a weight-gradient: a plan, or none of them (`rows` = 0: gemm_tc_kernel).
 typedef std::tuple<int, int, int, int, int, int, int, int, int, int, int, int> RowsKey;
 static std::map<RowsKey, WgradRowsParams> g_rows_cache;
+// Less work than this is start, additions and drain in either kernel, and gemm_tc_kernel adds it up from fewer parts, whose order
+// is left open: LeNet's second convolution at 17 images (0.09 GFLOP) 2 parts against 17 to 29, at 64 (0.33) 8 against 22. LeNet's
+// step without and with this kernel for the smaller: 17 images 87, 86 us; 32 images 94, 100; at 64 105, 102.
+constexpr double ROWS_MIN_FLOPS = 0.2e9;
 
 static int run_rows(WgradRowsParams p, const void* x, int N, int H, int W, const void* dy, long long lddy, int P, int Q, float* dw,
                     unsigned int* status, cudaStream_t stream) {
@@ -2874,6 +2878,7 @@ static int wgrad_by_plan(const void* x, int N, int H, int W, int Cp, const void*
     if (measure) return 0;
     return all.empty() ? plain() : run(all[std::min<size_t>((size_t)g_opt.force_rows, all.size()) - 1]);
   }
+  if (2.0 * N * P * Q * R * S * Cp * Kout < ROWS_MIN_FLOPS) return measure ? 0 : plain();
   const RowsKey key(N, H, W, Cp, Kout, R, S, pad_h, pad_w, P, Q, beside ? 1 : 0);
   std::unique_lock<std::mutex> lock(g_plan_mutex);
   const auto it = g_rows_cache.find(key);
