@@ -2685,6 +2685,8 @@ static int conv_dgrad(const void* dy, int N, int P, int Q, int Kp, const void* w
       all.push_back(f);
       if (taps) with_taps.push_back(f);
     }
+  // The phases' epilogue and fill_phase_kernel read and write 16 bytes at a time, without a map whose making would say no.
+  if (stride > 1 && (((uintptr_t)dx | (uintptr_t)mask) & 15u)) return -10;
   for (const DgradPhase& f : all) {
     if ((f.U > 0 && f.V > 0) || (add == dx && (!mask || add_masked))) continue;
     const int rc = fill_phase((const __nv_bfloat16*)add, (const __nv_bfloat16*)mask, (__nv_bfloat16*)dx, N, f.Hp, f.Wp, stride, f.a,
@@ -2938,7 +2940,7 @@ int rb_conv_fprop_norm(const void* x, int N, int H, int W, int Cp, const void* w
 //   positions (s i + a, s j + b), is a stride-1 convolution of dy with every s-th filter tap, whose rows the epilogue
 //   scatters. A phase without taps gets mask(add), and nothing has to be done when add is dx itself and there is no mask.
 //   wt: null, or the filters transposed and flipped (rb_pack_dgrad_filters): then these are read, as a K-major operand.
-//   add, mask: optional, layout of dx, add on a 16-byte boundary; add may be dx. Returns -20 for a strided geometry with a
+//   add, mask: optional, layout of dx; add may be dx. All three on a 16-byte boundary (else an error). Returns -20 for a strided geometry with a
 //   phase of negative padding.
 int rb_conv_dgrad_tc(const void* dy, int N, int P, int Q, int Kp, const void* w, const void* wt, int Kout, int Cp, int c_valid,
                      int R, int S, int stride, int pad_h, int pad_w, int H, int W, void* dx, const void* add,

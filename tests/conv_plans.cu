@@ -162,6 +162,28 @@ static void addends_are_aligned() {
   }
 }
 
+// The same for the output and the mask of a strided data-gradient, whose phases share one launch, have none (1 x 1) or are
+// too many for one (stride 3): refused before anything is launched. A geometry that is not taken keeps its own answer.
+static void strided_outputs_are_aligned() {
+  const struct { int R, stride, pad, rc; } tries[] = {{1, 2, 0, 0}, {2, 2, 0, 0}, {3, 2, 1, 0}, {5, 2, 2, 0}, {1, 3, 0, 0},
+                                                      {3, 3, 0, 0}, {5, 3, 2, 0}, {3, 2, 6, -20}, {2, 2, 1, -20}};
+  for (auto& t : tries)
+    for (int off = 0; off < 32; off += 2)
+      for (int form = 0; form < 3; ++form) {
+        const int P = (12 + 2 * t.pad - t.R) / t.stride + 1, before = g_launches;
+        // (an addend, which the third form's output is, is looked at first)
+        const int want = off % 16 != 0 && (form == 2 || !t.rc) ? -10 : t.rc;
+        void *const at = (void*)0x1000, *const odd = (void*)(0x2000 + (size_t)off);
+        void *const dx = form == 1 ? at : odd, *const mask = form == 0 ? nullptr : odd;
+        const int rc = form == 2 ? rb_conv_dgrad_onto_tc(at, 2, P, P, 32, at, nullptr, 32, 32, 32, t.R, t.R, t.stride, t.pad, t.pad, 12,
+                                                         12, dx, mask, nullptr, 0, nullptr, 0)
+                                 : rb_conv_dgrad_tc(at, 2, P, P, 32, at, nullptr, 32, 32, 32, t.R, t.R, t.stride, t.pad, t.pad, 12, 12,
+                                                    dx, nullptr, mask, nullptr, 0, nullptr, 0);
+        expect(rc == want, form == 1 ? "mask" : "output");
+        expect((g_launches != before) == (want == 0), "launched");
+      }
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
       {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
@@ -170,7 +192,8 @@ int main(int argc, char** argv) {
       {"deterministic_keeps_one_order", deterministic_keeps_one_order},
       {"pairs_win_by_a_margin", pairs_win_by_a_margin},
       {"flat_tiles_within_the_cap", flat_tiles_within_the_cap},
-      {"addends_are_aligned", addends_are_aligned}};
+      {"addends_are_aligned", addends_are_aligned},
+      {"strided_outputs_are_aligned", strided_outputs_are_aligned}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;
