@@ -2456,6 +2456,14 @@ constexpr double ROWS_MIN_FLOPS = 0.2e9;
 static int run_rows(WgradRowsParams p, const void* x, int N, int H, int W, const void* dy, long long lddy, int P, int Q, float* dw,
                     unsigned int* status, cudaStream_t stream) {
   p.status = status;
+  p.x = reinterpret_cast<const __nv_bfloat16*>(x);
+  p.dy = reinterpret_cast<const __nv_bfloat16*>(dy);
+  p.lddy = lddy;
+  p.N = N;
+  p.H = H;
+  p.W = W;
+  p.P = P;
+  p.Q = Q;
   const int wdy = p.dy_seg * 16 / (p.dyw * 2), wx = p.x_seg * 16 / (p.xw * 2);
   cuuint64_t dims_dy[4] = {(cuuint64_t)p.Kout, (cuuint64_t)Q, (cuuint64_t)P, (cuuint64_t)N};
   cuuint64_t dims_x[4] = {(cuuint64_t)p.Cp, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};

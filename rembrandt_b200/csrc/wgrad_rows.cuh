@@ -21,8 +21,10 @@
 //             end shared with the next row's beginning), and the whole chunk is one reduction: what bounds small images, whose
 //             rows are no multiple of 16 (13 x 13: 192 positions for 169 outputs instead of 208). Positions behind the boxes are
 //             zeros from the start of the kernel, in both operands.
-// Either way zero columns of one operand meet pixels of the other: finite ones add nothing, an infinity or a NaN makes the sums
-// that it meets NaN, also those of taps at a border that tap by tap would not have met it.
+// Either way zero columns of dy meet pixels at the border, which belong to no output of that tap. Finite ones add nothing; an
+// infinity or a NaN would turn sums into NaN that it has no part in. So a slab with a sum that is not finite is not added but taken
+// again, over the outputs alone (rows_again). For finite sums that costs the test: nothing to 0.5 us a launch (3 x 3, 32 -> 32 on
+// 128 x 16 x 16: 7.3 -> 7.5 us; 64 -> 64 on 32 x 64 x 64: 17.4 -> 17.5; 128 -> 128 on 256 x 19 x 19: 26.1 -> 26.2).
 //
 // A work item is 128 output channels x (filter rows x blocks of channels) of at most 512 accumulator columns over a range of
 // chunks; items that share a range run at the same time. The sums are added into dw by TMA.
@@ -47,6 +49,9 @@ struct alignas(64) WgradRowsParams {
   int dy_bytes, x_bytes;             // bytes that a box brings
   int stages, tile_bytes;
   int clear;                         // shared memory behind the boxes has to be zeros
+  const __nv_bfloat16 *x, *dy;       // for sums that are taken again
+  long long lddy;
+  int N, H, W, P, Q;
   unsigned int* status;
 };
 
@@ -110,6 +115,112 @@ __device__ __forceinline__ bool rows_item(const WgradRowsParams& p, SharedCtl* c
   return true;
 }
 
+// Item `work`: output channels, filter rows, channel blocks, chunks.
+struct RowsItem {
+  int m0, r0, cb0, ncb, c0, c1;
+};
+__device__ __forceinline__ RowsItem rows_item_of(const WgradRowsParams& p, int work) {
+  RowsItem it;
+  const int groups = p.groups_r * p.groups_c, t = work / p.m_tiles, sp = t / groups, g = t - sp * groups, gc = g / p.groups_r;
+  it.m0 = (work - t * p.m_tiles) * BM;
+  it.r0 = (g - gc * p.groups_r) * p.nr;
+  it.cb0 = gc * p.ncb;
+  it.ncb = min(p.ncb, p.cblocks - it.cb0);
+  it.c0 = (int)((long long)sp * p.chunks / p.splits);
+  it.c1 = (int)((long long)(sp + 1) * p.chunks / p.splits);
+  return it;
+}
+
+// What accumulator column `c` of an item holds: channel `chan` of tap (row r, `tap`).
+struct RowsColumn {
+  int r, tap, chan;
+};
+__device__ __forceinline__ RowsColumn rows_column_of(const WgradRowsParams& p, const RowsItem& it, int c) {
+  const int unit_cols = p.S * p.xw, unit = c / unit_cols, in_unit = c - unit * unit_cols, ri = unit / it.ncb;
+  RowsColumn at;
+  at.r = it.r0 + ri;
+  at.tap = in_unit / p.xw;
+  at.chan = (it.cb0 + unit - ri * it.ncb) * p.xw + in_unit - at.tap * p.xw;
+  return at;
+}
+
+// A slab of 32 accumulator columns (c ...) of an item on its way to dw: TMEM -> registers -> the warp's staging buffer.
+__device__ __forceinline__ void rows_load(uint32_t tmem, int c, uint32_t (&v)[32]) {
+  tmem_ld_32x32(tmem + (uint32_t)c + ((threadIdx.x >> 5 & 3u) << 21), v);
+  tmem_ld_wait();
+}
+__device__ __forceinline__ void rows_stage(uint8_t* staged, const uint32_t (&v)[32]) {
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) tma_store_wait_read<0>();
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    *reinterpret_cast<uint4*>(staged + lane * 128 + ((q ^ (lane & 7)) * 16)) = make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
+__device__ __forceinline__ bool rows_add(const WgradRowsParams& p, uint8_t* staged, const RowsItem& it, const RowsColumn& at, bool not_yet) {
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (__any_sync(0xffffffffu, not_yet)) return false;
+  if ((threadIdx.x & 31) == 0) {
+    tma_reduce_add_2d(&p.tm_dw, staged, (at.r * p.S + at.tap) * p.Cp + at.chan, it.m0 + (int)(threadIdx.x >> 5 & 3) * 32);
+    tma_store_commit();
+  }
+  return true;
+}
+
+// A slab with sums that are not finite: these are taken again, over output positions, pixels outside the image as zeros. In
+// doubles, so that the order does not matter; four columns at a time and one position after the other: slow, and only ever needed
+// for infinities and NaN. A sum that has become NaN is done: a launch whose operands are all NaN takes 1 to 2 ms, one with a single
+// infinite pixel 1 to 17, and where every sum is infinite and none NaN (512 -> 512 on 64 x 32 x 32, 22016 positions an item) 0.5 s,
+// which is below the limit that waits have.
+__device__ __forceinline__ void rows_again(const WgradRowsParams& p, uint8_t* staged, uint32_t tmem, int work, int c) {
+  const RowsItem it = rows_item_of(p, work);
+  const RowsColumn col = rows_column_of(p, it, c);
+  const int lane = threadIdx.x & 31, m = it.m0 + (int)(threadIdx.x >> 5 & 3) * 32 + lane;
+  {
+    uint32_t v[32];
+    rows_load(tmem, c, v);
+    rows_stage(staged, v);
+  }
+#pragma unroll 1
+  for (int j = 0; j < 32 && m < p.Kout; j += 4) {
+    float* const at = reinterpret_cast<float*>(staged + lane * 128 + ((j / 4) ^ (lane & 7)) * 16);
+    double sum[4] = {0.0, 0.0, 0.0, 0.0};
+    uint32_t again = 0u;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if ((__float_as_uint(at[e]) & 0x7f800000u) == 0x7f800000u) again |= 1u << e;
+    uint32_t open = again;      // those that are not NaN so far
+    for (int k = it.c0; k < it.c1 && open; ++k) {
+      const int grp = k / p.row_groups, h0 = (k - grp * p.row_groups) * p.rows;
+      const int n1 = min(p.N, (grp + 1) * p.images), h1 = min(p.P, h0 + p.rows);
+      for (int n = grp * p.images; n < n1; ++n)
+        for (int h = h0; h < h1; ++h) {
+          const int y = h + col.r - p.pad_h, w0 = p.pad_w - col.tap;
+          const int w1 = y >= 0 && y < p.H ? p.W : 0;      // pixels of this row
+          const __nv_bfloat16* dy = p.dy + ((long long)n * p.P + h) * p.Q * p.lddy + m;
+          const __nv_bfloat16* x = p.x + (((long long)n * p.H + y) * p.W - w0) * p.Cp + col.chan + j;
+#pragma unroll 1
+          for (int q = 0; q < p.Q; ++q, dy += p.lddy, x += p.Cp) {
+            const uint2 four = q >= w0 && q - w0 < w1 ? *reinterpret_cast<const uint2*>(x) : make_uint2(0u, 0u);
+            const double d = (double)__bfloat162float(*dy);
+            sum[0] += d * (double)__uint_as_float(four.x << 16);
+            sum[1] += d * (double)__uint_as_float(four.x & 0xffff0000u);
+            sum[2] += d * (double)__uint_as_float(four.y << 16);
+            sum[3] += d * (double)__uint_as_float(four.y & 0xffff0000u);
+          }
+        }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (isnan(sum[e])) open &= ~(1u << e);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (again & (1u << e)) at[e] = (float)sum[e];
+  }
+  rows_add(p, staged, it, col, false);
+}
+
 __global__ void __maxnreg__(LEAN_MAX_REGS) wgrad_rows_kernel(const __grid_constant__ WgradRowsParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -144,27 +255,13 @@ __global__ void __maxnreg__(LEAN_MAX_REGS) wgrad_rows_kernel(const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
-  // item `work`: output channels, filter rows, channel blocks, chunks
-  const int groups = p.groups_r * p.groups_c;
-  struct Item { int m0, r0, cb0, ncb, c0, c1; };
-  auto item = [&](int work) {
-    Item it;
-    const int t = work / p.m_tiles, sp = t / groups, g = t - sp * groups, gc = g / p.groups_r;
-    it.m0 = (work - t * p.m_tiles) * BM;
-    it.r0 = (g - gc * p.groups_r) * p.nr;
-    it.cb0 = gc * p.ncb;
-    it.ncb = min(p.ncb, p.cblocks - it.cb0);
-    it.c0 = (int)((long long)sp * p.chunks / p.splits);
-    it.c1 = (int)((long long)(sp + 1) * p.chunks / p.splits);
-    return it;
-  };
   if (warp == 0) {
     int s = 0, issued = 0;
     uint32_t ph = 0;
     bool ok = true;
     pdl_prolog();
     for (int work = blockIdx.x; work < p.work && ok; work += gridDim.x) {
-      const Item it = item(work);
+      const RowsItem it = rows_item_of(p, work);
       const int boxes = p.dy_blocks + it.ncb;
       int grp = it.c0 / p.row_groups, rg = it.c0 - grp * p.row_groups;
       for (int c = it.c0; c < it.c1; ++c) {
@@ -202,7 +299,7 @@ __global__ void __maxnreg__(LEAN_MAX_REGS) wgrad_rows_kernel(const __grid_consta
     const int pieces = (p.S + p.per_mma - 1) / p.per_mma;
     const uint32_t tiles_u32 = smem_u32(tiles);
     for (int work = blockIdx.x; work < p.work; work += gridDim.x) {
-      const Item it = item(work);
+      const RowsItem it = rows_item_of(p, work);
       if (!ctl_wait_warp(ctl, &ctl->acc_empty[0], acc_ph ^ 1u, p.status)) break;
       tc_fence_after();
       bool ok;
@@ -222,32 +319,28 @@ __global__ void __maxnreg__(LEAN_MAX_REGS) wgrad_rows_kernel(const __grid_consta
     uint8_t* const stg = staging + (warp - 2) * 4096;
     uint32_t acc_ph = 0;
     for (int work = blockIdx.x; work < p.work; work += gridDim.x) {
-      const Item it = item(work);
+      const RowsItem it = rows_item_of(p, work);
       if (!ctl_wait(ctl, &ctl->acc_full[0], acc_ph, p.status)) break;
       tc_fence_after();
-      const int unit_cols = p.S * p.xw, cols = p.nr * it.ncb * unit_cols;
+      const int cols = p.nr * it.ncb * p.S * p.xw;
+      uint32_t odd = 0u;      // slabs that rows_again takes
       for (int c = col_half * 32; c < cols; c += 64) {
-        const int unit = c / unit_cols, in_unit = c - unit * unit_cols;
-        const int ri = unit / it.ncb, tap = in_unit / p.xw;
-        const int chan = (it.cb0 + unit - ri * it.ncb) * p.xw + in_unit - tap * p.xw;
-        const int col = ((it.r0 + ri) * p.S + tap) * p.Cp + chan;
-        if (chan >= p.Cp || it.m0 + lane_base >= p.Kout) continue;
+        const RowsColumn at = rows_column_of(p, it, c);
+        if (at.chan >= p.Cp || it.m0 + lane_base >= p.Kout) continue;
         uint32_t v[32];
-        tmem_ld_32x32(tmem_base + (uint32_t)c + ((uint32_t)lane_base << 16), v);
-        tmem_ld_wait();
-        if (lane == 0) tma_store_wait_read<0>();
-        __syncwarp();
+        rows_load(tmem_base, c, v);
+        rows_stage(stg, v);
+        // One value that is not finite leaves the sum of all so (a sum that overflows is looked at for nothing). Worked out while
+        // the stores are on their way, and asked in place of the warp's own barrier.
+        float all[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *reinterpret_cast<uint4*>(stg + lane * 128 + ((q ^ (lane & 7)) * 16)) =
-              make_uint4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_reduce_add_2d(&p.tm_dw, stg, col, it.m0 + lane_base);
-          tma_store_commit();
-        }
+        for (int q = 0; q < 32; ++q) all[q & 3] += __uint_as_float(v[q]);
+        float one = (all[0] + all[1]) + (all[2] + all[3]);
+        asm volatile("" : "+f"(one));
+        const bool bad = (__float_as_uint(one) & 0x7f800000u) == 0x7f800000u && it.m0 + lane_base + lane < p.Kout;
+        if (!rows_add(p, stg, it, at, bad)) odd |= 1u << (c >> 5);
       }
+      for (; odd; odd &= odd - 1) rows_again(p, stg, tmem_base, work, (__ffs(odd) - 1) * 32);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->acc_empty[0]);

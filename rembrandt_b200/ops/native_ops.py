@@ -190,7 +190,8 @@ def tune_conv(N, H, W, Cp, Kout, R, S, stride, pad_h, pad_w, P, Q, ldy, relu=Fal
 
 
 def conv_wgrad_tc(x, N, H, W, Cp, dy, lddy, Kout, R, S, stride, pad_h, pad_w, P, Q, dw, split_k=0, beside=False):
-    """`beside`: leave room on the SMs for kernels that run at the same time."""
+    """`beside`: leave room on the SMs for kernels that run at the same time. Pixels outside the image count as zeros (which a NaN
+    or an infinity in dy turns into NaN)."""
     rc = _native.cuda().rb_conv_wgrad_tc(ptr(x), N, H, W, Cp, ptr(dy), lddy, Kout, R, S, stride, pad_h, pad_w, P, Q,
                                          ptr(dw), split_k, int(beside), ptr(status_word()), stream_handle())
     check(rc, "rb_conv_wgrad_tc")

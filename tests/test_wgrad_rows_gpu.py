@@ -88,6 +88,43 @@ def test_unequal_sides_and_outputs_cut_or_grown(shape):
             assert float((got - want).abs().max()) < 4e-6 * (N * P * Q) ** 0.5 * 4 + 2e-6      # as above
 
 
+BORDERS = [  # N, C, Ko, H, W, R, S, pad_h, pad_w
+    (2, 32, 32, 8, 8, 3, 3, 1, 1), (2, 64, 32, 11, 11, 3, 3, 1, 1), (1, 32, 64, 5, 20, 3, 3, 0, 0), (3, 32, 32, 7, 6, 5, 5, 2, 2),
+    (1, 32, 32, 12, 16, 3, 3, 1, 1), (2, 32, 32, 9, 7, 2, 4, 0, 3), (1, 32, 160, 7, 7, 3, 3, 2, 2), (17, 32, 32, 3, 3, 3, 3, 1, 1)]
+
+
+@pytest.mark.parametrize("shape", BORDERS)
+def test_infinities_and_nan_meet_what_they_belong_to(shape):
+    """A pixel at the border has no part in the taps that would put it against an output outside the image; pixels outside count as
+    zeros. So every sum is what the same products give in another order: as finite, as infinite, as much a NaN."""
+    N, C, Ko, H, W, R, S, ph, pw = shape
+    torch.manual_seed(sum(shape))
+    P, Q = H + 2 * ph - R + 1, W + 2 * pw - S + 1
+    x, dy = (torch.randn(N, c, *hw).bfloat16().double() for c, hw in ((C, (H, W)), (Ko, (P, Q))))
+    inf, nan = float("inf"), float("nan")
+    for c, (n, h, w, v) in enumerate([(0, 0, 0, inf), (0, 0, -1, -inf), (-1, -1, 0, nan), (-1, -1, -1, inf), (0, H // 2, -1, nan),
+                                      (-1, -1, W // 2, inf), (0, H // 2, W // 2, -inf), (-1, H // 2, 0, inf), (-1, 0, W // 2, nan)]):
+        x[n, c, h, w] = v
+    for k, (n, h, w, v) in enumerate([(0, 0, 0, inf), (-1, -1, -1, nan), (0, P // 2, Q // 2, -inf), (-1, P // 2, -1, inf)]):
+        dy[n, k, h, w] = v
+    dy[0, 4] = 0.0      # an infinite pixel against zeros inside the image
+    padded = F.pad(x, (pw, pw, ph, ph))
+    want = torch.stack([(dy[:, :, None] * padded[:, None, :, r: r + P, s: s + Q]).sum((0, 3, 4)) for r in range(R) for s in range(S)], 1)
+    assert int(want.isfinite().sum()) > want.numel() // 2      # [Ko][taps][C]
+    xi, dyi = (t.permute(0, 2, 3, 1).contiguous().bfloat16().to(DEV) for t in (x, dy))
+    for beside in (False, True):
+        for nth in range(1, 9):
+            out = torch.zeros((Ko, R * S, C), device=DEV)
+            with K.gemm_options(force_rows=nth):
+                K.conv_wgrad_tc(xi, N, H, W, C, dyi, Ko, Ko, R, S, 1, ph, pw, P, Q, out, beside=beside)
+            assert K.read_status() == 0 and K.gemm_last_launch()["a_mode"] == ROWS
+            got, plan = out.double().cpu(), K.gemm_last_launch()
+            assert torch.equal(got.isnan(), want.isnan()), (plan, (got.isnan() != want.isnan()).nonzero()[:9])
+            assert torch.equal(got == inf, want == inf) and torch.equal(got == -inf, want == -inf), plan
+            fine = want.isfinite()
+            assert float((got - want)[fine].abs().max()) < 4e-6 * (N * P * Q) ** 0.5 * 4      # as above
+
+
 @pytest.mark.parametrize("shape", [SHAPES[0], SHAPES[1], SHAPES[12]])
 def test_what_was_measured_is_what_runs(shape):
     args, check = _case(shape)
