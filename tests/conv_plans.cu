@@ -184,6 +184,38 @@ static void strided_outputs_are_aligned() {
       }
 }
 
+// Weight-gradients: row plans are taken where the best of them wins by 3 %, whichever is timed first; the first of equal ones.
+static float g_rows_ms[4];
+static int g_rows_seen;
+static float rows_take(const int* l) { return l[MODE] != A_ROWS ? 1.f : g_rows_ms[std::min(g_rows_seen++ / 3, 3)]; }
+static int wgrad(int N, int C, int Ko, int H, int R, int pad, int beside, bool measure = false, long long lddy = 0) {
+  void* const at = (void*)0x1000;
+  const int P = H + 2 * pad - R + 1;
+  if (measure) return rb_conv_wgrad_tune(at, N, H, H, C, at, Ko, Ko, R, R, pad, pad, P, P, (float*)at, beside, nullptr, 0);
+  return rb_conv_wgrad_tc(at, N, H, H, C, at, lddy ? lddy : Ko, Ko, R, R, 1, pad, pad, P, P, (float*)at, 0, beside, nullptr, 0);
+}
+static void row_plans_win_by_a_margin() {
+  g_time = rows_take;
+  const struct { float ms[4]; bool rows; const char* what; } tries[] = {
+      {{1.02f, 1.01f, 1.f, 1.f}, false, "slower"}, {{.98f, .99f, 1.f, 1.f}, false, "2 % faster"},
+      {{.98f, .96f, 1.f, .99f}, true, "the second 4 % faster"}, {{.9f, .96f, .91f, .99f}, true, "the first 10 % faster"},
+      {{.96f, .965f, .955f, .95f}, true, "all by little"}};
+  for (auto& t : tries)
+    for (int beside = 0; beside <= 1; ++beside) {
+      rb_gemm_clear_plans();
+      g_rows_seen = 0;
+      memcpy(g_rows_ms, t.ms, sizeof(g_rows_ms));
+      expect(wgrad(64, 32, 32, 32, 3, 1, beside, true) == 0, t.what);
+      expect(g_rows_seen == 12, "four row plans timed three times");
+      expect(wgrad(64, 32, 32, 32, 3, 1, beside) == 0 && (g_last_launch[MODE] == A_ROWS) == t.rows, t.what);
+      int took[9];
+      memcpy(took, g_last_launch, sizeof(took));
+      g_opt.force_rows = 1 + (int)(std::min_element(t.ms, t.ms + 4) - t.ms);
+      expect(wgrad(64, 32, 32, 32, 3, 1, beside) == 0 && (memcmp(took, g_last_launch, sizeof(took)) == 0) == t.rows, "the fastest");
+      g_opt.force_rows = -1;
+    }
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
       {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
@@ -193,7 +225,8 @@ int main(int argc, char** argv) {
       {"pairs_win_by_a_margin", pairs_win_by_a_margin},
       {"flat_tiles_within_the_cap", flat_tiles_within_the_cap},
       {"addends_are_aligned", addends_are_aligned},
-      {"strided_outputs_are_aligned", strided_outputs_are_aligned}};
+      {"strided_outputs_are_aligned", strided_outputs_are_aligned},
+      {"row_plans_win_by_a_margin", row_plans_win_by_a_margin}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;
