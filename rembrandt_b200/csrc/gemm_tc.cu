@@ -2453,8 +2453,8 @@ static std::map<RowsKey, WgradRowsParams> g_rows_cache;
 // step without and with this kernel for the smaller: 17 images 87, 86 us; 32 images 94, 100; at 64 105, 102.
 constexpr double ROWS_MIN_FLOPS = 0.2e9;
 // Row plans have to win by this much: two timings of one launch differ by up to 2 %, and between equals the general kernel adds up
-// fewer parts. 512 -> 512 on 64 x 32 x 32, general 188.6 us: measured four times without the margin a row plan of 189 to 193 us was
-// kept, with it the general kernel each time.
+// fewer parts. 512 -> 512 on 64 x 32 x 32: without the margin a row plan of 192.9 us was kept over 189.1; with it the general kernel
+// in four tunings of four.
 constexpr float ROWS_MARGIN = 0.97f;
 
 static int run_rows(WgradRowsParams p, const void* x, int N, int H, int W, const void* dy, long long lddy, int P, int Q, float* dw,
@@ -2881,15 +2881,15 @@ static int wgrad_by_plan(const void* x, int N, int H, int W, int Cp, const void*
   // options of the other kernel
   const bool forced = g_opt.force_mt || g_opt.force_taps || g_opt.force_box >= 0 || g_opt.force_resident >= 0 ||
                       (g_opt.bn_cap > 0 && g_opt.bn_cap < 256);
-  if (stride != 1 || R * S < 2 || split_k > 0 || g_opt.deterministic || g_opt.force_rows == 0 || forced || N < 1 || P < 1 || Q < 1)
-    return measure ? 0 : plain();
+  if (stride != 1 || R * S < 2 || split_k > 0 || N < 1 || P < 1 || Q < 1) return measure ? 0 : plain();
+  if (measure && (!g_opt.autotune || g_opt.deterministic || g_opt.force_rows >= 0 || forced)) return 1;
+  if (g_opt.deterministic || g_opt.force_rows == 0 || forced) return plain();
   auto run = [&](const WgradRowsParams& p) { return run_rows(p, x, N, H, W, dy, lddy, P, Q, dw, status, stream); };
   auto plans = [&]() {
     return rows_plans(N, H, W, Cp, Kout, R, S, pad_h, pad_w, P, Q, beside ? LEAN_TILE_BYTES : TILE_SMEM_BYTES);
   };
   if (g_opt.force_rows > 0) {
     const auto all = plans();
-    if (measure) return 0;
     return all.empty() ? plain() : run(all[std::min<size_t>((size_t)g_opt.force_rows, all.size()) - 1]);
   }
   if (2.0 * N * P * Q * R * S * Cp * Kout < ROWS_MIN_FLOPS) return measure ? 0 : plain();
@@ -2985,10 +2985,10 @@ int rb_conv_wgrad_tc(const void* x, int N, int H, int W, int Cp, const void* dy,
 
 // Times gemm_tc_kernel and the first four plans of wgrad_rows_kernel by its model on these operands, which are scratch (dw is
 // added into many times), and remembers which was the fastest. Synchronises the stream: never inside a capture. Does nothing for
-// a shape that has been measured, or that has no such plans.
+// a shape that has been measured, or that has no such plans. Returns 1 where an option is in the way of measuring: to be asked
+// again.
 int rb_conv_wgrad_tune(const void* x, int N, int H, int W, int Cp, const void* dy, long long lddy, int Kout, int R, int S,
                        int pad_h, int pad_w, int P, int Q, float* dw, int beside, unsigned int* status, cudaStream_t stream) {
-  if (!g_opt.autotune) return 0;
   return wgrad_by_plan(x, N, H, W, Cp, dy, lddy, Kout, R, S, 1, pad_h, pad_w, P, Q, dw, 0, beside, true, status, stream);
 }
 

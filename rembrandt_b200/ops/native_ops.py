@@ -131,6 +131,7 @@ def gemm_last_launch() -> dict:
 
 def gemm_clear_plans() -> None:
     OPTION_CHANGES[0] += 1
+    _tuned_convs.clear()
     _native.cuda().rb_gemm_clear_plans()
 
 
@@ -200,17 +201,19 @@ def conv_wgrad_tc(x, N, H, W, Cp, dy, lddy, Kout, R, S, stride, pad_h, pad_w, P,
 def tune_wgrad(N, H, W, Cp, Kout, Kp, R, S, stride, pad_h, pad_w, P, Q, beside=(False,)):
     """Measure which kernel and plan one weight-gradient takes, on scratch operands; `beside`: the forms that will be asked for.
     Idempotent per shape and process."""
-    forms = [b for b in beside if ("wgrad", torch.cuda.current_device(), N, H, W, Cp, Kout, Kp, R, S, stride, pad_h, pad_w, P, Q, b)
-             not in _tuned_convs]
-    if stride != 1 or R * S < 2 or not forms:
+    keys = {("wgrad", torch.cuda.current_device(), N, H, W, Cp, Kout, Kp, R, S, stride, pad_h, pad_w, P, Q, b): b for b in beside}
+    if stride != 1 or R * S < 2 or _tuned_convs.issuperset(keys):
         return
     x = torch.zeros((N, H, W, Cp), dtype=torch.bfloat16, device="cuda")
     dy = torch.zeros((N, P, Q, Kp), dtype=torch.bfloat16, device="cuda")
     dw = torch.zeros((Kout, R * S, Cp), dtype=torch.float32, device="cuda")
-    for b in forms:
-        _tuned_convs.add(("wgrad", torch.cuda.current_device(), N, H, W, Cp, Kout, Kp, R, S, stride, pad_h, pad_w, P, Q, b))
-        check(_native.cuda().rb_conv_wgrad_tune(ptr(x), N, H, W, Cp, ptr(dy), Kp, Kout, R, S, pad_h, pad_w, P, Q, ptr(dw), int(b),
-                                                ptr(status_word()), stream_handle()), "rb_conv_wgrad_tune")
+    for key, b in keys.items():
+        rc = _native.cuda().rb_conv_wgrad_tune(ptr(x), N, H, W, Cp, ptr(dy), Kp, Kout, R, S, pad_h, pad_w, P, Q, ptr(dw), int(b),
+                                               ptr(status_word()), stream_handle())
+        if rc == 1:     # an option was in the way: the next network of this shape asks again
+            continue
+        check(rc, "rb_conv_wgrad_tune")
+        _tuned_convs.add(key)
     torch.cuda.current_stream().synchronize()
 
 

@@ -216,6 +216,41 @@ static void row_plans_win_by_a_margin() {
     }
 }
 
+// What stands in the way of measuring a weight-gradient is said, and nothing is remembered; what was measured is for that shape, those
+// paddings and that form alone; shapes of little work and `deterministic` stay with the general kernel.
+static float rows_are_fastest(const int* l) { return l[MODE] == A_ROWS ? 1.f : 2.f; }
+static void row_plans_are_remembered() {
+  g_time = rows_are_fastest;
+  int* const in_the_way[] = {&g_opt.deterministic, &g_opt.force_mt, &g_opt.force_taps, &g_opt.force_box, &g_opt.force_resident,
+                             &g_opt.force_rows, &g_opt.bn_cap, &g_opt.autotune};
+  for (int* option : in_the_way) {
+    const int was = *option;
+    *option = option == &g_opt.bn_cap ? 128 : option == &g_opt.autotune ? 0 : 1;
+    expect(wgrad(64, 32, 32, 32, 3, 1, 0, true) == 1 && g_rows_cache.empty(), "an option in the way");
+    *option = was;
+    expect(wgrad(64, 32, 32, 32, 3, 1, 0) == 0 && g_last_launch[MODE] != A_ROWS, "not measured");
+  }
+  for (int beside = 0; beside <= 1; ++beside) {
+    expect(wgrad(64, 32, 32, 32, 3, 1, beside) == 0 && g_last_launch[MODE] != A_ROWS, "the other form was measured");
+    expect(wgrad(64, 32, 32, 32, 3, 1, beside, true) == 0 && g_rows_cache.size() == 1u + beside, "measured");
+    expect(wgrad(64, 32, 32, 32, 3, 1, beside) == 0 && g_last_launch[MODE] == A_ROWS, "measured");
+    const WgradRowsParams& p = g_rows_cache.rbegin()->second;
+    expect(p.stages * (p.dy_blocks * p.dy_block + p.ncb * p.x_block) <= (beside ? LEAN_TILE_BYTES : TILE_SMEM_BYTES), "fits");
+    expect(wgrad(63, 32, 32, 32, 3, 1, beside) == 0 && g_last_launch[MODE] != A_ROWS, "another batch");
+    expect(wgrad(64, 32, 32, 34, 3, 0, beside) == 0 && g_last_launch[MODE] != A_ROWS, "the same output at padding 0");
+    expect(wgrad(64, 32, 32, 32, 3, 1, beside, false, 64) == 0 && g_last_launch[MODE] == A_ROWS, "longer rows of dy");
+    g_opt.deterministic = 1;
+    expect(wgrad(64, 32, 32, 32, 3, 1, beside) == 0 && g_last_launch[MODE] != A_ROWS, "deterministic");
+    g_opt.deterministic = 0;
+  }
+  const size_t before = g_rows_cache.size();      // 0.199 GFLOP
+  expect(wgrad(42, 32, 32, 16, 3, 1, 0, true) == 0 && g_rows_cache.size() == before, "little work");
+  expect(wgrad(42, 32, 32, 16, 3, 1, 0) == 0 && g_last_launch[MODE] != A_ROWS, "little work");
+  expect(wgrad(43, 32, 32, 16, 3, 1, 0, true) == 0 && g_rows_cache.size() == before + 1, "enough work");
+  rb_gemm_clear_plans();
+  expect(wgrad(64, 32, 32, 32, 3, 1, 0) == 0 && g_last_launch[MODE] != A_ROWS, "forgotten");
+}
+
 int main(int argc, char** argv) {
   const struct { const char* name; void (*run)(); } scenarios[] = {
       {"remembered_flat_does_not_fit", remembered_flat_does_not_fit},
@@ -226,7 +261,8 @@ int main(int argc, char** argv) {
       {"flat_tiles_within_the_cap", flat_tiles_within_the_cap},
       {"addends_are_aligned", addends_are_aligned},
       {"strided_outputs_are_aligned", strided_outputs_are_aligned},
-      {"row_plans_win_by_a_margin", row_plans_win_by_a_margin}};
+      {"row_plans_win_by_a_margin", row_plans_win_by_a_margin},
+      {"row_plans_are_remembered", row_plans_are_remembered}};
   g_encode_tiled = no_tiled;
   g_encode_im2col = no_im2col;
   g_num_sms = 148;

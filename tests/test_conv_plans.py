@@ -25,7 +25,8 @@ def program(tmp_path_factory):
 
 @pytest.mark.parametrize("scenario", ["remembered_flat_does_not_fit", "paddings_are_measured_apart", "sub_tiles_of_other_modes",
                                       "deterministic_keeps_one_order", "pairs_win_by_a_margin", "flat_tiles_within_the_cap",
-                                      "addends_are_aligned", "strided_outputs_are_aligned", "row_plans_win_by_a_margin"])
+                                      "addends_are_aligned", "strided_outputs_are_aligned", "row_plans_win_by_a_margin",
+                                      "row_plans_are_remembered"])
 def test_plans(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=60,
                        env={k: v for k, v in os.environ.items() if not k.startswith("RB_GEMM_")})

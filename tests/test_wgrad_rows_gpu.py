@@ -2,7 +2,8 @@
 filter rows per item, one or more channel blocks), channel blocks of 32 and 64 that are and are not full, one and two blocks of
 output channels, rows that are and are not multiples of 16 positions, chunks of several images and of part of one, images wider
 than high, filters of 2 to 8 taps a row, paddings from none to the filter's width; values that must not be added into (channels of
-the padding); and what is remembered of a measurement."""
+the padding); and what is
+remembered of a measurement."""
 import pytest
 import torch
 import torch.nn.functional as F
@@ -125,21 +126,31 @@ def test_infinities_and_nan_meet_what_they_belong_to(shape):
             assert float((got - want)[fine].abs().max()) < 4e-6 * (N * P * Q) ** 0.5 * 4      # as above
 
 
-@pytest.mark.parametrize("shape", [SHAPES[0], SHAPES[1], SHAPES[12]])
+# (row plans take three quarters of the general kernel's time here: which is kept does not hang on a percent)
+@pytest.mark.parametrize("shape", [(32, 32, 32, 16, 16, 5, 2), (64, 32, 64, 12, 12, 5, 2)])
 def test_what_was_measured_is_what_runs(shape):
     args, check = _case(shape)
-    run = lambda a, dw: K.conv_wgrad_tc(*a, dw)
-    K.gemm_clear_plans()
-    check(run)
-    assert K.gemm_last_launch()["a_mode"] != ROWS      # not measured: the general kernel
+
+    def runs_rows(beside):
+        check(lambda a, dw: K.conv_wgrad_tc(*a, dw, beside=beside))
+        return K.gemm_last_launch()["a_mode"] == ROWS
+
     N, H, W, Cp, _, Kp, Ko, k = args[1:9]
-    K._tuned_convs.clear()
-    K.tune_wgrad(N, H, W, Cp, Ko, Kp, k, k, 1, *args[11:])
-    check(run)
-    first = K.gemm_last_launch()
-    check(run)
-    assert K.gemm_last_launch() == first
-    with K.gemm_options(deterministic=1):
-        check(run)
-        assert K.gemm_last_launch()["a_mode"] != ROWS
+    tune = lambda *beside: K.tune_wgrad(N, H, W, Cp, Ko, Kp, k, k, 1, *args[11:], beside=beside)
     K.gemm_clear_plans()
+    assert not runs_rows(False) and not runs_rows(True)      # not measured: the general kernel
+    with K.gemm_options(autotune=0):
+        tune(False, True)
+    assert not runs_rows(False) and not runs_rows(True)      # nor with measuring switched off
+    for first in (False, True):
+        tune(first)
+        assert runs_rows(first) and not runs_rows(not first)      # each form by itself
+        launch = (runs_rows(first), K.gemm_last_launch())
+        assert (runs_rows(first), K.gemm_last_launch()) == launch
+        with K.gemm_options(deterministic=1):
+            K.conv_wgrad_tc(*args, torch.zeros((Ko, k * k, Cp), device=DEV), beside=first)
+            assert K.gemm_last_launch()["a_mode"] != ROWS
+        tune(False, True)
+        assert runs_rows(False) and runs_rows(True)
+        K.gemm_clear_plans()
+        assert not runs_rows(first)      # forgotten, and measured again when asked for
