@@ -75,3 +75,67 @@ def test_captured_passes_take_the_gradients_of_eager_ones(model, batch, c, hw, c
             if seg.name.endswith(".w"):
                 u, v = (t[seg.offset: seg.offset + seg.numel] for t in (got, want))
                 assert float((u - v).norm()) <= limit * float(v.norm()), seg.name
+
+
+ROWS = 6      # how gemm_last_launch names the kernel for whole rows
+
+
+@pytest.mark.parametrize("model,batch,c,hw,classes,rows", [("lenet", 9, 1, 28, 10, False), ("cifar", 24, 3, 32, 10, True),
+                                                           ("resnet20_cifar", 64, 3, 32, 10, True),
+                                                           ("go_policy_resnet", 12, 32, 19, 361, True), ("resnet18", 4, 3, 256, 1000, True)])
+def test_captured_weight_gradients_are_those_of_what_lies_in_their_operands(model, batch, c, hw, classes, rows, monkeypatch):
+    """After a pass every operand of its weight-gradients still lies where they read it: each taken again from there, by itself, has
+    to give what the captured launch beside other kernels gave, but for the order of its sums."""
+    eng = build_replica(model, batch, seed=(3, 4))
+    net = eng.net
+    taken = []
+    conv, gemm = K.conv_wgrad_tc, K.gemm_tc
+
+    def conv_wgrad(x, *a, beside=False):
+        conv(x, *a, beside=beside)
+        taken.append(((x,) + a, K.gemm_last_launch()["a_mode"], torch.cuda.current_stream() == net._side))
+
+    def gemm_tc(a, a_mn, *rest, **kw):
+        gemm(a, a_mn, *rest, **kw)
+        if a_mn and rest[2]:      # both operands as they lie: an affine layer's weight-gradient, or that of a layer of windows
+            taken.append(((a, a_mn) + rest, None, torch.cuda.current_stream() == net._side))
+
+    def one_pass():
+        net.forward(True)
+        net.backward()
+
+    g = torch.Generator().manual_seed(12)
+    graph = None
+    for _ in range(4):
+        net.load_batch(torch.randint(0, 256, (batch, c, hw, hw), dtype=torch.uint8, generator=g).to(DEV),
+                       torch.randint(0, classes, (batch,), dtype=torch.int32, generator=g).to(DEV))
+        with torch.cuda.stream(eng.compute_stream):
+            if graph is None:
+                one_pass()
+                torch.cuda.synchronize()
+                monkeypatch.setattr(K, "conv_wgrad_tc", conv_wgrad)
+                monkeypatch.setattr(K, "gemm_tc", gemm_tc)
+                graph = torch.cuda.CUDAGraph()
+                graph.capture_begin(capture_error_mode="thread_local")
+                one_pass()
+                graph.capture_end()
+                monkeypatch.undo()
+                assert any(side for *_, side in taken) and any(mode == ROWS for _, mode, _ in taken) == rows
+            net.grads.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            for args, mode, side in taken:
+                if mode is None:
+                    a, _, lda, b, _, ldb, M, N, k, out = args[:10]
+                    if not side:
+                        continue      # into a scratch that the layer clears
+                    want = a.reshape(-1, lda)[:k, :M].double().T @ b.reshape(-1, ldb)[:k, :N].double()
+                else:
+                    out = args[15]
+                    want = torch.zeros_like(out)
+                    with K.gemm_options(force_rows=0):
+                        conv(*args[:15], want)
+                    torch.cuda.synchronize()
+                off = float((out.double() - want.double().view_as(out)).norm() / want.double().norm())
+                # sums of up to 65536 products in parts of another number: 6e-6 of their norm seen; one lost part of 148 is 7e-3
+                assert off < 2.5e-5, (off, args[1:15], mode, side)
