@@ -165,20 +165,14 @@ __device__ __forceinline__ void pixel_coords(int P, int Q, int stride, int lower
 struct WorkItem {
   int tm, tn, kb0, kb1, tail, phase;
 };
-__device__ __forceinline__ const GemmPhase& phase_of(const GemmPhasesParams& p, int k) { return p.ph[k]; }
-__device__ __forceinline__ const GemmPhase& phase_of(const GemmTcParams& p, int) {      // never looked at
-  return *reinterpret_cast<const GemmPhase*>(&p);
-}
-__device__ __forceinline__ int phases_of(const GemmPhasesParams& p) { return p.phases; }
-__device__ __forceinline__ int phases_of(const GemmTcParams&) { return 0; }
 template <bool PHASES, class Params>
 __device__ __forceinline__ WorkItem decode_work(const Params& p, int work, int m_items, int direct, int kb_per_split) {
   WorkItem w;
   int rem;
   w.phase = 0;
-  if (PHASES) {
-    for (int k = 1; k < phases_of(p); ++k) w.phase = work >= phase_of(p, k).work0 ? k : w.phase;
-    const GemmPhase& ph = phase_of(p, w.phase);
+  if constexpr (PHASES) {
+    for (int k = 1; k < p.phases; ++k) w.phase = work >= p.ph[k].work0 ? k : w.phase;
+    const GemmPhase& ph = p.ph[w.phase];
     rem = work - ph.work0;
     m_items = ph.m_items;
     w.kb0 = 0;
@@ -488,8 +482,8 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
   const int n_tiles = p.n_tiles;
   // whole items first, then the parts of the cut items of the last wave (tail cut; never in flat mode)
   const int direct = m_items * n_tiles - p.tail_items;
-  const int num_work = PHASES ? phase_of(p, phases_of(p) - 1).work0 + phase_of(p, phases_of(p) - 1).m_items * n_tiles
-                     : p.tail_items > 0 ? direct + p.tail_items * p.tail_split : m_items * n_tiles * p.split_k;
+  int num_work = p.tail_items > 0 ? direct + p.tail_items * p.tail_split : m_items * n_tiles * p.split_k;
+  if constexpr (PHASES) num_work = p.ph[p.phases - 1].work0 + p.ph[p.phases - 1].m_items * n_tiles;
   // flat mode: [A ring: fl_a_stages x fl_a_bytes][B ring: stages x b_bytes, or the resident panel]
   uint8_t* const b_ring = FLAT ? tiles + p.fl_a_stages * p.fl_a_bytes : tiles;
   const int kb_per_split = (p.num_kb + p.split_k - 1) / p.split_k;
@@ -512,8 +506,8 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
     for (int w = 0; w < EPI_WARPS; ++w) mbar_init(&ctl->mask_bar[w], 1);
     ctl->abort_flag = 0;
     mbar_fence_init();
-    if (PHASES)
-      for (int k = 0; k < phases_of(p); ++k) tma_prefetch_desc(&phase_of(p, k).tm_a);
+    if constexpr (PHASES)
+      for (int k = 0; k < p.phases; ++k) tma_prefetch_desc(&p.ph[k].tm_a);
     else
       tma_prefetch_desc(&p.tm_a);
     tma_prefetch_desc(&p.tm_b);
@@ -685,19 +679,22 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
       const int wg_t = lane / wg_apt, wg_c = 64 * (lane - wg_t * wg_apt);
       for (int work = cta_id; work < num_work && ok; work += cta_step) {
         const WorkItem it = decode_work<PHASES>(p, work, m_items, direct, kb_per_split);
-        const GemmPhase& phase = phase_of(p, it.phase);
-        if (PHASES) {
-          taps_w = phase.S;
-          dg_base = phase.dg_base;
-          map_a = &phase.tm_a;
+        if constexpr (PHASES) {
+          taps_w = p.ph[it.phase].S;
+          dg_base = p.ph[it.phase].dg_base;
+          map_a = &p.ph[it.phase].tm_a;
         }
         const int tn = it.tn, kb0 = it.kb0, kb1 = it.kb1;
         const int tm = pair ? it.tm * 2 + (int)cta_rank : it.tm;
         const int m0 = tm * BM * mt;
         int a_w = 0, a_h = 0, a_n = 0;   // first pixel of this lane's A load
         if (mode == A_IM2COL_K && lane < nload) {
-          if (PHASES) pixel_coords(phase.P, phase.Q, 1, phase.lower_h, phase.lower_w, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
-          else pixel_coords(p.cv_P, p.cv_Q, p.cv_stride, p.cv_lower_h, p.cv_lower_w, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
+          if constexpr (PHASES) {
+            const GemmPhase& ph = p.ph[it.phase];
+            pixel_coords(ph.P, ph.Q, 1, ph.lower_h, ph.lower_w, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
+          } else {
+            pixel_coords(p.cv_P, p.cv_Q, p.cv_stride, p.cv_lower_h, p.cv_lower_w, m0 + aj * BM + aq * a_rows, a_w, a_h, a_n);
+          }
         }
         if (mode == A_BOX_K) {   // lane j loads sub-tile j: image a_n, first output row a_h
           a_n = tm / bx_groups;
@@ -971,8 +968,6 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
     bool ok = true;
     for (int work = cta_id; work < num_work && ok; work += cta_step) {
       const WorkItem it = decode_work<PHASES>(p, work, m_items, direct, kb_per_split);
-      const GemmPhase& phase = phase_of(p, it.phase);
-      const int rows_d = PHASES ? phase.M : p.M;
       const int tn = it.tn;
       const int tm = pair ? it.tm * 2 + (int)cta_rank : it.tm;
       const bool tail = it.tail >= 0;
@@ -1017,9 +1012,10 @@ __global__ void __maxnreg__(LEAN ? LEAN_MAX_REGS : GEMM_MAX_REGS) gemm_tc_kernel
           const bool addend = EXT && p.add_src != nullptr;
           long long drow_of = -1;
           if (FLAT) drow_of = flat_row(p, (tm * mt + j) * p.fl_step + lane_base + lane);
-          else if (PHASES) {
-            if (row0 + lane < rows_d)
-              drow_of = scatter_row(row0 + lane, phase.P, phase.Q, p.sc_stride, phase.sc_a, phase.sc_b, p.sc_H, p.sc_W);
+          else if constexpr (PHASES) {
+            const GemmPhase& ph = p.ph[it.phase];
+            if (row0 + lane < ph.M)
+              drow_of = scatter_row(row0 + lane, ph.P, ph.Q, p.sc_stride, ph.sc_a, ph.sc_b, p.sc_H, p.sc_W);
           } else if ((scatter || addend) && lane < band_rows && row0 + lane < p.M)
             drow_of = scatter ? scatter_row(row0 + lane, p.cv_P, p.cv_Q, p.sc_stride, p.sc_a, p.sc_b, p.sc_H, p.sc_W)
                               : (long long)(row0 + lane);
