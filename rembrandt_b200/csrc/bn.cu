@@ -189,8 +189,11 @@ __global__ void __launch_bounds__(256) bn_reduce_kernel(const bf16* __restrict__
 
 static void launch_bn_reduce(const bf16* x, const bf16* dy, const bf16* y, const float* mean, const float* istd,
                              long long rows, int C, float* plain, int backward, const BnScratch& ws, cudaStream_t st) {
-  // Two blocks per SM: every block adds 2 * C sums to the same addresses, and in the backward pass the weight-gradient beside it
-  // leaves room for one or two. With four, the Go network's step at 256 boards took 1511 us, with two 1457, with one 1515.
+  // Two blocks per SM: every block adds 2 * C sums to the same addresses, and in the backward pass of a captured step the
+  // weight-gradient beside it leaves room for one or two. Fastest or equal without a neighbour too, on the 14 sizes tried: forward
+  // (us a layer with its application; 1, 2, 3, 4 blocks) 92416 x 128: 20.7, 18.9, 18.7, 20.9, 131072 x 64: 17.0, 15.2, 15.5, 16.6,
+  // 8192 x 64: 6.0, 5.9, 6.0, 6.0; backward (2, 4) 92416 x 128: 24.1, 26.5, 2048 x 512: 9.0, 9.0. The Go network's step at 256
+  // boards, weight-gradients beside and in line, with four 1421 and 1531 us, with two 1408 and 1521.
   const dim3 grid = row_grid(rows, C, 8, 148 * 2);
   auto go = [&](auto kern) { launch_pdl(kern, grid, dim3(256), 0, st, x, dy, y, mean, istd, rows, C, plain, ws); };
   if (!backward) go(bn_reduce_kernel<0, 0>);
@@ -452,8 +455,9 @@ __global__ void __launch_bounds__(256) bn_bwd_apply_kernel(const bf16* __restric
 static void launch_bn_bwd_apply(const bf16* x, const bf16* dy, const bf16* y, const float* mean, const float* istd,
                                 const float* gamma, const float* plain, const BnScratch& ws, float* dgamma,
                                 float* dbeta, bf16* dx, long long rows, int C, int c_valid, cudaStream_t st) {
-  // (no more blocks than find room beside the weight-gradient: with eight per SM the Go network's step took 1436 us, now 1420;
-  // ResNet-18's at 32 images 1465, now 1451)
+  // Two blocks per SM, which find room beside a weight-gradient and are the fastest alone: 92416 x 128, us a layer with its sums, by
+  // 2, 4, 8 blocks: 24.1, 25.2, 28.3, 32768 x 128: 14.1, 15.8, 15.8. Steps with weight-gradients beside and in line, with eight and
+  // with two: the Go network at 256 boards 1432 and 1569 us, 1408 and 1521; ResNet-18 at 32 images 1417 and 1595, 1406 and 1582.
   dim3 grid = row_grid(rows, C, 4, 148 * 2);
   if (ws.sums) ++grid.x;   // the blocks that store what exists once per channel
   auto go = [&](auto kern) {

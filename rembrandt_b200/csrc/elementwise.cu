@@ -221,8 +221,8 @@ __global__ void zero_s2d_structural_kernel(float* __restrict__ dw, int Kout, int
   }
 }
 
-// Loss and number of correct samples of a step into page-locked host memory, and the accumulators cleared: the last launch
-// of a step, in place of two copies, a conversion, a copy to the host and two fills. With `turn` the two rows of `host` are
+// Loss and number of correct samples of a step into page-locked host memory, and the accumulators cleared: one launch behind
+// the loss (captured steps run it beside their backward pass), in place of two copies, a conversion, a copy to the host and two fills. With `turn` the two rows of `host` are
 // written in turn.
 __global__ void publish_stats_kernel(float* loss_sum, int* correct, volatile float* host, unsigned int* turn) {
   pdl_prolog();

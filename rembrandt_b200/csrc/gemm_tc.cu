@@ -2444,9 +2444,11 @@ static std::vector<WgradRowsParams> rows_plans(int N, int H, int W, int Cp, int 
 // What was measured as the fastest for a weight-gradient: a plan, or none of them (`rows` = 0: gemm_tc_kernel).
 typedef std::tuple<int, int, int, int, int, int, int, int, int, int, int, int> RowsKey;
 static std::map<RowsKey, WgradRowsParams> g_rows_cache;
-// Less work than this is start, additions and drain in either kernel, and gemm_tc_kernel adds it up from fewer parts, whose order
-// is left open: LeNet's second convolution at 17 images (0.09 GFLOP) 2 parts against 17 to 29, at 64 (0.33) 8 against 22. LeNet's
-// step without and with this kernel for the smaller: 17 images 87, 86 us; 32 images 94, 100; at 64 105, 102.
+// With less work than this the general kernel adds up from 1 to 16 parts, row plans from 24 to 49, whose order is left open, and runs
+// repeat less closely: LeNet's parameters after eight steps at 17 images, two captured runs, differ by 4e-4 of an update in the median
+// with the general kernel and by 2.7e-2 with row plans (one value at a rounding edge falls either way). It is not the faster of the
+// two everywhere below the line: a launch of row plans takes 0.3 to 2.5 us less of 6 to 8 (32 -> 32 channels on 8 x 32 x 32, 0.15
+// GFLOP: 8.1 -> 5.6) or up to 2.5 more (256 -> 256 on 4 x 4 x 4: 4.3 -> 6.8).
 constexpr double ROWS_MIN_FLOPS = 0.2e9;
 // Row plans have to win by this much: two timings of one launch differ by up to 2 %, and between equals the general kernel adds up
 // fewer parts. 512 -> 512 on 64 x 32 x 32: without the margin a row plan of 192.9 us was kept over 189.1; with it the general kernel

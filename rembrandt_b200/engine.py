@@ -9,8 +9,8 @@ kernel individually, the engine
 * captures forward + backward (+ exchange + update when the backend's kernels can be captured) + the publication of
   loss / accuracy in one CUDA graph per slot and replays it per step (the learning rate is read from device memory, so
   a schedule captures nothing again); an inference pass is a graph as well;
-* returns loss / accuracy with a one-step lag through a pinned host mirror that the last kernel of the step writes, so
-  the host never blocks on the step it has just launched.
+* returns loss / accuracy with a one-step lag through a pinned host mirror that a kernel of the step writes (beside backward
+  in a captured step, behind the update in an eager one), so the host never blocks on the step it has just launched.
 
 On CPU the same interface runs the reference path eagerly.
 """

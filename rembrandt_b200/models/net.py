@@ -130,9 +130,11 @@ class Net:
         if not self.is_cuda:
             self.params.requires_grad_(True)
             self.params.grad = self.grads
-        # Small kernels that depend on nothing the main stream is about to produce (bias-gradient column sums, the
-        # re-packing of filters for the data-grad) run on a side stream beside the tensor-core kernels, which leave
-        # DRAM and most of the register file idle; `side` forks, `join_side` joins (both are captured into graphs).
+        # What the rest of a pass does not wait for runs on a side stream: small kernels beside the tensor-core kernels, which
+        # leave DRAM and most of the register file idle (bias-gradient column sums, the re-packing of filters for the
+        # data-grad); in captured steps also weight-gradients beside normalisations and data-gradients (`beside`), the
+        # publication of the loss beside backward and the count of steps beside the update. What it reads is not written
+        # again before `join_side`. `side` forks, `join_side` joins (both are captured into graphs).
         self._side = None
         self._side_dirty = False
         self._collected = False  # backward hands every operator's gradients on as soon as they are there

@@ -698,9 +698,13 @@ class Conv2dOp(Op):
                 if self.s2d:
                     K.zero_s2d_structural(gw, ko, self.r2, self.cp, self.f, self.in_c, self.cfg.conv_size)
 
-            # A small one is all latency, and the data-gradient, which does not depend on it, runs in the same time (LeNet's
-            # step at 64 images 127 -> 113 us, affine layers included). One that fills the SMs only gets into the way of the
-            # data-gradient's blocks (NIN at 64 images: 897 us as it is, 938 with all of them beside).
+            # A small one is all latency, and the data-gradient, which does not depend on it, runs in the same time; one that
+            # fills the SMs only gets into the way of the data-gradient's blocks. Forward and backward in a graph, us, with none
+            # of these beside, with those under the line, and with all: LeNet at 16 images 82, 79, 79, at 64 100, 97, 97; CIFAR
+            # network at 16 108, 98, 98, at 64 129, 124, 124; NIN at 8 412, 401, 396, at 64 838, 838, 870; VGG-A at 32 1945, 1999,
+            # 1940 (noise). Above the line some gain (CIFAR network at 128, 0.6 GFLOP: 152 -> 148, NIN at 16, 0.8 to 1.5: 498 -> 472)
+            # and some lose (NIN at 37, 1.8 to 2: 660 -> 669). The neighbour is a GEMM that takes whole SMs, so the form that leaves
+            # room on one (`beside` of the kernel) gives nothing: 401 and 404, 498 and 497 us for NIN at 8 and 16.
             if 2.0 * rows * r * r * self.cp * self.out_cp < self.SMALL_WGRAD_FLOPS:
                 self.net.beside(wgrad)
             else:
